@@ -141,3 +141,32 @@ def test_batch_small_grid_matches_oracle(cuda, ctas):
     views = w.views[:1] + w.views[1:5] + w.views[5:9] + w.views[21:30]
     _check_batch(w, views, max_ctas=ctas)
 
+
+
+@pytest.mark.parametrize("capacity", [1, 255, 256, 257, 1024, 2000, 5000])
+def test_pack_draws_unit_edges(cuda, capacity):
+    """Views of 1, 255, 256, 257, 513 and 1024 draws and views without any (a camera that
+    looks away) packed into buffers that end before, at and after the 256-draw units."""
+    import torch
+    from helio_b200 import scene as S
+
+    sc, v = benchmark_scene(64, 64)
+    away = S.View(S.perspective((0, 0, 0), (0, 0, 1), (0, 1, 0), 60.0, 16 / 9), v.width, v.height, v.depth)
+    views = [away, v, v, away, away, v, v, v, v, away]
+    caps = [9, 1, 255, 9, 9, 256, 257, 513, 1024, 9]
+    b, vs, _ = run_batch(sc, views, span_visibility=False, capacities=caps)
+    per = [gather(b, i, len(sc.objects)) for i in range(len(views))]
+    counts = [len(p["indirect"]) for p in per]
+    assert counts == [0 if w is away else c for w, c in zip(views, caps)]
+    room = capacity + 3
+    ind = torch.full((room, 5), -1, dtype=torch.int32, device="cuda")
+    drw = torch.full((room, 4), -1, dtype=torch.int32, device="cuda")
+    off = torch.full((len(views) + 1,), -1, dtype=torch.int32, device="cuda")
+    b.pack_draws(ind[:capacity], drw[:capacity], off)
+    torch.cuda.synchronize()
+    ends = np.minimum(np.concatenate([[0], np.cumsum(counts)]), capacity)
+    np.testing.assert_array_equal(off.cpu().numpy(), ends)
+    n = int(ends[-1])
+    np.testing.assert_array_equal(u32(ind[:n]), np.concatenate([p["indirect"] for p in per])[:n])
+    np.testing.assert_array_equal(u32(drw[:n]), np.concatenate([p["draws"] for p in per])[:n])
+    assert (ind[n:].cpu().numpy() == -1).all() and (drw[n:].cpu().numpy() == -1).all()
