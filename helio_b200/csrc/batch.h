@@ -92,8 +92,11 @@ constexpr uint32_t kBatchPhaseStamps = 10;
 // instance in range and a valid transform), as float bits, for the per-view reject
 // boxes: bounds[0] = largest world radius max(local_radius * max_scale, 0),
 // bounds[1] = largest |c.x| + |c.y| + |c.z| of a world centre c (computed exactly as
-// the select computes them). `bounds` must be zero before the launch.
-cudaError_t launch_scene_bounds(const VgSceneDev& scene, uint32_t* bounds, cudaStream_t stream);
+// the select computes them). With `totals` (or null), also sums over all objects: totals[0] =
+// lod_meshlet_counts[0], totals[1] = 64-meshlet spans and totals[2] = meshlets of the largest
+// of the object's LODs. `bounds` and `totals` must be zero before the launch.
+cudaError_t launch_scene_bounds(const VgSceneDev& scene, uint32_t* bounds, unsigned long long* totals,
+                                cudaStream_t stream);
 
 // Packs the published draws of every view (min(counters[0], capacity) each) into
 // one pair of arrays, view after view; offsets[v] = first draw of view v, offsets[V] =
