@@ -643,7 +643,7 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
             if (P.views[v].hiz.mip_count <= 7u) continue;
             load_hiz_job(P, v, sm);
             __syncwarp();
-            hiz_tail_warp(J);
+            hiz_tail_call(J, 0u, 1u);
             __syncwarp();
         }
     }

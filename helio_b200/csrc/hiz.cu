@@ -2,12 +2,11 @@
 //
 // The reference runs one depth-copy dispatch and then mip_count-1 dispatches
 // separated by barriers (crates/helio-pass-hiz/src/lib.rs:503-531). Here one launch
-// builds every level of one or several views: each 64x64 tile of level 0 is reduced
-// by one CTA to levels 1..6 (hiz_tile.cuh), and the CTA of the last tile of each view
-// finishes the levels above 6. A single view whose depth TMA can address (16-byte
-// aligned, row pitch a multiple of 4 floats) runs the persistent form below, which
-// streams the tiles into shared memory with TMA loads; other inputs and multi-view
-// launches read the tile with 128-bit loads.
+// builds every level: each 64x64 tile of level 0 is reduced by one CTA to levels 1..6
+// (hiz_tile.cuh), and the CTA of the last tile finishes the levels above 6. A view whose
+// depth TMA can address (16-byte aligned, row pitch a multiple of 4 floats) runs the
+// persistent form, which streams the tiles into shared memory with TMA loads; other inputs
+// are read straight into registers, a tile per CTA.
 
 #include <cudaTypedefs.h>  // PFN_cuTensorMapEncodeTiled
 
@@ -23,32 +22,18 @@ namespace helio {
 
 namespace {
 
-// `single` is used when jobs == nullptr (one view, job passed by value);
-// otherwise jobs[] holds n_jobs views. The job is copied to shared memory so
-// that its level arrays can be indexed at run time.
-__global__ void __launch_bounds__(256, 3) hiz_build_kernel(HizJob single, const HizJob* __restrict__ jobs,
-                                                        uint32_t n_jobs, uint32_t* tickets) {
-    __shared__ float s_m3[8][9];
-    __shared__ HizJob s_J;
-    __shared__ uint32_t s_job;
-    const uint32_t tile = blockIdx.x;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0;
-        if (jobs) {
-            uint32_t hi = n_jobs - 1;
-            while (lo < hi) {  // last job with tile_begin <= tile
-                uint32_t mid = (lo + hi + 1) >> 1;
-                if (jobs[mid].tile_begin <= tile) lo = mid;
-                else hi = mid - 1;
-            }
-            s_J = jobs[lo];
-        } else {
-            s_J = single;
-        }
-        s_job = lo;
-    }
+// One tile per CTA of four warps, its level 0 loaded into registers (128-bit loads where the
+// rows allow them, else 32 independent 4-byte loads per lane). 1367x769, whose rows no wide load
+// fits: 8.2 us per launch back to back, 10.1 with 256 threads per tile, the job copied by one
+// thread and the tail level by level. 8 CTAs per SM hide the loads' latency; the job is copied to shared memory for the tail, whose fields of levels 7.. no tile
+// reads (from the parameter space each would wait for a cold constant-cache line).
+__global__ void __launch_bounds__(kHizBlockThreads, 8)
+    hiz_build_kernel(const __grid_constant__ HizJob J, uint32_t* ticket) {
+    __shared__ __align__(16) HizJob s_J;
+    for (uint32_t i = threadIdx.x; i < sizeof(HizJob) / 4u; i += kHizBlockThreads)
+        reinterpret_cast<uint32_t*>(&s_J)[i] = reinterpret_cast<const uint32_t*>(&J)[i];
     __syncthreads();
-    hiz_tile(s_J, s_job, tile - s_J.tile_begin, tickets, s_m3);
+    hiz_tile_block(s_J, blockIdx.x, ticket);
 }
 
 // Persistent form for one view whose level 0 TMA can address: CTA b takes tiles b, b + G,
@@ -57,15 +42,12 @@ __global__ void __launch_bounds__(256, 3) hiz_build_kernel(HizJob single, const 
 // (32x32 texels; q = 2 * row + column) of a landed tile on its own: each lane holds an
 // 8-row x 4-column block, registers give levels 1 and 2, warp shuffles levels 3..5. The
 // quadrants' level-5 texels meet in shared memory and thread 0 forms the tile's level-6
-// texel after the next tile's barrier, so a tile costs one barrier of 4 warps. Every 2x2
-// step takes its four texels in the order of hiz_build_kernel (top-left, top-right,
-// bottom-left, bottom-right) through hiz_red4, so both forms give identical pyramids.
+// texel after the next tile's barrier, so a tile costs one barrier of 4 warps.
 constexpr int kHizStages = 2;
 constexpr int kHizTmaThreads = 128;
 constexpr int kHizTmaCtasPerSm = 6;
 constexpr uint32_t kHizTileBytes = kHizTile * kHizTile * 4u;
 constexpr uint32_t kHizWaitPolls = 1u << 20;  // bounded wait for a landed tile
-static_assert(2 * kHizTailBuf <= kHizStages * kHizTile * kHizTile, "the tail's two level buffers fit the staging");
 
 __global__ void __launch_bounds__(kHizTmaThreads, kHizTmaCtasPerSm)
     hiz_build_tma_kernel(const __grid_constant__ CUtensorMap src, const __grid_constant__ HizJob J, uint32_t* ticket,
@@ -143,8 +125,8 @@ __global__ void __launch_bounds__(kHizTmaThreads, kHizTmaCtasPerSm)
         }
         prev = t;
     }
-    // A wait that gave up leaves later loads in flight: wait for them (bounded) before
-    // the tail reuses the staging buffers or the CTA's shared memory is released.
+    // A wait that gave up leaves later loads in flight: wait for them (bounded) before the
+    // CTA's shared memory is released.
     if (tid == 0) {
         for (uint32_t j = k; j < k + kHizStages; ++j)
             if (blockIdx.x + j * G < tiles)
@@ -166,8 +148,7 @@ __global__ void __launch_bounds__(kHizTmaThreads, kHizTmaCtasPerSm)
         }
         __syncthreads();
         if (deferred) hiz_quad_copy0(J, dX0, dY0, q, v);
-        // Every tile has landed and been read: the staging buffers hold the tail's levels.
-        if (s_last) hiz_tail_body<4, 4>(s_J, s_stage, s_stage + kHizTailBuf);
+        if (s_last) hiz_tail(s_J, (uint32_t)q, 4u);
     }
 }
 
@@ -246,14 +227,6 @@ void hiz_assign(HizJob* job, const float* depth, float* levels_base) {
     }
 }
 
-void launch_hiz_build(const HizJob* jobs_dev, uint32_t n_jobs, uint32_t total_tiles, uint32_t* tickets_dev,
-                      cudaStream_t stream) {
-    if (total_tiles == 0 || n_jobs == 0) return;
-    helio_launch_begin("hiz_build", stream);
-    hiz_build_kernel<<<total_tiles, 256, 0, stream>>>(HizJob{}, jobs_dev, n_jobs, tickets_dev);
-    helio_launch_end(stream);
-}
-
 void launch_hiz_build_tma(const CUtensorMap& src, const HizJob& job, uint32_t* ticket_dev, uint32_t* error_dev,
                           cudaStream_t stream) {
     const uint32_t tiles = job.tiles_x * job.tiles_y;
@@ -290,7 +263,7 @@ void launch_hiz_build_single(const HizJob& job, uint32_t* ticket_dev, cudaStream
     const uint32_t tiles = job.tiles_x * job.tiles_y;
     if (tiles == 0) return;
     helio_launch_begin("hiz_build", stream);
-    hiz_build_kernel<<<tiles, 256, 0, stream>>>(job, nullptr, 1u, ticket_dev);
+    hiz_build_kernel<<<tiles, kHizBlockThreads, 0, stream>>>(job, ticket_dev);
     helio_launch_end(stream);
 }
 

@@ -35,11 +35,8 @@ size_t hiz_layout(uint32_t width, uint32_t height, uint32_t depth_pitch, bool co
                   HizJob* job);
 void hiz_assign(HizJob* job, const float* depth, float* levels_base);
 
-// jobs_dev: n_jobs jobs in device memory, tile_begin ascending; tickets_dev:
-// n_jobs zero-initialised counters (left zero after the launch).
-void launch_hiz_build(const HizJob* jobs_dev, uint32_t n_jobs, uint32_t total_tiles,
-                      uint32_t* tickets_dev, cudaStream_t stream);
-// One view, job passed by value (tile_begin must be 0).
+// One view, job passed by value (tile_begin must be 0); ticket_dev: one zero-initialised
+// counter (left zero after the launch).
 void launch_hiz_build_single(const HizJob& job, uint32_t* ticket_dev, cudaStream_t stream);
 
 // Tensor map of a 2-D float array (width x height, row pitch in floats) read in boxes of

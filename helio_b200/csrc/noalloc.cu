@@ -48,27 +48,23 @@ struct NoAllocJobs {
 
 static __device__ __align__(256) unsigned char g_noalloc_hiz_scratch[sizeof(NoAllocScratch)];
 
-// The multi-view Hi-Z build of hiz.cu, reading its job table from the parameter
-// instead of device memory: one CTA per 64x64 tile, the job found by a binary search
-// over tile_begin, the last CTA of each view building levels 7.. (tickets[view]).
-__global__ void __launch_bounds__(256) hiz_build_noalloc_kernel(const __grid_constant__ NoAllocJobs table,
-                                                                uint32_t n_jobs, uint32_t* tickets) {
-    __shared__ float s_m3[8][9];
-    __shared__ helio::HizJob s_J;
-    __shared__ uint32_t s_job;
+// One CTA of four warps per 64x64 tile of any view, the view's job found by a binary search
+// over tile_begin in the parameter and copied to shared memory; the last CTA of each view
+// builds levels 7.. (tickets[view]).
+__global__ void __launch_bounds__(helio::kHizBlockThreads, 8)
+    hiz_build_noalloc_kernel(const __grid_constant__ NoAllocJobs table, uint32_t n_jobs, uint32_t* tickets) {
+    __shared__ __align__(16) helio::HizJob s_J;
     const uint32_t tile = blockIdx.x;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {  // last job with tile_begin <= tile
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (table.jobs[mid].tile_begin <= tile) lo = mid;
-            else hi = mid - 1;
-        }
-        s_J = table.jobs[lo];
-        s_job = lo;
+    uint32_t lo = 0, hi = n_jobs - 1;
+    while (lo < hi) {  // last job with tile_begin <= tile
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (table.jobs[mid].tile_begin <= tile) lo = mid;
+        else hi = mid - 1;
     }
+    for (uint32_t i = threadIdx.x; i < sizeof(helio::HizJob) / 4u; i += helio::kHizBlockThreads)
+        reinterpret_cast<uint32_t*>(&s_J)[i] = reinterpret_cast<const uint32_t*>(&table.jobs[lo])[i];
     __syncthreads();
-    helio::hiz_tile(s_J, s_job, tile - s_J.tile_begin, tickets, s_m3);
+    helio::hiz_tile_block(s_J, tile - s_J.tile_begin, tickets + lo);
 }
 
 constexpr int kMaxDevices = 64;
@@ -152,7 +148,7 @@ extern "C" int32_t helio_hiz_build_noalloc(uint32_t view_count, const helio_hiz_
         return noalloc_fail(HELIO_ERR_CUDA, "helio_hiz_build_noalloc: clearing the tickets failed");
     if (tiles == 0) return HELIO_OK;
     helio_launch_begin("hiz_build_noalloc", s);
-    hiz_build_noalloc_kernel<<<tiles, 256, 0, s>>>(table, view_count, dev_scratch->tickets);
+    hiz_build_noalloc_kernel<<<tiles, helio::kHizBlockThreads, 0, s>>>(table, view_count, dev_scratch->tickets);
     helio_launch_end(s);
     if (cudaGetLastError() != cudaSuccess)
         return noalloc_fail(HELIO_ERR_CUDA, "helio_hiz_build_noalloc: kernel launch failed");

@@ -115,3 +115,33 @@ def test_hiz_repeated_launches_stable(cuda):
     torch.cuda.synchronize()
     got = [hz.level(l).cpu().numpy() for l in range(hz.publish().mip_count)]
     _levels_equal(got, O.hiz_build(depth))
+
+
+@pytest.mark.parametrize("w,h", [(127, 129), (128, 64), (2047, 130), (2048, 128), (2112, 65), (2111, 2113),
+                                 (4095, 191), (4161, 2049), (130, 6209), (12345, 67)])
+def test_hiz_tail_quadrant_edges(cuda, w, h):
+    """Level 6 just below, at and above one 32x32 quadrant, one row or column high, and several
+    quadrants wide, through the TMA form (even pitch), the register form (odd pitch, TMA off)
+    and the no-allocation call."""
+    import ctypes as C
+
+    import torch
+    from helio_b200 import native as N
+
+    rng = np.random.default_rng(w * 13 + h)
+    depth = rng.random((h, w), dtype=np.float32)
+    ref = O.hiz_build(depth)
+    for kw in ({"pitch": (w + 7) // 4 * 4}, {"pitch": w + 5}, {"tma": False}, {"alias": True}):
+        _, g = gpu_hiz(depth, **kw)
+        _levels_equal(g, ref)
+    lib, d = N.cull_lib(), torch.from_numpy(depth).cuda()
+    views = (N.HizViewInput * 2)(*[N.HizViewInput(d.data_ptr(), w, h, 0, 0)] * 2)
+    pyr = (N.HizPyramid * 2)()
+    out = torch.zeros(2 * sum((x.shape[1] + 3) // 4 * 4 * x.shape[0] for x in ref) + 8, device="cuda")
+    N.check(lib.helio_hiz_build_noalloc(2, views, out.data_ptr(), out.numel(), pyr, None))
+    torch.cuda.synchronize()
+    for p in pyr:
+        for l, r in enumerate(ref):
+            at = (p.levels[l] - out.data_ptr()) // 4
+            got = out[at:at + p.pitch[l] * p.height[l]].cpu().numpy().reshape(p.height[l], p.pitch[l])[:, :p.width[l]]
+            np.testing.assert_array_equal(got.view(np.uint32), r.view(np.uint32), err_msg=f"level {l}")
