@@ -251,12 +251,11 @@ class PlainWorkload:
 
     def kernel_bytes(self) -> tuple[dict, int]:
         """Bytes an ideal implementation must move per launch, from the step's outputs:
-        hiz_build = depth read + level-0 copy + levels 1.. written; vg_select = 164 B per
+        hiz_build = depth read + level-0 copy + levels 1.. written; vg_frame = 148 B per
         object (64 B head / bounds / LOD errors, 64 B model, 16 B InstanceCullData, 4 B
-        selected-LOD write, 16 B selected-range record); vg_cull_test = 24 B per work item
-        (item, selected range, visibility words) + 80 B per active item (model + cull
-        data) + 44 B per tested meshlet (centre, radius, cone apex, cutoff, axis);
-        vg_cull_emit = 48 B per visible draw (12 B read, 36 B written)."""
+        selected-LOD write) + 16 B per work item (item, visibility words) + 44 B per tested
+        meshlet (centre, radius, cone apex, cutoff, axis) + 48 B per visible draw (12 B read,
+        36 B written)."""
         v, depth, cam, hz, vg = self.passes[0]
         o = vg.outputs()
         counters = o["counters"].cpu().numpy().view(np.uint32)
@@ -266,10 +265,10 @@ class PlainWorkload:
         sp1 = selected.astype(np.int64)
         cnt = np.where(sp1 > 0, obj["lod_meshlet_counts"][np.arange(len(obj)), np.maximum(sp1 - 1, 0)], 0)
         n = np.clip(cnt[items["object_index"].astype(np.int64)] - items["local_meshlet_base"].astype(np.int64), 0, 64)
-        tested, active = int(n.sum()), int((n > 0).sum())
+        tested = int(n.sum())
         hz = hiz_bytes(v.width, v.height, True)  # the TMA form or the 128-bit-load form, whichever ran
-        return {"hiz_build_tma": hz, "hiz_build": hz, "vg_select": 164 * len(obj),
-                "vg_cull_test": 24 * len(items) + 80 * active + 44 * tested, "vg_cull_emit": 48 * visible}, visible
+        return {"hiz_build_tma": hz, "hiz_build": hz,
+                "vg_frame": 148 * len(obj) + 16 * len(items) + 44 * tested + 48 * visible}, visible
 
     def e2e(self):
         import torch

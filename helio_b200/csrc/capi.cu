@@ -181,15 +181,14 @@ struct helio_vg_pass {
     // Scene (device resident).
     DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, items, staging;
     // Outputs and scratch.
-    DevBuf indirect, draws, visibility, sel, scratch;
+    DevBuf indirect, draws, visibility;
+    DevBuf scratch;  // published counters (16 words) | kVgStateWords state words | tile statuses
     uint32_t capacity = 0;
     uint32_t meshlet_count = 0, object_count = 0, work_item_count = 0, max_draw_count = 0;
     uint64_t last_version = 0, last_instance_version = 0;
     bool have_version = false;
     uint32_t num_tiles = 0;
-    uint32_t items_per_warp = 32;
-    size_t scratch_clear_bytes = 0;
-    size_t view_offset = 0;
+    uint32_t tile_items = helio::kMaxTileItems;
 };
 
 // ════════════════════════════════════════════════════════════════════════════
@@ -604,7 +603,6 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->instances.ensure(O * sizeof(HelioGpuInstanceData)));
         HELIO_CK(p->cull.ensure(O * sizeof(HelioInstanceCullData)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
-        HELIO_CK(p->sel.ensure(O * sizeof(helio::SelRecord)));
         HELIO_CK(p->visibility.ensure(W * 8));
         const HelioGpuMeshletEntry* aos = f->meshlets;
         if (M) {
@@ -641,14 +639,11 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
             p->capacity = cap;
         }
         p->max_draw_count = bounded;
-        p->items_per_warp = helio::vg_cull_items_per_warp(p->work_item_count);
-        p->num_tiles = helio::vg_cull_tiles(p->work_item_count, p->items_per_warp);
-        // scratch: counters (16 words) | tile counts (both cleared per execute) | warp counts |
-        //          window bits | view constants (16-byte aligned)
-        p->scratch_clear_bytes = 64 + (size_t)p->num_tiles * 4;
-        p->view_offset = (64 + helio::vg_cull_scratch_words(p->num_tiles) * 4 + 15) & ~(size_t)15;
-        HELIO_CK(p->scratch.ensure(p->view_offset + sizeof(helio::CullView)));
-        HELIO_CK(cudaMemsetAsync(p->scratch.ptr, 0, p->scratch_clear_bytes, s));
+        p->tile_items = helio::vg_tile_items(p->work_item_count);
+        p->num_tiles = helio::vg_tiles(p->work_item_count, p->tile_items);
+        const size_t scratch_bytes = (16 + helio::kVgStateWords) * 4 + (size_t)p->num_tiles * 8;
+        HELIO_CK(p->scratch.ensure(scratch_bytes));
+        HELIO_CK(cudaMemsetAsync(p->scratch.ptr, 0, scratch_bytes, s));
         p->last_version = f->buffer_version;
         p->last_instance_version = f->instance_version;
         p->have_version = true;
@@ -678,7 +673,6 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
     if (st != HELIO_OK) return st;
     cudaStream_t s = as_stream(stream);
     uint32_t* scratch = p->scratch.as<uint32_t>();
-    HELIO_CK(cudaMemsetAsync(p->scratch.ptr, 0, p->scratch_clear_bytes, s));
     if (p->cfg.flags & HELIO_VG_CLEAR_INDIRECT)  // rendering.rs:1128-1130
         HELIO_CK(cudaMemsetAsync(p->indirect.ptr, 0, (size_t)p->capacity * sizeof(HelioDrawIndexedIndirectArgs), s));
 
@@ -696,48 +690,24 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
     scene.instance_count = p->object_count;
     scene.work_item_count = p->work_item_count;
 
-    helio::CullView* view =
-        reinterpret_cast<helio::CullView*>(reinterpret_cast<char*>(p->scratch.ptr) + p->view_offset);
-    helio::ViewSetupParams vs{};
-    vs.camera = camera_dev;
-    vs.out = view;
-    vs.hiz = to_view(*hiz);
-    vs.screen_height = p->cfg.height;
-    vs.hiz_mip_count = mip_levels(p->cfg.width, p->cfg.height);  // unclamped, rendering.rs:828-829
-    vs.lod_threshold_px = p->lod_threshold;
-
-    helio::VgSelectParams sp{};
-    // The select blocks build the view constants themselves (block 0 publishes them for
-    // the meshlet kernels); only an empty scene, with no select launch, needs the setup launch.
-    if (p->object_count) {
-        sp.compute_view = 1u;
-        sp.setup = vs;
-    } else {
-        helio::launch_vg_view_setup(vs, s);
-    }
-    sp.scene = scene;
-    sp.view = view;
-    sp.sel = p->sel.as<helio::SelRecord>();
-    sp.counters = scratch;
-    sp.counter_count = p->counter_count;
-    sp.write_reserved = 1u;
-    helio::launch_vg_select(sp, s);
-
-    helio::VgCullParams cp{};
-    cp.scene = scene;
-    cp.view = view;
-    cp.sel = p->sel.as<helio::SelRecord>();
-    cp.indirect = p->indirect.as<HelioDrawIndexedIndirectArgs>();
-    cp.draws = p->draws.as<HelioGpuVgDraw>();
-    cp.counters = scratch;
-    cp.visibility = p->visibility.as<uint32_t>();
-    cp.scratch.tile_counts = scratch + 16;
-    cp.scratch.warp_counts = cp.scratch.tile_counts + p->num_tiles;
-    cp.scratch.bits = cp.scratch.warp_counts + (size_t)p->num_tiles * helio::kCullWarps;
-    cp.capacity = p->max_draw_count;  // min(draw_capacity, buffer lengths), vg_cull.wgsl:248-251
-    cp.num_tiles = p->num_tiles;
-    cp.items_per_warp = p->items_per_warp;
-    HELIO_CK(helio::launch_vg_cull(cp, s));
+    helio::VgFrameParams fp{};
+    fp.scene = scene;
+    fp.setup.camera = camera_dev;
+    fp.setup.hiz = to_view(*hiz);
+    fp.setup.screen_height = p->cfg.height;
+    fp.setup.hiz_mip_count = mip_levels(p->cfg.width, p->cfg.height);  // unclamped, rendering.rs:828-829
+    fp.setup.lod_threshold_px = p->lod_threshold;
+    fp.indirect = p->indirect.as<HelioDrawIndexedIndirectArgs>();
+    fp.draws = p->draws.as<HelioGpuVgDraw>();
+    fp.counters = scratch;
+    fp.visibility = p->visibility.as<uint32_t>();
+    fp.state = scratch + 16;
+    fp.status = reinterpret_cast<unsigned long long*>(fp.state + helio::kVgStateWords);
+    fp.capacity = p->max_draw_count;  // min(draw_capacity, buffer lengths), vg_cull.wgsl:248-251
+    fp.num_tiles = p->num_tiles;
+    fp.tile_items = p->tile_items;
+    fp.counter_count = p->counter_count;
+    HELIO_CK(helio::launch_vg_frame(fp, s));
     HELIO_CK(cudaGetLastError());
     return HELIO_OK;
 }
@@ -773,10 +743,13 @@ int32_t helio_vg_publish(const helio_vg_pass* p, helio_vg_outputs* out) {
 
 int32_t helio_vg_device_status(helio_vg_pass* p, void* stream) {
     HELIO_ARG(p, "null pointer");
-    // The VG kernels never wait on one another inside a launch; this reports any
-    // asynchronous CUDA error of the work queued so far.
+    uint32_t err = 0;
+    if (p->scratch.ptr)
+        HELIO_CK(cudaMemcpyAsync(&err, p->scratch.as<uint32_t>() + 16 + helio::kVgError, 4, cudaMemcpyDeviceToHost,
+                                 as_stream(stream)));
     HELIO_CK(cudaStreamSynchronize(as_stream(stream)));
     HELIO_CK(cudaGetLastError());
+    if (err & helio::kDevTimeout) return fail(HELIO_ERR_TIMEOUT, "a meshlet tile's wait for the tiles before it gave up");
     return HELIO_OK;
 }
 

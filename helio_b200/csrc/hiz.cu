@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "hiz_tile.cuh"
+#include "host_util.h"
 #include "kernels.h"
 #include "tma.cuh"
 
@@ -30,9 +31,11 @@ namespace {
 __global__ void __launch_bounds__(kHizBlockThreads, 8)
     hiz_build_kernel(const __grid_constant__ HizJob J, uint32_t* ticket) {
     __shared__ __align__(16) HizJob s_J;
+    pdl_launch_dependents();
     for (uint32_t i = threadIdx.x; i < sizeof(HizJob) / 4u; i += kHizBlockThreads)
         reinterpret_cast<uint32_t*>(&s_J)[i] = reinterpret_cast<const uint32_t*>(&J)[i];
     __syncthreads();
+    pdl_wait();  // the depth, and the readers of the previous pyramid
     hiz_tile_block(s_J, blockIdx.x, ticket);
 }
 
@@ -68,9 +71,13 @@ __global__ void __launch_bounds__(kHizTmaThreads, kHizTmaCtasPerSm)
         tma_load_2d(s_stage + s * (kHizTile * kHizTile), &src, &s_full[s], (int32_t)(tx * kHizTile),
                     (int32_t)(ty * kHizTile));
     };
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < kHizStages; ++s) mbar_init(&s_full[s], 1u);
         mbar_init_fence();
+    }
+    pdl_wait();  // the depth, and the readers of the previous pyramid
+    if (tid == 0) {
         for (int s = 0; s < kHizStages; ++s)
             if (blockIdx.x + s * G < tiles) issue(blockIdx.x + s * G, s);
     }
@@ -255,7 +262,7 @@ void launch_hiz_build_tma(const CUtensorMap& src, const HizJob& job, uint32_t* t
     }
     const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)full);
     helio_launch_begin("hiz_build_tma", stream);
-    hiz_build_tma_kernel<<<grid, kHizTmaThreads, smem, stream>>>(src, job, ticket_dev, error_dev);
+    launch_after(hiz_build_tma_kernel, grid, kHizTmaThreads, smem, stream, src, job, ticket_dev, error_dev);
     helio_launch_end(stream);
 }
 
@@ -263,7 +270,7 @@ void launch_hiz_build_single(const HizJob& job, uint32_t* ticket_dev, cudaStream
     const uint32_t tiles = job.tiles_x * job.tiles_y;
     if (tiles == 0) return;
     helio_launch_begin("hiz_build", stream);
-    hiz_build_kernel<<<tiles, kHizBlockThreads, 0, stream>>>(job, ticket_dev);
+    launch_after(hiz_build_kernel, tiles, kHizBlockThreads, 0, stream, job, ticket_dev);
     helio_launch_end(stream);
 }
 

@@ -63,6 +63,25 @@ struct DevBuf {
     }
 };
 
+// Launches `kernel` with programmatic stream serialization: its CTAs may be scheduled while the
+// stream's previous kernel finishes, and wait in pdl_wait before their first global access,
+// which hides a launch gap.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t stream,
+                                A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 inline uint32_t host_mip_levels(uint32_t w, uint32_t h) {
     uint32_t m = w > h ? w : h, bits = 0;
     while (m) {

@@ -1,28 +1,31 @@
 // vg_cull.cu — virtual-geometry object select and meshlet cull (VirtualGeometryPass).
 //
 // References (crates/helio-pass-virtual-geometry/):
-//   shaders/vg_cull.wgsl:282-352   cs_select_objects  -> vg_select_kernel
+//   shaders/vg_cull.wgsl:282-352   cs_select_objects  -> select_object
 //   shaders/vg_cull.wgsl:135-264   cull_meshlet       -> meshlet_visible + emission
-//   shaders/vg_cull.wgsl:354-405   cs_cull_meshlets   -> vg_cull_test_kernel + vg_cull_emit_kernel
+//   shaders/vg_cull.wgsl:354-405   cs_cull_meshlets   -> vg_frame_kernel
 //   src/lib.rs:132-167             InstanceCullData::from_instance -> instance_cull_data_kernel
 //
 // Layout and scheduling (B200 design, not a translation of the WGSL dispatches):
 //   * meshlet descriptors are re-laid once per upload into four 16-byte streams;
-//   * a warp owns 32 consecutive work items (one per lane); the lanes read their
-//     item and the object's selected-LOD record, then the warp packs the active
-//     meshlets of all 32 items densely into 32-lane windows, so a work item whose
-//     LOD has 13 meshlets occupies 13 lanes instead of a 64-lane group;
-//   * visible meshlets are compacted deterministically in two launches without
-//     any device-side wait: the test kernel stores each warp's window ballots and
-//     the per-tile / per-warp visible counts; the emit kernel runs only for tiles
-//     with visible meshlets, sums the counts of the tiles before it, and writes
-//     each draw at slot = (visible meshlets before it in (work item, lane) order).
-//     The reference appends with atomicAdd (vg_cull.wgsl:247), so its order is
-//     unspecified; this order is reproducible and first_instance = slot.
+//   * one launch does the whole view. A tile CTA takes up to 256 consecutive work items, one
+//     per thread, and selects their objects itself (an object's few items repeat its select,
+//     from L2, which costs less than a launch and a round trip of records in between); it then
+//     packs the items' active meshlets densely into 32-lane windows shared out over its warps,
+//     so a work item whose LOD has 13 meshlets occupies 13 lanes and a warp whose items are all
+//     visible does not run on alone;
+//   * further CTAs run the select once per object for its outputs (objects[i].reserved, the
+//     LOD histogram), in the shadow of the tiles;
+//   * visible meshlets are compacted deterministically: tiles are handed out in order by a
+//     ticket, each publishes its count and takes its first slot from the tiles before it
+//     (decoupled look-back, bounded), so each draw lands at slot = (visible meshlets before it
+//     in (work item, lane) order). The reference appends with atomicAdd (vg_cull.wgsl:247), so
+//     its order is unspecified; this order is reproducible and first_instance = slot.
 
 #include <algorithm>
 
 #include "common.cuh"
+#include "host_util.h"
 #include "kernels.h"
 #include "vg.h"
 #include "vg_device.cuh"
@@ -90,13 +93,18 @@ __global__ void instance_cull_data_kernel(const HelioGpuInstanceData* __restrict
     }
 }
 
-// ── View constants (one warp per launch) ──────────────────────────────────────
+// ── View constants ────────────────────────────────────────────────────────────
 
 // The view constants of P's camera into v (shared memory), by one warp (every lane of
-// the warp calls it; lanes 0..5 build the planes, lane 0 the rest).
+// the warp calls it; lanes 0..5 build the planes, lane 0 the camera's fields, all of them copy
+// the pyramid descriptor).
 __device__ __forceinline__ void view_setup_warp(const ViewSetupParams& P, CullView& v) {
+    const uint32_t lane = threadIdx.x & 31u;
     publish_planes_warp(P.camera->view_proj, v.planes);
-    if ((threadIdx.x & 31) == 0) {
+    static_assert(sizeof(HizView) % 4 == 0, "copied word by word");
+    for (uint32_t k = lane; k < sizeof(HizView) / 4; k += 32u)
+        reinterpret_cast<uint32_t*>(&v.hiz)[k] = reinterpret_cast<const uint32_t*>(&P.hiz)[k];
+    if (lane == 0) {
         const HelioGpuCameraUniforms* cam = P.camera;
         v.vp = ldg_mat4(cam->view_proj);
         v.pos_near = __ldg(reinterpret_cast<const float4*>(cam->position_near));
@@ -104,7 +112,6 @@ __device__ __forceinline__ void view_setup_warp(const ViewSetupParams& P, CullVi
         v.p11 = __ldg(&cam->proj[5]);
         v.focal = fmul(fmul(fabsf(v.p11), (float)P.screen_height), 0.5f);
         v.lod_threshold_px = P.lod_threshold_px;
-        v.hiz = P.hiz;
         v.screen_height = P.screen_height;
         v.hiz_mip_count = P.hiz_mip_count;
         v.pad[0] = v.pad[1] = 0u;
@@ -112,271 +119,352 @@ __device__ __forceinline__ void view_setup_warp(const ViewSetupParams& P, CullVi
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(32) vg_view_setup_kernel(ViewSetupParams P) {
-    __shared__ CullView s_view;
-    view_setup_warp(P, s_view);
-    if (threadIdx.x == 0) *P.out = s_view;
-}
-
 // ── Object select: cs_select_objects (vg_cull.wgsl:282-352) ───────────────────
 
-__global__ void __launch_bounds__(256) vg_select_kernel(VgSelectParams P) {
-    __shared__ CullView s_view;
-    pdl_launch_dependents();  // the meshlet tests may be scheduled (they wait for this grid)
-    if (P.compute_view) {
-        // The view setup folded in: warp 0 builds the constants; block 0 publishes them.
-        if (threadIdx.x < 32) view_setup_warp(P.setup, s_view);
-        __syncthreads();
-        if (blockIdx.x == 0) {
-            const uint4* src = reinterpret_cast<const uint4*>(&s_view);
-            uint4* dst = reinterpret_cast<uint4*>(P.setup.out);
-            for (uint32_t k = threadIdx.x; k < sizeof(CullView) / 16; k += blockDim.x) dst[k] = src[k];
-        }
-    } else {
-        load_view(P.view, s_view, threadIdx.x, blockDim.x);
-        __syncthreads();
+struct Selected {
+    uint32_t sel;  // LOD + 1, 0 = culled
+    uint32_t lod_count, instance;
+};
+
+// The instance index and LOD count only: `reserved`, in the same 16 bytes, is written by this
+// launch.
+__device__ __forceinline__ uint2 object_head(const HelioGpuVgObject* o) {
+    return __ldg(reinterpret_cast<const uint2*>(o));
+}
+
+__device__ __forceinline__ Selected select_object(const VgSceneDev& S, const CullView& view,
+                                                  const HelioGpuVgObject* o, uint2 head) {
+    Selected r{0u, min(head.y, 8u), head.x};
+    if (r.lod_count == 0u || r.instance >= S.instance_count) return r;
+    // The object's fields and the instance's in one round trip.
+    const float4 lb = __ldg(reinterpret_cast<const float4*>(o->local_bounds));
+    const float4 e0 = __ldg(reinterpret_cast<const float4*>(o->lod_errors));
+    const float4 e1 = __ldg(reinterpret_cast<const float4*>(o->lod_errors + 4));
+    const HelioInstanceCullData cd = load_cull(S.cull + r.instance);
+    const Mat4 model = ldg_mat4(S.instances[r.instance].model);
+    if (cd.valid_transform == 0u) return r;
+    const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
+    const float wr = fmaxf(fmul(lb.w, cd.max_scale), 0.0f);
+    if (!sphere_visible_vg(view.planes, c, wr)) return r;
+    const float4 pn = view.pos_near;
+    const F3 d = sub3(c, f3(pn.x, pn.y, pn.z));
+    const float dist = fsqrt(dot3(d, d));
+    const float closest = fmaxf(fsub(dist, wr), fmaxf(pn.w, 1.0e-4f));
+    const float focal = view.focal;
+    const QuotientBound qb = quotient_bound(view.lod_threshold_px);
+    const float rc = quotient_rcp(closest);
+    const float err[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+    uint32_t lod = 0;
+#pragma unroll
+    for (uint32_t level = 1; level < 8; ++level) {
+        if (level >= r.lod_count) break;
+        // px = err * max_scale * focal / closest; px <= threshold keeps the level.
+        if (quotient_le(fmul(fmul(err[level], cd.max_scale), focal), closest, rc, qb)) lod = level;
+        else break;
     }
-    const Planes& s_planes = s_view.planes;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
+    r.sel = lod + 1u;
+    return r;
+}
+
+// Object CTA: the select's outputs of 256 objects. The CTA that finishes last (an atomic count)
+// publishes the histogram and leaves the accumulators at zero for the next launch.
+__device__ void object_block(const VgFrameParams& P, const CullView& view, uint32_t block, uint32_t blocks,
+                             uint32_t* s_hist, uint32_t* s_flag) {
     const VgSceneDev& S = P.scene;
-    bool vis = false;
-    uint32_t selected = 0, lod_count = 0;
+    const uint32_t i = block * (kCullWarps * 32u) + threadIdx.x, lane = threadIdx.x & 31u;
+    if (threadIdx.x < 9) s_hist[threadIdx.x] = 0u;
+    Selected r{0u, 0u, 0u};
     if (i < S.object_count) {
-        const HelioGpuVgObject* o = S.objects + i;
-        // One round trip for the object fields, one for the instance fields.
-        const uint4 head = __ldg(reinterpret_cast<const uint4*>(o));  // instance_index, lod_count, max_meshlet_count, reserved
-        const float4 lb = __ldg(reinterpret_cast<const float4*>(o->local_bounds));
-        const float4 e0 = __ldg(reinterpret_cast<const float4*>(o->lod_errors));
-        const float4 e1 = __ldg(reinterpret_cast<const float4*>(o->lod_errors + 4));
-        lod_count = min(head.y, 8u);
-        const uint32_t ii = head.x;
-        uint32_t sel = 0;
-        if (lod_count > 0u && ii < S.instance_count) {
-            const HelioInstanceCullData cd = load_cull(S.cull + ii);
-            const Mat4 model = ldg_mat4(S.instances[ii].model);
-            if (cd.valid_transform != 0u) {
-                const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
-                const float wr = fmaxf(fmul(lb.w, cd.max_scale), 0.0f);
-                if (sphere_visible_vg(s_planes, c, wr)) {
-                    const float4 pn = s_view.pos_near;
-                    const F3 d = sub3(c, f3(pn.x, pn.y, pn.z));
-                    const float dist = fsqrt(dot3(d, d));
-                    const float closest = fmaxf(fsub(dist, wr), fmaxf(pn.w, 1.0e-4f));
-                    const float focal = s_view.focal;
-                    const QuotientBound qb = quotient_bound(s_view.lod_threshold_px);
-                    const float r = quotient_rcp(closest);
-                    const float err[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-                    uint32_t lod = 0;
-#pragma unroll
-                    for (uint32_t level = 1; level < 8; ++level) {
-                        if (level >= lod_count) break;
-                        // px = err * max_scale * focal / closest; px <= threshold keeps the level.
-                        if (quotient_le(fmul(fmul(err[level], cd.max_scale), focal), closest, r, qb)) lod = level;
-                        else break;
-                    }
-                    selected = lod;
-                    sel = lod + 1;
-                    vis = true;
-                }
-            }
-        }
-        SelRecord rec = make_uint4(0u, 0u, ii, sel);
-        if (sel) {
-            rec.x = __ldg(&o->lod_first_meshlets[sel - 1]);
-            rec.y = __ldg(&o->lod_meshlet_counts[sel - 1]);
-        }
-        P.sel[i] = rec;
-        if (P.write_reserved) S.objects[i].reserved = sel;
+        r = select_object(S, view, S.objects + i, object_head(S.objects + i));
+        S.objects[i].reserved = r.sel;
     }
-    if (P.counter_count >= 11u) {
+    if (P.counter_count < 11u) return;  // uniform over the grid
+    __syncthreads();
 #pragma unroll
-        for (uint32_t l = 0; l < 8; ++l) {
-            const uint32_t n = __popc(__ballot_sync(0xffffffffu, vis && selected == l));
-            if (lane == 0 && n) atomicAdd(P.counters + 2 + l, n);
-        }
-        uint32_t mx = vis ? lod_count - 1u : 0u;
-        const bool any = __ballot_sync(0xffffffffu, vis) != 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0 && any) atomicMax(P.counters + 10, mx);
+    for (uint32_t l = 0; l < 8; ++l) {
+        const uint32_t n = __popc(__ballot_sync(0xffffffffu, r.sel == l + 1u));
+        if (lane == 0 && n) atomicAdd(s_hist + l, n);
     }
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, r.sel ? r.lod_count - 1u : 0u);
+    if (lane == 0 && mx) atomicMax(s_hist + 8, mx);
+    __syncthreads();
+    uint32_t* hist = P.state + kVgHist;
+    if (threadIdx.x < 8 && s_hist[threadIdx.x]) atomicAdd(hist + threadIdx.x, s_hist[threadIdx.x]);
+    if (threadIdx.x == 8 && s_hist[8]) atomicMax(hist + 8, s_hist[8]);
+    __threadfence();  // this CTA's sums before its count
+    __syncthreads();
+    if (threadIdx.x == 0) *s_flag = atomicAdd(P.state + kVgDone, 1u) + 1u == blocks;
+    __syncthreads();
+    if (!*s_flag) return;
+    __threadfence();
+    if (threadIdx.x < 9) {
+        P.counters[2 + threadIdx.x] = __ldcg(hist + threadIdx.x);
+        hist[threadIdx.x] = 0u;
+    }
+    if (threadIdx.x == 0) P.state[kVgDone] = 0u;
 }
 
 // ── Meshlet cull ──────────────────────────────────────────────────────────────
 
-// The 32 work items of one warp (lane = item): active meshlet range and packing offsets.
-struct WarpItems {
-    uint32_t n, first, inst, lod, off, total;
+constexpr uint32_t kThreads = kCullWarps * 32u;
+constexpr uint32_t kMaxWindows = kMaxTileItems * HELIO_VG_MESHLETS_PER_WORK_ITEM / 32u;  // of a tile
+static_assert(kMaxTileItems <= kThreads && kMaxWindows == 2u * kThreads, "one item and two windows per thread");
+
+// Exclusive scan over the CTA; `total` gets the CTA's sum. s: kCullWarps words.
+__device__ __forceinline__ uint32_t tile_scan(uint32_t x, uint32_t* s, uint32_t& total) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t inc = x;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    __syncthreads();
+    if (lane == 31u) s[warp] = inc;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kCullWarps; ++w) {
+        const uint32_t t = s[w];
+        if (w < warp) before += t;
+        total += t;
+    }
+    return before + inc - x;
+}
+
+// The active items of a tile in item order (rank = position among the active ones).
+struct TileItems {
+    uint32_t off[kMaxTileItems];    // packed position of the item's first meshlet
+    uint32_t first[kMaxTileItems];  // its first meshlet
+    uint32_t inst[kMaxTileItems];
+    uint8_t lod[kMaxTileItems];
+    uint32_t heads[kMaxWindows];    // bit p of word w: an item starts at position 32 w + p
+    uint16_t owner[kMaxWindows];    // rank of the item that holds position 32 w
 };
 
-__device__ __forceinline__ WarpItems load_warp_items(const VgSceneDev& S, const SelRecord* sel, uint32_t w_idx) {
-    const int lane = threadIdx.x & 31;
-    WarpItems w{0u, 0u, 0u, 0u, 0u, 0u};
-    if (w_idx < S.work_item_count) {
-        const HelioGpuVgWorkItem it = S.items[w_idx];
-        if (it.object_index < S.object_count) {
-            const SelRecord r = __ldg(sel + it.object_index);
-            if (r.w != 0u && it.local_meshlet_base < r.y) {
-                w.n = min(64u, r.y - it.local_meshlet_base);
-                w.first = r.x + it.local_meshlet_base;
-                w.inst = r.z;
-                w.lod = r.w - 1u;
+// Rank of the item that holds position 32 w + lane.
+__device__ __forceinline__ uint32_t item_at(const TileItems& t, uint32_t w) {
+    const uint32_t le = 0xffffffffu >> (31u - (threadIdx.x & 31u));
+    return t.owner[w] + __popc(t.heads[w] & le & ~1u);
+}
+
+enum : uint32_t { kTileSum = 1u, kTilePrefix = 2u };  // a status holds the tile's count, or all up to it
+
+__device__ __forceinline__ unsigned long long tile_status(uint32_t epoch, uint32_t kind, uint32_t value) {
+    return ((unsigned long long)(epoch & 0x3FFFFFFFu) << 34) | ((unsigned long long)kind << 32) | value;
+}
+// Relaxed GPU-scope accesses: a status carries its whole message.
+__device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_status(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Visible meshlets of the tiles before `tile`, by the whole CTA: thread t waits (bounded) for
+// the status of tile hi - 1 - t; the nearest one that holds a prefix ends the walk, the counts
+// nearer than it are added. Every earlier ticket is held by a CTA that runs and publishes its
+// count without waiting, so the waits end. Returns false, uniformly, when one gave up.
+__device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t epoch, uint32_t* s_red,
+                               uint32_t& prefix) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    prefix = 0;
+    for (uint32_t hi = tile; hi > 0;) {
+        const bool mine = threadIdx.x < hi;
+        unsigned long long st = 0;
+        int lost = 0;
+        if (mine) {
+            const unsigned long long* p = P.status + (hi - 1u - threadIdx.x);
+            uint32_t polls = 0;
+            while (st = ld_status(p), (uint32_t)(st >> 34) != (epoch & 0x3FFFFFFFu)) {
+                if (++polls > kSpinLimit) {
+                    lost = 1;
+                    break;
+                }
+                if (polls > 32u) __nanosleep(polls < 512u ? 32 : 256);
+            }
+        }
+        if (__syncthreads_or(lost)) return false;
+        // The nearest prefix: the lowest thread that saw one.
+        const bool is_prefix = mine && ((uint32_t)(st >> 32) & 3u) == kTilePrefix;
+        const uint32_t bal = __ballot_sync(0xffffffffu, is_prefix);
+        if (lane == 0) s_red[warp] = bal ? warp * 32u + (uint32_t)__ffs(bal) - 1u : 0xFFFFFFFFu;
+        __syncthreads();
+        uint32_t near = 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t w = 0; w < kCullWarps; ++w) near = min(near, s_red[w]);
+        uint32_t sum = mine && threadIdx.x <= near ? (uint32_t)st : 0u;
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        __syncthreads();
+        if (lane == 0) s_red[warp] = sum;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t w = 0; w < kCullWarps; ++w) prefix += s_red[w];
+        if (near != 0xFFFFFFFFu) break;
+        hi = hi > kThreads ? hi - kThreads : 0u;
+        __syncthreads();
+    }
+    return true;
+}
+
+// kWide: the form for large scenes, whose launch has more CTAs than fit at four per SM: they
+// gain more from a fifth resident CTA than they lose to loading the cone inputs after the
+// frustum test. In smaller scenes each warp's latency dominates, and the loads stay together.
+//
+// Bound by the latency of its dependent loads (item, object, instance, meshlet, pyramid texel)
+// and by the launch. Against a select, a test and an emission launch with the counters cleared
+// before them, a frame (Hi-Z build included) went 29.3 -> 21.7 us with 4,096 instances x 64
+// meshlets at 1024x1024, 42.1 -> 31.8 with 10,000 x 100 (500 of them moved) at 1920x1080, and
+// 60.3 -> 54.3 with 100,000 x 100 at 3840x2160.
+template <bool kWide>
+__global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const __grid_constant__ VgFrameParams P) {
+    __shared__ CullView s_view;
+    __shared__ TileItems s_it;
+    __shared__ uint32_t s_bits[kMaxWindows + 2];  // window ballots (+2 so bit-field reads stay in bounds)
+    __shared__ uint32_t s_pre[kMaxWindows];       // visible meshlets of the tile before each window
+    __shared__ uint32_t s_tmp[kCullWarps + 1];
+    __shared__ uint32_t s_tile, s_epoch;
+
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const VgSceneDev& S = P.scene;
+    pdl_launch_dependents();
+    for (uint32_t k = tid; k < kMaxWindows + 2; k += kThreads) s_bits[k] = 0u;
+    for (uint32_t k = tid; k < kMaxWindows; k += kThreads) s_it.heads[k] = 0u;
+    pdl_wait();  // the kernel before may be the Hi-Z build, or the previous launch of this one
+    const bool object_cta = blockIdx.x >= P.num_tiles;
+    if (warp == 1) view_setup_warp(P.setup, s_view);
+    if (tid == 0 && !object_cta) {
+        uint32_t epoch, ticket;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(epoch) : "l"(P.state + kVgEpoch) : "memory");
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(P.state + kVgTicket) : "memory");
+        if (ticket == P.num_tiles - 1u) {  // the last one: every tile CTA has read the epoch
+            P.state[kVgTicket] = 0u;
+            P.state[kVgEpoch] = epoch + 1u;
+        }
+        s_tile = ticket;
+        s_epoch = epoch + 1u;  // never the zeros of a fresh status
+    }
+    __syncthreads();
+    if (object_cta) {
+        object_block(P, s_view, blockIdx.x - P.num_tiles, gridDim.x - P.num_tiles, s_it.off, s_tmp);
+        return;
+    }
+    const uint32_t tile = s_tile, epoch = s_epoch;
+
+    // The tile's items, one per thread: the object's selected LOD and the item's share of it.
+    const uint32_t w_idx = tile * P.tile_items + tid;
+    const bool mine = tid < P.tile_items && w_idx < S.work_item_count;
+    uint32_t n = 0, first = 0, inst = 0, lod = 0;
+    if (mine) {
+        const uint2 it = __ldg(reinterpret_cast<const uint2*>(S.items + w_idx));  // object, local meshlet base
+        if (it.x < S.object_count) {
+            const HelioGpuVgObject* o = S.objects + it.x;
+            const Selected r = select_object(S, s_view, o, object_head(o));
+            if (r.sel) {
+                const uint32_t count = __ldg(&o->lod_meshlet_counts[r.sel - 1u]);
+                if (it.y < count) {
+                    n = min(64u, count - it.y);
+                    first = __ldg(&o->lod_first_meshlets[r.sel - 1u]) + it.y;
+                    inst = r.instance;
+                    lod = r.sel - 1u;
+                }
             }
         }
     }
-    uint32_t incl = w.n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+    // Packed positions and ranks in one scan (at most 2^14 positions, 2^8 ranks).
+    uint32_t sums;
+    const uint32_t ex = tile_scan(n ? (1u << 16) | n : 0u, s_tmp, sums);
+    const uint32_t off = ex & 0xFFFFu, total = sums & 0xFFFFu, windows = (total + 31u) >> 5;
+    if (n) {
+        const uint32_t rank = ex >> 16;
+        s_it.off[rank] = off;
+        s_it.first[rank] = first;
+        s_it.inst[rank] = inst;
+        s_it.lod[rank] = (uint8_t)lod;
+        atomicOr(s_it.heads + (off >> 5), 1u << (off & 31u));
+        for (uint32_t w = (off + 31u) >> 5; 32u * w < off + n; ++w) s_it.owner[w] = (uint16_t)rank;
     }
-    w.off = incl - w.n;
-    w.total = __shfl_sync(0xffffffffu, incl, 31);
-    return w;
-}
+    __syncthreads();
 
-constexpr int kBitWordsPerWarp = kWindowsPerWarp + 2;  // +2 so bit-field reads stay in bounds
-
-// kWide: the form for large scenes, whose warps each walk many windows (32 work items per
-// warp) and whose launch has more tiles than fit at four CTAs per SM: they gain more from a
-// fifth resident CTA than they lose to loading the cone inputs after the frustum test (10M
-// meshlets at 3840x2160: 27.3 -> 25.0 us). With fewer items per warp each warp's latency
-// dominates, and the loads stay together (1M meshlets: 43.6 against 45.5 us per step).
-template <bool kWide>
-__global__ void __launch_bounds__(kCullWarps * 32, kWide ? 5 : 4) vg_cull_test_kernel(VgCullParams P) {
-    __shared__ CullView s_view;
-    __shared__ uint32_t s_bits[kCullWarps][kBitWordsPerWarp];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const VgSceneDev& S = P.scene;
-    const uint32_t tile = blockIdx.x;
-    pdl_launch_dependents();  // the emission may be scheduled (it waits for this grid)
-    for (int k = lane; k < kBitWordsPerWarp; k += 32) s_bits[warp][k] = 0u;
-    pdl_wait();  // the select's records and view constants
-    const bool mine = (uint32_t)lane < P.items_per_warp;
-    const uint32_t w_idx = (tile * kCullWarps + warp) * P.items_per_warp + lane;
-    const WarpItems it = load_warp_items(S, P.sel, mine ? w_idx : 0xFFFFFFFFu);
-
-    // View constants are staged only when some warp of the tile has work.
-    if (__syncthreads_or(it.total > 0u)) {
-        load_view(P.view, s_view, tid, blockDim.x);
-        __syncthreads();
-    }
-
-    uint32_t warp_count = 0;
-    const uint32_t windows = (it.total + 31u) >> 5;
-    for (uint32_t win = 0; win < windows; ++win) {
-        const uint32_t s = win * 32u + lane;
-        const int j = owner_lane(it.off, s);
-        const uint32_t j_off = __shfl_sync(0xffffffffu, it.off, j);
-        const uint32_t j_first = __shfl_sync(0xffffffffu, it.first, j);
-        const uint32_t j_inst = __shfl_sync(0xffffffffu, it.inst, j);
+    for (uint32_t w = warp; w < windows; w += kCullWarps) {
+        const uint32_t s = w * 32u + lane;
         bool vis = false;
-        if (s < it.total) {
-            const uint32_t mi = j_first + (s - j_off);
+        if (s < total) {
+            const uint32_t k = item_at(s_it, w);
+            const uint32_t mi = s_it.first[k] + (s - s_it.off[k]);
             if (mi < S.meshlet_count) {
-                const HelioGpuInstanceData* in = S.instances + j_inst;
-                const HelioInstanceCullData cd = load_cull(S.cull + j_inst);
+                const uint32_t ji = s_it.inst[k];
+                const HelioGpuInstanceData* in = S.instances + ji;
+                const HelioInstanceCullData cd = load_cull(S.cull + ji);
                 const Mat4 model = ldg_mat4(in->model);
                 vis = meshlet_visible<false, kWide>(S, s_view, mi, model, cd, in);
             }
         }
         const uint32_t bits = __ballot_sync(0xffffffffu, vis);
-        if (lane == 0) s_bits[warp][win] = bits;
-        warp_count += __popc(bits);
+        if (lane == 0) s_bits[w] = bits;
     }
-    __syncwarp();
-    const size_t wslot = (size_t)tile * kCullWarps + warp;
-    if (lane == 0) {
-        P.scratch.warp_counts[wslot] = warp_count;
-        if (warp_count) {
-            atomicAdd(P.scratch.tile_counts + tile, warp_count);
-            atomicAdd(P.counters + 0, warp_count);
-        }
-    }
-    if (warp_count) {
-        for (uint32_t k = lane; k < windows; k += 32) P.scratch.bits[wslot * kWindowsPerWarp + k] = s_bits[warp][k];
-    }
-    // Per-work-item visibility words: bits [off, off + n) of the warp's window bits.
-    if (P.visibility && mine && w_idx < S.work_item_count) {
-        uint32_t lo = 0, hi = 0;
-        if (it.n) {
-            const uint32_t w0 = it.off >> 5, sh = it.off & 31u;
-            const unsigned long long a = (unsigned long long)s_bits[warp][w0] |
-                                         ((unsigned long long)s_bits[warp][w0 + 1] << 32);
-            const unsigned long long c = s_bits[warp][w0 + 2];
-            unsigned long long field = sh ? ((a >> sh) | (c << (64 - sh))) : a;
-            if (it.n < 64) field &= (1ull << it.n) - 1ull;
-            lo = (uint32_t)field;
-            hi = (uint32_t)(field >> 32);
-        }
-        reinterpret_cast<uint2*>(P.visibility)[w_idx] = make_uint2(lo, hi);
-    }
-}
-
-__global__ void __launch_bounds__(kCullWarps * 32) vg_cull_emit_kernel(VgCullParams P) {
-    __shared__ uint32_t s_red[kCullWarps];
-    __shared__ uint32_t s_prefix;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t tile = blockIdx.x;
-    pdl_wait();  // the meshlet tests' counts and window bits
-    const uint32_t count = P.scratch.tile_counts[tile];
-    if (count == 0u) return;  // uniform: the whole CTA leaves
-
-    // Exclusive prefix: visible meshlets of all earlier tiles.
-    uint32_t sum = 0;
-    for (uint32_t i = tid; i < tile; i += blockDim.x) sum += P.scratch.tile_counts[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) s_red[warp] = sum;
     __syncthreads();
+
+    // Visible meshlets before each window, and of the tile.
+    uint32_t count;
+    {
+        const uint32_t c0 = __popc(s_bits[2u * tid]), c1 = __popc(s_bits[2u * tid + 1u]);
+        const uint32_t before = tile_scan(c0 + c1, s_tmp, count);
+        s_pre[2u * tid] = before;
+        s_pre[2u * tid + 1u] = before + c0;
+    }
+    if (tid == 0) st_status(P.status + tile, tile_status(epoch, tile == 0u ? kTilePrefix : kTileSum, count));
+    // Per-work-item visibility words: bits [off, off + n) of the tile's window bits.
+    if (mine) reinterpret_cast<uint2*>(P.visibility)[w_idx] = bit_field64(s_bits, off, n);
+    const bool last = tile == P.num_tiles - 1u;
+    if (count == 0u && !last) return;  // uniform: nothing to place
+
+    uint32_t base;
+    if (!tile_look_back(P, tile, epoch, s_tmp, base)) {
+        if (tid == 0) atomicOr(P.state + kVgError, (uint32_t)kDevTimeout);
+        return;
+    }
     if (tid == 0) {
-        uint32_t p = 0;
-#pragma unroll
-        for (int w = 0; w < (int)kCullWarps; ++w) p += s_red[w];
-        s_prefix = p;
-        const unsigned long long end = (unsigned long long)p + count;
-        const unsigned long long lo = p > P.capacity ? p : P.capacity;
-        if (end > lo) atomicAdd(P.counters + 1, (uint32_t)(end - lo));
+        if (tile != 0u) st_status(P.status + tile, tile_status(epoch, kTilePrefix, base + count));
+        if (last) {
+            const uint32_t all = base + count;
+            P.counters[0] = all;
+            P.counters[1] = all > P.capacity ? all - P.capacity : 0u;
+        }
     }
+    // Emission, four windows at a time per warp: their draw records are loaded before any is
+    // written. (tile_look_back ended with s_pre visible to every thread.)
     __syncthreads();
-
-    const size_t wslot0 = (size_t)tile * kCullWarps;
-    const uint32_t wc = P.scratch.warp_counts[wslot0 + warp];
-    if (wc == 0u) return;  // uniform per warp; no block barrier follows
-    uint32_t base = s_prefix;
-    for (int w = 0; w < warp; ++w) base += P.scratch.warp_counts[wslot0 + w];
-
-    const VgSceneDev& S = P.scene;
-    const uint32_t w_idx = (tile * kCullWarps + warp) * P.items_per_warp + lane;
-    const WarpItems it = load_warp_items(S, P.sel, (uint32_t)lane < P.items_per_warp ? w_idx : 0xFFFFFFFFu);
-    const uint32_t windows = (it.total + 31u) >> 5;
-    const uint32_t* wbits = P.scratch.bits + (wslot0 + warp) * kWindowsPerWarp;
-    for (uint32_t win = 0; win < windows; ++win) {
-        const uint32_t bits = wbits[win];
-        if (bits == 0u) continue;
-        const uint32_t s = win * 32u + lane;
-        const int j = owner_lane(it.off, s);
-        const uint32_t j_off = __shfl_sync(0xffffffffu, it.off, j);
-        const uint32_t j_first = __shfl_sync(0xffffffffu, it.first, j);
-        const uint32_t j_inst = __shfl_sync(0xffffffffu, it.inst, j);
-        const uint32_t j_lod = __shfl_sync(0xffffffffu, it.lod, j);
-        if ((bits >> lane) & 1u) {
-            const uint32_t slot = base + __popc(bits & ((1u << lane) - 1u));
-            if (slot < P.capacity) {
-                const uint32_t mi = j_first + (s - j_off);
-                const uint4 d = __ldg(S.m_draw + mi);
-                uint32_t* o = reinterpret_cast<uint32_t*>(P.indirect + slot);
-                o[0] = d.y;  // index_count
-                o[1] = 1u;
-                o[2] = d.x;  // first_index
-                o[3] = d.z;  // vertex_offset
-                o[4] = slot; // first_instance
-                reinterpret_cast<uint4*>(P.draws)[slot] = make_uint4(j_inst, mi, j_lod, 0u);
+    for (uint32_t w0 = warp; w0 < windows; w0 += 4u * kCullWarps) {
+        uint4 d[4];
+        uint32_t b[4], mi[4], k[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t w = w0 + (uint32_t)q * kCullWarps;
+            b[q] = w < windows ? s_bits[w] : 0u;
+            if ((b[q] >> lane) & 1u) {
+                k[q] = item_at(s_it, w);
+                mi[q] = s_it.first[k[q]] + (w * 32u + lane - s_it.off[k[q]]);
+                d[q] = __ldg(S.m_draw + mi[q]);
             }
         }
-        base += __popc(bits);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (!((b[q] >> lane) & 1u)) continue;
+            const uint32_t w = w0 + (uint32_t)q * kCullWarps;
+            const uint32_t slot = base + s_pre[w] + __popc(b[q] & ((1u << lane) - 1u));
+            if (slot >= P.capacity) continue;
+            uint32_t* o = reinterpret_cast<uint32_t*>(P.indirect + slot);
+            o[0] = d[q].y;  // index_count
+            o[1] = 1u;
+            o[2] = d[q].x;  // first_index
+            o[3] = d[q].z;  // vertex_offset
+            o[4] = slot;    // first_instance
+            reinterpret_cast<uint4*>(P.draws)[slot] = make_uint4(s_it.inst[k[q]], mi[q], s_it.lod[k[q]], 0u);
+        }
     }
 }
 
@@ -402,51 +490,15 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
     helio_launch_end(stream);
 }
 
-void launch_vg_view_setup(const ViewSetupParams& p, cudaStream_t stream) {
-    helio_launch_begin("vg_view_setup", stream);
-    vg_view_setup_kernel<<<1, 32, 0, stream>>>(p);
-    helio_launch_end(stream);
-}
-
-void launch_vg_select(const VgSelectParams& p, cudaStream_t stream) {
-    if (!p.scene.object_count) return;
-    helio_launch_begin("vg_select", stream);
-    vg_select_kernel<<<(p.scene.object_count + 255u) / 256u, 256, 0, stream>>>(p);
-    helio_launch_end(stream);
-}
-
-namespace {
-
-// The meshlet tests and the emission are launched with programmatic stream serialization:
-// each may be scheduled while the kernel before it finishes (its CTAs wait in pdl_wait), which
-// hides a launch gap per kernel.
-cudaError_t launch_after(void (*kernel)(VgCullParams), uint32_t grid, const VgCullParams& p, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kCullWarps * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
-}  // namespace
-
-cudaError_t launch_vg_cull(const VgCullParams& p, cudaStream_t stream) {
+cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream) {
     if (!p.num_tiles) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const bool wide = p.items_per_warp >= 32u && p.num_tiles > 4u * (uint32_t)std::max(sms, 1);
-    helio_launch_begin("vg_cull_test", stream);
-    cudaError_t e = launch_after(wide ? vg_cull_test_kernel<true> : vg_cull_test_kernel<false>, p.num_tiles, p, stream);
-    helio_launch_end(stream);
-    if (e != cudaSuccess) return e;
-    helio_launch_begin("vg_cull_emit", stream);
-    e = launch_after(vg_cull_emit_kernel, p.num_tiles, p, stream);
+    const uint32_t grid = p.num_tiles + (uint32_t)(((uint64_t)p.scene.object_count + kThreads - 1) / kThreads);
+    const bool wide = grid > 4u * (uint32_t)std::max(sms, 1);
+    helio_launch_begin("vg_frame", stream);
+    const cudaError_t e = launch_after(wide ? vg_frame_kernel<true> : vg_frame_kernel<false>, grid, kThreads, 0, stream, p);
     helio_launch_end(stream);
     return e;
 }

@@ -455,8 +455,9 @@ int32_t helio_vg_execute(helio_vg_pass* pass, const HelioGpuCameraUniforms* came
 int32_t helio_vg_resize(helio_vg_pass* pass, uint32_t width, uint32_t height);
 int32_t helio_vg_set_lod_quality(helio_vg_pass* pass, uint32_t lod_quality);
 int32_t helio_vg_publish(const helio_vg_pass* pass, helio_vg_outputs* out);
-/* Synchronises `stream` and reports any asynchronous CUDA error of the queued
- * work (the cull kernels themselves never wait on one another). */
+/* Synchronises `stream` and reports any asynchronous CUDA error of the queued work, or
+ * HELIO_ERR_TIMEOUT when a tile's bounded wait for the draw counts of the tiles before it
+ * gave up in an execute since the last full upload (that execute's outputs are invalid). */
 int32_t helio_vg_device_status(helio_vg_pass* pass, void* stream);
 void helio_vg_destroy(helio_vg_pass* pass);
 

@@ -168,3 +168,38 @@ def test_vg_empty_scene_is_a_no_op(cuda):
     vg.prepare(S.frame_data(empty))
     vg.execute(torch.from_numpy(camera_bytes(w.views[0].camera)).cuda(), hz.publish())
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("objects,meshlets", [(1, 1), (7, 64), (8, 65), (9, 200), (443, 1), (445, 33), (3553, 64),
+                                              (7105, 20), (56833, 3), (60000, 100), (130000, 1)])
+def test_frame_tiles_match_oracle(cuda, objects, meshlets):
+    """Scenes around the steps of the tile size (8 to 256 work items) and of the look-back
+    (one tile, a few, more than one window of 256 tiles), executed twice."""
+    from helio_b200 import scene as S
+    from oracle import oracle as O
+
+    sc = S.make_scene(91 + objects, objects, meshlets, 4, 0, 20.0)
+    v = S.main_view(5, 256, 144, 40)
+    g = gpu_vg_view(sc, v, execute_times=2, publication_limit=400000)
+    o = oracle_vg_view(sc, v, O.hiz_build(v.depth), capacity=min(sc.max_draw_count, 400000))
+    assert_vg_equal(g, o)
+
+
+@pytest.mark.parametrize("counter_count", [2, 11])
+def test_frame_arbitrary_work_items(cuda, counter_count):
+    """Work items in any order: repeated objects, bases off the 64 grid and past the LOD's end,
+    object indices past the array, objects that no item names (still selected)."""
+    from helio_b200 import scene as S
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(17)
+    sc = S.make_scene(23, 3000, 150, 4, 0, 20.0)
+    items = np.zeros(9001, S.DT_ITEM)
+    items["object_index"] = rng.integers(0, 2000, len(items))
+    items["object_index"][rng.random(len(items)) < 0.02] = 3000 + 5
+    items["local_meshlet_base"] = rng.integers(0, 200, len(items))
+    sc = S.Scene(sc.meshlets, sc.objects, sc.instances, items, sc.aabbs, sc.draw_calls, 500000, 150)
+    v = S.main_view(5, 200, 120, 30)
+    g = gpu_vg_view(sc, v, publication_limit=500000, counter_count=counter_count)
+    o = oracle_vg_view(sc, v, O.hiz_build(v.depth), capacity=500000, counter_count=counter_count)
+    assert_vg_equal(g, o, counter_count)
