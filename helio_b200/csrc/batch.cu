@@ -30,8 +30,6 @@
 // always ends and reads nothing a timed-out phase left incomplete; the host then
 // reports HELIO_ERR_TIMEOUT.
 
-#include <algorithm>
-
 #include "batch.h"
 #include "hiz_tile.cuh"
 #include "vg_device.cuh"
@@ -442,7 +440,7 @@ __device__ void phase_hiz_tile(const BatchParams& P, uint32_t tile, char* sm) {
 // Exact sphere test and LOD walk of the pair (view v_begin + k, object of lane j) on
 // each active lane (vg_cull.wgsl:315-336). Every lane of the warp calls it.
 __device__ void select_batch(const BatchParams& P, uint32_t chunk, uint32_t v_begin, bool active, uint32_t k,
-                             uint32_t j, F3 c, float wr, float max_scale, char* sm) {
+                             uint32_t j, F3 c, float wr, float max_scale, uint32_t lods, char* sm) {
     const SelView* s_sv = reinterpret_cast<const SelView*>(sm + kSmSelViews);
     uint8_t* s_lod = reinterpret_cast<uint8_t*>(sm + kSmSelLod);
     uint32_t* s_spans = reinterpret_cast<uint32_t*>(sm + kSmSelSpans);
@@ -452,12 +450,12 @@ __device__ void select_batch(const BatchParams& P, uint32_t chunk, uint32_t v_be
     const F3 cj = f3(__shfl_sync(0xffffffffu, c.x, j), __shfl_sync(0xffffffffu, c.y, j),
                      __shfl_sync(0xffffffffu, c.z, j));
     const float wrj = __shfl_sync(0xffffffffu, wr, j), msj = __shfl_sync(0xffffffffu, max_scale, j);
+    const uint32_t lod_count = __shfl_sync(0xffffffffu, lods, j);
     if (!active) return;
     const SelView& sv = s_sv[v_begin + k];
     if (!sphere_visible_vg(sv.planes, cj, wrj)) return;
     const uint32_t slot = warp * 32u + j;
     const HelioGpuVgObject* obj = P.scene.objects + (chunk * kBatchChunk + slot);
-    const uint32_t lod_count = min(__ldg(&obj->lod_count), 8u);
     const float4 e0 = __ldg(reinterpret_cast<const float4*>(obj->lod_errors));
     const float4 e1 = __ldg(reinterpret_cast<const float4*>(obj->lod_errors + 4));
     const float err[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
@@ -547,21 +545,14 @@ __device__ void phase_select_chunk(const BatchParams& P, uint32_t chunk, uint32_
     bool valid = false;
     F3 c = f3(0.f, 0.f, 0.f);
     float wr = 0.0f, max_scale = 0.0f;
+    uint32_t lod_count = 0;
     if (o < S.object_count) {
-        const HelioGpuVgObject* obj = S.objects + o;
-        const uint4 head = __ldg(reinterpret_cast<const uint4*>(obj));
-        const float4 lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
-        const uint32_t lod_count = min(head.y, 8u), ii = head.x;
-        if (lod_count > 0u && ii < S.instance_count) {
-            const HelioInstanceCullData cd = load_cull(S.cull + ii);
-            const Mat4 model = ldg_mat4(S.instances[ii].model);
-            if (cd.valid_transform != 0u) {
-                valid = true;
-                max_scale = cd.max_scale;
-                c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
-                wr = fmaxf(fmul(lb.w, cd.max_scale), 0.0f);
-            }
-        }
+        const ObjectWorld w = load_world(S, o);
+        valid = w.lod_count != 0u;
+        lod_count = w.lod_count;
+        max_scale = w.max_scale;
+        c = f3(w.sphere.x, w.sphere.y, w.sphere.z);
+        wr = w.sphere.w;
     }
     __syncthreads();  // the previous unit is done with the tile and the counters
     constexpr uint32_t kRow4 = kBatchChunk / 16;  // 16-byte words per tile row
@@ -599,7 +590,7 @@ __device__ void phase_select_chunk(const BatchParams& P, uint32_t chunk, uint32_
         const uint32_t before = __shfl_sync(0xffffffffu, hit_inc - hit_count, j);
         const bool active = i < total;
         const uint32_t k = active ? select_bit(hj, i - before) : 0u;
-        select_batch(P, chunk, v_begin, active, k, j, c, wr, max_scale, sm);
+        select_batch(P, chunk, v_begin, active, k, j, c, wr, max_scale, lod_count, sm);
     }
     __syncthreads();
     for (uint32_t i = tid; i < nv * kRow4; i += kBatchThreads) {
@@ -1164,73 +1155,6 @@ __global__ void __launch_bounds__(kBatchThreads, 5) batch_cull_kernel(BatchParam
     }
 }
 
-// Bounds over the valid objects, and (kTotals) the sums that size a batch's buffers: LOD0
-// meshlets, 64-meshlet spans and meshlets of each object's largest LOD. Bound by memory (64
-// of an object's 128 bytes and 80 of its instance): a grid of 8 CTAs per SM strides over the
-// objects, and sums and maxima meet in the block, so that a block costs at most five atomics
-// (two per warp on the same two words, without the sums, took 37 us for 475,000 objects).
-template <bool kTotals>
-__global__ void __launch_bounds__(kBatchThreads) scene_bounds_kernel(VgSceneDev S, uint32_t* bounds,
-                                                                     unsigned long long* totals) {
-    __shared__ uint32_t s_max[2];
-    __shared__ unsigned long long s_sum[3];
-    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
-    if (kTotals && threadIdx.x < 3) s_sum[threadIdx.x] = 0ull;
-    __syncthreads();
-    uint32_t a = 0u, b = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
-    unsigned long long lod0 = 0, spans = 0, draws = 0;
-    const uint32_t stride = gridDim.x * kBatchThreads;
-    for (uint64_t o = blockIdx.x * kBatchThreads + threadIdx.x; o < S.object_count; o += stride) {
-        const HelioGpuVgObject* obj = S.objects + o;
-        const uint4 head = __ldg(reinterpret_cast<const uint4*>(obj));
-        const uint32_t lod_count = min(head.y, 8u), ii = head.x;
-        if (kTotals) {
-            const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts));
-            const uint4 c1 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts + 4));
-            const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            uint32_t mx = 0;
-#pragma unroll
-            for (uint32_t l = 0; l < 8; ++l) mx = l < lod_count ? max(mx, c[l]) : mx;
-            lod0 += c[0];
-            spans += (mx + 63u) / 64u;
-            draws += mx;
-        }
-        if (lod_count > 0u && ii < S.instance_count) {
-            const HelioInstanceCullData cd = load_cull(S.cull + ii);
-            if (cd.valid_transform != 0u) {
-                const float4 lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
-                const F3 c = mat4_point3(ldg_mat4(S.instances[ii].model), f3(lb.x, lb.y, lb.z));
-                const float wr = fmaxf(fmul(lb.w, cd.max_scale), 0.0f);
-                const float cl1 = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);  // rounding up is not needed: 2^-20 slack
-                a = max(a, __float_as_uint(wr));  // (NaN above +inf)
-                b = max(b, __float_as_uint(cl1));
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 16; k > 0; k >>= 1) {
-        a = max(a, __shfl_xor_sync(0xffffffffu, a, k));
-        b = max(b, __shfl_xor_sync(0xffffffffu, b, k));
-        if (kTotals) {
-            lod0 += __shfl_xor_sync(0xffffffffu, lod0, k);
-            spans += __shfl_xor_sync(0xffffffffu, spans, k);
-            draws += __shfl_xor_sync(0xffffffffu, draws, k);
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(s_max, a);
-        atomicMax(s_max + 1, b);
-        if (kTotals) {
-            atomicAdd(s_sum, lod0);
-            atomicAdd(s_sum + 1, spans);
-            atomicAdd(s_sum + 2, draws);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 && s_max[threadIdx.x]) atomicMax(bounds + threadIdx.x, s_max[threadIdx.x]);
-    if (kTotals && threadIdx.x < 3 && s_sum[threadIdx.x]) atomicAdd(totals + threadIdx.x, s_sum[threadIdx.x]);
-}
-
 }  // namespace
 
 // The views' published draws, end to end. Every CTA computes the views' packing table itself
@@ -1304,21 +1228,6 @@ __global__ void __launch_bounds__(kBatchThreads) pack_draws_kernel(const BatchVi
         }
         if (tid < count) dst_d[tid] = rec;
     }
-}
-
-cudaError_t launch_scene_bounds(const VgSceneDev& scene, uint32_t* bounds, unsigned long long* totals,
-                                cudaStream_t stream) {
-    const uint32_t n = scene.object_count;
-    if (n) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const uint32_t blocks = std::min<uint32_t>((uint32_t)(((uint64_t)n + kBatchThreads - 1) / kBatchThreads),
-                                                   (uint32_t)(sms > 0 ? sms : 1) * 8u);
-        if (totals) scene_bounds_kernel<true><<<blocks, kBatchThreads, 0, stream>>>(scene, bounds, totals);
-        else scene_bounds_kernel<false><<<blocks, kBatchThreads, 0, stream>>>(scene, bounds, nullptr);
-    }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_pack_draws(const BatchViewDev* views, uint32_t view_count, HelioDrawIndexedIndirectArgs* indirect,

@@ -45,7 +45,7 @@ enum : uint32_t { kBatchErrTimeout = 1u, kBatchErrSpanCapacity = 2u };
 
 struct BatchParams {
     VgSceneDev scene;
-    const uint32_t* scene_bounds;  // [2] launch_scene_bounds output
+    const uint32_t* scene_bounds;  // [2] bounds of launch_scene_update
     BatchViewDev* views;      // [view_count]
     CullView* cviews;         // [view_count], written by phase 0
     uint8_t* lod;             // [view_count * lod_pitch]: LOD + 1 per (view, object), 0 = culled
@@ -87,16 +87,6 @@ struct BatchParams {
 // [0..7] phase boundaries, [8] / [9] largest per-CTA time spent on Hi-Z tiles /
 // object chunks in phase 1 (ns).
 constexpr uint32_t kBatchPhaseStamps = 10;
-
-// Bounds over the valid objects of a scene (an object with lod_count > 0, an
-// instance in range and a valid transform), as float bits, for the per-view reject
-// boxes: bounds[0] = largest world radius max(local_radius * max_scale, 0),
-// bounds[1] = largest |c.x| + |c.y| + |c.z| of a world centre c (computed exactly as
-// the select computes them). With `totals` (or null), also sums over all objects: totals[0] =
-// lod_meshlet_counts[0], totals[1] = 64-meshlet spans and totals[2] = meshlets of the largest
-// of the object's LODs. `bounds` and `totals` must be zero before the launch.
-cudaError_t launch_scene_bounds(const VgSceneDev& scene, uint32_t* bounds, unsigned long long* totals,
-                                cudaStream_t stream);
 
 // Packs the published draws of every view (min(counters[0], capacity) each) into
 // one pair of arrays, view after view; offsets[v] = first draw of view v, offsets[V] =

@@ -17,8 +17,8 @@ using helio::as_stream;
 using helio::DevBuf;
 
 struct helio_vg_scene {
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, staging;
-    DevBuf bounds;  // launch_scene_bounds of the current objects and instances: u32[2], then u64[3] totals
+    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, world, staging;
+    DevBuf bounds;  // launch_scene_update of the current objects and instances: u32[2], then u64[3] totals
     uint32_t meshlet_count = 0, object_count = 0;
     uint64_t lod0_meshlets = 0, max_spans = 0, max_draw_count = 0;
     uint64_t version = 0, instance_version = 0;
@@ -33,6 +33,7 @@ struct helio_vg_scene {
         s.objects = objects.as<HelioGpuVgObject>();
         s.instances = instances.as<HelioGpuInstanceData>();
         s.cull = cull.as<HelioInstanceCullData>();
+        s.world = world.as<uint4>();
         s.items = nullptr;
         s.meshlet_count = meshlet_count;
         s.object_count = object_count;
@@ -93,15 +94,34 @@ int32_t copy_in(void* dst, const void* src, size_t bytes, uint32_t memory, cudaS
 
 constexpr size_t kBoundsBytes = 8 + 3 * 8;
 
-// The scene's bounds, and with `totals` the sums of launch_scene_bounds, read back (waits for
-// the stream). Summing the objects on the host, read back whole, took 15 to 33 ms for 475,000
-// objects (61 MB through pageable memory); the kernel reads them once at device bandwidth: a pass
-// that rebuilds, uploads and culls such a scene went from 33.1 ms to 0.47 ms.
-int32_t refresh_bounds(helio_vg_scene* sc, const helio::VgSceneDev& dev, uint64_t* totals, cudaStream_t s) {
+// Instances [first, first + count) of a scene of `objects` objects from `src` (the caller's rows
+// of that range) and everything derived from them, the bounds included; with `totals` also the
+// sums of launch_scene_update, read back (waits for the stream). Device rows that 16-byte loads
+// can read are copied by the update kernel itself. (Summing the objects on the host, read back
+// whole, took 15 to 33 ms for 475,000 objects.)
+int32_t scene_update(helio_vg_scene* sc, uint32_t objects, uint32_t first, uint32_t count,
+                     const HelioGpuInstanceData* src, uint32_t memory, uint64_t* totals, cudaStream_t s) {
     HELIO_CK(sc->bounds.ensure(kBoundsBytes));
     HELIO_CK(cudaMemsetAsync(sc->bounds.ptr, 0, kBoundsBytes, s));
+    const bool direct = memory == HELIO_MEM_DEVICE && count && src && (reinterpret_cast<uintptr_t>(src) & 15u) == 0u;
+    if (!direct) {
+        int32_t st = copy_in(sc->instances.as<HelioGpuInstanceData>() + first, src,
+                             (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
+        if (st) return st;
+    }
     unsigned long long* sums = reinterpret_cast<unsigned long long*>(sc->bounds.as<char>() + 8);
-    HELIO_CK(helio::launch_scene_bounds(dev, sc->bounds.as<uint32_t>(), totals ? sums : nullptr, s));
+    helio::SceneUpdate u{};
+    u.scene = sc->dev();
+    u.scene.object_count = u.scene.instance_count = objects;
+    u.src = direct ? src : nullptr;
+    u.instances = sc->instances.as<HelioGpuInstanceData>();
+    u.cull = sc->cull.as<HelioInstanceCullData>();
+    u.world = sc->world.as<uint4>();
+    u.first = first;
+    u.count = count;
+    u.bounds = sc->bounds.as<uint32_t>();
+    u.totals = totals ? sums : nullptr;
+    HELIO_CK(helio::launch_scene_update(u, s));
     if (totals) {
         HELIO_CK(cudaMemcpyAsync(totals, sums, 3 * 8, cudaMemcpyDeviceToHost, s));
         HELIO_CK(cudaStreamSynchronize(s));
@@ -218,6 +238,7 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->objects.ensure(O * sizeof(HelioGpuVgObject)));
         HELIO_CK(sc->instances.ensure(O * sizeof(HelioGpuInstanceData)));
         HELIO_CK(sc->cull.ensure(O * sizeof(HelioInstanceCullData)));
+        HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
         const HelioGpuMeshletEntry* aos = f->meshlets;
         if (M) {
             if (f->memory == HELIO_MEM_HOST) {
@@ -232,18 +253,10 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
             HELIO_CK(cudaGetLastError());
         }
         if ((st = copy_in(sc->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
-        if ((st = copy_in(sc->instances.ptr, f->instances, O * sizeof(HelioGpuInstanceData), f->memory, s)))
-            return st;
-        helio::launch_instance_cull_data(sc->instances.as<HelioGpuInstanceData>(), (uint32_t)O,
-                                         sc->cull.as<HelioInstanceCullData>(), s);
-        HELIO_CK(cudaGetLastError());
-        // Per-object span bound and LOD0 size, for capacities and the metric; the wait for them
-        // also ends the use of the staging copy.
-        helio::VgSceneDev now = sc->dev();
-        now.meshlet_count = f->meshlet_count;
-        now.object_count = now.instance_count = f->object_count;
+        // With the per-object span bound and LOD0 size, for capacities and the metric; the wait
+        // for them also ends the use of the staging copy.
         uint64_t totals[3] = {0, 0, 0};
-        if ((st = refresh_bounds(sc, now, totals, s))) return st;
+        if ((st = scene_update(sc, f->object_count, 0, f->object_count, f->instances, f->memory, totals, s))) return st;
         if (f->memory == HELIO_MEM_HOST) sc->staging.release();
         sc->meshlet_count = f->meshlet_count;
         sc->object_count = f->object_count;
@@ -256,14 +269,10 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
     } else if (f->instance_version != sc->instance_version) {
         const uint64_t start = f->instance_dirty_start, count = f->instance_dirty_count;
         HELIO_ARG(count > 0 && start + count <= sc->object_count, "invalid dirty instance range");
-        if ((st = copy_in(sc->instances.as<HelioGpuInstanceData>() + start, f->instances + start,
-                          count * sizeof(HelioGpuInstanceData), f->memory, s)))
+        if ((st = scene_update(sc, sc->object_count, (uint32_t)start, (uint32_t)count,
+                               f->instances ? f->instances + start : nullptr, f->memory, nullptr, s)))
             return st;
-        helio::launch_instance_cull_data(sc->instances.as<HelioGpuInstanceData>() + start, (uint32_t)count,
-                                         sc->cull.as<HelioInstanceCullData>() + start, s);
-        HELIO_CK(cudaGetLastError());
         sc->instance_version = f->instance_version;
-        if ((st = refresh_bounds(sc, sc->dev(), nullptr, s))) return st;
     }
     return HELIO_OK;
 }
@@ -275,7 +284,7 @@ int32_t helio_vg_scene_info_get(const helio_vg_scene* sc, helio_vg_scene_info* o
     out->lod0_meshlets = sc->lod0_meshlets;
     out->max_spans = sc->max_spans;
     out->device_bytes = sc->m_bounds.bytes + sc->m_cone.bytes + sc->m_axis.bytes + sc->m_draw.bytes +
-                        sc->objects.bytes + sc->instances.bytes + sc->cull.bytes;
+                        sc->objects.bytes + sc->instances.bytes + sc->cull.bytes + sc->world.bytes;
     return HELIO_OK;
 }
 

@@ -179,7 +179,7 @@ struct helio_vg_pass {
     uint32_t publication_limit = HELIO_VG_DEFAULT_PUBLICATION_LIMIT;
     uint32_t counter_count = HELIO_VG_COUNTER_COUNT;
     // Scene (device resident).
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, items, staging;
+    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, world, items, staging;
     // Outputs and scratch.
     DevBuf indirect, draws, visibility;
     DevBuf scratch;  // published counters (16 words) | kVgStateWords state words | tile statuses
@@ -587,6 +587,30 @@ static int32_t vg_copy(void* dst, const void* src, size_t bytes, uint32_t memory
     return HELIO_OK;
 }
 
+// Instances [first, first + count) of a scene of `objects` objects from `src` (the caller's rows
+// of that range), and everything derived from them. Device rows that 16-byte loads can read are
+// copied by the update kernel itself.
+static int32_t vg_update(helio_vg_pass* p, uint32_t objects, uint32_t first, uint32_t count,
+                         const HelioGpuInstanceData* src, uint32_t memory, cudaStream_t s) {
+    const bool direct = memory == HELIO_MEM_DEVICE && count && src && (reinterpret_cast<uintptr_t>(src) & 15u) == 0u;
+    if (!direct) {
+        int32_t st = vg_copy(p->instances.as<HelioGpuInstanceData>() + first, src,
+                             (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
+        if (st) return st;
+    }
+    helio::SceneUpdate u{};
+    u.scene.objects = p->objects.as<HelioGpuVgObject>();
+    u.scene.object_count = u.scene.instance_count = objects;
+    u.scene.world = u.world = p->world.as<uint4>();
+    u.src = direct ? src : nullptr;
+    u.instances = p->instances.as<HelioGpuInstanceData>();
+    u.cull = p->cull.as<HelioInstanceCullData>();
+    u.first = first;
+    u.count = count;
+    HELIO_CK(helio::launch_scene_update(u, s));
+    return HELIO_OK;
+}
+
 int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* stream) {
     HELIO_ARG(p && f, "null pointer");
     HELIO_ARG(f->memory == HELIO_MEM_HOST || f->memory == HELIO_MEM_DEVICE, "unknown memory space");
@@ -602,6 +626,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->objects.ensure(O * sizeof(HelioGpuVgObject)));
         HELIO_CK(p->instances.ensure(O * sizeof(HelioGpuInstanceData)));
         HELIO_CK(p->cull.ensure(O * sizeof(HelioInstanceCullData)));
+        HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
         HELIO_CK(p->visibility.ensure(W * 8));
         const HelioGpuMeshletEntry* aos = f->meshlets;
@@ -617,11 +642,8 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
             HELIO_CK(cudaGetLastError());
         }
         if ((st = vg_copy(p->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
-        if ((st = vg_copy(p->instances.ptr, f->instances, O * sizeof(HelioGpuInstanceData), f->memory, s))) return st;
         if ((st = vg_copy(p->items.ptr, f->work_items, W * sizeof(HelioGpuVgWorkItem), f->memory, s))) return st;
-        helio::launch_instance_cull_data(p->instances.as<HelioGpuInstanceData>(), (uint32_t)O,
-                                         p->cull.as<HelioInstanceCullData>(), s);
-        HELIO_CK(cudaGetLastError());
+        if ((st = vg_update(p, f->object_count, 0, f->object_count, f->instances, f->memory, s))) return st;
         if (f->memory == HELIO_MEM_HOST && M) {
             // The staging copy is consumed by the pack kernel; release it once it ran.
             HELIO_CK(cudaStreamSynchronize(s));
@@ -651,13 +673,9 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         // Dirty-instance patch (rendering.rs:787-819).
         const uint64_t start = f->instance_dirty_start, count = f->instance_dirty_count;
         HELIO_ARG(count > 0 && start + count <= p->object_count, "invalid dirty instance range");
-        const HelioGpuInstanceData* src = f->instances + start;
-        int32_t st2 = vg_copy(p->instances.as<HelioGpuInstanceData>() + start, src,
-                              count * sizeof(HelioGpuInstanceData), f->memory, s);
-        if (st2) return st2;
-        helio::launch_instance_cull_data(p->instances.as<HelioGpuInstanceData>() + start, (uint32_t)count,
-                                         p->cull.as<HelioInstanceCullData>() + start, s);
-        HELIO_CK(cudaGetLastError());
+        if ((st = vg_update(p, p->object_count, (uint32_t)start, (uint32_t)count,
+                            f->instances ? f->instances + start : nullptr, f->memory, s)))
+            return st;
         p->last_instance_version = f->instance_version;
     }
     return HELIO_OK;
@@ -684,6 +702,7 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
     scene.objects = p->objects.as<HelioGpuVgObject>();
     scene.instances = p->instances.as<HelioGpuInstanceData>();
     scene.cull = p->cull.as<HelioInstanceCullData>();
+    scene.world = p->world.as<uint4>();
     scene.items = p->items.as<HelioGpuVgWorkItem>();
     scene.meshlet_count = p->meshlet_count;
     scene.object_count = p->object_count;

@@ -48,49 +48,141 @@ __global__ void pack_meshlets_kernel(const HelioGpuMeshletEntry* __restrict__ ao
     }
 }
 
-// InstanceCullData::from_instance (lib.rs:132-167), Rust f32 evaluation order.
+// InstanceCullData::from_instance (lib.rs:132-167), Rust f32 evaluation order, of the
+// column-major model matrix m.
+__device__ __forceinline__ HelioInstanceCullData cull_data_of(const Mat4& mm) {
+    const float m[16] = {mm.c0.x, mm.c0.y, mm.c0.z, mm.c0.w, mm.c1.x, mm.c1.y, mm.c1.z, mm.c1.w,
+                         mm.c2.x, mm.c2.y, mm.c2.z, mm.c2.w, mm.c3.x, mm.c3.y, mm.c3.z, mm.c3.w};
+    const float sx = fsqrt(fadd(fadd(fmul(m[0], m[0]), fmul(m[1], m[1])), fmul(m[2], m[2])));
+    const float sy = fsqrt(fadd(fadd(fmul(m[4], m[4]), fmul(m[5], m[5])), fmul(m[6], m[6])));
+    const float sz = fsqrt(fadd(fadd(fmul(m[8], m[8]), fmul(m[9], m[9])), fmul(m[10], m[10])));
+    const float max_scale = fmaxf(fmaxf(sx, sy), sz);
+    const float min_scale = fminf(fminf(sx, sy), sz);
+    const float dot_xy = fadd(fadd(fmul(m[0], m[4]), fmul(m[1], m[5])), fmul(m[2], m[6]));
+    const float dot_xz = fadd(fadd(fmul(m[0], m[8]), fmul(m[1], m[9])), fmul(m[2], m[10]));
+    const float dot_yz = fadd(fadd(fmul(m[4], m[8]), fmul(m[5], m[9])), fmul(m[6], m[10]));
+    const float det = fadd(fsub(fmul(m[0], fsub(fmul(m[5], m[10]), fmul(m[6], m[9]))),
+                                fmul(m[4], fsub(fmul(m[1], m[10]), fmul(m[2], m[9])))),
+                           fmul(m[8], fsub(fmul(m[1], m[6]), fmul(m[2], m[5]))));
+    const bool affine = fabsf(m[3]) <= 1.0e-6f && fabsf(m[7]) <= 1.0e-6f && fabsf(m[11]) <= 1.0e-6f &&
+                        fabsf(fsub(m[15], 1.0f)) <= 1.0e-4f;
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) finite = finite && isfinite(m[k]);
+    const bool valid = finite && isfinite(max_scale) && min_scale > 1.0e-8f && affine;
+    const float ut = fmul(max_scale, 1.0e-4f);
+    const float ot = fmul(fmul(max_scale, max_scale), 1.0e-4f);
+    const bool ap = fsub(max_scale, min_scale) <= ut && fabsf(dot_xy) <= ot && fabsf(dot_xz) <= ot &&
+                    fabsf(dot_yz) <= ot;
+    const bool cone = valid && ap && det > 0.0f;
+    HelioInstanceCullData r;
+    r.max_scale = valid ? max_scale : 0.0f;
+    r.min_scale = valid ? min_scale : 0.0f;
+    r.cone_cull_enabled = cone ? 1u : 0u;
+    r.valid_transform = valid ? 1u : 0u;
+    return r;
+}
+
 __global__ void instance_cull_data_kernel(const HelioGpuInstanceData* __restrict__ inst, uint32_t n,
                                           HelioInstanceCullData* __restrict__ out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float m[16];
-        const float4* src = reinterpret_cast<const float4*>(inst[i].model);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float4 q = __ldg(src + k);
-            m[4 * k + 0] = q.x;
-            m[4 * k + 1] = q.y;
-            m[4 * k + 2] = q.z;
-            m[4 * k + 3] = q.w;
-        }
-        const float sx = fsqrt(fadd(fadd(fmul(m[0], m[0]), fmul(m[1], m[1])), fmul(m[2], m[2])));
-        const float sy = fsqrt(fadd(fadd(fmul(m[4], m[4]), fmul(m[5], m[5])), fmul(m[6], m[6])));
-        const float sz = fsqrt(fadd(fadd(fmul(m[8], m[8]), fmul(m[9], m[9])), fmul(m[10], m[10])));
-        const float max_scale = fmaxf(fmaxf(sx, sy), sz);
-        const float min_scale = fminf(fminf(sx, sy), sz);
-        const float dot_xy = fadd(fadd(fmul(m[0], m[4]), fmul(m[1], m[5])), fmul(m[2], m[6]));
-        const float dot_xz = fadd(fadd(fmul(m[0], m[8]), fmul(m[1], m[9])), fmul(m[2], m[10]));
-        const float dot_yz = fadd(fadd(fmul(m[4], m[8]), fmul(m[5], m[9])), fmul(m[6], m[10]));
-        const float det = fadd(fsub(fmul(m[0], fsub(fmul(m[5], m[10]), fmul(m[6], m[9]))),
-                                    fmul(m[4], fsub(fmul(m[1], m[10]), fmul(m[2], m[9])))),
-                               fmul(m[8], fsub(fmul(m[1], m[6]), fmul(m[2], m[5]))));
-        const bool affine = fabsf(m[3]) <= 1.0e-6f && fabsf(m[7]) <= 1.0e-6f && fabsf(m[11]) <= 1.0e-6f &&
-                            fabsf(fsub(m[15], 1.0f)) <= 1.0e-4f;
-        bool finite = true;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) finite = finite && isfinite(m[k]);
-        const bool valid = finite && isfinite(max_scale) && min_scale > 1.0e-8f && affine;
-        const float ut = fmul(max_scale, 1.0e-4f);
-        const float ot = fmul(fmul(max_scale, max_scale), 1.0e-4f);
-        const bool ap = fsub(max_scale, min_scale) <= ut && fabsf(dot_xy) <= ot && fabsf(dot_xz) <= ot &&
-                        fabsf(dot_yz) <= ot;
-        const bool cone = valid && ap && det > 0.0f;
-        HelioInstanceCullData r;
-        r.max_scale = valid ? max_scale : 0.0f;
-        r.min_scale = valid ? min_scale : 0.0f;
-        r.cone_cull_enabled = cone ? 1u : 0u;
-        r.valid_transform = valid ? 1u : 0u;
-        out[i] = r;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        out[i] = cull_data_of(ldg_mat4(inst[i].model));
+}
+
+// launch_scene_update: the rows copied as 16-byte words in order, their cull data, the world
+// records, each a grid-stride loop that reads the source rows only (no loop waits for another's
+// results; an object recomputes its instance's scale). Bound by memory: 288 bytes per copied row,
+// 64 to 128 per object. Bounds and sums meet in the block, so that a block costs at most five
+// atomics (two per warp on the same two words took 37 us for 475,000 objects, without the sums).
+constexpr uint32_t kUpdateThreads = 256;
+
+template <bool kTotals>
+__global__ void __launch_bounds__(kUpdateThreads) scene_update_kernel(const __grid_constant__ SceneUpdate U) {
+    const VgSceneDev& S = U.scene;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t t0 = blockIdx.x * kUpdateThreads + threadIdx.x, stride = gridDim.x * kUpdateThreads;
+    const HelioGpuInstanceData* rows = U.src ? U.src : U.instances + U.first;  // row i = instance first + i
+    if (U.src) {
+        const uint4* src = reinterpret_cast<const uint4*>(U.src);
+        uint4* dst = reinterpret_cast<uint4*>(U.instances + U.first);
+        const uint64_t words = (uint64_t)U.count * (sizeof(HelioGpuInstanceData) / 16);
+        for (uint64_t w = t0; w < words; w += stride) dst[w] = __ldg(src + w);
     }
+    for (uint64_t i = t0; i < U.count; i += stride) U.cull[U.first + i] = cull_data_of(ldg_mat4(rows[i].model));
+    uint32_t rad = 0u, far1 = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
+    unsigned long long lod0 = 0, spans = 0, draws = 0;
+    for (uint64_t o = t0; o < S.object_count; o += stride) {
+        const HelioGpuVgObject* obj = S.objects + o;
+        const uint2 head = __ldg(reinterpret_cast<const uint2*>(obj));  // instance_index, lod_count
+        const uint32_t lods = min(head.y, 8u);
+        if (kTotals) {
+            const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts));
+            const uint4 c1 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts + 4));
+            const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+            uint32_t mx = 0;
+#pragma unroll
+            for (uint32_t l = 0; l < 8; ++l) mx = l < lods ? max(mx, c[l]) : mx;
+            lod0 += c[0];
+            spans += (mx + 63u) / 64u;
+            draws += mx;
+        }
+        float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t live = 0;
+        const bool named = head.x < S.instance_count;
+        if (named && head.x - U.first < U.count) {
+            const Mat4 model = ldg_mat4(rows[head.x - U.first].model);
+            const HelioInstanceCullData cd = cull_data_of(model);
+            if (lods && cd.valid_transform) {
+                const float4 lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
+                const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
+                sphere = make_float4(c.x, c.y, c.z, fmaxf(fmul(lb.w, cd.max_scale), 0.0f));
+                live = lods;
+            }
+            U.world[2u * o] = make_uint4(__float_as_uint(sphere.x), __float_as_uint(sphere.y),
+                                         __float_as_uint(sphere.z), __float_as_uint(sphere.w));
+            U.world[2u * o + 1u] = make_uint4(__float_as_uint(cd.max_scale), live, head.x, 0u);
+        } else if (!named) {
+            U.world[2u * o] = U.world[2u * o + 1u] = make_uint4(0u, 0u, 0u, 0u);
+        } else if (U.bounds) {
+            const ObjectWorld w = load_world(S, (uint32_t)o);
+            sphere = w.sphere;
+            live = w.lod_count;
+        }
+        if (live) {
+            rad = max(rad, __float_as_uint(sphere.w));  // (NaN above +inf)
+            // Rounding up is not needed: the reject boxes leave 2^-20 of slack.
+            far1 = max(far1, __float_as_uint(fabsf(sphere.x) + fabsf(sphere.y) + fabsf(sphere.z)));
+        }
+    }
+    if (!U.bounds && !kTotals) return;
+    __shared__ uint32_t s_max[2];
+    __shared__ unsigned long long s_sum[3];
+    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0ull;
+    __syncthreads();
+    rad = __reduce_max_sync(0xffffffffu, rad);
+    far1 = __reduce_max_sync(0xffffffffu, far1);
+    if (kTotals) {
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) {
+            lod0 += __shfl_xor_sync(0xffffffffu, lod0, k);
+            spans += __shfl_xor_sync(0xffffffffu, spans, k);
+            draws += __shfl_xor_sync(0xffffffffu, draws, k);
+        }
+    }
+    if ((threadIdx.x & 31u) == 0) {
+        atomicMax(s_max, rad);
+        atomicMax(s_max + 1, far1);
+        if (kTotals) {
+            atomicAdd(s_sum, lod0);
+            atomicAdd(s_sum + 1, spans);
+            atomicAdd(s_sum + 2, draws);
+        }
+    }
+    __syncthreads();
+    if (U.bounds && threadIdx.x < 2 && s_max[threadIdx.x]) atomicMax(U.bounds + threadIdx.x, s_max[threadIdx.x]);
+    if (kTotals && threadIdx.x < 3 && s_sum[threadIdx.x]) atomicAdd(U.totals + threadIdx.x, s_sum[threadIdx.x]);
 }
 
 // ── View constants ────────────────────────────────────────────────────────────
@@ -126,26 +218,15 @@ struct Selected {
     uint32_t lod_count, instance;
 };
 
-// The instance index and LOD count only: `reserved`, in the same 16 bytes, is written by this
-// launch.
-__device__ __forceinline__ uint2 object_head(const HelioGpuVgObject* o) {
-    return __ldg(reinterpret_cast<const uint2*>(o));
-}
-
-__device__ __forceinline__ Selected select_object(const VgSceneDev& S, const CullView& view,
-                                                  const HelioGpuVgObject* o, uint2 head) {
-    Selected r{0u, min(head.y, 8u), head.x};
-    if (r.lod_count == 0u || r.instance >= S.instance_count) return r;
-    // The object's fields and the instance's in one round trip.
-    const float4 lb = __ldg(reinterpret_cast<const float4*>(o->local_bounds));
+__device__ __forceinline__ Selected select_object(const VgSceneDev& S, const CullView& view, uint32_t i) {
+    const ObjectWorld w = load_world(S, i);
+    Selected r{0u, w.lod_count, w.instance};
+    const F3 c = f3(w.sphere.x, w.sphere.y, w.sphere.z);
+    const float wr = w.sphere.w;
+    if (w.lod_count == 0u || !sphere_visible_vg(view.planes, c, wr)) return r;
+    const HelioGpuVgObject* o = S.objects + i;
     const float4 e0 = __ldg(reinterpret_cast<const float4*>(o->lod_errors));
     const float4 e1 = __ldg(reinterpret_cast<const float4*>(o->lod_errors + 4));
-    const HelioInstanceCullData cd = load_cull(S.cull + r.instance);
-    const Mat4 model = ldg_mat4(S.instances[r.instance].model);
-    if (cd.valid_transform == 0u) return r;
-    const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
-    const float wr = fmaxf(fmul(lb.w, cd.max_scale), 0.0f);
-    if (!sphere_visible_vg(view.planes, c, wr)) return r;
     const float4 pn = view.pos_near;
     const F3 d = sub3(c, f3(pn.x, pn.y, pn.z));
     const float dist = fsqrt(dot3(d, d));
@@ -159,7 +240,7 @@ __device__ __forceinline__ Selected select_object(const VgSceneDev& S, const Cul
     for (uint32_t level = 1; level < 8; ++level) {
         if (level >= r.lod_count) break;
         // px = err * max_scale * focal / closest; px <= threshold keeps the level.
-        if (quotient_le(fmul(fmul(err[level], cd.max_scale), focal), closest, rc, qb)) lod = level;
+        if (quotient_le(fmul(fmul(err[level], w.max_scale), focal), closest, rc, qb)) lod = level;
         else break;
     }
     r.sel = lod + 1u;
@@ -175,7 +256,7 @@ __device__ void object_block(const VgFrameParams& P, const CullView& view, uint3
     if (threadIdx.x < 9) s_hist[threadIdx.x] = 0u;
     Selected r{0u, 0u, 0u};
     if (i < S.object_count) {
-        r = select_object(S, view, S.objects + i, object_head(S.objects + i));
+        r = select_object(S, view, i);
         S.objects[i].reserved = r.sel;
     }
     if (P.counter_count < 11u) return;  // uniform over the grid
@@ -318,7 +399,7 @@ __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t e
 // and by the launch. Against a select, a test and an emission launch with the counters cleared
 // before them, a frame (Hi-Z build included) went 29.3 -> 21.7 us with 4,096 instances x 64
 // meshlets at 1024x1024, 42.1 -> 31.8 with 10,000 x 100 (500 of them moved) at 1920x1080, and
-// 60.3 -> 54.3 with 100,000 x 100 at 3840x2160.
+// 60.3 -> 54.3 with 100,000 x 100 at 3840x2160 (46.8 with the objects' world records).
 template <bool kWide>
 __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const __grid_constant__ VgFrameParams P) {
     __shared__ CullView s_view;
@@ -362,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
         const uint2 it = __ldg(reinterpret_cast<const uint2*>(S.items + w_idx));  // object, local meshlet base
         if (it.x < S.object_count) {
             const HelioGpuVgObject* o = S.objects + it.x;
-            const Selected r = select_object(S, s_view, o, object_head(o));
+            const Selected r = select_object(S, s_view, it.x);
             if (r.sel) {
                 const uint32_t count = __ldg(&o->lod_meshlet_counts[r.sel - 1u]);
                 if (it.y < count) {
@@ -488,6 +569,22 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
     helio_launch_begin("instance_cull_data", stream);
     instance_cull_data_kernel<<<blocks, 256, 0, stream>>>(inst, n, out);
     helio_launch_end(stream);
+}
+
+cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream) {
+    const uint64_t words = u.src ? (uint64_t)u.count * (sizeof(HelioGpuInstanceData) / 16) : u.count;
+    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(words / 4, u.count), u.scene.object_count);
+    if (!n) return cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kUpdateThreads - 1) / kUpdateThreads,
+                                                       (uint64_t)std::max(sms, 1) * 8u);
+    helio_launch_begin("scene_update", stream);
+    const cudaError_t e = launch_after(u.totals ? scene_update_kernel<true> : scene_update_kernel<false>, grid,
+                                       kUpdateThreads, 0, stream, u);
+    helio_launch_end(stream);
+    return e;
 }
 
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream) {

@@ -17,11 +17,15 @@ __device__ __forceinline__ HelioInstanceCullData load_cull(const HelioInstanceCu
     return r;
 }
 
-// Cooperative copy of view constants into shared memory (16-byte words).
-__device__ __forceinline__ void load_view(const CullView* src, CullView& dst, int tid, int nthreads) {
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-    uint4* d = reinterpret_cast<uint4*>(&dst);
-    for (int k = tid; k < (int)(sizeof(CullView) / 16); k += nthreads) d[k] = __ldg(s + k);
+__device__ __forceinline__ ObjectWorld load_world(const VgSceneDev& S, uint32_t o) {
+    const uint4 a = __ldg(S.world + 2u * (size_t)o), b = __ldg(S.world + 2u * (size_t)o + 1u);
+    ObjectWorld w;
+    w.sphere = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w));
+    w.max_scale = __uint_as_float(b.x);
+    w.lod_count = b.y;
+    w.instance = b.z;
+    w.pad = 0u;
+    return w;
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {

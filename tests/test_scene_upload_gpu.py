@@ -35,3 +35,55 @@ def test_upload_totals_match_host_sums(cuda, n):
         assert got.object_count == n
         assert got.lod0_meshlets == int(counts[:, 0].sum())
         assert got.max_spans == int(spans.sum())
+
+
+@pytest.mark.parametrize("memory", ["host", "device", "device_unaligned"])
+@pytest.mark.parametrize("start,count", [(0, 3000), (0, 1), (2999, 1), (700, 1111)])
+def test_moved_instances_reach_every_object_that_names_them(cuda, memory, start, count):
+    """A dirty range of instances (rows of host memory, device rows the update copies itself,
+    device rows 4 bytes off its 16-byte loads) in a scene whose objects name instances in any
+    order, several the same and some none: the single-view pass and the batch give the oracle's
+    results for the moved scene."""
+    import torch
+    from helpers import assert_vg_equal, check_view, gather, gpu_hiz, gpu_vg_view, oracle_vg_view, u32
+    from helio_b200 import native as N
+    from helio_b200 import scene as S
+    from helio_b200.passes import BatchedCull, VgScene, VirtualGeometryPass
+    from oracle import oracle as O
+
+    n = 3000
+    rng = np.random.default_rng(start + count)
+    sc = S.make_scene(7, n, 40, 4, 0, 20.0)
+    sc.objects["instance_index"] = rng.integers(0, n, n)
+    sc.objects["instance_index"][:20] = n + 3
+    moved = S.make_scene(8, n, 40, 4, 0, 20.0).instances[start:start + count].copy()
+    moved["model"][::97, 3] = 0.5  # not affine: an invalid transform
+    new = S.Scene(sc.meshlets, sc.objects, sc.instances.copy(), sc.work_items, sc.aabbs, sc.draw_calls,
+                  sc.max_draw_count, sc.lod0_meshlets)
+    new.instances[start:start + count] = moved
+    v = S.main_view(5, 200, 120, 30)
+    frame = S.frame_data(sc)
+    raw = np.zeros(n * 144 + 16, np.uint8)
+    at = 4 if memory == "device_unaligned" else 0
+    raw[at:at + n * 144] = new.instances.view(np.uint8).reshape(-1)
+    rows = torch.from_numpy(raw).cuda() if memory != "host" else raw
+    base = (rows.data_ptr() if memory != "host" else raw.ctypes.data) + at
+    patch = N.VgFrameData(frame.meshlets, frame.objects, base, frame.work_items, frame.meshlet_count,
+                          frame.object_count, frame.work_item_count, frame.max_draw_count, 1, 2, start, count,
+                          N.HELIO_MEM_HOST if memory == "host" else N.HELIO_MEM_DEVICE, 0)
+    levels = O.hiz_build(v.depth)
+    hz, _ = gpu_hiz(v.depth)
+    vg = VirtualGeometryPass(v.width, v.height)
+    gpu_vg_view(sc, v, hz=hz, frame=frame, vg_pass=vg)
+    assert_vg_equal(gpu_vg_view(new, v, hz=hz, frame=patch, vg_pass=vg), oracle_vg_view(new, v, levels))
+    vs, b = VgScene(), BatchedCull(2)
+    vs.upload(frame)
+    d = torch.from_numpy(v.depth).cuda()
+    b.prepare(vs, [{"camera": v.camera, "depth": d}] * 2)
+    b.execute()
+    vs.upload(patch)
+    b.execute()
+    torch.cuda.synchronize()
+    for i in range(2):
+        got = gather(b, i, n)
+        check_view(new, v, got, None, None, got["capacity"])
