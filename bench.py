@@ -1390,7 +1390,7 @@ def run_shadow(args, rank, world, local_rank):
     peak, peak_kind = peaks()
     roofline = {"bound": "hbm", "kernel": "shadow_cull", "achieved": achieved, "peak": peak,
                 "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
-                "note": "three launches per step (graph replay); latency-bound at this size"}
+                "note": "two launches per step (graph replay); latency-bound at this size"}
     e2e = None
     if not args.no_e2e:
         hs = torch.from_numpy(np.ascontiguousarray(src.view(np.int32))).pin_memory()

@@ -719,7 +719,7 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
             __syncthreads();
             const uint32_t b = *s_claim;
             if (b >= P.shadow_blocks) break;
-            shadow_place_block(P.shadow, b, 0u, kShadowFaces, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
+            shadow_place_block<true>(P.shadow, b, 0u, 1u, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
         }
     }
 }
@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
             uint32_t next = 0;
             if (threadIdx.x == 0) next = atomicAdd(P.work, 1u);
             if (S && (q + 1u) % K == 0u && (q + 1u) / K <= S) {
-                shadow_test_block(P.shadow, (q + 1u) / K - 1u, 0u, kShadowFaces,
+                shadow_test_block(P.shadow, (q + 1u) / K - 1u, 0u, 1u,
                                   *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
                 __syncthreads();  // every thread has read *s_unit
                 if (threadIdx.x == 0) *s_unit = next;
@@ -1117,11 +1117,13 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
     }
     if (!grid_sync(P)) return;
     stamp(P, 2);
-    // The attached shadow cull's scan: CTA j takes the j-th dirty face (and clears face
-    // j's count when face j is clean); done before the phase's last barrier.
-    if (P.shadow_blocks)
-        for (uint32_t j = blockIdx.x; j < kShadowFaces; j += gridDim.x)
-            shadow_scan_face(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
+    // The attached shadow cull's scan: CTA j takes the j-th chunk of dirty faces, CTA 0 also
+    // clears the clean faces' counts; done before the phase's last barrier.
+    if (P.shadow_blocks) {
+        if (blockIdx.x == 0) shadow_clear_clean(P.shadow);
+        for (uint32_t j = blockIdx.x; j < kShadowChunks; j += gridDim.x)
+            shadow_scan_chunk(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
+    }
 
     if (!grid_exclusive_scan(P, P.chunk_counts, P.chunk_offs, P.view_count * P.object_chunks, s_tmp)) return;
     stamp(P, 3);

@@ -724,14 +724,14 @@ int32_t helio_shadow_cull_create(helio_shadow_cull_pass** out);
 /* Binds the inputs (kept until the next prepare) and grows the scratch for draw_count.
  * shadow_matrices and instances must be 16-byte aligned. */
 int32_t helio_shadow_cull_prepare(helio_shadow_cull_pass* pass, const helio_shadow_cull_inputs* in);
-/* Three launches on `stream`; no allocation, no read-back. */
+/* One to three launches on `stream`; no allocation, no read-back. */
 int32_t helio_shadow_cull_execute(helio_shadow_cull_pass* pass, void* stream);
 int32_t helio_shadow_cull_publish(const helio_shadow_cull_pass* pass, helio_shadow_cull_outputs* out);
 void helio_shadow_cull_destroy(helio_shadow_cull_pass* pass);
 
 /* Folds a prepared shadow cull pass into a batch: from the next helio_batch_execute on,
  * the pass's test, scan and placement run as units of the batch's own phases (the
- * persistent launch's work queue and barriers) instead of three launches of their own,
+ * persistent launch's work queue and barriers) instead of launches of their own,
  * with the outputs of helio_shadow_cull_execute, read with helio_shadow_cull_publish.
  * The pass stays the caller's: it must stay alive, and its inputs valid, while it is
  * attached; a pass with no face or no draw in use does nothing, as in the standalone

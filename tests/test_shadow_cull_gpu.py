@@ -179,3 +179,28 @@ def test_shadow_cull_folded_into_a_batch(cuda, max_ctas):
         np.testing.assert_array_equal(c, wc)
         np.testing.assert_array_equal(ind, wind)
         np.testing.assert_array_equal(dr, wdr)
+
+
+@pytest.mark.parametrize("draws", [1, 31, 256, 257, 2048, 2049, 6145, 8192, 8193, 262144, 262145])
+@pytest.mark.parametrize("faces", [1, 32, 33, 256])
+def test_shadow_cull_launch_forms(cuda, draws, faces):
+    """Draw counts at the edges of a block, of the one-launch cluster form and its rounds, of the
+    form whose place blocks sum the counts and of the one with a scan; dirty faces that fill
+    part of a chunk of 32, exactly one, just over one, and all eight. Two frames in a row."""
+    from helio_b200 import scene as S
+
+    if draws > 100000 and faces == 256:
+        draws = 262145  # one form is enough at this size
+    mats, nf = S.shadow_faces(9, 12, 40)
+    assert nf == 256
+    inst, src = shadow_scene(draws, 4000, draws, spread=150.0)
+    rng = np.random.default_rng(draws + faces)
+    g = Gpu()
+    ref_dst = ref_counts = None
+    for _ in range(2):
+        dirty = np.zeros(256, np.uint32)
+        dirty[rng.permutation(256)[:faces]] = 1
+        dst, counts = g.run(mats, inst, src, dirty, nf)
+        ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf, dst=ref_dst, counts=ref_counts)
+        assert ran
+        check_frame(dst, counts, ref_dst, ref_counts, np.nonzero(dirty)[0])
