@@ -196,3 +196,20 @@ def test_built_scene_culls_like_the_oracle(cuda):
     for i, v in enumerate(views):
         got = gather(bc, i, len(built.objects))
         check_view(built, v, got, None, None, got["capacity"])
+
+
+@pytest.mark.parametrize("slots,meshes", [(1, 1), (3, 2), (1023, 5), (1024, 8192), (1025, 300), (4096, 4096), (4100, 4097),
+                                          (3000, 8193), (1024 * 1024, 256), (1024 * 1024 + 1, 5000),
+                                          (1500000, 9000)])
+def test_build_forms_match_oracle(cuda, slots, meshes):
+    """Slot counts at the edges of a 1024-slot block and of the form that scans the block sums,
+    library sizes at the edges of the shared table and of the last block's fold; run twice."""
+    from helio_b200.passes import VgBuilder
+
+    lib = random_library(slots + meshes, pool=2000, meshes=meshes, slots=slots, max_count=200)
+    ref = O.vg_rebuild(lib.pool, lib.meshes, lib.slot_mesh, lib.slot_instances)
+    assert ref is not None
+    b = VgBuilder()
+    for _ in range(2):
+        _, host, _ = gpu_build(lib, b)
+        assert_same(host, ref)
