@@ -94,31 +94,29 @@ int32_t copy_in(void* dst, const void* src, size_t bytes, uint32_t memory, cudaS
 
 constexpr size_t kBoundsBytes = 8 + 3 * 8;
 
-// Instances [first, first + count) of a scene of `objects` objects from `src` (the caller's rows
-// of that range) and everything derived from them, the bounds included; with `totals` also the
-// sums of launch_scene_update, read back (waits for the stream). Device rows that 16-byte loads
-// can read are copied by the update kernel itself. (Summing the objects on the host, read back
+// Runs the update `u` with the instances [first, first + count) of a scene of `objects` objects from
+// `src` (the caller's rows of that range) and the scene's bounds; with `totals` also the sums of
+// launch_scene_update, read back (waits for the stream). Device rows that 16-byte loads
+// can read are copied by the update itself. (Summing the objects on the host, read back
 // whole, took 15 to 33 ms for 475,000 objects.)
-int32_t scene_update(helio_vg_scene* sc, uint32_t objects, uint32_t first, uint32_t count,
+int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects, uint32_t first, uint32_t count,
                      const HelioGpuInstanceData* src, uint32_t memory, uint64_t* totals, cudaStream_t s) {
     HELIO_CK(sc->bounds.ensure(kBoundsBytes));
     HELIO_CK(cudaMemsetAsync(sc->bounds.ptr, 0, kBoundsBytes, s));
-    const bool direct = memory == HELIO_MEM_DEVICE && count && src && (reinterpret_cast<uintptr_t>(src) & 15u) == 0u;
-    if (!direct) {
-        int32_t st = copy_in(sc->instances.as<HelioGpuInstanceData>() + first, src,
-                             (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
-        if (st) return st;
-    }
-    unsigned long long* sums = reinterpret_cast<unsigned long long*>(sc->bounds.as<char>() + 8);
-    helio::SceneUpdate u{};
     u.scene = sc->dev();
     u.scene.object_count = u.scene.instance_count = objects;
-    u.src = direct ? src : nullptr;
     u.instances = sc->instances.as<HelioGpuInstanceData>();
     u.cull = sc->cull.as<HelioInstanceCullData>();
     u.world = sc->world.as<uint4>();
     u.first = first;
     u.count = count;
+    if (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16)) {
+        u.src_rows = src;
+    } else {
+        int32_t st = copy_in(u.instances + first, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
+        if (st) return st;
+    }
+    unsigned long long* sums = reinterpret_cast<unsigned long long*>(sc->bounds.as<char>() + 8);
     u.bounds = sc->bounds.as<uint32_t>();
     u.totals = totals ? sums : nullptr;
     HELIO_CK(helio::launch_scene_update(u, s));
@@ -239,25 +237,28 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->instances.ensure(O * sizeof(HelioGpuInstanceData)));
         HELIO_CK(sc->cull.ensure(O * sizeof(HelioInstanceCullData)));
         HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
-        const HelioGpuMeshletEntry* aos = f->meshlets;
-        if (M) {
-            if (f->memory == HELIO_MEM_HOST) {
-                HELIO_CK(sc->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
-                if ((st = copy_in(sc->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s)))
-                    return st;
-                aos = sc->staging.as<HelioGpuMeshletEntry>();
-            }
-            HELIO_ARG(aos, "meshlet array missing");
-            helio::launch_pack_meshlets(aos, (uint32_t)M, sc->m_bounds.as<float4>(), sc->m_cone.as<float4>(),
-                                        sc->m_axis.as<float4>(), sc->m_draw.as<uint4>(), s);
-            HELIO_CK(cudaGetLastError());
+        // Device arrays that 16-byte loads can read are copied by the update launch itself.
+        helio::SceneUpdate u{};
+        const bool device = f->memory == HELIO_MEM_DEVICE;
+        u.src_meshlets = f->meshlets;
+        if (M && !(device && helio::update_reads(f->meshlets, 16))) {
+            HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
+            HELIO_CK(sc->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
+            if ((st = copy_in(sc->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
+            u.src_meshlets = sc->staging.as<HelioGpuMeshletEntry>();
         }
-        if ((st = copy_in(sc->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
+        u.meshlet_count = f->meshlet_count;
+        u.m_bounds = sc->m_bounds.as<float4>();
+        u.m_cone = sc->m_cone.as<float4>();
+        u.m_axis = sc->m_axis.as<float4>();
+        u.m_draw = sc->m_draw.as<uint4>();
+        if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
+        else if ((st = copy_in(sc->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
         // With the per-object span bound and LOD0 size, for capacities and the metric; the wait
         // for them also ends the use of the staging copy.
         uint64_t totals[3] = {0, 0, 0};
-        if ((st = scene_update(sc, f->object_count, 0, f->object_count, f->instances, f->memory, totals, s))) return st;
-        if (f->memory == HELIO_MEM_HOST) sc->staging.release();
+        if ((st = scene_update(sc, u, f->object_count, 0, f->object_count, f->instances, f->memory, totals, s))) return st;
+        sc->staging.release();
         sc->meshlet_count = f->meshlet_count;
         sc->object_count = f->object_count;
         sc->lod0_meshlets = totals[0];
@@ -269,7 +270,8 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
     } else if (f->instance_version != sc->instance_version) {
         const uint64_t start = f->instance_dirty_start, count = f->instance_dirty_count;
         HELIO_ARG(count > 0 && start + count <= sc->object_count, "invalid dirty instance range");
-        if ((st = scene_update(sc, sc->object_count, (uint32_t)start, (uint32_t)count,
+        helio::SceneUpdate u{};
+        if ((st = scene_update(sc, u, sc->object_count, (uint32_t)start, (uint32_t)count,
                                f->instances ? f->instances + start : nullptr, f->memory, nullptr, s)))
             return st;
         sc->instance_version = f->instance_version;

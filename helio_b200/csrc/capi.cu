@@ -587,27 +587,19 @@ static int32_t vg_copy(void* dst, const void* src, size_t bytes, uint32_t memory
     return HELIO_OK;
 }
 
-// Instances [first, first + count) of a scene of `objects` objects from `src` (the caller's rows
-// of that range), and everything derived from them. Device rows that 16-byte loads can read are
-// copied by the update kernel itself.
-static int32_t vg_update(helio_vg_pass* p, uint32_t objects, uint32_t first, uint32_t count,
-                         const HelioGpuInstanceData* src, uint32_t memory, cudaStream_t s) {
-    const bool direct = memory == HELIO_MEM_DEVICE && count && src && (reinterpret_cast<uintptr_t>(src) & 15u) == 0u;
-    if (!direct) {
-        int32_t st = vg_copy(p->instances.as<HelioGpuInstanceData>() + first, src,
-                             (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
-        if (st) return st;
-    }
-    helio::SceneUpdate u{};
-    u.scene.objects = p->objects.as<HelioGpuVgObject>();
-    u.scene.object_count = u.scene.instance_count = objects;
-    u.scene.world = u.world = p->world.as<uint4>();
-    u.src = direct ? src : nullptr;
-    u.instances = p->instances.as<HelioGpuInstanceData>();
-    u.cull = p->cull.as<HelioInstanceCullData>();
-    u.first = first;
-    u.count = count;
-    HELIO_CK(helio::launch_scene_update(u, s));
+// A scene update of the pass's buffers: instances [first, first + count) of a scene of `objects`
+// objects from `src` (the caller's rows of that range).
+static int32_t vg_rows(helio_vg_pass* p, helio::SceneUpdate* u, uint32_t objects, uint32_t first, uint32_t count,
+                       const HelioGpuInstanceData* src, uint32_t memory, cudaStream_t s) {
+    u->scene.objects = p->objects.as<HelioGpuVgObject>();
+    u->scene.object_count = u->scene.instance_count = objects;
+    u->scene.world = u->world = p->world.as<uint4>();
+    u->instances = p->instances.as<HelioGpuInstanceData>();
+    u->cull = p->cull.as<HelioInstanceCullData>();
+    u->first = first;
+    u->count = count;
+    if (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16)) u->src_rows = src;
+    else return vg_copy(u->instances + first, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
     return HELIO_OK;
 }
 
@@ -629,23 +621,31 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
         HELIO_CK(p->visibility.ensure(W * 8));
-        const HelioGpuMeshletEntry* aos = f->meshlets;
-        if (M) {
-            if (f->memory == HELIO_MEM_HOST) {
-                HELIO_CK(p->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
-                if ((st = vg_copy(p->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
-                aos = p->staging.as<HelioGpuMeshletEntry>();
-            }
-            HELIO_ARG(aos, "meshlet array missing");
-            helio::launch_pack_meshlets(aos, (uint32_t)M, p->m_bounds.as<float4>(), p->m_cone.as<float4>(),
-                                        p->m_axis.as<float4>(), p->m_draw.as<uint4>(), s);
-            HELIO_CK(cudaGetLastError());
+        // Device arrays that 16-byte loads can read are copied by the update launch itself.
+        helio::SceneUpdate u{};
+        const bool device = f->memory == HELIO_MEM_DEVICE;
+        u.src_meshlets = f->meshlets;
+        if (M && !(device && helio::update_reads(f->meshlets, 16))) {
+            HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
+            HELIO_CK(p->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
+            if ((st = vg_copy(p->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
+            u.src_meshlets = p->staging.as<HelioGpuMeshletEntry>();
         }
-        if ((st = vg_copy(p->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
-        if ((st = vg_copy(p->items.ptr, f->work_items, W * sizeof(HelioGpuVgWorkItem), f->memory, s))) return st;
-        if ((st = vg_update(p, f->object_count, 0, f->object_count, f->instances, f->memory, s))) return st;
-        if (f->memory == HELIO_MEM_HOST && M) {
-            // The staging copy is consumed by the pack kernel; release it once it ran.
+        u.meshlet_count = f->meshlet_count;
+        u.m_bounds = p->m_bounds.as<float4>();
+        u.m_cone = p->m_cone.as<float4>();
+        u.m_axis = p->m_axis.as<float4>();
+        u.m_draw = p->m_draw.as<uint4>();
+        if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
+        else if ((st = vg_copy(p->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
+        u.items = p->items.as<HelioGpuVgWorkItem>();
+        u.item_count = f->work_item_count;
+        if (device && helio::update_reads(f->work_items, 8)) u.src_items = f->work_items;
+        else if ((st = vg_copy(p->items.ptr, f->work_items, W * sizeof(HelioGpuVgWorkItem), f->memory, s))) return st;
+        if ((st = vg_rows(p, &u, f->object_count, 0, f->object_count, f->instances, f->memory, s))) return st;
+        HELIO_CK(helio::launch_scene_update(u, s));
+        if (p->staging.ptr) {
+            // The staging copy is consumed by the update; release it once it ran.
             HELIO_CK(cudaStreamSynchronize(s));
             p->staging.release();
         }
@@ -673,9 +673,11 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         // Dirty-instance patch (rendering.rs:787-819).
         const uint64_t start = f->instance_dirty_start, count = f->instance_dirty_count;
         HELIO_ARG(count > 0 && start + count <= p->object_count, "invalid dirty instance range");
-        if ((st = vg_update(p, p->object_count, (uint32_t)start, (uint32_t)count,
-                            f->instances ? f->instances + start : nullptr, f->memory, s)))
+        helio::SceneUpdate u{};
+        if ((st = vg_rows(p, &u, p->object_count, (uint32_t)start, (uint32_t)count,
+                          f->instances ? f->instances + start : nullptr, f->memory, s)))
             return st;
+        HELIO_CK(helio::launch_scene_update(u, s));
         p->last_instance_version = f->instance_version;
     }
     return HELIO_OK;

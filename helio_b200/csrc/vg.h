@@ -103,30 +103,36 @@ inline uint32_t vg_tiles(uint32_t work_items, uint32_t tile_items) {
     return (uint32_t)(((uint64_t)work_items + tile_items - 1) / tile_items);
 }
 
-void launch_pack_meshlets(const HelioGpuMeshletEntry* aos, uint32_t n, float4* bounds, float4* cone, float4* axis,
-                          uint4* draw, cudaStream_t stream);
 void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, HelioInstanceCullData* out,
                                cudaStream_t stream);
 
-// Brings a scene's derived data up to date with the instances [first, first + count): their
-// InstanceCullData and the ObjectWorld records of the objects that name them, in one launch. With
-// `src` (device, 16-byte aligned) also copies the `count` rows from it; null: the rows are in
-// scene.instances already.
+// Brings a device-resident scene up to date in one launch: copies what the caller gives in device
+// memory, and derives from the instances [first, first + count) their InstanceCullData and the
+// ObjectWorld records of the objects that name them. A null source: the data is in the
+// destination already.
 // With `bounds` (u32[2], zero before the launch), bounds over all valid objects as float bits, for
 // the batch's reject boxes: bounds[0] = largest world radius max(local_radius * max_scale, 0),
 // bounds[1] = largest |c.x| + |c.y| + |c.z| of a world centre c. With `totals` (u64[3], zero before
 // the launch), sums over all objects: totals[0] = lod_meshlet_counts[0], totals[1] = 64-meshlet
 // spans and totals[2] = meshlets of the largest of the object's LODs.
 struct SceneUpdate {
-    VgSceneDev scene;
-    const HelioGpuInstanceData* src;
+    VgSceneDev scene;  // object_count, instance_count, objects (written too, with src_objects) and world
+    const HelioGpuInstanceData* src_rows;     // [count], 16-byte aligned
+    const HelioGpuVgObject* src_objects;      // [object_count], 16-byte aligned
+    const HelioGpuVgWorkItem* src_items;      // [item_count], 8-byte aligned
+    const HelioGpuMeshletEntry* src_meshlets; // [meshlet_count], 16-byte aligned, packed into the four streams
     HelioGpuInstanceData* instances;
     HelioInstanceCullData* cull;
     uint4* world;
-    uint32_t first, count;
+    HelioGpuVgWorkItem* items;
+    float4 *m_bounds, *m_cone, *m_axis;
+    uint4* m_draw;
+    uint32_t first, count, item_count, meshlet_count;
     uint32_t* bounds;
     unsigned long long* totals;
 };
+// Whether the update kernel can read an array of device memory itself.
+inline bool update_reads(const void* p, size_t align) { return p && (reinterpret_cast<uintptr_t>(p) & (align - 1)) == 0; }
 cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream);
 // Object select, meshlet cull and emission of one view, in one launch.
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream);

@@ -36,18 +36,6 @@ namespace {
 
 // ── Scene preparation ─────────────────────────────────────────────────────────
 
-__global__ void pack_meshlets_kernel(const HelioGpuMeshletEntry* __restrict__ aos, uint32_t n,
-                                     float4* __restrict__ bounds, float4* __restrict__ cone,
-                                     float4* __restrict__ axis, uint4* __restrict__ draw) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4* src = reinterpret_cast<const float4*>(aos + i);
-        bounds[i] = __ldcs(src + 0);
-        cone[i] = __ldcs(src + 1);
-        axis[i] = __ldcs(src + 2);
-        draw[i] = __ldcs(reinterpret_cast<const uint4*>(src + 3));
-    }
-}
-
 // InstanceCullData::from_instance (lib.rs:132-167), Rust f32 evaluation order, of the
 // column-major model matrix m.
 __device__ __forceinline__ HelioInstanceCullData cull_data_of(const Mat4& mm) {
@@ -89,31 +77,90 @@ __global__ void instance_cull_data_kernel(const HelioGpuInstanceData* __restrict
         out[i] = cull_data_of(ldg_mat4(inst[i].model));
 }
 
-// launch_scene_update: the rows copied as 16-byte words in order, their cull data, the world
-// records, each a grid-stride loop that reads the source rows only (no loop waits for another's
-// results; an object recomputes its instance's scale). Bound by memory: 288 bytes per copied row,
-// 64 to 128 per object. Bounds and sums meet in the block, so that a block costs at most five
-// atomics (two per warp on the same two words took 37 us for 475,000 objects, without the sums).
+// launch_scene_update. CTAs come in three kinds: one per 256 rows and 256 objects (the same
+// indices, since an object mostly names the instance of its own index, whose row is then in L1), one
+// per 2048 work items, one per 512 meshlets. Copies have all their loads in flight before the
+// first store. No kind waits for another's results: rows are read from their source, and an object
+// recomputes its instance's scale. Bound by memory: 288 bytes per copied row, 256 per copied object.
+// Bounds and sums meet in the block, so that a block costs at most five atomics (two per warp on
+// the same two words took 37 us for 475,000 objects).
 constexpr uint32_t kUpdateThreads = 256;
+constexpr uint32_t kUpdateItems = 8 * kUpdateThreads;
+constexpr uint32_t kUpdateMeshlets = 2 * kUpdateThreads;
+
+// Copies n 16-byte words (at most kEach per thread) from src to dst, loads first.
+template <int kEach>
+__device__ __forceinline__ void copy_words(uint4* dst, const uint4* src, uint32_t n) {
+    uint4 x[kEach];
+#pragma unroll
+    for (int k = 0; k < kEach; ++k)
+        if (k * kUpdateThreads + threadIdx.x < n) x[k] = __ldg(src + k * kUpdateThreads + threadIdx.x);
+#pragma unroll
+    for (int k = 0; k < kEach; ++k)
+        if (k * kUpdateThreads + threadIdx.x < n) dst[k * kUpdateThreads + threadIdx.x] = x[k];
+}
+
+__device__ __forceinline__ void update_items(const SceneUpdate& U, uint32_t block) {
+    const uint2* src = reinterpret_cast<const uint2*>(U.src_items);
+    uint2* dst = reinterpret_cast<uint2*>(U.items);
+    uint2 x[8];
+    const uint64_t i0 = (uint64_t)block * kUpdateItems + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (i0 + k * kUpdateThreads < U.item_count) x[k] = __ldg(src + i0 + k * kUpdateThreads);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (i0 + k * kUpdateThreads < U.item_count) dst[i0 + k * kUpdateThreads] = x[k];
+}
+
+// Meshlets into the four streams.
+__device__ __forceinline__ void update_meshlets(const SceneUpdate& U, uint32_t block) {
+    const uint4* src = reinterpret_cast<const uint4*>(U.src_meshlets);
+    uint4* streams[4] = {reinterpret_cast<uint4*>(U.m_bounds), reinterpret_cast<uint4*>(U.m_cone),
+                         reinterpret_cast<uint4*>(U.m_axis), U.m_draw};
+    const uint64_t m0 = (uint64_t)block * kUpdateMeshlets;
+    uint4 x[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint64_t m = m0 + (uint32_t)r * kUpdateThreads + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (m < U.meshlet_count) x[r][k] = __ldcs(src + 4u * m + k);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint64_t m = m0 + (uint32_t)r * kUpdateThreads + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (m < U.meshlet_count) streams[k][m] = x[r][k];
+    }
+}
 
 template <bool kTotals>
-__global__ void __launch_bounds__(kUpdateThreads) scene_update_kernel(const __grid_constant__ SceneUpdate U) {
+__global__ void __launch_bounds__(kUpdateThreads, 4)
+    scene_update_kernel(const __grid_constant__ SceneUpdate U, uint32_t object_blocks, uint32_t item_blocks) {
     const VgSceneDev& S = U.scene;
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t t0 = blockIdx.x * kUpdateThreads + threadIdx.x, stride = gridDim.x * kUpdateThreads;
-    const HelioGpuInstanceData* rows = U.src ? U.src : U.instances + U.first;  // row i = instance first + i
-    if (U.src) {
-        const uint4* src = reinterpret_cast<const uint4*>(U.src);
-        uint4* dst = reinterpret_cast<uint4*>(U.instances + U.first);
-        const uint64_t words = (uint64_t)U.count * (sizeof(HelioGpuInstanceData) / 16);
-        for (uint64_t w = t0; w < words; w += stride) dst[w] = __ldg(src + w);
+    if (blockIdx.x >= object_blocks) {
+        const uint32_t b = blockIdx.x - object_blocks;
+        if (b < item_blocks) update_items(U, b);
+        else update_meshlets(U, b - item_blocks);
+        return;
     }
-    for (uint64_t i = t0; i < U.count; i += stride) U.cull[U.first + i] = cull_data_of(ldg_mat4(rows[i].model));
+    const uint32_t i0 = blockIdx.x * kUpdateThreads, i = i0 + threadIdx.x;
+    const HelioGpuInstanceData* rows = U.src_rows ? U.src_rows : U.instances + U.first;  // row k = instance first + k
+    if (U.src_rows && i0 < U.count)
+        copy_words<9>(reinterpret_cast<uint4*>(U.instances + U.first + i0), reinterpret_cast<const uint4*>(rows + i0),
+                      min(kUpdateThreads, U.count - i0) * (uint32_t)(sizeof(HelioGpuInstanceData) / 16));
+    if (U.src_objects && i0 < S.object_count)
+        copy_words<8>(reinterpret_cast<uint4*>(S.objects + i0), reinterpret_cast<const uint4*>(U.src_objects + i0),
+                      min(kUpdateThreads, S.object_count - i0) * (uint32_t)(sizeof(HelioGpuVgObject) / 16));
+    if (i < U.count) U.cull[U.first + i] = cull_data_of(ldg_mat4(rows[i].model));
     uint32_t rad = 0u, far1 = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
     unsigned long long lod0 = 0, spans = 0, draws = 0;
-    for (uint64_t o = t0; o < S.object_count; o += stride) {
-        const HelioGpuVgObject* obj = S.objects + o;
+    if (i < S.object_count) {
+        const HelioGpuVgObject* obj = (U.src_objects ? U.src_objects : S.objects) + i;
         const uint2 head = __ldg(reinterpret_cast<const uint2*>(obj));  // instance_index, lod_count
         const uint32_t lods = min(head.y, 8u);
         if (kTotals) {
@@ -123,9 +170,9 @@ __global__ void __launch_bounds__(kUpdateThreads) scene_update_kernel(const __gr
             uint32_t mx = 0;
 #pragma unroll
             for (uint32_t l = 0; l < 8; ++l) mx = l < lods ? max(mx, c[l]) : mx;
-            lod0 += c[0];
-            spans += (mx + 63u) / 64u;
-            draws += mx;
+            lod0 = c[0];
+            spans = (mx + 63u) / 64u;
+            draws = mx;
         }
         float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t live = 0;
@@ -139,20 +186,20 @@ __global__ void __launch_bounds__(kUpdateThreads) scene_update_kernel(const __gr
                 sphere = make_float4(c.x, c.y, c.z, fmaxf(fmul(lb.w, cd.max_scale), 0.0f));
                 live = lods;
             }
-            U.world[2u * o] = make_uint4(__float_as_uint(sphere.x), __float_as_uint(sphere.y),
-                                         __float_as_uint(sphere.z), __float_as_uint(sphere.w));
-            U.world[2u * o + 1u] = make_uint4(__float_as_uint(cd.max_scale), live, head.x, 0u);
+            U.world[2u * (size_t)i] = make_uint4(__float_as_uint(sphere.x), __float_as_uint(sphere.y),
+                                                 __float_as_uint(sphere.z), __float_as_uint(sphere.w));
+            U.world[2u * (size_t)i + 1u] = make_uint4(__float_as_uint(cd.max_scale), live, head.x, 0u);
         } else if (!named) {
-            U.world[2u * o] = U.world[2u * o + 1u] = make_uint4(0u, 0u, 0u, 0u);
+            U.world[2u * (size_t)i] = U.world[2u * (size_t)i + 1u] = make_uint4(0u, 0u, 0u, 0u);
         } else if (U.bounds) {
-            const ObjectWorld w = load_world(S, (uint32_t)o);
+            const ObjectWorld w = load_world(S, i);
             sphere = w.sphere;
             live = w.lod_count;
         }
         if (live) {
-            rad = max(rad, __float_as_uint(sphere.w));  // (NaN above +inf)
+            rad = __float_as_uint(sphere.w);  // (NaN above +inf)
             // Rounding up is not needed: the reject boxes leave 2^-20 of slack.
-            far1 = max(far1, __float_as_uint(fabsf(sphere.x) + fabsf(sphere.y) + fabsf(sphere.z)));
+            far1 = __float_as_uint(fabsf(sphere.x) + fabsf(sphere.y) + fabsf(sphere.z));
         }
     }
     if (!U.bounds && !kTotals) return;
@@ -551,16 +598,6 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
 
 }  // namespace
 
-void launch_pack_meshlets(const HelioGpuMeshletEntry* aos, uint32_t n, float4* bounds, float4* cone, float4* axis,
-                          uint4* draw, cudaStream_t stream) {
-    if (!n) return;
-    uint32_t blocks = (n + 255u) / 256u;
-    if (blocks > 148u * 16u) blocks = 148u * 16u;
-    helio_launch_begin("pack_meshlets", stream);
-    pack_meshlets_kernel<<<blocks, 256, 0, stream>>>(aos, n, bounds, cone, axis, draw);
-    helio_launch_end(stream);
-}
-
 void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, HelioInstanceCullData* out,
                                cudaStream_t stream) {
     if (!n) return;
@@ -572,17 +609,14 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
 }
 
 cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream) {
-    const uint64_t words = u.src ? (uint64_t)u.count * (sizeof(HelioGpuInstanceData) / 16) : u.count;
-    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(words / 4, u.count), u.scene.object_count);
-    if (!n) return cudaSuccess;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kUpdateThreads - 1) / kUpdateThreads,
-                                                       (uint64_t)std::max(sms, 1) * 8u);
+    auto blocks = [](uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / per); };
+    const uint32_t objects = blocks(std::max(u.count, u.scene.object_count), kUpdateThreads);
+    const uint32_t items = u.src_items ? blocks(u.item_count, kUpdateItems) : 0u;
+    const uint32_t meshlets = u.src_meshlets ? blocks(u.meshlet_count, kUpdateMeshlets) : 0u;
+    if (objects + items + meshlets == 0u) return cudaSuccess;
     helio_launch_begin("scene_update", stream);
-    const cudaError_t e = launch_after(u.totals ? scene_update_kernel<true> : scene_update_kernel<false>, grid,
-                                       kUpdateThreads, 0, stream, u);
+    const cudaError_t e = launch_after(u.totals ? scene_update_kernel<true> : scene_update_kernel<false>,
+                                       objects + items + meshlets, kUpdateThreads, 0, stream, u, objects, items);
     helio_launch_end(stream);
     return e;
 }
