@@ -285,7 +285,7 @@ __device__ __forceinline__ bool outputs_fit(const BuildOut& o, uint64_t objects,
 // scan_blocks_kernel); the warp sums of all rounds meet behind one barrier and give every slot its
 // own. Bound by latency: the sums, the slots' mesh indices, the mesh heads.
 template <bool kScanned>
-__global__ void __launch_bounds__(kThreads) place_kernel(const __grid_constant__ helio_vg_build_inputs in,
+__global__ void __launch_bounds__(kThreads, 4) place_kernel(const __grid_constant__ helio_vg_build_inputs in,
                                                          const __grid_constant__ BuildWork w,
                                                          const uint64_t* block_base,
                                                          const __grid_constant__ BuildOut out) {
@@ -354,7 +354,8 @@ __global__ void __launch_bounds__(kThreads) place_kernel(const __grid_constant__
     for (uint32_t j = 0; j < kSub; ++j) {
         const bool ok = m[j] < in.mesh_count;
         h[j] = ok ? mesh_word(in.meshes, m[j], 0) : make_uint4(0u, 0u, 0u, 0u);
-        fr[j] = ok ? __ldcg(w.first_ref + m[j]) : 0u;
+        // Through L1: past it, a small library's table is a few L2 lines that every slot asks for.
+        fr[j] = ok ? __ldg(w.first_ref + m[j]) : 0u;
     }
     uint32_t ex[kSub][4];  // exclusive within the warp and round
 #pragma unroll
@@ -425,7 +426,8 @@ __device__ __forceinline__ void write_objects(const helio_vg_build_inputs& in, c
     if (!used_mask) return;
     const uint32_t obj0 = __shfl_sync(0xffffffffu, obj, __ffs(used_mask) - 1);
     const uint32_t n_used = __popc(used_mask);
-    const bool full = used_mask == 0xffffffffu;
+    // Lane k holds the k-th used lane: found once, then read by shuffles.
+    const uint32_t nth = nth_set_bit(used_mask, min(lane, n_used - 1u));
     {
         constexpr uint32_t kW = sizeof(HelioGpuInstanceData) / 16;  // 9 words per instance
         const uint4* src = reinterpret_cast<const uint4*>(in.slot_instances) + (o - lane) * kW;
@@ -435,7 +437,8 @@ __device__ __forceinline__ void write_objects(const helio_vg_build_inputs& in, c
 #pragma unroll
         for (uint32_t r = 0; r < kW; ++r) {
             const uint32_t w = r * 32u + lane, k = w / kW;  // k-th used lane of the warp
-            if (w < words) x[r] = __ldcs(src + (full ? w : nth_set_bit(used_mask, k) * kW + (w - k * kW)));
+            const uint32_t from = __shfl_sync(0xffffffffu, nth, k);
+            if (w < words) x[r] = __ldcs(src + from * kW + (w - k * kW));
         }
 #pragma unroll
         for (uint32_t r = 0; r < kW; ++r)
@@ -448,8 +451,7 @@ __device__ __forceinline__ void write_objects(const helio_vg_build_inputs& in, c
 #pragma unroll
     for (uint32_t r = 0; r < 8; ++r) {
         const uint32_t k = 4u * r + (lane >> 3);
-        const uint32_t from = full ? k : nth_set_bit(used_mask, min(k, n_used - 1u));
-        const uint32_t mk = __shfl_sync(0xffffffffu, m, from);
+        const uint32_t mk = __shfl_sync(0xffffffffu, m, __shfl_sync(0xffffffffu, nth, k));
         if (k >= n_used) continue;
         x[r] = mesh_word(in.meshes, mk, (int)w);
         base[r] = w == 4u || w == 5u ? __ldg(out.mesh_base + mk) : 0u;
