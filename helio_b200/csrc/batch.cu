@@ -19,8 +19,8 @@
 //   2  exclusive scan of the (view, chunk) span counts
 //   3  expansion into one list of active spans, view-major, each view padded to a
 //      multiple of 32 spans so every group of 32 spans belongs to one view
-//   4  meshlet tests: a warp takes a group of 32 spans and packs their meshlets
-//      densely into 32-lane windows (window ballots and per-group counts stored)
+//   4  meshlet tests: a warp takes a group of 32 spans (16 or 8 in small batches) and packs
+//      their meshlets densely into 32-lane windows (window ballots and per-group counts stored)
 //   5  exclusive scan of the group counts
 //   6  emission of each view's draws at slot = position in the view's order
 //
@@ -56,7 +56,7 @@ struct SelBox {
 // Dynamic shared memory layout (bytes).
 constexpr uint32_t kSelectMaxViews = 32;  // views per select unit, at most
 constexpr uint32_t kHizTailUnits = 3;      // Hi-Z units per CTA held back for the end of the work queue
-constexpr uint32_t kExpandBatch = 8;       // (view, chunk) units per claim of the expansion queue
+constexpr uint32_t kExpandBatch = 8;       // (view, chunk) units per claim of the expansion queue, at most
 static_assert(kSelectMaxViews * 8 <= kBatchThreads, "one thread per (view, mask word) in the write-out");
 constexpr size_t kSmSelViews = 0;                                               // SelView[kBatchMaxViews]
 constexpr size_t kSmSelBox = kSmSelViews + sizeof(SelView) * kBatchMaxViews;    // SelBox[kBatchMaxViews]
@@ -640,24 +640,27 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
     }
     const VgSceneDev& S = P.scene;
     const uint32_t n_units = V * C;
-    // Warps claim batches of kExpandBatch units from a queue; batch b holds the units
-    // b + k * NB (lane k < kExpandBatch), strided so that the heavy consecutive chunks of
+    // Warps claim batches of eb units from a queue; batch b holds the units
+    // b + k * NB (lane k < eb), strided so that the heavy consecutive chunks of
     // a large view spread over many batches, and small enough that warps which drew light
-    // batches draw more of them. A warp flattens its batch's visible lists into one
+    // batches draw more of them: 8 units when every warp then still finds several batches, down to
+    // one for small batches, whose few units would otherwise leave most warps idle (9 views over
+    // 30,000 objects: 1,062 units on 3,552 warps). A warp flattens its batch's visible lists into one
     // sequence: round r gives lane i the entry 32 r + i, so the list and object loads of
     // every unit are in flight together (two round trips per round instead of two per
     // unit). The spans of an entry go to its unit's first span + the spans of the unit's
     // earlier entries: a scan of the span counts within the round, less the scan before
     // the unit's first entry in the round, plus what the unit wrote in earlier rounds
     // (carried by the unit's lane).
-    const uint32_t NB = (n_units + kExpandBatch - 1) / kExpandBatch;
+    const uint32_t eb = min(max(n_units / (gridDim.x * (kBatchThreads / 32)), 1u), kExpandBatch);
+    const uint32_t NB = (n_units + eb - 1) / eb;
     for (;;) {
         uint32_t bq = 0;
         if (lane == 0) bq = atomicAdd(P.expand_work, 1u);
         bq = __shfl_sync(0xffffffffu, bq, 0);
         if (bq >= NB) break;
         const size_t u = bq + (size_t)lane * NB;
-        const bool live = (uint32_t)lane < kExpandBatch && u < n_units;
+        const bool live = (uint32_t)lane < eb && u < n_units;
         const uint32_t vis = live ? ld_cg(P.chunk_vis + u) : 0u;
         if (!__any_sync(0xffffffffu, vis != 0u)) continue;
         const uint32_t v = live ? (uint32_t)(u / C) : 0u, ch = live ? (uint32_t)(u - (size_t)v * C) : 0u;
@@ -724,14 +727,32 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
     }
 }
 
-// The 32 spans of a group (lane = span): meshlet range and packing offsets.
+// ── Groups of the meshlet tests and the emission ─────────────────────────────
+// A group is 32, 16 or 8 consecutive spans of the list (32 >> shift), so it belongs to one view. A
+// warp works through its group's windows one after the other; with few groups per warp that
+// chain, and the rounding of groups over warps, set the time, so small batches take smaller
+// groups: groups are halved while there is not one per warp. 2,880 groups of 32 on 5,920 warps
+// (9 views over 30,000 objects): tests 54 us, 43 as groups of 8, emission 14.8 -> 12.1. With
+// more than one group per warp halving gains nothing (11,895 groups: 72.4 us either way, the
+// emission 19.2 -> 22.3).
+constexpr uint32_t kMaxGroupShift = 2;
+constexpr uint32_t kGroupsPerWarp = 1;
+
+__device__ __forceinline__ uint32_t group_shift(uint32_t spans) {
+    const uint32_t warps = gridDim.x * (kBatchThreads / 32);
+    uint32_t s = 0;
+    while (s < kMaxGroupShift && ((spans >> 5) << s) < kGroupsPerWarp * warps) ++s;
+    return s;
+}
+
+// The spans of a group (lane = span; none past the group): meshlet range and packing offsets.
 struct GroupSpans {
     uint32_t n, first, inst, lod, off, total, view;
 };
 
-__device__ __forceinline__ GroupSpans load_group(const BatchParams& P, uint32_t g) {
-    const int lane = threadIdx.x & 31;
-    const ActiveSpan s = __ldcg(P.spans + (size_t)g * 32u + lane);
+__device__ __forceinline__ GroupSpans load_group(const BatchParams& P, uint32_t g, uint32_t shift) {
+    const uint32_t lane = threadIdx.x & 31, size = 32u >> shift;
+    const ActiveSpan s = lane < size ? __ldcg(P.spans + (size_t)g * size + lane) : make_uint4(0u, 0u, 0u, 0u);
     GroupSpans r;
     r.n = span_n(s);
     r.first = s.x;
@@ -744,7 +765,7 @@ __device__ __forceinline__ GroupSpans load_group(const BatchParams& P, uint32_t 
     return r;
 }
 
-// ── Phase 4: meshlet tests of every group of 32 spans ────────────────────────
+// ── Phase 4: meshlet tests of every group of spans ───────────────────────────
 // Hi-Z tests of n <= 32 queued candidates of a group: lane i takes entry i, a
 // meshlet position s of the group with the world sphere the frustum test computed;
 // visible ones set bit s of the group's bits.
@@ -757,11 +778,11 @@ __device__ void test_hiz_batch(const CullView& cv, const uint16_t* q, const floa
     if (meshlet_hiz_visible<true>(cv, f3(sp.x, sp.y, sp.z), sp.w)) atomicOr(bits + (s >> 5), 1u << (s & 31u));
 }
 
-// Per group of 32 spans, the warp runs the frustum and cone tests window by window
+// Per group, the warp runs the frustum and cone tests window by window
 // (32 meshlets packed densely across the spans) and queues the meshlets that pass;
 // every 32 queued meshlets take the Hi-Z test together, so that the costly Hi-Z
 // test runs on full warps although about half the meshlets leave earlier.
-__device__ void phase_test(const BatchParams& P, uint32_t groups, char* sm) {
+__device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift, char* sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     CullView& cv = *reinterpret_cast<CullView*>(sm + kSmTestViews + sizeof(CullView) * warp);
     uint32_t* bits = reinterpret_cast<uint32_t*>(sm + kSmTestBits) + warp * kBits;
@@ -781,7 +802,7 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, char* sm) {
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= groups) break;
         g = groups - 1u - g;
-        const GroupSpans gs = load_group(P, g);
+        const GroupSpans gs = load_group(P, g, shift);
         if (gs.view >= P.view_count) continue;  // never true: every span below the group count is written
         if (gs.view != cached_view) {
             const uint4* src = reinterpret_cast<const uint4*>(P.cviews + gs.view);
@@ -845,10 +866,11 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, char* sm) {
         for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
         if (lane == 0) P.group_counts[g] = count;
         if (count)
-            for (uint32_t k = lane; k < windows; k += 32) P.group_bits[(size_t)g * kWindowsPerWarp + k] = bits[k];
-        if (P.span_vis) {
+            for (uint32_t k = lane; k < windows; k += 32)
+                P.group_bits[(size_t)g * (kWindowsPerWarp >> shift) + k] = bits[k];
+        if (P.span_vis && (uint32_t)lane < (32u >> shift)) {
             const uint2 w = bit_field64(bits, gs.off, gs.n);
-            reinterpret_cast<uint2*>(P.span_vis)[(size_t)g * 32u + lane] = w;
+            reinterpret_cast<uint2*>(P.span_vis)[(size_t)g * (32u >> shift) + lane] = w;
         }
         __syncwarp();
     }
@@ -866,24 +888,24 @@ __device__ __forceinline__ uint32_t cnt_of(uint32_t lo, uint32_t hi) {
 // ── Phase 6: emission, per view, in the canonical order ───────────────────────
 // The loads of one group that do not depend on another group's data: its scan offset,
 // lane k's span and lane k's two window ballots (windows k and k + 32; the ballot row has
-// kWindowsPerWarp entries, read whole and masked to the group's windows later).
+// kWindowsPerWarp >> shift entries, read whole and masked to the group's windows later).
 struct EmitLoads {
     uint32_t goff, bits_lo, bits_hi;
     ActiveSpan span;
 };
 
-__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t g) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t g, uint32_t shift) {
+    const uint32_t lane = threadIdx.x & 31, size = 32u >> shift, windows = kWindowsPerWarp >> shift;
     EmitLoads e;
     e.goff = ld_cg(P.group_offs + g);
-    e.span = __ldcg(P.spans + (size_t)g * 32u + lane);
-    const uint32_t* gbits = P.group_bits + (size_t)g * kWindowsPerWarp;
-    e.bits_lo = ld_cg(gbits + lane);
-    e.bits_hi = ld_cg(gbits + lane + 32);
+    e.span = lane < size ? __ldcg(P.spans + (size_t)g * size + lane) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t* gbits = P.group_bits + (size_t)g * windows;
+    e.bits_lo = lane < windows ? ld_cg(gbits + lane) : 0u;
+    e.bits_hi = lane + 32u < windows ? ld_cg(gbits + lane + 32) : 0u;
     return e;
 }
 
-__device__ void phase_emit(const BatchParams& P, uint32_t groups) {
+__device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const VgSceneDev& S = P.scene;
     const uint32_t gw = blockIdx.x * (kBatchThreads / 32) + warp, GW = gridDim.x * (kBatchThreads / 32);
@@ -898,13 +920,13 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups) {
         if (!mask) continue;
         uint32_t g = gw + (k0 + (__ffs(mask) - 1)) * GW;
         mask &= mask - 1u;
-        EmitLoads cur = emit_loads(P, g);
+        EmitLoads cur = emit_loads(P, g, shift);
         for (;;) {
             const bool more = mask != 0u;
             const uint32_t g_next = more ? gw + (k0 + (__ffs(mask) - 1)) * GW : 0u;
             mask &= mask - 1u;
             EmitLoads nxt{};
-            if (more) nxt = emit_loads(P, g_next);
+            if (more) nxt = emit_loads(P, g_next, shift);
             // The current group: its spans' packing offsets, then its view's table entry.
             GroupSpans gs;
             gs.n = span_n(cur.span);
@@ -917,7 +939,7 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups) {
             gs.total = __shfl_sync(0xffffffffu, inc, 31);
             if (gs.view < P.view_count) {
                 const BatchViewDev& V = P.views[gs.view];
-                const uint32_t first_group = ld_cg(P.view_span_start + gs.view) >> 5;
+                const uint32_t first_group = ld_cg(P.view_span_start + gs.view) >> (5u - shift);
                 const uint32_t cap = V.capacity;
                 HelioDrawIndexedIndirectArgs* indirect = V.indirect;
                 HelioGpuVgDraw* draws = V.draws;
@@ -1140,14 +1162,14 @@ __global__ void __launch_bounds__(kBatchThreads, 5) batch_cull_kernel(BatchParam
     if (ld_cg(P.error) & kBatchErrTimeout) return;
     stamp(P, 4);
     const uint32_t total_spans = min(ld_cg(P.view_span_start + P.view_count), P.span_capacity);
-    const uint32_t groups = total_spans >> 5;
-    phase_test(P, groups, sm);
+    const uint32_t shift = group_shift(total_spans), groups = total_spans >> (5u - shift);
+    phase_test(P, groups, shift, sm);
     if (!grid_sync(P)) return;
     stamp(P, 5);
 
     if (!grid_exclusive_scan(P, P.group_counts, P.group_offs, groups, s_tmp)) return;
     stamp(P, 6);
-    phase_emit(P, groups);
+    phase_emit(P, groups, shift);
     // End of the launch: the latest block end (no barrier needed).
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -71,8 +71,8 @@ struct BatchParams {
     uint32_t* view_span_start;  // [view_count + 1] first span of each view (views padded to 32)
     ActiveSpan* spans;        // [span_capacity]
     uint32_t span_capacity;   // multiple of 32
-    uint32_t* group_counts;   // [span_capacity / 32] visible meshlets per group of 32 spans
-    uint32_t* group_offs;     // [span_capacity / 32 + 1]
+    uint32_t* group_counts;   // [span_capacity / 8] visible meshlets per group of 32, 16 or 8 spans
+    uint32_t* group_offs;     // [span_capacity / 8 + 1]
     uint32_t* group_bits;     // [span_capacity / 32 * kWindowsPerWarp] window ballots
     uint32_t* span_vis;       // [span_capacity * 2] per-span visibility words, or null
     unsigned long long* phase_ns;  // [kBatchPhaseStamps] %globaltimer at launch and after each phase

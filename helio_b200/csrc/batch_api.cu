@@ -204,8 +204,8 @@ int32_t plan_batch(const helio_batch_config& cfg, const helio_vg_scene* sc, uint
     p.need[kBufSegTotals] = (size_t)std::max(p.grid, helio::batch_cull_max_grid()) * 4;
     p.need[kBufViewSpanStart] = (size_t)(n + 1) * 4;
     p.need[kBufSpans] = (size_t)p.span_capacity * sizeof(helio::ActiveSpan);
-    p.need[kBufGroupCounts] = (groups + 1) * 4;
-    p.need[kBufGroupOffs] = (groups + 1) * 4;
+    p.need[kBufGroupCounts] = (groups * 4 + 1) * 4;  // groups of 8 spans at the least
+    p.need[kBufGroupOffs] = (groups * 4 + 1) * 4;
     p.need[kBufGroupBits] = (groups + 1) * helio::kWindowsPerWarp * 4;
     p.need[kBufSpanVis] = (cfg.flags & HELIO_BATCH_SPAN_VISIBILITY) ? (size_t)p.span_capacity * 8 : 0;
     for (size_t& x : p.need) x = x ? x : 16;  // DevBuf::ensure allocates at least 16 bytes

@@ -170,3 +170,19 @@ def test_pack_draws_unit_edges(cuda, capacity):
     np.testing.assert_array_equal(u32(ind[:n]), np.concatenate([p["indirect"] for p in per])[:n])
     np.testing.assert_array_equal(u32(drw[:n]), np.concatenate([p["draws"] for p in per])[:n])
     assert (ind[n:].cpu().numpy() == -1).all() and (drw[n:].cpu().numpy() == -1).all()
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_batch_group_sizes_match_oracle(cuda, shift):
+    """Groups of 32, 16 and 8 spans: a meshlet-test grid with fewer warps than groups of 32, with
+    as many as one and a half times them, and with six times as many."""
+    from helio_b200 import scene as S
+
+    w = S.config(3, scale=0.05)
+    views = w.views[:1] + w.views[1:5] + w.views[21:30]
+    b, _, _ = run_batch(w.scene, views)
+    groups = int(u32(b.spans()["view_span_start"])[-1]) // 32
+    warps = {0: groups // 2, 1: groups * 3 // 2, 2: groups * 6}[shift]
+    ctas = max(1, warps // 8)
+    assert {0: groups >= 8 * ctas, 1: groups < 8 * ctas <= 2 * groups, 2: 2 * groups < 8 * ctas}[shift]
+    _check_batch(w, views, cull_ctas=ctas)
