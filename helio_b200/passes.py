@@ -82,10 +82,12 @@ def device_view(ptr: int, shape, dtype: str = "<i4", strides=None) -> torch.Tens
     return torch.as_tensor(_CudaArray(ptr, shape, dtype, strides), device="cuda")
 
 
-def _stream_ptr(stream) -> C.c_void_p:
+def _stream_ptr(stream) -> int:
+    # The raw handle: building torch's Stream object takes 3 us, as long as the launch of a pass
+    # (4,099 draws through both instance passes: 20.4 -> 14.2 us a pass with the handle alone).
     if stream is None:
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 def _ptr(t) -> C.c_void_p:
