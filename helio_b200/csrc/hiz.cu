@@ -31,7 +31,6 @@ namespace {
 __global__ void __launch_bounds__(kHizBlockThreads, 8)
     hiz_build_kernel(const __grid_constant__ HizJob J, uint32_t* ticket) {
     __shared__ __align__(16) HizJob s_J;
-    pdl_launch_dependents();
     for (uint32_t i = threadIdx.x; i < sizeof(HizJob) / 4u; i += kHizBlockThreads)
         reinterpret_cast<uint32_t*>(&s_J)[i] = reinterpret_cast<const uint32_t*>(&J)[i];
     __syncthreads();
@@ -71,7 +70,6 @@ __global__ void __launch_bounds__(kHizTmaThreads, kHizTmaCtasPerSm)
         tma_load_2d(s_stage + s * (kHizTile * kHizTile), &src, &s_full[s], (int32_t)(tx * kHizTile),
                     (int32_t)(ty * kHizTile));
     };
-    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < kHizStages; ++s) mbar_init(&s_full[s], 1u);
         mbar_init_fence();

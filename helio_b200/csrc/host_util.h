@@ -63,9 +63,9 @@ struct DevBuf {
     }
 };
 
-// Launches `kernel` with programmatic stream serialization: its CTAs may be scheduled while the
-// stream's previous kernel finishes, and wait in pdl_wait before their first global access,
-// which hides a launch gap.
+// Launches `kernel` with programmatic stream serialization: its CTAs are scheduled as those of the
+// stream's previous kernel end, and wait in pdl_wait before their first global access, which
+// hides a launch gap.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t stream,
                                 A&&... args) {

@@ -232,7 +232,6 @@ __global__ void __launch_bounds__(256, 4) instance_cull_kernel(const __grid_cons
     __shared__ HizView s_hiz;
     __shared__ uint32_t s_stats[8];
     if (threadIdx.x < 8) s_stats[threadIdx.x] = 0u;
-    pdl_launch_dependents();
     if (kOcclusion)
         for (uint32_t k = threadIdx.x; k < sizeof(HizView) / 4; k += blockDim.x)
             reinterpret_cast<uint32_t*>(&s_hiz)[k] = reinterpret_cast<const uint32_t*>(&P.hiz)[k];

@@ -49,7 +49,6 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
     __shared__ ShadowSmem s;
     __shared__ uint32_t s_total[kShadowChunk];  // this CTA's visible draws per face
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, x = blockIdx.x, c = blockIdx.y;
-    pdl_launch_dependents();
     pdl_wait();
     float4 sphere[kMaxRounds];
     uint32_t live_mask[kMaxRounds];
@@ -119,14 +118,12 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
 // Larger lists: test and place over (block of 256 draws) x (chunks y, y + gridDim.y, ...).
 __global__ void __launch_bounds__(kThreads) shadow_test_kernel(const __grid_constant__ ShadowDev D) {
     __shared__ ShadowSmem s;
-    pdl_launch_dependents();
     pdl_wait();
     shadow_test_block(D, blockIdx.x, blockIdx.y, gridDim.y, s);
 }
 
 __global__ void __launch_bounds__(kThreads) shadow_scan_kernel(const __grid_constant__ ShadowDev D) {
     __shared__ ShadowSmem s;
-    pdl_launch_dependents();
     pdl_wait();
     shadow_scan_chunk(D, blockIdx.x, s);
 }
@@ -134,7 +131,6 @@ __global__ void __launch_bounds__(kThreads) shadow_scan_kernel(const __grid_cons
 template <bool kScanned>
 __global__ void __launch_bounds__(kThreads) shadow_place_kernel(const __grid_constant__ ShadowDev D) {
     __shared__ ShadowSmem s;
-    pdl_launch_dependents();
     pdl_wait();
     if (blockIdx.x == 0 && blockIdx.y == 0) shadow_clear_clean(D);
     shadow_place_block<kScanned>(D, blockIdx.x, blockIdx.y, gridDim.y, s);

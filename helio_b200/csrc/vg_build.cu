@@ -102,7 +102,6 @@ __global__ void __launch_bounds__(kThreads) first_ref_kernel(const __grid_consta
     extern __shared__ uint32_t s_first[];
     __shared__ unsigned long long s_sum[3];
     __shared__ uint32_t s_last;
-    helio::pdl_launch_dependents();
     const bool local = in.mesh_count <= kSharedMeshes;
     if (local)
         for (uint32_t k = threadIdx.x; k < in.mesh_count; k += kThreads) s_first[k] = 0u;
@@ -164,7 +163,6 @@ __global__ void __launch_bounds__(kThreads) first_ref_kernel(const __grid_consta
 
 __global__ void __launch_bounds__(kThreads) fold_kernel(const __grid_constant__ helio_vg_build_inputs in,
                                                         const __grid_constant__ BuildWork w) {
-    helio::pdl_launch_dependents();
     helio::pdl_wait();
     const uint32_t m = blockIdx.x * kThreads + threadIdx.x;
     if (m < in.mesh_count) fold_mesh(in, w, m);
@@ -235,7 +233,6 @@ constexpr uint32_t kScanThreads = 512;
 __global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(const __grid_constant__ BuildWork w,
                                                                    uint64_t* block_base, uint64_t* totals) {
     __shared__ uint64_t s[kVals][kScanThreads / 32];
-    helio::pdl_launch_dependents();
     helio::pdl_wait();
     uint64_t carry[kVals] = {0, 0, 0, 0, 0};
     for (uint32_t b0 = 0; b0 < w.blocks; b0 += kScanThreads) {
@@ -292,7 +289,6 @@ __global__ void __launch_bounds__(kThreads, 4) place_kernel(const __grid_constan
     __shared__ uint64_t s_sums[2 * kVals][kThreads / 32];
     __shared__ uint32_t s_scan[4][kSub * kThreads / 32];  // per (value, round and warp)
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    helio::pdl_launch_dependents();
     helio::pdl_wait();
     // The slots' meshes are on their way while the sums are taken.
     const uint64_t o0 = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x;
@@ -502,7 +498,6 @@ __device__ __forceinline__ void copy_descriptors(const helio_vg_build_inputs& in
 __global__ void __launch_bounds__(kThreads) outputs_kernel(const __grid_constant__ helio_vg_build_inputs in,
                                                            const __grid_constant__ BuildOut out, uint32_t mesh_ctas,
                                                            uint32_t* error) {
-    helio::pdl_launch_dependents();
     helio::pdl_wait();
     if (!outputs_fit(out, __ldcg(out.totals), __ldcg(out.totals + 1), __ldcg(out.totals + 2), __ldcg(out.totals + 4)))
         return;  // uniform over the grid

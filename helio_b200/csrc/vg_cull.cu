@@ -140,7 +140,6 @@ template <bool kTotals>
 __global__ void __launch_bounds__(kUpdateThreads, 4)
     scene_update_kernel(const __grid_constant__ SceneUpdate U, uint32_t object_blocks, uint32_t item_blocks) {
     const VgSceneDev& S = U.scene;
-    pdl_launch_dependents();
     pdl_wait();
     if (blockIdx.x >= object_blocks) {
         const uint32_t b = blockIdx.x - object_blocks;
@@ -458,7 +457,6 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const VgSceneDev& S = P.scene;
-    pdl_launch_dependents();
     for (uint32_t k = tid; k < kMaxWindows + 2; k += kThreads) s_bits[k] = 0u;
     for (uint32_t k = tid; k < kMaxWindows; k += kThreads) s_it.heads[k] = 0u;
     pdl_wait();  // the kernel before may be the Hi-Z build, or the previous launch of this one
