@@ -8,7 +8,7 @@
 //
 // Layout and scheduling (B200 design, not a translation of the WGSL dispatches):
 //   * meshlet descriptors are re-laid once per upload into four 16-byte streams;
-//   * one launch does the whole view. A tile CTA takes up to 256 consecutive work items, one
+//   * one launch does the whole view. A tile CTA takes up to 512 consecutive work items, two
 //     per thread, and selects their objects itself (an object's few items repeat its select,
 //     from L2, which costs less than a launch and a round trip of records in between); it then
 //     packs the items' active meshlets densely into 32-lane windows shared out over its warps,
@@ -293,26 +293,40 @@ __device__ __forceinline__ Selected select_object(const VgSceneDev& S, const Cul
     return r;
 }
 
-// Object CTA: the select's outputs of 256 objects. The CTA that finishes last (an atomic count)
-// publishes the histogram and leaves the accumulators at zero for the next launch.
+// Object CTA: the select's outputs of kObjectBlock objects. The CTA that finishes last (an atomic
+// count) publishes the histogram and leaves the accumulators at zero for the next launch.
+constexpr uint32_t kObjectRounds = 4;
+constexpr uint32_t kObjectBlock = kObjectRounds * kCullWarps * 32u;
+
 __device__ void object_block(const VgFrameParams& P, const CullView& view, uint32_t block, uint32_t blocks,
                              uint32_t* s_hist, uint32_t* s_flag) {
     const VgSceneDev& S = P.scene;
-    const uint32_t i = block * (kCullWarps * 32u) + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t i0 = block * kObjectBlock + threadIdx.x, lane = threadIdx.x & 31u;
     if (threadIdx.x < 9) s_hist[threadIdx.x] = 0u;
-    Selected r{0u, 0u, 0u};
-    if (i < S.object_count) {
-        r = select_object(S, view, i);
-        S.objects[i].reserved = r.sel;
+    Selected r[kObjectRounds];
+#pragma unroll
+    for (uint32_t k = 0; k < kObjectRounds; ++k) {
+        const uint32_t i = i0 + k * kCullWarps * 32u;
+        r[k] = Selected{0u, 0u, 0u};
+        if (i < S.object_count) {
+            r[k] = select_object(S, view, i);
+            S.objects[i].reserved = r[k].sel;
+        }
     }
     if (P.counter_count < 11u) return;  // uniform over the grid
     __syncthreads();
+    uint32_t mx = 0;
 #pragma unroll
-    for (uint32_t l = 0; l < 8; ++l) {
-        const uint32_t n = __popc(__ballot_sync(0xffffffffu, r.sel == l + 1u));
-        if (lane == 0 && n) atomicAdd(s_hist + l, n);
+    for (uint32_t k = 0; k < kObjectRounds; ++k) {
+        mx = max(mx, r[k].sel ? r[k].lod_count - 1u : 0u);
+        if (!__any_sync(0xffffffffu, r[k].sel != 0u)) continue;
+#pragma unroll
+        for (uint32_t l = 0; l < 8; ++l) {
+            const uint32_t n = __popc(__ballot_sync(0xffffffffu, r[k].sel == l + 1u));
+            if (lane == 0 && n) atomicAdd(s_hist + l, n);
+        }
     }
-    const uint32_t mx = __reduce_max_sync(0xffffffffu, r.sel ? r.lod_count - 1u : 0u);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0 && mx) atomicMax(s_hist + 8, mx);
     __syncthreads();
     uint32_t* hist = P.state + kVgHist;
@@ -335,7 +349,11 @@ __device__ void object_block(const VgFrameParams& P, const CullView& view, uint3
 
 constexpr uint32_t kThreads = kCullWarps * 32u;
 constexpr uint32_t kMaxWindows = kMaxTileItems * HELIO_VG_MESHLETS_PER_WORK_ITEM / 32u;  // of a tile
-static_assert(kMaxTileItems <= kThreads && kMaxWindows == 2u * kThreads, "one item and two windows per thread");
+constexpr uint32_t kItemRounds = kMaxTileItems / kThreads;  // items per thread
+constexpr uint32_t kThreadWindows = kMaxWindows / kThreads;  // windows per thread, counted after the tests
+static_assert(kItemRounds == 2u && kThreadWindows * kThreads == kMaxWindows, "the tile's rounds");
+// A packed position and a rank share a word (rank << 16 | position).
+static_assert(kMaxTileItems * HELIO_VG_MESHLETS_PER_WORK_ITEM < (1u << 16) && kMaxTileItems < (1u << 16), "packed scan");
 
 // Exclusive scan over the CTA; `total` gets the CTA's sum. s: kCullWarps words.
 __device__ __forceinline__ uint32_t tile_scan(uint32_t x, uint32_t* s, uint32_t& total) {
@@ -460,7 +478,9 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     for (uint32_t k = tid; k < kMaxWindows + 2; k += kThreads) s_bits[k] = 0u;
     for (uint32_t k = tid; k < kMaxWindows; k += kThreads) s_it.heads[k] = 0u;
     pdl_wait();  // the kernel before may be the Hi-Z build, or the previous launch of this one
-    const bool object_cta = blockIdx.x >= P.num_tiles;
+    // The object CTAs come first: they are short, and the tiles beyond the first wave start behind them.
+    const uint32_t object_ctas = gridDim.x - P.num_tiles;
+    const bool object_cta = blockIdx.x < object_ctas;
     if (warp == 1) view_setup_warp(P.setup, s_view);
     if (tid == 0 && !object_cta) {
         uint32_t epoch, ticket;
@@ -475,44 +495,52 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     }
     __syncthreads();
     if (object_cta) {
-        object_block(P, s_view, blockIdx.x - P.num_tiles, gridDim.x - P.num_tiles, s_it.off, s_tmp);
+        object_block(P, s_view, blockIdx.x, object_ctas, s_it.off, s_tmp);
         return;
     }
     const uint32_t tile = s_tile, epoch = s_epoch;
 
-    // The tile's items, one per thread: the object's selected LOD and the item's share of it.
-    const uint32_t w_idx = tile * P.tile_items + tid;
-    const bool mine = tid < P.tile_items && w_idx < S.work_item_count;
-    uint32_t n = 0, first = 0, inst = 0, lod = 0;
-    if (mine) {
-        const uint2 it = __ldg(reinterpret_cast<const uint2*>(S.items + w_idx));  // object, local meshlet base
-        if (it.x < S.object_count) {
-            const HelioGpuVgObject* o = S.objects + it.x;
-            const Selected r = select_object(S, s_view, it.x);
-            if (r.sel) {
-                const uint32_t count = __ldg(&o->lod_meshlet_counts[r.sel - 1u]);
-                if (it.y < count) {
-                    n = min(64u, count - it.y);
-                    first = __ldg(&o->lod_first_meshlets[r.sel - 1u]) + it.y;
-                    inst = r.instance;
-                    lod = r.sel - 1u;
-                }
-            }
+    // The tile's items, in rounds of one per thread: the object's selected LOD and the item's share
+    // of it.
+    const uint32_t w0 = tile * P.tile_items + tid;
+    uint32_t n[kItemRounds], first[kItemRounds], inst[kItemRounds], lod[kItemRounds], off[kItemRounds];
+#pragma unroll
+    for (uint32_t r = 0; r < kItemRounds; ++r) {
+        n[r] = first[r] = inst[r] = lod[r] = 0u;
+        if (r * kThreads + tid >= P.tile_items || w0 + r * kThreads >= S.work_item_count) continue;
+        const uint2 it = __ldg(reinterpret_cast<const uint2*>(S.items + w0 + r * kThreads));  // object, local meshlet base
+        if (it.x >= S.object_count) continue;
+        const HelioGpuVgObject* o = S.objects + it.x;
+        const Selected sel = select_object(S, s_view, it.x);
+        if (!sel.sel) continue;
+        const uint32_t count = __ldg(&o->lod_meshlet_counts[sel.sel - 1u]);
+        if (it.y >= count) continue;
+        n[r] = min(64u, count - it.y);
+        first[r] = __ldg(&o->lod_first_meshlets[sel.sel - 1u]) + it.y;
+        inst[r] = sel.instance;
+        lod[r] = sel.sel - 1u;
+    }
+    // Packed positions and ranks, a scan per round.
+    uint32_t total = 0, ranks = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < kItemRounds; ++r) {
+        if (r * kThreads >= P.tile_items) break;  // uniform
+        uint32_t sums;
+        const uint32_t ex = tile_scan(n[r] ? (1u << 16) | n[r] : 0u, s_tmp, sums);
+        off[r] = total + (ex & 0xFFFFu);
+        if (n[r]) {
+            const uint32_t rank = ranks + (ex >> 16);
+            s_it.off[rank] = off[r];
+            s_it.first[rank] = first[r];
+            s_it.inst[rank] = inst[r];
+            s_it.lod[rank] = (uint8_t)lod[r];
+            atomicOr(s_it.heads + (off[r] >> 5), 1u << (off[r] & 31u));
+            for (uint32_t w = (off[r] + 31u) >> 5; 32u * w < off[r] + n[r]; ++w) s_it.owner[w] = (uint16_t)rank;
         }
+        total += sums & 0xFFFFu;
+        ranks += sums >> 16;
     }
-    // Packed positions and ranks in one scan (at most 2^14 positions, 2^8 ranks).
-    uint32_t sums;
-    const uint32_t ex = tile_scan(n ? (1u << 16) | n : 0u, s_tmp, sums);
-    const uint32_t off = ex & 0xFFFFu, total = sums & 0xFFFFu, windows = (total + 31u) >> 5;
-    if (n) {
-        const uint32_t rank = ex >> 16;
-        s_it.off[rank] = off;
-        s_it.first[rank] = first;
-        s_it.inst[rank] = inst;
-        s_it.lod[rank] = (uint8_t)lod;
-        atomicOr(s_it.heads + (off >> 5), 1u << (off & 31u));
-        for (uint32_t w = (off + 31u) >> 5; 32u * w < off + n; ++w) s_it.owner[w] = (uint16_t)rank;
-    }
+    const uint32_t windows = (total + 31u) >> 5;
     __syncthreads();
 
     for (uint32_t w = warp; w < windows; w += kCullWarps) {
@@ -537,14 +565,25 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     // Visible meshlets before each window, and of the tile.
     uint32_t count;
     {
-        const uint32_t c0 = __popc(s_bits[2u * tid]), c1 = __popc(s_bits[2u * tid + 1u]);
-        const uint32_t before = tile_scan(c0 + c1, s_tmp, count);
-        s_pre[2u * tid] = before;
-        s_pre[2u * tid + 1u] = before + c0;
+        uint32_t c[kThreadWindows], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kThreadWindows; ++k) {
+            c[k] = __popc(s_bits[kThreadWindows * tid + k]);
+            sum += c[k];
+        }
+        uint32_t before = tile_scan(sum, s_tmp, count);
+#pragma unroll
+        for (uint32_t k = 0; k < kThreadWindows; ++k) {
+            s_pre[kThreadWindows * tid + k] = before;
+            before += c[k];
+        }
     }
     if (tid == 0) st_status(P.status + tile, tile_status(epoch, tile == 0u ? kTilePrefix : kTileSum, count));
     // Per-work-item visibility words: bits [off, off + n) of the tile's window bits.
-    if (mine) reinterpret_cast<uint2*>(P.visibility)[w_idx] = bit_field64(s_bits, off, n);
+#pragma unroll
+    for (uint32_t r = 0; r < kItemRounds; ++r)
+        if (r * kThreads + tid < P.tile_items && w0 + r * kThreads < S.work_item_count)
+            reinterpret_cast<uint2*>(P.visibility)[w0 + r * kThreads] = bit_field64(s_bits, off[r], n[r]);
     const bool last = tile == P.num_tiles - 1u;
     if (count == 0u && !last) return;  // uniform: nothing to place
 
@@ -564,12 +603,12 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     // Emission, four windows at a time per warp: their draw records are loaded before any is
     // written. (tile_look_back ended with s_pre visible to every thread.)
     __syncthreads();
-    for (uint32_t w0 = warp; w0 < windows; w0 += 4u * kCullWarps) {
+    for (uint32_t wb = warp; wb < windows; wb += 4u * kCullWarps) {
         uint4 d[4];
         uint32_t b[4], mi[4], k[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t w = w0 + (uint32_t)q * kCullWarps;
+            const uint32_t w = wb + (uint32_t)q * kCullWarps;
             b[q] = w < windows ? s_bits[w] : 0u;
             if ((b[q] >> lane) & 1u) {
                 k[q] = item_at(s_it, w);
@@ -580,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             if (!((b[q] >> lane) & 1u)) continue;
-            const uint32_t w = w0 + (uint32_t)q * kCullWarps;
+            const uint32_t w = wb + (uint32_t)q * kCullWarps;
             const uint32_t slot = base + s_pre[w] + __popc(b[q] & ((1u << lane) - 1u));
             if (slot >= P.capacity) continue;
             uint32_t* o = reinterpret_cast<uint32_t*>(P.indirect + slot);
@@ -624,7 +663,7 @@ cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t grid = p.num_tiles + (uint32_t)(((uint64_t)p.scene.object_count + kThreads - 1) / kThreads);
+    const uint32_t grid = p.num_tiles + (uint32_t)(((uint64_t)p.scene.object_count + kObjectBlock - 1) / kObjectBlock);
     const bool wide = grid > 4u * (uint32_t)std::max(sms, 1);
     helio_launch_begin("vg_frame", stream);
     const cudaError_t e = launch_after(wide ? vg_frame_kernel<true> : vg_frame_kernel<false>, grid, kThreads, 0, stream, p);

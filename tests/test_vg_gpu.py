@@ -171,9 +171,10 @@ def test_vg_empty_scene_is_a_no_op(cuda):
 
 
 @pytest.mark.parametrize("objects,meshlets", [(1, 1), (7, 64), (8, 65), (9, 200), (443, 1), (445, 33), (3553, 64),
-                                              (7105, 20), (56833, 3), (60000, 100), (130000, 1)])
+                                              (7105, 20), (56833, 3), (60000, 100), (130000, 1), (1183, 9),
+                                              (1185, 64), (37889, 2), (75775, 1), (75777, 65)])
 def test_frame_tiles_match_oracle(cuda, objects, meshlets):
-    """Scenes around the steps of the tile size (8 to 256 work items) and of the look-back
+    """Scenes around the steps of the tile size (8 to 512 work items) and of the look-back
     (one tile, a few, more than one window of 256 tiles), executed twice."""
     from helio_b200 import scene as S
     from oracle import oracle as O
