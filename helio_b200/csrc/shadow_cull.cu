@@ -10,11 +10,10 @@
 // defined; here it is the draw order, and face_counts[f] counts all of them as the
 // reference's counter does (only the first 4096 are stored).
 //
-// Stages and layout: shadow_device.cuh. Up to 8,192 draws one launch does everything, a cluster
+// Stages and layout: shadow_device.cuh. Up to 2,048 draws one launch does everything, a cluster
 // of 8 CTAs per chunk of 32 dirty faces; beyond that a test and a place launch, with a scan
 // between them from 1,024 blocks of 256 draws on. Against three launches in every case: 2,000
-// draws x 10 dirty faces 16.4 -> 10.3 us a pass (6.7 us of it on the device; the host's calls are
-// the rest), 100,000 x 44 35.0 -> 20.4 us.
+// draws x 10 dirty faces 16.4 -> 6.7 us a pass, 4,188 x 19 18.4 -> 8.7, 100,000 x 44 35.5 -> 20.8.
 
 #include <algorithm>
 #include <new>
@@ -34,62 +33,46 @@ constexpr uint32_t kWarps = kShadowWarps;
 constexpr uint32_t kFaces = kShadowFaces;
 constexpr uint32_t kChunks = kShadowChunks;
 
-// Small draw lists in one launch: cluster y is chunk y, its CTA x takes the draws
-// [x * rounds * 256, ...), `rounds` per thread, and learns the counts of the CTAs before it
-// through distributed shared memory, so that nothing but the results touches global memory.
-// Bound by latency: the dirty list, the draws' instances and spheres, the planes and one cluster
-// barrier.
+// Small draw lists in one launch: cluster y is chunk y, its CTA x takes the draws [256 x, ...), one
+// per thread, and learns the counts of the CTAs before it through distributed shared memory, so
+// that nothing but the results touches global memory. Bound by latency: the dirty list, the draws'
+// instances and spheres, the planes and one cluster barrier. Up to 2,048 draws it takes 5.5 to 9.2
+// us on the device (10 to 60 dirty faces), the two launches below 6.9 to 10.2; with several draws
+// per thread it fell behind them (3,000 draws x 19 faces: 12.5 against 8.9 us).
 constexpr uint32_t kClusterCtas = 8;
-constexpr uint32_t kMaxRounds = 4;
-constexpr uint32_t kClusterDraws = kClusterCtas * kMaxRounds * kThreads;
+constexpr uint32_t kClusterDraws = kClusterCtas * kThreads;
 
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
-    shadow_cluster_kernel(const __grid_constant__ ShadowDev D, uint32_t rounds) {
+    shadow_cluster_kernel(const __grid_constant__ ShadowDev D) {
     namespace cg = cooperative_groups;
     __shared__ ShadowSmem s;
-    __shared__ uint32_t s_total[kShadowChunk];  // this CTA's visible draws per face
+    __shared__ uint32_t s_cnt[kWarps][kShadowChunk];  // visible draws per (warp, face)
+    __shared__ uint32_t s_total[kShadowChunk];        // this CTA's visible draws per face
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, x = blockIdx.x, c = blockIdx.y;
     pdl_wait();
-    float4 sphere[kMaxRounds];
-    uint32_t live_mask[kMaxRounds];
-#pragma unroll
-    for (uint32_t k = 0; k < kMaxRounds; ++k) {  // loaded while the dirty faces are listed
-        bool live = false;
-        if (k < rounds) sphere[k] = shadow_draw_sphere(D, (x * rounds + k) * kThreads + threadIdx.x, live);
-        live_mask[k] = __ballot_sync(0xffffffffu, live);
-    }
+    const uint32_t d = x * kThreads + threadIdx.x;
+    bool live;  // loaded while the dirty faces are listed
+    const float4 sphere = shadow_draw_sphere(D, d, live);
+    HelioDrawIndexedIndirectArgs draw{};
+    if (d < D.draw_count) draw = D.src[d];
+    const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
     const uint32_t n_active = shadow_list_dirty(D.face_dirty, s);
     if (x == 0 && c == 0) shadow_clear_clean(D);
     if (c * kShadowChunk >= n_active) return;  // uniform over the cluster
-    const uint32_t nf = min(kShadowChunk, n_active - c * kShadowChunk);
-    const uint32_t width = shadow_width(nf);
+    const uint32_t nf = min(kShadowChunk, n_active - c * kShadowChunk), width = shadow_width(nf);
+    shadow_put_sphere(s.sphere[warp], sphere);
     const ShadowPlanes p = shadow_chunk_planes(D, c * kShadowChunk, nf, width, s);
-    uint32_t word[kMaxRounds], n = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < kMaxRounds; ++k) {
-        word[k] = 0u;
-        if (k >= rounds || live_mask[k] == 0u) continue;  // uniform over the warp
-        __syncwarp();
-        shadow_put_sphere(s.sphere[warp], sphere[k]);
-        __syncwarp();
-        const uint32_t all = shadow_test_word(p, s.sphere[warp], width) & live_mask[k];
-        word[k] = lane < nf ? all : 0u;
-        n += __popc(word[k]);
-    }
-    // The counts per (round, warp): the draw order is round by round within a CTA.
-    __shared__ uint32_t s_cnt[kMaxRounds][kWarps][kShadowChunk];
-#pragma unroll
-    for (uint32_t k = 0; k < kMaxRounds; ++k) s_cnt[k][warp][lane] = __popc(word[k]);
+    uint32_t word = 0u;
+    if (live_mask) word = shadow_test_word(p, s.sphere[warp], width) & live_mask;  // uniform over the warp
+    if (lane >= nf) word = 0u;
+    s_cnt[warp][lane] = __popc(word);
     __syncthreads();
-    if (warp == 0) {
-        uint32_t total = 0;
-        for (uint32_t k = 0; k < rounds; ++k)
-            for (uint32_t w = 0; w < kWarps; ++w) total += s_cnt[k][w][lane];
-        s_total[lane] = total;
-    }
+    uint32_t at = 0;
+    for (uint32_t w = 0; w < warp; ++w) at += s_cnt[w][lane];
+    if (warp == kWarps - 1) s_total[lane] = at + __popc(word);
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    uint32_t at = 0, all = 0;
+    uint32_t all = 0;
     for (uint32_t r = 0; r < kClusterCtas; ++r) {
         const uint32_t t = *cluster.map_shared_rank(s_total + lane, r);
         if (r < x) at += t;
@@ -98,21 +81,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
     cluster.sync();  // no CTA leaves while another reads its totals
     const uint32_t face = lane < nf ? s.active[c * kShadowChunk + lane] : 0u;
     if (x == 0 && warp == 0 && lane < nf) D.face_counts[face] = all;
-#pragma unroll
-    for (uint32_t k = 0; k < kMaxRounds; ++k) {
-        if (k >= rounds) break;
-        uint32_t a = at;
-        for (uint32_t w = 0; w < kWarps; ++w) {
-            const uint32_t t = s_cnt[k][w][lane];
-            if (w < warp) a += t;
-            at += t;
-        }
-        if (!__any_sync(0xffffffffu, word[k] != 0u)) continue;
-        const uint32_t d = (x * rounds + k) * kThreads + threadIdx.x;
-        HelioDrawIndexedIndirectArgs draw{};
-        if (d < D.draw_count) draw = D.src[d];
-        shadow_place_words(D, draw, word[k], a, face);
-    }
+    shadow_place_words(D, draw, word, at, face);
 }
 
 // Larger lists: test and place over (block of 256 draws) x (chunks y, y + gridDim.y, ...).
@@ -142,7 +111,6 @@ constexpr uint32_t kSumBlocks = 1024;
 
 cudaError_t launch_shadow(const ShadowDev& D, cudaStream_t s) {
     if (D.draw_count <= kClusterDraws) {
-        const uint32_t rounds = (D.draw_count + kClusterCtas * kThreads - 1) / (kClusterCtas * kThreads);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kClusterCtas, kChunks);
         cfg.blockDim = dim3(kThreads);
@@ -152,7 +120,7 @@ cudaError_t launch_shadow(const ShadowDev& D, cudaStream_t s) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, shadow_cluster_kernel, D, rounds);
+        return cudaLaunchKernelEx(&cfg, shadow_cluster_kernel, D);
     }
     // One CTA takes all chunks of its draws when the blocks alone fill the device; below that the
     // chunks are shared out, so that a CTA's chain of loads and planes is not repeated per chunk.
