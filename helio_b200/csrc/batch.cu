@@ -80,11 +80,17 @@ constexpr size_t kSmTestBits = kSmTestViews + sizeof(CullView) * 8;      // u32[
 constexpr int kBits = kWindowsPerWarp + 2;
 constexpr size_t kSmTestQueue = kSmTestBits + 8 * kBits * 4;            // u16[8][64]
 constexpr size_t kSmVStart = 0;                                          // u32[kBatchMaxViews + 1]
+// Phases 2 and 3 of a small batch: the chunk offsets in shared memory (local_exclusive_scan).
+constexpr size_t kSmOffs = 1024;                                         // u32[kLocalChunks + 1]
+constexpr uint32_t kLocalChunks = (uint32_t)((kSmSelLod - kSmOffs) / 4) - 1;
+static_assert(kSmVStart + 4 * (kBatchMaxViews + 1) <= kSmOffs, "the view starts lie below the offsets");
 constexpr size_t kSmTestSpheres = ((kSmTestQueue + 8 * 64 * 2) + 15) / 16 * 16;  // float4[8][64]
 // The cull kernel (phases 4..6) has its own, small layout: the test phase's region
 // from offset 0, then the scan scratch.
 constexpr size_t kSm2Misc = kSmTestSpheres + 8 * 64 * 16;  // u32[64]
 constexpr size_t kSm2Total = kSm2Misc + 64 * 4;
+// Phases 5 and 6 of a small batch: the group offsets, in the test phase's region.
+constexpr uint32_t kLocalGroups = (uint32_t)(kSm2Misc / 4) - 1;
 
 __device__ __forceinline__ uint32_t ld_cg(const uint32_t* p) { return __ldcg(p); }
 
@@ -205,6 +211,35 @@ __device__ bool grid_exclusive_scan(const BatchParams& P, const uint32_t* in, ui
     return grid_sync(P);
 }
 
+// The same sums in shared memory (n + 1 words of s_out), by every CTA for itself: no grid barrier
+// after the one that ended the phase of the counts. For counts that fit a CTA's shared memory; at a
+// few thousand, loading them costs each CTA one round trip where the two barriers cost 5 us.
+__device__ void local_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* s_out, uint32_t* s_tmp) {
+    const uint32_t tid = threadIdx.x;
+    constexpr uint32_t kPer = 8;  // counts per thread and round
+    uint32_t base = 0;
+    for (uint32_t t0 = 0; t0 < n; t0 += kPer * kBatchThreads) {
+        uint32_t x[kPer], sum = 0, total;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            const uint32_t i = t0 + tid * kPer + k;
+            x[k] = i < n ? ld_cg(in + i) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) sum += x[k];
+        uint32_t at = base + block_exclusive(sum, s_tmp, total);
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            const uint32_t i = t0 + tid * kPer + k;
+            if (i < n) s_out[i] = at;
+            at += x[k];
+        }
+        base += total;
+    }
+    if (tid == 0) s_out[n] = base;
+    __syncthreads();
+}
+
 // ── Reject box of a view ──────────────────────────────────────────────────────
 // sphere_visible_vg rejects (c, r) when some plane gives fl(d_i) < -r, where d_i =
 // dot(n_i, c) + w_i is evaluated with 4 roundings, so |fl(d_i) - d_i| <= 5u S_i
@@ -228,19 +263,21 @@ __device__ bool grid_exclusive_scan(const BatchParams& P, const uint32_t* in, ui
 // direction of Q is a cross product of two normals (lanes 0..14, both signs) that
 // no plane rejects.
 struct PlaneD {
-    double x, y, z, w;  // normal and offset pushed out by s_i
-    __device__ double norm() const { return sqrt(x * x + y * y + z * z); }
+    double x, y, z, w, len;  // normal, offset pushed out by s_i, length of the normal
     __device__ double at(double px, double py, double pz) const { return x * px + y * py + z * pz + w; }
 };
 
-// Plane i of `pl` (shared memory, so a lane-dependent i costs no local memory) with
-// its offset pushed out by rmax + 2^-20 (cl1 + |w| + rmax).
+// Plane i of `pl` with its offset pushed out by rmax + 2^-20 (cl1 + |w| + rmax).
 __device__ __forceinline__ PlaneD pushed_plane(const Planes& pl, int i, double rmax, double cl1) {
     const float4 p = pl.p[i];
-    return PlaneD{p.x, p.y, p.z, (double)p.w + rmax + 0x1p-20 * (cl1 + fabs((double)p.w) + rmax)};
+    PlaneD q{p.x, p.y, p.z, (double)p.w + rmax + 0x1p-20 * (cl1 + fabs((double)p.w) + rmax), 0.0};
+    q.len = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
+    return q;
 }
 
-__device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, float box[6]) {
+// s_q: six planes of shared memory, one built by each of lanes 0..5 (a double square root apiece,
+// where every use of a length had one of its own).
+__device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, PlaneD* s_q, float box[6]) {
     const int lane = threadIdx.x & 31;
     bool finite = isfinite(rmax_f) && isfinite(cl1_f);
     const double rmax = rmax_f, cl1 = cl1_f;
@@ -250,8 +287,10 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, flo
         finite = finite && isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(p.w);
     }
     auto scale = [&](const PlaneD& q, double x, double y, double z) {
-        return (fabs(x) + fabs(y) + fabs(z)) * q.norm() + fabs(q.w) + 1e-30;
+        return (fabs(x) + fabs(y) + fabs(z)) * q.len + fabs(q.w) + 1e-30;
     };
+    if (lane < 6) s_q[lane] = pushed_plane(pl, lane, rmax, cl1);
+    __syncwarp();
     bool bad = !finite;
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (finite && lane < 20) {
@@ -266,13 +305,12 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, flo
                 c = b + 1;
             }
         }
-        const PlaneD A = pushed_plane(pl, a, rmax, cl1), B = pushed_plane(pl, b, rmax, cl1),
-                     Cc = pushed_plane(pl, c, rmax, cl1);
+        const PlaneD A = s_q[a], B = s_q[b], Cc = s_q[c];
         const double bc[3] = {B.y * Cc.z - B.z * Cc.y, B.z * Cc.x - B.x * Cc.z, B.x * Cc.y - B.y * Cc.x};
         const double ca[3] = {Cc.y * A.z - Cc.z * A.y, Cc.z * A.x - Cc.x * A.z, Cc.x * A.y - Cc.y * A.x};
         const double ab[3] = {A.y * B.z - A.z * B.y, A.z * B.x - A.x * B.z, A.x * B.y - A.y * B.x};
         const double det = A.x * bc[0] + A.y * bc[1] + A.z * bc[2];
-        const double rel = fabs(det) / (A.norm() * B.norm() * Cc.norm() + 1e-300);
+        const double rel = fabs(det) / (A.len * B.len * Cc.len + 1e-300);
         const bool corner = a < 2 && b >= 2 && b < 4 && c >= 4;
         double p[3] = {0.0, 0.0, 0.0};
         bool feasible = false, loose = false;
@@ -283,7 +321,7 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, flo
             loose = feasible;
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
-                const PlaneD q = pushed_plane(pl, j, rmax, cl1);
+                const PlaneD q = s_q[j];
                 const double sl = q.at(p[0], p[1], p[2]), sc = scale(q, p[0], p[1], p[2]);
                 feasible = feasible && sl >= -1e-7 * sc;
                 loose = loose && sl >= -1e-3 * sc;
@@ -301,16 +339,16 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, flo
                 ++a;
                 b = a + 1;
             }
-        const PlaneD A = pushed_plane(pl, a, rmax, cl1), B = pushed_plane(pl, b, rmax, cl1);
+        const PlaneD A = s_q[a], B = s_q[b];
         const double d[3] = {A.y * B.z - A.z * B.y, A.z * B.x - A.x * B.z, A.x * B.y - A.y * B.x};
         const double len = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-        if (len > 1e-12 * A.norm() * B.norm()) {
+        if (len > 1e-12 * A.len * B.len) {
             for (int sgn = -1; sgn <= 1; sgn += 2) {
                 bool ray = true;
 #pragma unroll
                 for (int j = 0; j < 6; ++j) {
-                    const PlaneD q = pushed_plane(pl, j, rmax, cl1);
-                    ray = ray && sgn * (q.x * d[0] + q.y * d[1] + q.z * d[2]) >= -1e-9 * q.norm() * len;
+                    const PlaneD q = s_q[j];
+                    ray = ray && sgn * (q.x * d[0] + q.y * d[1] + q.z * d[2]) >= -1e-9 * q.len * len;
                 }
                 if (ray) bad = true;
             }
@@ -336,38 +374,45 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, flo
 }
 
 // ── Phase 0: view constants ──────────────────────────────────────────────────
+// One warp per view. The constants are put together in shared memory by all lanes and stored
+// as 16-byte words; lane 0 then publishes the view.
 __device__ void phase_setup(const BatchParams& P) {
+    __shared__ CullView s_c;
+    __shared__ PlaneD s_q[6];
+    if (threadIdx.x >= 32) return;
+    const uint32_t lane = threadIdx.x;
     for (uint32_t v = blockIdx.x; v < P.view_count; v += gridDim.x) {
-        if (threadIdx.x >= 32) continue;
-        const BatchViewDev& V = P.views[v];
-        __shared__ Planes s_pl;
-        publish_planes_warp(V.camera.view_proj, s_pl);
-        float box[6];
-        reject_box_warp(s_pl, __uint_as_float(__ldg(P.scene_bounds)), __uint_as_float(__ldg(P.scene_bounds + 1)),
-                        box);
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < 6; ++k) P.views[v].reject_box[k] = box[k];
-            CullView c;
-            c.planes = s_pl;
-            c.vp = ldg_mat4(V.camera.view_proj);
-            c.pos_near = __ldg(reinterpret_cast<const float4*>(V.camera.position_near));
-            c.p00 = __ldg(&V.camera.proj[0]);
-            c.p11 = __ldg(&V.camera.proj[5]);
-            c.focal = fmul(fmul(fabsf(c.p11), (float)V.height), 0.5f);
-            c.lod_threshold_px = V.lod_threshold_px;
-            for (int l = 0; l < HELIO_HIZ_MAX_MIPS; ++l) {
-                c.hiz.levels[l] = V.hiz.levels[l];
-                c.hiz.width[l] = V.hiz.lw[l];
-                c.hiz.height[l] = V.hiz.lh[l];
-                c.hiz.pitch[l] = V.hiz.lpitch[l];
-            }
-            c.hiz.mip_count = V.hiz.mip_count;
-            c.screen_height = V.height;
-            c.hiz_mip_count = V.hiz_mip_count;
-            c.pad[0] = c.pad[1] = 0u;
-            P.cviews[v] = c;
-            red_add_release(P.setup_done, 1u);  // the select units wait for every view
+        BatchViewDev& V = P.views[v];
+        const uint32_t rad = __ldg(P.scene_bounds), far1 = __ldg(P.scene_bounds + 1);
+        if (lane >= 8 && lane < 8 + HELIO_HIZ_MAX_MIPS) {
+            const uint32_t l = lane - 8;
+            s_c.hiz.levels[l] = V.hiz.levels[l];
+            s_c.hiz.width[l] = V.hiz.lw[l];
+            s_c.hiz.height[l] = V.hiz.lh[l];
+            s_c.hiz.pitch[l] = V.hiz.lpitch[l];
+        } else if (lane == 0) {
+            s_c.vp = ldg_mat4(V.camera.view_proj);
+            s_c.pos_near = __ldg(reinterpret_cast<const float4*>(V.camera.position_near));
+            s_c.p00 = __ldg(&V.camera.proj[0]);
+            s_c.p11 = __ldg(&V.camera.proj[5]);
+            s_c.focal = fmul(fmul(fabsf(s_c.p11), (float)V.height), 0.5f);
+            s_c.lod_threshold_px = V.lod_threshold_px;
+            s_c.hiz.mip_count = V.hiz.mip_count;
+            s_c.screen_height = V.height;
+            s_c.hiz_mip_count = V.hiz_mip_count;
+            s_c.pad[0] = s_c.pad[1] = 0u;
         }
+        publish_planes_warp(V.camera.view_proj, s_c.planes);
+        float box[6];
+        reject_box_warp(s_c.planes, __uint_as_float(rad), __uint_as_float(far1), s_q, box);
+        const uint4* src = reinterpret_cast<const uint4*>(&s_c);
+        uint4* dst = reinterpret_cast<uint4*>(P.cviews + v);
+        for (uint32_t k = lane; k < sizeof(CullView) / 16; k += 32u) dst[k] = src[k];
+#pragma unroll
+        for (uint32_t k = 0; k < 6; ++k)
+            if (lane == k) V.reject_box[k] = box[k];
+        __syncwarp();
+        if (lane == 0) red_add_release(P.setup_done, 1u);  // the select units wait for every view
         __syncwarp();
     }
 }
@@ -603,16 +648,18 @@ __device__ void phase_select_chunk(const BatchParams& P, uint32_t chunk, uint32_
 }
 
 // ── Phase 3: expansion into the view-major list of active spans ──────────────
-__device__ void phase_expand(const BatchParams& P, char* sm) {
+// offs: the chunk offsets in shared memory, or null (then P.chunk_offs holds them).
+__device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* sm) {
     uint32_t* s_vstart = reinterpret_cast<uint32_t*>(sm + kSmVStart);
     uint32_t* s_tmp = reinterpret_cast<uint32_t*>(sm + kSmMisc);
     const uint32_t V = P.view_count, C = P.object_chunks, tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
+    auto offset_of = [&](size_t i) { return offs ? offs[i] : ld_cg(P.chunk_offs + i); };
     // Padded first span of every view (a multiple of 32).
     {
         uint32_t padded = 0;
         if (tid < V) {
-            const uint32_t a = ld_cg(P.chunk_offs + (size_t)tid * C), e = ld_cg(P.chunk_offs + (size_t)(tid + 1) * C);
+            const uint32_t a = offset_of((size_t)tid * C), e = offset_of((size_t)(tid + 1) * C);
             padded = (e - a + 31u) & ~31u;
         }
         uint32_t total;
@@ -654,10 +701,19 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
     // (carried by the unit's lane).
     const uint32_t eb = min(max(n_units / (gridDim.x * (kBatchThreads / 32)), 1u), kExpandBatch);
     const uint32_t NB = (n_units + eb - 1) / eb;
-    for (;;) {
+    // With at most one batch per warp there is nothing to balance: warp w takes batch w, without
+    // the round trips of the claims.
+    const uint32_t warps = gridDim.x * (kBatchThreads / 32);
+    const bool fixed = NB <= warps;
+    for (bool first = true;; first = false) {
         uint32_t bq = 0;
-        if (lane == 0) bq = atomicAdd(P.expand_work, 1u);
-        bq = __shfl_sync(0xffffffffu, bq, 0);
+        if (fixed) {
+            if (!first) break;
+            bq = (uint32_t)warp * gridDim.x + blockIdx.x;
+        } else {
+            if (lane == 0) bq = atomicAdd(P.expand_work, 1u);
+            bq = __shfl_sync(0xffffffffu, bq, 0);
+        }
         if (bq >= NB) break;
         const size_t u = bq + (size_t)lane * NB;
         const bool live = (uint32_t)lane < eb && u < n_units;
@@ -665,7 +721,7 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
         if (!__any_sync(0xffffffffu, vis != 0u)) continue;
         const uint32_t v = live ? (uint32_t)(u / C) : 0u, ch = live ? (uint32_t)(u - (size_t)v * C) : 0u;
         uint32_t pos = 0;  // the unit's first span in the view-major list
-        if (vis) pos = s_vstart[v] + (ld_cg(P.chunk_offs + u) - ld_cg(P.chunk_offs + (size_t)v * C));
+        if (vis) pos = s_vstart[v] + (offset_of(u) - offset_of((size_t)v * C));
         const uint32_t inc_vis = warp_inclusive(vis);
         const uint32_t first_e = inc_vis - vis, total = __shfl_sync(0xffffffffu, inc_vis, 31);
         uint32_t written = 0;  // spans this lane's unit has written in earlier rounds
@@ -708,7 +764,7 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
     }
     // Padding spans (n = 0) complete every view to a multiple of 32.
     for (uint32_t v = blockIdx.x; v < V; v += gridDim.x) {
-        const uint32_t end = ld_cg(P.chunk_offs + (size_t)(v + 1) * C) - ld_cg(P.chunk_offs + (size_t)v * C);
+        const uint32_t end = offset_of((size_t)(v + 1) * C) - offset_of((size_t)v * C);
         for (uint32_t p = s_vstart[v] + end + tid; p < s_vstart[v + 1]; p += kBatchThreads)
             if (p < P.span_capacity) P.spans[p] = make_uint4(0u, v << 16, 0u, 0u);
     }
@@ -894,10 +950,17 @@ struct EmitLoads {
     ActiveSpan span;
 };
 
-__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t g, uint32_t shift) {
+// Draws of the batch before group g: from shared memory in a small batch (no pointer to either
+// place is kept: the cull kernel has no register for it).
+__device__ __forceinline__ uint32_t group_offset(const BatchParams& P, uint32_t groups, uint32_t g) {
+    extern __shared__ __align__(16) char sm[];
+    return groups <= kLocalGroups ? reinterpret_cast<const uint32_t*>(sm)[g] : ld_cg(P.group_offs + g);
+}
+
+__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t groups, uint32_t g, uint32_t shift) {
     const uint32_t lane = threadIdx.x & 31, size = 32u >> shift, windows = kWindowsPerWarp >> shift;
     EmitLoads e;
-    e.goff = ld_cg(P.group_offs + g);
+    e.goff = group_offset(P, groups, g);
     e.span = lane < size ? __ldcg(P.spans + (size_t)g * size + lane) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t* gbits = P.group_bits + (size_t)g * windows;
     e.bits_lo = lane < windows ? ld_cg(gbits + lane) : 0u;
@@ -920,13 +983,13 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift
         if (!mask) continue;
         uint32_t g = gw + (k0 + (__ffs(mask) - 1)) * GW;
         mask &= mask - 1u;
-        EmitLoads cur = emit_loads(P, g, shift);
+        EmitLoads cur = emit_loads(P, groups, g, shift);
         for (;;) {
             const bool more = mask != 0u;
             const uint32_t g_next = more ? gw + (k0 + (__ffs(mask) - 1)) * GW : 0u;
             mask &= mask - 1u;
             EmitLoads nxt{};
-            if (more) nxt = emit_loads(P, g_next, shift);
+            if (more) nxt = emit_loads(P, groups, g_next, shift);
             // The current group: its spans' packing offsets, then its view's table entry.
             GroupSpans gs;
             gs.n = span_n(cur.span);
@@ -948,7 +1011,7 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift
                 const uint32_t bits_lo = (uint32_t)lane < windows ? cur.bits_lo : 0u;
                 const uint32_t bits_hi = (uint32_t)lane + 32u < windows ? cur.bits_hi : 0u;
                 const uint32_t count = cnt_of(bits_lo, bits_hi);
-                uint32_t slot0 = cur.goff - ld_cg(P.group_offs + first_group);
+                uint32_t slot0 = cur.goff - group_offset(P, groups, first_group);
                 if (lane == 0) {
                     atomicAdd(counters + 0, count);
                     const unsigned long long end = (unsigned long long)slot0 + count;
@@ -1140,16 +1203,24 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
     if (!grid_sync(P)) return;
     stamp(P, 2);
     // The attached shadow cull's scan: CTA j takes the j-th chunk of dirty faces, CTA 0 also
-    // clears the clean faces' counts; done before the phase's last barrier.
+    // clears the clean faces' counts; done before the phase's last barrier (so an attached pass
+    // always takes the scan with barriers).
     if (P.shadow_blocks) {
         if (blockIdx.x == 0) shadow_clear_clean(P.shadow);
         for (uint32_t j = blockIdx.x; j < kShadowChunks; j += gridDim.x)
             shadow_scan_chunk(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
     }
 
-    if (!grid_exclusive_scan(P, P.chunk_counts, P.chunk_offs, P.view_count * P.object_chunks, s_tmp)) return;
+    const uint32_t n_chunks = P.view_count * P.object_chunks;
+    uint32_t* offs = n_chunks <= kLocalChunks && P.shadow_blocks == 0u ? reinterpret_cast<uint32_t*>(sm + kSmOffs) : nullptr;
+    if (offs) {
+        __syncthreads();  // the region is the select's
+        local_exclusive_scan(P.chunk_counts, n_chunks, offs, s_tmp);
+    } else if (!grid_exclusive_scan(P, P.chunk_counts, P.chunk_offs, n_chunks, s_tmp)) {
+        return;
+    }
     stamp(P, 3);
-    phase_expand(P, sm);
+    phase_expand(P, offs, sm);
 }
 
 // Phases 4..6 as a second cooperative launch: the meshlet tests need fewer registers
@@ -1167,7 +1238,8 @@ __global__ void __launch_bounds__(kBatchThreads, 5) batch_cull_kernel(BatchParam
     if (!grid_sync(P)) return;
     stamp(P, 5);
 
-    if (!grid_exclusive_scan(P, P.group_counts, P.group_offs, groups, s_tmp)) return;
+    if (groups <= kLocalGroups) local_exclusive_scan(P.group_counts, groups, reinterpret_cast<uint32_t*>(sm), s_tmp);
+    else if (!grid_exclusive_scan(P, P.group_counts, P.group_offs, groups, s_tmp)) return;
     stamp(P, 6);
     phase_emit(P, groups, shift);
     // End of the launch: the latest block end (no barrier needed).

@@ -186,3 +186,14 @@ def test_batch_group_sizes_match_oracle(cuda, shift):
     ctas = max(1, warps // 8)
     assert {0: groups >= 8 * ctas, 1: groups < 8 * ctas <= 2 * groups, 2: 2 * groups < 8 * ctas}[shift]
     _check_batch(w, views, cull_ctas=ctas)
+
+
+@pytest.mark.parametrize("views,objects", [(43, 32000), (42, 32513), (42, 32768), (1, 255)])
+def test_batch_scan_forms_match_oracle(cuda, views, objects):
+    """(view, chunk) counts that just fit a CTA's shared memory (43 x 125 = 5375), one more
+    (42 x 128 = 5376, a part-filled and a full last chunk), and a single one."""
+    from helio_b200 import scene as S
+
+    sc = S.make_scene(objects, objects, 3, 4, 0, 40.0)
+    w = S.Workload(3, sc, S.multiview_set(S.SEED_BASE + 9, True, 0.05)[5:5 + views])
+    _check_batch(w, w.views)
