@@ -882,10 +882,7 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift
             if (s < gs.total) {
                 const uint32_t mi = j_first + (s - j_off);
                 if (mi < S.meshlet_count) {
-                    const HelioGpuInstanceData* in = S.instances + j_inst;
-                    const HelioInstanceCullData cd = load_cull(S.cull + j_inst);
-                    const Mat4 model = ldg_mat4(in->model);
-                    cand = meshlet_frustum_cone_lazy(cv, S, mi, in, model, cd, c, wr);
+                    cand = meshlet_frustum_cone<true>(cv, S, mi, j_inst, c, wr);
                 }
             }
             const uint32_t b = __ballot_sync(0xffffffffu, cand);

@@ -17,7 +17,9 @@ using helio::as_stream;
 using helio::DevBuf;
 
 struct helio_vg_scene {
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, world, staging;
+    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, xform, world;
+    DevBuf staging;      // meshlets on their way to the update launch
+    DevBuf row_staging;  // instance rows on their way there, for the whole scene: a patch never allocates
     DevBuf bounds;  // launch_scene_update of the current objects and instances: u32[2], then u64[3] totals
     uint32_t meshlet_count = 0, object_count = 0;
     uint64_t lod0_meshlets = 0, max_spans = 0, max_draw_count = 0;
@@ -31,8 +33,7 @@ struct helio_vg_scene {
         s.m_axis = m_axis.as<float4>();
         s.m_draw = m_draw.as<uint4>();
         s.objects = objects.as<HelioGpuVgObject>();
-        s.instances = instances.as<HelioGpuInstanceData>();
-        s.cull = cull.as<HelioInstanceCullData>();
+        s.xform = xform.as<float4>();
         s.world = world.as<uint4>();
         s.items = nullptr;
         s.meshlet_count = meshlet_count;
@@ -105,15 +106,14 @@ int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects
     HELIO_CK(cudaMemsetAsync(sc->bounds.ptr, 0, kBoundsBytes, s));
     u.scene = sc->dev();
     u.scene.object_count = u.scene.instance_count = objects;
-    u.instances = sc->instances.as<HelioGpuInstanceData>();
-    u.cull = sc->cull.as<HelioInstanceCullData>();
+    u.xform = sc->xform.as<float4>();
     u.world = sc->world.as<uint4>();
     u.first = first;
     u.count = count;
-    if (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16)) {
-        u.src_rows = src;
-    } else {
-        int32_t st = copy_in(u.instances + first, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
+    u.rows = src;
+    if (count && !(memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16))) {
+        u.rows = sc->row_staging.as<HelioGpuInstanceData>();
+        int32_t st = copy_in(sc->row_staging.ptr, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
         if (st) return st;
     }
     unsigned long long* sums = reinterpret_cast<unsigned long long*>(sc->bounds.as<char>() + 8);
@@ -234,8 +234,8 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->m_axis.ensure(M * 16));
         HELIO_CK(sc->m_draw.ensure(M * 16));
         HELIO_CK(sc->objects.ensure(O * sizeof(HelioGpuVgObject)));
-        HELIO_CK(sc->instances.ensure(O * sizeof(HelioGpuInstanceData)));
-        HELIO_CK(sc->cull.ensure(O * sizeof(HelioInstanceCullData)));
+        HELIO_CK(sc->row_staging.ensure(O * sizeof(HelioGpuInstanceData)));
+        HELIO_CK(sc->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
         // Device arrays that 16-byte loads can read are copied by the update launch itself.
         helio::SceneUpdate u{};
@@ -286,7 +286,7 @@ int32_t helio_vg_scene_info_get(const helio_vg_scene* sc, helio_vg_scene_info* o
     out->lod0_meshlets = sc->lod0_meshlets;
     out->max_spans = sc->max_spans;
     out->device_bytes = sc->m_bounds.bytes + sc->m_cone.bytes + sc->m_axis.bytes + sc->m_draw.bytes +
-                        sc->objects.bytes + sc->instances.bytes + sc->cull.bytes + sc->world.bytes;
+                        sc->objects.bytes + sc->row_staging.bytes + sc->xform.bytes + sc->world.bytes;
     return HELIO_OK;
 }
 

@@ -179,7 +179,9 @@ struct helio_vg_pass {
     uint32_t publication_limit = HELIO_VG_DEFAULT_PUBLICATION_LIMIT;
     uint32_t counter_count = HELIO_VG_COUNTER_COUNT;
     // Scene (device resident).
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, instances, cull, world, items, staging;
+    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, xform, world, items;
+    DevBuf staging;      // meshlets on their way to the update launch
+    DevBuf row_staging;  // instance rows on their way there, for the whole scene: a patch never allocates
     // Outputs and scratch.
     DevBuf indirect, draws, visibility;
     DevBuf scratch;  // published counters (16 words) | kVgStateWords state words | tile statuses
@@ -594,13 +596,13 @@ static int32_t vg_rows(helio_vg_pass* p, helio::SceneUpdate* u, uint32_t objects
     u->scene.objects = p->objects.as<HelioGpuVgObject>();
     u->scene.object_count = u->scene.instance_count = objects;
     u->scene.world = u->world = p->world.as<uint4>();
-    u->instances = p->instances.as<HelioGpuInstanceData>();
-    u->cull = p->cull.as<HelioInstanceCullData>();
+    u->xform = p->xform.as<float4>();
     u->first = first;
     u->count = count;
-    if (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16)) u->src_rows = src;
-    else return vg_copy(u->instances + first, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
-    return HELIO_OK;
+    u->rows = src;
+    if (count == 0 || (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16))) return HELIO_OK;
+    u->rows = p->row_staging.as<HelioGpuInstanceData>();
+    return vg_copy(p->row_staging.ptr, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
 }
 
 int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* stream) {
@@ -616,8 +618,8 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->m_axis.ensure(M * 16));
         HELIO_CK(p->m_draw.ensure(M * 16));
         HELIO_CK(p->objects.ensure(O * sizeof(HelioGpuVgObject)));
-        HELIO_CK(p->instances.ensure(O * sizeof(HelioGpuInstanceData)));
-        HELIO_CK(p->cull.ensure(O * sizeof(HelioInstanceCullData)));
+        HELIO_CK(p->row_staging.ensure(O * sizeof(HelioGpuInstanceData)));
+        HELIO_CK(p->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
         HELIO_CK(p->visibility.ensure(W * 8));
@@ -702,8 +704,7 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
     scene.m_axis = p->m_axis.as<float4>();
     scene.m_draw = p->m_draw.as<uint4>();
     scene.objects = p->objects.as<HelioGpuVgObject>();
-    scene.instances = p->instances.as<HelioGpuInstanceData>();
-    scene.cull = p->cull.as<HelioInstanceCullData>();
+    scene.xform = p->xform.as<float4>();
     scene.world = p->world.as<uint4>();
     scene.items = p->items.as<HelioGpuVgWorkItem>();
     scene.meshlet_count = p->meshlet_count;

@@ -13,8 +13,7 @@ struct VgSceneDev {
     const float4* m_axis;    // cone_axis.xyz, lod_error
     const uint4* m_draw;     // first_index, index_count, vertex_offset, instance_index
     HelioGpuVgObject* objects;
-    const HelioGpuInstanceData* instances;
-    const HelioInstanceCullData* cull;
+    const float4* xform;  // [6 * instance_count] InstanceXform
     const uint4* world;  // [2 * object_count] ObjectWorld, kept up to date by launch_scene_update
     const HelioGpuVgWorkItem* items;
     uint32_t meshlet_count;
@@ -35,6 +34,21 @@ struct ObjectWorld {
     uint32_t pad;
 };
 static_assert(sizeof(ObjectWorld) == 32, "one sector");
+
+// What the meshlet tests read of an instance: the affine rows of its model matrix, its
+// InstanceCullData and its normal matrix in three 32-byte words, where the 144-byte
+// GpuInstanceData and the cull data took eight 16-byte loads in two places. The frustum test reads
+// the first two words, the cone test the third. (Meshlet tests of the batch: 73.0 -> 69.7 us with 85
+// views over 200,000 objects, 94.5 -> 88.0 with 4 views over 475,000.)
+struct InstanceXform {
+    float4 c0;  // model column 0 (xyz), max_scale
+    float4 c1;  // model column 1 (xyz), flags as bits: 1 = valid_transform, 2 = cone_cull_enabled
+    float4 c2;  // model column 2 (xyz), normal column 0 x
+    float4 c3;  // model column 3 (xyz), normal column 0 y
+    float4 na;  // normal column 0 z, normal column 1 xyz
+    float4 nb;  // normal column 2 xyz, unused
+};
+static_assert(sizeof(InstanceXform) == 96, "three 32-byte words");
 
 // View constants of the select / cull stages (vg_cull.wgsl:266-280 planes; fields of
 // GpuCameraUniforms) and the Hi-Z pyramid descriptor, held in shared memory.
@@ -112,9 +126,9 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
                                cudaStream_t stream);
 
 // Brings a device-resident scene up to date in one launch: copies what the caller gives in device
-// memory, and derives from the instances [first, first + count) their InstanceCullData and the
+// memory, and derives from the instances [first, first + count) their InstanceXform and the
 // ObjectWorld records of the objects that name them. A null source: the data is in the
-// destination already.
+// destination already (rows are never kept: everything reads what is derived from them).
 // With `bounds` (u32[2], zero before the launch), bounds over all valid objects as float bits, for
 // the batch's reject boxes: bounds[0] = largest world radius max(local_radius * max_scale, 0),
 // bounds[1] = largest |c.x| + |c.y| + |c.z| of a world centre c. With `totals` (u64[3], zero before
@@ -122,12 +136,11 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
 // spans and totals[2] = meshlets of the largest of the object's LODs.
 struct SceneUpdate {
     VgSceneDev scene;  // object_count, instance_count, objects (written too, with src_objects) and world
-    const HelioGpuInstanceData* src_rows;     // [count], 16-byte aligned
+    const HelioGpuInstanceData* rows;         // [count], 16-byte aligned
     const HelioGpuVgObject* src_objects;      // [object_count], 16-byte aligned
     const HelioGpuVgWorkItem* src_items;      // [item_count], 8-byte aligned
     const HelioGpuMeshletEntry* src_meshlets; // [meshlet_count], 16-byte aligned, packed into the four streams
-    HelioGpuInstanceData* instances;
-    HelioInstanceCullData* cull;
+    float4* xform;
     uint4* world;
     HelioGpuVgWorkItem* items;
     float4 *m_bounds, *m_cone, *m_axis;

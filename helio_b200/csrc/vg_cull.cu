@@ -81,12 +81,19 @@ __global__ void instance_cull_data_kernel(const HelioGpuInstanceData* __restrict
 // indices, since an object mostly names the instance of its own index, whose row is then in L1), one
 // per 2048 work items, one per 512 meshlets. Copies have all their loads in flight before the
 // first store. No kind waits for another's results: rows are read from their source, and an object
-// recomputes its instance's scale. Bound by memory: 288 bytes per copied row, 256 per copied object.
+// recomputes its instance's scale. Bound by memory: 240 bytes per row, 256 per copied object.
 // Bounds and sums meet in the block, so that a block costs at most five atomics (two per warp on
 // the same two words took 37 us for 475,000 objects).
 constexpr uint32_t kUpdateThreads = 256;
 constexpr uint32_t kUpdateItems = 8 * kUpdateThreads;
 constexpr uint32_t kUpdateMeshlets = 2 * kUpdateThreads;
+
+// 32 bytes in one store (sm_100), a whole sector; p is 32-byte aligned.
+__device__ __forceinline__ void st_pair(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 
 // Copies n 16-byte words (at most kEach per thread) from src to dst, loads first.
 template <int kEach>
@@ -148,19 +155,33 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
         return;
     }
     const uint32_t i0 = blockIdx.x * kUpdateThreads, i = i0 + threadIdx.x;
-    const HelioGpuInstanceData* rows = U.src_rows ? U.src_rows : U.instances + U.first;  // row k = instance first + k
-    if (U.src_rows && i0 < U.count)
-        copy_words<9>(reinterpret_cast<uint4*>(U.instances + U.first + i0), reinterpret_cast<const uint4*>(rows + i0),
-                      min(kUpdateThreads, U.count - i0) * (uint32_t)(sizeof(HelioGpuInstanceData) / 16));
+    const HelioGpuInstanceData* rows = U.rows;  // row k = instance first + k
     if (U.src_objects && i0 < S.object_count)
         copy_words<8>(reinterpret_cast<uint4*>(S.objects + i0), reinterpret_cast<const uint4*>(U.src_objects + i0),
                       min(kUpdateThreads, S.object_count - i0) * (uint32_t)(sizeof(HelioGpuVgObject) / 16));
-    if (i < U.count) U.cull[U.first + i] = cull_data_of(ldg_mat4(rows[i].model));
+    // The object's fields are on their way while the instance's record is made.
+    const HelioGpuVgObject* obj = (U.src_objects ? U.src_objects : S.objects) + i;
+    uint2 head = make_uint2(0u, 0u);  // instance_index, lod_count
+    float4 lb = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < S.object_count) {
+        head = __ldg(reinterpret_cast<const uint2*>(obj));
+        lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
+    }
+    if (i < U.count) {
+        const float4* row = reinterpret_cast<const float4*>(rows + i);
+        const Mat4 m{__ldg(row), __ldg(row + 1), __ldg(row + 2), __ldg(row + 3)};
+        const float4 n0 = __ldg(row + 4), n1 = __ldg(row + 5), n2 = __ldg(row + 6);
+        const HelioInstanceCullData cd = cull_data_of(m);
+        const uint32_t flags = (cd.valid_transform ? 1u : 0u) | (cd.cone_cull_enabled ? 2u : 0u);
+        float4* x = U.xform + 6u * (size_t)(U.first + i);
+        st_pair(x, make_float4(m.c0.x, m.c0.y, m.c0.z, cd.max_scale),
+                make_float4(m.c1.x, m.c1.y, m.c1.z, __uint_as_float(flags)));
+        st_pair(x + 2, make_float4(m.c2.x, m.c2.y, m.c2.z, n0.x), make_float4(m.c3.x, m.c3.y, m.c3.z, n0.y));
+        st_pair(x + 4, make_float4(n0.z, n1.x, n1.y, n1.z), make_float4(n2.x, n2.y, n2.z, 0.0f));
+    }
     uint32_t rad = 0u, far1 = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
     unsigned long long lod0 = 0, spans = 0, draws = 0;
     if (i < S.object_count) {
-        const HelioGpuVgObject* obj = (U.src_objects ? U.src_objects : S.objects) + i;
-        const uint2 head = __ldg(reinterpret_cast<const uint2*>(obj));  // instance_index, lod_count
         const uint32_t lods = min(head.y, 8u);
         if (kTotals) {
             const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts));
@@ -180,7 +201,6 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
             const Mat4 model = ldg_mat4(rows[head.x - U.first].model);
             const HelioInstanceCullData cd = cull_data_of(model);
             if (lods && cd.valid_transform) {
-                const float4 lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
                 const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
                 sphere = make_float4(c.x, c.y, c.z, fmaxf(fmul(lb.w, cd.max_scale), 0.0f));
                 live = lods;
@@ -550,11 +570,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
             const uint32_t k = item_at(s_it, w);
             const uint32_t mi = s_it.first[k] + (s - s_it.off[k]);
             if (mi < S.meshlet_count) {
-                const uint32_t ji = s_it.inst[k];
-                const HelioGpuInstanceData* in = S.instances + ji;
-                const HelioInstanceCullData cd = load_cull(S.cull + ji);
-                const Mat4 model = ldg_mat4(in->model);
-                vis = meshlet_visible<false, kWide>(S, s_view, mi, model, cd, in);
+                vis = meshlet_visible<false, kWide>(S, s_view, mi, s_it.inst[k]);
             }
         }
         const uint32_t bits = __ballot_sync(0xffffffffu, vis);

@@ -7,14 +7,39 @@
 
 namespace helio {
 
-__device__ __forceinline__ HelioInstanceCullData load_cull(const HelioInstanceCullData* p) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
-    HelioInstanceCullData r;
-    r.max_scale = __uint_as_float(q.x);
-    r.min_scale = __uint_as_float(q.y);
-    r.cone_cull_enabled = q.z;
-    r.valid_transform = q.w;
-    return r;
+// 32 bytes in one load (sm_100); p is 32-byte aligned.
+__device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// The frustum test's share of an instance: model holds xyz of each column (the w of columns 0 and 1
+// carry max_scale and the flags, those of 2 and 3 the start of the normal matrix).
+struct InstanceView {
+    Mat4 model;
+    __device__ float max_scale() const { return model.c0.w; }
+    __device__ bool valid() const { return (__float_as_uint(model.c1.w) & 1u) != 0u; }
+    __device__ bool cone() const { return (__float_as_uint(model.c1.w) & 2u) != 0u; }
+};
+
+__device__ __forceinline__ InstanceView load_instance(const VgSceneDev& S, uint32_t i) {
+    const float4* p = S.xform + 6u * (size_t)i;
+    InstanceView v;
+    ldg_pair(p, v.model.c0, v.model.c1);
+    ldg_pair(p + 2, v.model.c2, v.model.c3);
+    return v;
+}
+
+// The rest of the normal matrix of instance i.
+__device__ __forceinline__ void load_normal(const VgSceneDev& S, uint32_t i, float4& na, float4& nb) {
+    ldg_pair(S.xform + 6u * (size_t)i + 4u, na, nb);
+}
+
+// mat3(normal matrix) * axis, in the order of mat3_vec.
+__device__ __forceinline__ F3 normal_vec(const InstanceView& v, float4 na, float4 nb, float4 axis) {
+    return mat3_vec(make_float4(v.model.c2.w, v.model.c3.w, na.x, 0.0f), make_float4(na.y, na.z, na.w, 0.0f), nb,
+                    f3(axis.x, axis.y, axis.z));
 }
 
 __device__ __forceinline__ ObjectWorld load_world(const VgSceneDev& S, uint32_t o) {
@@ -59,82 +84,41 @@ __device__ __forceinline__ bool cone_rejects(F3 a, F3 cta, float ads, float cuto
     return dot3(divs3(cta, fsqrt(ads)), axis_ws) >= cutoff;
 }
 
-// World-space bounding sphere of meshlet mi of an instance (vg_cull.wgsl:150-152).
-__device__ __forceinline__ void meshlet_sphere(const VgSceneDev& S, uint32_t mi, const Mat4& model,
-                                               const HelioInstanceCullData& cd, F3& c, float& wr) {
-    const float4 b = __ldg(S.m_bounds + mi);
-    c = mat4_point3(model, f3(b.x, b.y, b.z));
-    wr = fmaxf(fmul(b.w, cd.max_scale), 0.0f);
-}
-
-// Everything the frustum and cone tests read of one meshlet of one instance,
-// loaded in one go (one memory round trip instead of one per test).
-struct MeshletInputs {
-    float4 bounds, cone, axis;
-    float4 n0, n1, n2;  // the instance's normal matrix columns
-};
-
-__device__ __forceinline__ MeshletInputs load_meshlet(const VgSceneDev& S, uint32_t mi,
-                                                      const HelioGpuInstanceData* inst) {
-    MeshletInputs m;
-    m.bounds = __ldg(S.m_bounds + mi);
-    m.cone = __ldg(S.m_cone + mi);
-    m.axis = __ldg(S.m_axis + mi);
-    const float4* nm = reinterpret_cast<const float4*>(inst->normal_mat);
-    m.n0 = __ldg(nm);
-    m.n1 = __ldg(nm + 1);
-    m.n2 = __ldg(nm + 2);
-    return m;
-}
-
 // cull_meshlet, first part (vg_cull.wgsl:143-182): the frustum and normal-cone
 // tests. True = the meshlet is still a candidate and the Hi-Z test decides it;
-// (c, wr) is its world-space sphere.
-__device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const MeshletInputs& m, const Mat4& model,
-                                                     const HelioInstanceCullData& cd, F3& c, float& wr) {
-    if (cd.valid_transform == 0u) return false;
-    c = mat4_point3(model, f3(m.bounds.x, m.bounds.y, m.bounds.z));
-    wr = fmaxf(fmul(m.bounds.w, cd.max_scale), 0.0f);
+// (c, wr) is its world-space sphere (:150-152). kLazyCone: the cone inputs (apex, axis, the rest of
+// the normal matrix) are loaded only for meshlets whose sphere passes the frustum: fewer registers
+// live at a time, for kernels that run more warps per SM instead of more loads per warp. Otherwise
+// everything is loaded in one go (one memory round trip instead of one per test).
+template <bool kLazyCone>
+__device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const VgSceneDev& S, uint32_t mi,
+                                                     uint32_t instance, F3& c, float& wr) {
+    const InstanceView in = load_instance(S, instance);
+    const float4 b = __ldg(S.m_bounds + mi);
+    float4 cone, axis, na, nb;
+    if (!kLazyCone) {
+        cone = __ldg(S.m_cone + mi);
+        axis = __ldg(S.m_axis + mi);
+        load_normal(S, instance, na, nb);
+    }
+    if (!in.valid()) return false;
+    c = mat4_point3(in.model, f3(b.x, b.y, b.z));
+    wr = fmaxf(fmul(b.w, in.max_scale()), 0.0f);
     if (!sphere_visible_vg(C.planes, c, wr)) return false;
     // Perspective normal-cone test (:159-182).
-    if (cd.cone_cull_enabled != 0u) {
+    if (in.cone()) {
         const F3 cam = f3(C.pos_near.x, C.pos_near.y, C.pos_near.z);
         const F3 ctc = sub3(c, cam);
         const float cam_dist_sq = dot3(ctc, ctc);
         const float guard = fmul(wr, 1.5f);
-        if (cam_dist_sq > fmul(guard, guard) && m.cone.w <= 1.0f) {
-            const F3 a = mat3_vec(m.n0, m.n1, m.n2, f3(m.axis.x, m.axis.y, m.axis.z));
-            const F3 apex = mat4_point3(model, f3(m.cone.x, m.cone.y, m.cone.z));
-            const F3 cta = sub3(apex, cam);
-            const float ads = dot3(cta, cta);
-            if (ads > 1.0e-12f && cone_rejects(a, cta, ads, m.cone.w)) return false;
-        }
-    }
-    return true;
-}
-
-// The same tests with the cone inputs (apex, axis, the instance's normal matrix) loaded
-// only for meshlets whose sphere passes the frustum: fewer registers live at a time, for
-// kernels that run more warps per SM instead of more loads per warp.
-__device__ __forceinline__ bool meshlet_frustum_cone_lazy(const CullView& C, const VgSceneDev& S, uint32_t mi,
-                                                          const HelioGpuInstanceData* inst, const Mat4& model,
-                                                          const HelioInstanceCullData& cd, F3& c, float& wr) {
-    if (cd.valid_transform == 0u) return false;
-    const float4 b = __ldg(S.m_bounds + mi);
-    c = mat4_point3(model, f3(b.x, b.y, b.z));
-    wr = fmaxf(fmul(b.w, cd.max_scale), 0.0f);
-    if (!sphere_visible_vg(C.planes, c, wr)) return false;
-    if (cd.cone_cull_enabled != 0u) {
-        const F3 cam = f3(C.pos_near.x, C.pos_near.y, C.pos_near.z);
-        const F3 ctc = sub3(c, cam);
-        const float cam_dist_sq = dot3(ctc, ctc);
-        const float guard = fmul(wr, 1.5f);
-        const float4 cone = __ldg(S.m_cone + mi);
+        if (kLazyCone) cone = __ldg(S.m_cone + mi);
         if (cam_dist_sq > fmul(guard, guard) && cone.w <= 1.0f) {
-            const float4 axis = __ldg(S.m_axis + mi);
-            const float4* nm = reinterpret_cast<const float4*>(inst->normal_mat);
-            const F3 a = mat3_vec(__ldg(nm), __ldg(nm + 1), __ldg(nm + 2), f3(axis.x, axis.y, axis.z));
-            const F3 apex = mat4_point3(model, f3(cone.x, cone.y, cone.z));
+            if (kLazyCone) {
+                axis = __ldg(S.m_axis + mi);
+                load_normal(S, instance, na, nb);
+            }
+            const F3 a = normal_vec(in, na, nb, axis);
+            const F3 apex = mat4_point3(in.model, f3(cone.x, cone.y, cone.z));
             const F3 cta = sub3(apex, cam);
             const float ads = dot3(cta, cta);
             if (ads > 1.0e-12f && cone_rejects(a, cta, ads, cone.w)) return false;
@@ -185,17 +169,13 @@ __device__ __forceinline__ bool meshlet_hiz_visible(const CullView& C, F3 c, flo
     return true;
 }
 
-// cull_meshlet decision part (vg_cull.wgsl:143-240): true = emit a draw. kLazyCone: the
-// cone inputs are loaded after the frustum test (fewer live registers), else with the sphere.
+// cull_meshlet decision part (vg_cull.wgsl:143-240): true = emit a draw.
 template <bool kCoherentHiz = false, bool kLazyCone = false>
 __device__ __forceinline__ bool meshlet_visible(const VgSceneDev& S, const CullView& C, uint32_t mi,
-                                                const Mat4& model, const HelioInstanceCullData& cd,
-                                                const HelioGpuInstanceData* inst) {
+                                                uint32_t instance) {
     F3 c;
     float wr;
-    const bool cand = kLazyCone ? meshlet_frustum_cone_lazy(C, S, mi, inst, model, cd, c, wr)
-                                : meshlet_frustum_cone(C, load_meshlet(S, mi, inst), model, cd, c, wr);
-    if (!cand) return false;
+    if (!meshlet_frustum_cone<kLazyCone>(C, S, mi, instance, c, wr)) return false;
     return meshlet_hiz_visible<kCoherentHiz>(C, c, wr);
 }
 
