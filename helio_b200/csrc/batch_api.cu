@@ -17,7 +17,7 @@ using helio::as_stream;
 using helio::DevBuf;
 
 struct helio_vg_scene {
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, xform, world;
+    DevBuf m_bounds, m_axis, m_draw, objects, xform, world;
     DevBuf staging;      // meshlets on their way to the update launch
     DevBuf row_staging;  // instance rows on their way there, for the whole scene: a patch never allocates
     DevBuf bounds;  // launch_scene_update of the current objects and instances: u32[2], then u64[3] totals
@@ -29,7 +29,6 @@ struct helio_vg_scene {
     helio::VgSceneDev dev() const {
         helio::VgSceneDev s{};
         s.m_bounds = m_bounds.as<float4>();
-        s.m_cone = m_cone.as<float4>();
         s.m_axis = m_axis.as<float4>();
         s.m_draw = m_draw.as<uint4>();
         s.objects = objects.as<HelioGpuVgObject>();
@@ -229,8 +228,7 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
     int32_t st;
     if (!sc->have || f->buffer_version != sc->version) {
         const size_t M = f->meshlet_count, O = f->object_count;
-        HELIO_CK(sc->m_bounds.ensure(M * 16));
-        HELIO_CK(sc->m_cone.ensure(M * 16));
+        HELIO_CK(sc->m_bounds.ensure(M * 32));
         HELIO_CK(sc->m_axis.ensure(M * 16));
         HELIO_CK(sc->m_draw.ensure(M * 16));
         HELIO_CK(sc->objects.ensure(O * sizeof(HelioGpuVgObject)));
@@ -249,7 +247,6 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         }
         u.meshlet_count = f->meshlet_count;
         u.m_bounds = sc->m_bounds.as<float4>();
-        u.m_cone = sc->m_cone.as<float4>();
         u.m_axis = sc->m_axis.as<float4>();
         u.m_draw = sc->m_draw.as<uint4>();
         if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
@@ -285,7 +282,7 @@ int32_t helio_vg_scene_info_get(const helio_vg_scene* sc, helio_vg_scene_info* o
     out->object_count = sc->object_count;
     out->lod0_meshlets = sc->lod0_meshlets;
     out->max_spans = sc->max_spans;
-    out->device_bytes = sc->m_bounds.bytes + sc->m_cone.bytes + sc->m_axis.bytes + sc->m_draw.bytes +
+    out->device_bytes = sc->m_bounds.bytes + sc->m_axis.bytes + sc->m_draw.bytes +
                         sc->objects.bytes + sc->row_staging.bytes + sc->xform.bytes + sc->world.bytes;
     return HELIO_OK;
 }

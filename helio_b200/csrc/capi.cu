@@ -179,7 +179,7 @@ struct helio_vg_pass {
     uint32_t publication_limit = HELIO_VG_DEFAULT_PUBLICATION_LIMIT;
     uint32_t counter_count = HELIO_VG_COUNTER_COUNT;
     // Scene (device resident).
-    DevBuf m_bounds, m_cone, m_axis, m_draw, objects, xform, world, items;
+    DevBuf m_bounds, m_axis, m_draw, objects, xform, world, items;
     DevBuf staging;      // meshlets on their way to the update launch
     DevBuf row_staging;  // instance rows on their way there, for the whole scene: a patch never allocates
     // Outputs and scratch.
@@ -613,8 +613,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
     if (!p->have_version || f->buffer_version != p->last_version) {
         // Full upload (rendering.rs:715-786).
         const size_t M = f->meshlet_count, O = f->object_count, W = f->work_item_count;
-        HELIO_CK(p->m_bounds.ensure(M * 16));
-        HELIO_CK(p->m_cone.ensure(M * 16));
+        HELIO_CK(p->m_bounds.ensure(M * 32));
         HELIO_CK(p->m_axis.ensure(M * 16));
         HELIO_CK(p->m_draw.ensure(M * 16));
         HELIO_CK(p->objects.ensure(O * sizeof(HelioGpuVgObject)));
@@ -635,7 +634,6 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         }
         u.meshlet_count = f->meshlet_count;
         u.m_bounds = p->m_bounds.as<float4>();
-        u.m_cone = p->m_cone.as<float4>();
         u.m_axis = p->m_axis.as<float4>();
         u.m_draw = p->m_draw.as<uint4>();
         if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
@@ -700,7 +698,6 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
 
     helio::VgSceneDev scene{};
     scene.m_bounds = p->m_bounds.as<float4>();
-    scene.m_cone = p->m_cone.as<float4>();
     scene.m_axis = p->m_axis.as<float4>();
     scene.m_draw = p->m_draw.as<uint4>();
     scene.objects = p->objects.as<HelioGpuVgObject>();

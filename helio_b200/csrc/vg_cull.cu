@@ -7,7 +7,7 @@
 //   src/lib.rs:132-167             InstanceCullData::from_instance -> instance_cull_data_kernel
 //
 // Layout and scheduling (B200 design, not a translation of the WGSL dispatches):
-//   * meshlet descriptors are re-laid once per upload into four 16-byte streams;
+//   * meshlet descriptors are re-laid once per upload into three streams;
 //   * one launch does the whole view. A tile CTA takes up to 512 consecutive work items, two
 //     per thread, and selects their objects itself (an object's few items repeat its select,
 //     from L2, which costs less than a launch and a round trip of records in between); it then
@@ -120,10 +120,10 @@ __device__ __forceinline__ void update_items(const SceneUpdate& U, uint32_t bloc
         if (i0 + k * kUpdateThreads < U.item_count) dst[i0 + k * kUpdateThreads] = x[k];
 }
 
-// Meshlets into the four streams.
+// Meshlets into the three streams.
 __device__ __forceinline__ void update_meshlets(const SceneUpdate& U, uint32_t block) {
     const uint4* src = reinterpret_cast<const uint4*>(U.src_meshlets);
-    uint4* streams[4] = {reinterpret_cast<uint4*>(U.m_bounds), reinterpret_cast<uint4*>(U.m_cone),
+    uint4* streams[4] = {reinterpret_cast<uint4*>(U.m_bounds), reinterpret_cast<uint4*>(U.m_bounds) + 1,
                          reinterpret_cast<uint4*>(U.m_axis), U.m_draw};
     const uint64_t m0 = (uint64_t)block * kUpdateMeshlets;
     uint4 x[2][4];
@@ -139,7 +139,7 @@ __device__ __forceinline__ void update_meshlets(const SceneUpdate& U, uint32_t b
         const uint64_t m = m0 + (uint32_t)r * kUpdateThreads + threadIdx.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (m < U.meshlet_count) streams[k][m] = x[r][k];
+            if (m < U.meshlet_count) streams[k][k < 2 ? 2u * m : m] = x[r][k];
     }
 }
 

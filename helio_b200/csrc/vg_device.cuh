@@ -86,7 +86,7 @@ __device__ __forceinline__ bool cone_rejects(F3 a, F3 cta, float ads, float cuto
 
 // cull_meshlet, first part (vg_cull.wgsl:143-182): the frustum and normal-cone
 // tests. True = the meshlet is still a candidate and the Hi-Z test decides it;
-// (c, wr) is its world-space sphere (:150-152). kLazyCone: the cone inputs (apex, axis, the rest of
+// (c, wr) is its world-space sphere (:150-152). kLazyCone: the cone's other inputs (axis, the rest of
 // the normal matrix) are loaded only for meshlets whose sphere passes the frustum: fewer registers
 // live at a time, for kernels that run more warps per SM instead of more loads per warp. Otherwise
 // everything is loaded in one go (one memory round trip instead of one per test).
@@ -94,10 +94,9 @@ template <bool kLazyCone>
 __device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const VgSceneDev& S, uint32_t mi,
                                                      uint32_t instance, F3& c, float& wr) {
     const InstanceView in = load_instance(S, instance);
-    const float4 b = __ldg(S.m_bounds + mi);
-    float4 cone, axis, na, nb;
+    float4 b, cone, axis, na, nb;
+    ldg_pair(S.m_bounds + 2u * (size_t)mi, b, cone);
     if (!kLazyCone) {
-        cone = __ldg(S.m_cone + mi);
         axis = __ldg(S.m_axis + mi);
         load_normal(S, instance, na, nb);
     }
@@ -111,7 +110,6 @@ __device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const Vg
         const F3 ctc = sub3(c, cam);
         const float cam_dist_sq = dot3(ctc, ctc);
         const float guard = fmul(wr, 1.5f);
-        if (kLazyCone) cone = __ldg(S.m_cone + mi);
         if (cam_dist_sq > fmul(guard, guard) && cone.w <= 1.0f) {
             if (kLazyCone) {
                 axis = __ldg(S.m_axis + mi);
