@@ -386,9 +386,7 @@ __device__ void phase_setup(const BatchParams& P) {
         const uint32_t rad = __ldg(P.scene_bounds), far1 = __ldg(P.scene_bounds + 1);
         if (lane >= 8 && lane < 8 + HELIO_HIZ_MAX_MIPS) {
             const uint32_t l = lane - 8;
-            s_c.hiz.levels[l] = V.hiz.levels[l];
-            s_c.hiz.width[l] = V.hiz.lw[l];
-            s_c.hiz.height[l] = V.hiz.lh[l];
+            s_c.hiz.level[l] = HizLevel{V.hiz.levels[l], V.hiz.lw[l], V.hiz.lh[l]};
             s_c.hiz.pitch[l] = V.hiz.lpitch[l];
         } else if (lane == 0) {
             s_c.vp = ldg_mat4(V.camera.view_proj);

@@ -121,9 +121,7 @@ uint32_t mip_levels(uint32_t w, uint32_t h) { return helio::host_mip_levels(w, h
 helio::HizView to_view(const helio_hiz_pyramid& p) {
     helio::HizView v{};
     for (int l = 0; l < HELIO_HIZ_MAX_MIPS; ++l) {
-        v.levels[l] = p.levels[l];
-        v.width[l] = p.width[l];
-        v.height[l] = p.height[l];
+        v.level[l] = helio::HizLevel{p.levels[l], p.width[l], p.height[l]};
         v.pitch[l] = p.pitch[l];
     }
     v.mip_count = p.mip_count;

@@ -117,39 +117,42 @@ __device__ __forceinline__ uint32_t ceil_log2_exact(float d) {
     return (bits & 0x7FFFFFu) ? e + 1u : e;
 }
 
-// Hi-Z pyramid as passed to kernels (a copy of helio_hiz_pyramid in param space).
-struct HizView {
-    const float* levels[HELIO_HIZ_MAX_MIPS];
-    uint32_t width[HELIO_HIZ_MAX_MIPS];
-    uint32_t height[HELIO_HIZ_MAX_MIPS];
+// Hi-Z pyramid as passed to kernels (a copy of helio_hiz_pyramid in param space). What a sample needs
+// of its level but the pitch is one 16-byte word: lanes sample levels of their own.
+struct HizLevel {
+    const float* texels;
+    uint32_t width, height;
+};
+static_assert(sizeof(HizLevel) == 16, "one load");
+struct alignas(16) HizView {
+    HizLevel level[HELIO_HIZ_MAX_MIPS];
     uint32_t pitch[HELIO_HIZ_MAX_MIPS];
     uint32_t mip_count;
+    uint32_t pad[3];
 };
 
-// Copy with static indices (kernel parameters must not be indexed dynamically).
-__device__ __forceinline__ void copy_hiz(const HizView& src, HizView& dst) {
-#pragma unroll
-    for (int l = 0; l < HELIO_HIZ_MAX_MIPS; ++l) {
-        dst.levels[l] = src.levels[l];
-        dst.width[l] = src.width[l];
-        dst.height[l] = src.height[l];
-        dst.pitch[l] = src.pitch[l];
-    }
-    dst.mip_count = src.mip_count;
+__device__ __forceinline__ HizLevel hiz_level(const HizView& hz, uint32_t l) {
+    const uint4 q = *reinterpret_cast<const uint4*>(&hz.level[l]);
+    HizLevel r;
+    r.texels = reinterpret_cast<const float*>(((uint64_t)q.y << 32) | q.x);
+    r.width = q.z;
+    r.height = q.w;
+    return r;
 }
 
 // kCoherent: the pyramid was written earlier in the same launch, so it is read
 // through L2 (ld.global.cg) instead of the read-only path.
 template <bool kCoherent = false>
 __device__ __forceinline__ float hiz_sample(const HizView& hz, float u, float v, uint32_t mip) {
-    uint32_t l = min(mip, hz.mip_count - 1u);
-    uint32_t w = hz.width[l], h = hz.height[l];
+    const uint32_t l = min(mip, hz.mip_count - 1u);
+    const HizLevel lv = hiz_level(hz, l);
+    const uint32_t w = lv.width, h = lv.height;
     // u, v lie in [0, 1] at every call site, so the products lie in [0, w] / [0, h].
     int ix = (int)floorf(fmul(u, (float)w));
     int iy = (int)floorf(fmul(v, (float)h));
     ix = min(max(ix, 0), (int)w - 1);
     iy = min(max(iy, 0), (int)h - 1);
-    const float* p = hz.levels[l] + (size_t)iy * hz.pitch[l] + ix;
+    const float* p = lv.texels + (size_t)iy * hz.pitch[l] + ix;
     return kCoherent ? __ldcg(p) : __ldg(p);
 }
 
