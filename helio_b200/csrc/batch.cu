@@ -927,15 +927,6 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift
     }
 }
 
-// Visible meshlets of a group: the set bits of all its window ballots (lane k holds
-// windows k and k + 32).
-__device__ __forceinline__ uint32_t cnt_of(uint32_t lo, uint32_t hi) {
-    uint32_t c = __popc(lo) + __popc(hi);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    return c;
-}
-
 // ── Phase 6: emission, per view, in the canonical order ───────────────────────
 // The loads of one group that do not depend on another group's data: its scan offset,
 // lane k's span and lane k's two window ballots (windows k and k + 32; the ballot row has
@@ -1005,48 +996,70 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift
                 const uint32_t windows = (gs.total + 31u) >> 5;
                 const uint32_t bits_lo = (uint32_t)lane < windows ? cur.bits_lo : 0u;
                 const uint32_t bits_hi = (uint32_t)lane + 32u < windows ? cur.bits_hi : 0u;
-                const uint32_t count = cnt_of(bits_lo, bits_hi);
-                uint32_t slot0 = cur.goff - group_offset(P, groups, first_group);
+                const uint32_t inc_lo = warp_inclusive(__popc(bits_lo));
+                const uint32_t inc_hi = windows > 32u ? warp_inclusive(__popc(bits_hi)) : 0u;
+                const uint32_t n_lo = __shfl_sync(0xffffffffu, inc_lo, 31);
+                const uint32_t count = n_lo + __shfl_sync(0xffffffffu, inc_hi, 31);
+                const uint32_t slot0 = cur.goff - group_offset(P, groups, first_group);
                 if (lane == 0) {
                     atomicAdd(counters + 0, count);
                     const unsigned long long end = (unsigned long long)slot0 + count;
                     const unsigned long long lo = slot0 > cap ? slot0 : cap;
                     if (end > lo) atomicAdd(counters + 1, (uint32_t)(end - lo));
                 }
-                // Windows in groups of 4: the draw records of 4 windows are loaded before
-                // any of them is written.
-                for (uint32_t w0 = 0; w0 < windows; w0 += 4) {
-                    uint4 d[4];
-                    uint32_t b[4], mi[4], ji[4], jl[4];
+                // Draw by draw: lane i of a round takes the group's i-th next visible meshlet (its
+                // window by a search over the windows' counts, its bit, its span), so that every lane
+                // loads and stores one and the stores of a round are contiguous; window by window, only
+                // the visible third of the lanes did (emission of 858,000 draws of 85 views 19.9 ->
+                // 14.4 us, of 748,000 of 4 views 26.0 -> 19.2). Two rounds' draw records are loaded
+                // before either is written.
+                for (uint32_t i0 = 0; i0 < count; i0 += 64u) {
+                    uint4 d[2];
+                    uint32_t mi[2], ji[2], jl[2];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint32_t win = w0 + k;
-                        const uint32_t src = win < 32u ? bits_lo : bits_hi;
-                        b[k] = win < windows ? __shfl_sync(0xffffffffu, src, win & 31u) : 0u;
-                        const uint32_t s = win * 32u + lane;
+                    for (int k = 0; k < 2; ++k) {
+                        const uint32_t i = i0 + 32u * k + lane;
+                        uint32_t win = 0, rank = i, word;
+#pragma unroll
+                        for (uint32_t step = 16; step; step >>= 1)
+                            if (__shfl_sync(0xffffffffu, inc_lo, win + step - 1u) <= i) win += step;
+                        rank -= __shfl_sync(0xffffffffu, inc_lo - __popc(bits_lo), win);
+                        word = __shfl_sync(0xffffffffu, bits_lo, win);
+                        if (windows > 32u) {  // uniform
+                            const uint32_t ih = i - n_lo;  // (only used past n_lo)
+                            uint32_t wh = 0;
+#pragma unroll
+                            for (uint32_t step = 16; step; step >>= 1)
+                                if (__shfl_sync(0xffffffffu, inc_hi, wh + step - 1u) <= ih) wh += step;
+                            const uint32_t rh = ih - __shfl_sync(0xffffffffu, inc_hi - __popc(bits_hi), wh);
+                            const uint32_t bh = __shfl_sync(0xffffffffu, bits_hi, wh);
+                            if (i >= n_lo) {
+                                win = 32u + wh;
+                                rank = rh;
+                                word = bh;
+                            }
+                        }
+                        const bool live = i < count;
+                        const uint32_t s = live ? win * 32u + select_bit(word, rank) : 0u;
                         const int j = owner_lane(gs.off, s);
                         const uint32_t j_off = __shfl_sync(0xffffffffu, gs.off, j);
                         const uint32_t j_first = __shfl_sync(0xffffffffu, gs.first, j);
                         ji[k] = __shfl_sync(0xffffffffu, gs.inst, j);
                         jl[k] = __shfl_sync(0xffffffffu, gs.lod, j);
                         mi[k] = j_first + (s - j_off);
-                        if ((b[k] >> lane) & 1u) d[k] = __ldg(S.m_draw + mi[k]);
+                        if (live) d[k] = __ldg(S.m_draw + mi[k]);
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if ((b[k] >> lane) & 1u) {
-                            const uint32_t slot = slot0 + __popc(b[k] & ((1u << lane) - 1u));
-                            if (slot < cap) {
-                                uint32_t* out = reinterpret_cast<uint32_t*>(indirect + slot);
-                                out[0] = d[k].y;
-                                out[1] = 1u;
-                                out[2] = d[k].x;
-                                out[3] = d[k].z;
-                                out[4] = slot;
-                                reinterpret_cast<uint4*>(draws)[slot] = make_uint4(ji[k], mi[k], jl[k], 0u);
-                            }
-                        }
-                        slot0 += __popc(b[k]);
+                    for (int k = 0; k < 2; ++k) {
+                        const uint32_t i = i0 + 32u * k + lane, slot = slot0 + i;
+                        if (i >= count || slot >= cap) continue;
+                        uint32_t* out = reinterpret_cast<uint32_t*>(indirect + slot);
+                        out[0] = d[k].y;
+                        out[1] = 1u;
+                        out[2] = d[k].x;
+                        out[3] = d[k].z;
+                        out[4] = slot;
+                        reinterpret_cast<uint4*>(draws)[slot] = make_uint4(ji[k], mi[k], jl[k], 0u);
                     }
                 }
             }
