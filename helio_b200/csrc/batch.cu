@@ -86,12 +86,8 @@ constexpr size_t kSmOffs = 1024;                                         // u32[
 constexpr uint32_t kLocalChunks = (uint32_t)((kSmSelLod - kSmOffs) / 4) - 1;
 static_assert(kSmVStart + 4 * (kBatchMaxViews + 1) <= kSmOffs, "the view starts lie below the offsets");
 constexpr size_t kSmTestSpheres = ((kSmTestQueue + 8 * 64 * 2) + 15) / 16 * 16;  // float4[8][64]
-// The cull kernel (phases 4..6) has its own, small layout: the test phase's region
-// from offset 0, then the scan scratch.
-constexpr size_t kSm2Misc = kSmTestSpheres + 8 * 64 * 16;  // u32[64]
-constexpr size_t kSm2Total = kSm2Misc + 64 * 4;
-// Phases 5 and 6 of a small batch: the group offsets, in the test phase's region.
-constexpr uint32_t kLocalGroups = (uint32_t)(kSm2Misc / 4) - 1;
+// The cull kernel (phases 4..6) has its own, small layout: the test phase's region.
+constexpr size_t kSm2Total = kSmTestSpheres + 8 * 64 * 16;
 
 __device__ __forceinline__ uint32_t ld_cg(const uint32_t* p) { return __ldcg(p); }
 
@@ -399,7 +395,7 @@ __device__ void phase_setup(const BatchParams& P) {
             s_c.hiz.mip_count = V.hiz.mip_count;
             s_c.screen_height = V.height;
             s_c.hiz_mip_count = V.hiz_mip_count;
-            s_c.pad[0] = s_c.pad[1] = 0u;
+            s_c.first_span = s_c.pad = 0u;  // (phase_expand sets the first span)
         }
         publish_planes_warp(V.camera.view_proj, s_c.planes);
         float box[6];
@@ -667,7 +663,18 @@ __device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* s
         if (tid == 0) s_vstart[V] = total;
         __syncthreads();
         if (blockIdx.x == 0)
-            for (uint32_t v = tid; v <= V; v += kBatchThreads) P.view_span_start[v] = s_vstart[v];
+            for (uint32_t v = tid; v <= V; v += kBatchThreads) {
+                P.view_span_start[v] = s_vstart[v];
+                if (v < V) P.cviews[v].first_span = s_vstart[v];
+            }
+        // The sums that the tests add to; a group has at least 8 spans.
+        const uint32_t groups = min(total, P.span_capacity) >> 3;
+#pragma unroll
+        for (uint32_t k = 0; k < kGroupSumLevels; ++k) {
+            uint32_t* level = P.group_sums + group_sum_words(P.span_capacity >> 3, V, k);
+            const uint32_t n = (groups >> group_sum_shift(k)) + V + 1u;
+            for (uint32_t i = blockIdx.x * kBatchThreads + tid; i < n; i += gridDim.x * kBatchThreads) level[i] = 0u;
+        }
         if (tid == 0 && total > P.span_capacity) atomicOr(P.error, kBatchErrSpanCapacity);
     }
     // Hi-Z levels 7.. of each view, by warp 0 of CTA v (mod grid), from the level 6
@@ -923,7 +930,13 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift
         uint32_t count = __popc(bits[lane]) + __popc(bits[lane + 32]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-        if (lane == 0) P.group_counts[g] = count;
+        if (count && lane < (int)kGroupSumLevels) {
+            const uint32_t f = cv.first_span >> (5u - shift), k = group_sum_shift(lane);
+            atomicAdd(P.group_sums + group_sum_words(P.span_capacity >> 3, P.view_count, lane) + (f >> k) + gs.view +
+                          ((g - f) >> k),
+                      count);
+        }
+        if (lane == 0) P.group_counts[g] = make_uint2(count | (gs.view << 16), cv.first_span >> (5u - shift));
         if (count)
             for (uint32_t k = lane; k < windows; k += 32)
                 P.group_bits[(size_t)g * (kWindowsPerWarp >> shift) + k] = bits[k];
@@ -936,25 +949,39 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift
 }
 
 // ── Phase 6: emission, per view, in the canonical order ───────────────────────
-// The loads of one group that do not depend on another group's data: its scan offset,
-// lane k's span and lane k's two window ballots (windows k and k + 32; the ballot row has
-// kWindowsPerWarp >> shift entries, read whole and masked to the group's windows later).
+// The loads of one group: lane k's span, lane k's two window ballots (windows k and k + 32; the
+// ballot row has kWindowsPerWarp >> shift entries, read whole and masked to the group's windows
+// later), and lane k's parts of the view's draws before the group.
+// Those draws are not a scan's result: the tests add every group's count to the sums of its runs of
+// 16, 256 and 8,192 groups of the view, and a warp adds up, in one round trip beside its other
+// loads, the counts before the group in its run of 16 (lanes 0..15), the runs of 16 before it in its run
+// of 256 (lanes 16..31), and the runs of 256 in its run of 8,192; only past the view's first 8,192
+// groups also the runs of those.
 struct EmitLoads {
-    uint32_t goff, bits_lo, bits_hi;
+    uint32_t view, before_lo, before_hi, bits_lo, bits_hi;
     ActiveSpan span;
 };
 
-// Draws of the batch before group g: from shared memory in a small batch (no pointer to either
-// place is kept: the cull kernel has no register for it).
-__device__ __forceinline__ uint32_t group_offset(const BatchParams& P, uint32_t groups, uint32_t g) {
-    extern __shared__ __align__(16) char sm[];
-    return groups <= kLocalGroups ? reinterpret_cast<const uint32_t*>(sm)[g] : ld_cg(P.group_offs + g);
-}
-
-__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t groups, uint32_t g, uint32_t shift) {
+// head is the group's entry of P.group_counts.
+__device__ __forceinline__ EmitLoads emit_loads(const BatchParams& P, uint32_t g, uint2 head, uint32_t shift) {
     const uint32_t lane = threadIdx.x & 31, size = 32u >> shift, windows = kWindowsPerWarp >> shift;
+    const uint32_t f = head.y, l = g - f, cap = P.span_capacity >> 3;
     EmitLoads e;
-    e.goff = group_offset(P, groups, g);
+    e.view = head.x >> 16;
+    const uint32_t* runs = P.group_sums + (f >> 4) + e.view;
+    const uint32_t k = lane & 15u;
+    e.before_lo = 0u;
+    if (lane < 16u) {
+        if (k < (l & 15u)) e.before_lo = ld_cg(&P.group_counts[f + (l & ~15u) + k].x) & 0xFFFFu;
+    } else if (k < ((l >> 4) & 15u)) {
+        e.before_lo = ld_cg(runs + ((l >> 4) & ~15u) + k);
+    }
+    runs = P.group_sums + group_sum_words(cap, P.view_count, 1u) + (f >> 8) + e.view;
+    e.before_hi = lane < ((l >> 8) & 31u) ? ld_cg(runs + ((l >> 8) & ~31u) + lane) : 0u;
+    if (l >> 13) {
+        runs = P.group_sums + group_sum_words(cap, P.view_count, 2u) + (f >> 13) + e.view;
+        for (uint32_t i = lane; i < l >> 13; i += 32u) e.before_hi += ld_cg(runs + i);
+    }
     e.span = lane < size ? __ldcg(P.spans + (size_t)g * size + lane) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t* gbits = P.group_bits + (size_t)g * windows;
     e.bits_lo = lane < windows ? ld_cg(gbits + lane) : 0u;
@@ -972,31 +999,32 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift
     // current group's draws are written, so that those round trips overlap the writes.
     for (uint32_t k0 = 0; gw + (size_t)k0 * GW < groups; k0 += 32u) {
         const size_t gl = gw + (size_t)(k0 + lane) * GW;
-        const uint32_t cnt = gl < groups ? ld_cg(P.group_counts + gl) : 0u;
-        uint32_t mask = __ballot_sync(0xffffffffu, cnt != 0u);
+        const uint2 head = gl < groups ? __ldcg(P.group_counts + gl) : make_uint2(0u, 0u);
+        uint32_t mask = __ballot_sync(0xffffffffu, (head.x & 0xFFFFu) != 0u);
         if (!mask) continue;
-        uint32_t g = gw + (k0 + (__ffs(mask) - 1)) * GW;
-        mask &= mask - 1u;
-        EmitLoads cur = emit_loads(P, groups, g, shift);
+        auto next_loads = [&] {
+            const uint32_t k = __ffs(mask) - 1;
+            mask &= mask - 1u;
+            const uint2 h = make_uint2(__shfl_sync(0xffffffffu, head.x, k), __shfl_sync(0xffffffffu, head.y, k));
+            return emit_loads(P, gw + (k0 + k) * GW, h, shift);
+        };
+        EmitLoads cur = next_loads();
         for (;;) {
             const bool more = mask != 0u;
-            const uint32_t g_next = more ? gw + (k0 + (__ffs(mask) - 1)) * GW : 0u;
-            mask &= mask - 1u;
             EmitLoads nxt{};
-            if (more) nxt = emit_loads(P, groups, g_next, shift);
+            if (more) nxt = next_loads();
             // The current group: its spans' packing offsets, then its view's table entry.
             GroupSpans gs;
             gs.n = span_n(cur.span);
             gs.first = cur.span.x;
             gs.inst = cur.span.z;
             gs.lod = span_lod(cur.span);
-            gs.view = __shfl_sync(0xffffffffu, span_view(cur.span), 0);
+            gs.view = cur.view;
             const uint32_t inc = warp_inclusive(gs.n);
             gs.off = inc - gs.n;
             gs.total = __shfl_sync(0xffffffffu, inc, 31);
             if (gs.view < P.view_count) {
                 const BatchViewDev& V = P.views[gs.view];
-                const uint32_t first_group = ld_cg(P.view_span_start + gs.view) >> (5u - shift);
                 const uint32_t cap = V.capacity;
                 HelioDrawIndexedIndirectArgs* indirect = V.indirect;
                 HelioGpuVgDraw* draws = V.draws;
@@ -1008,7 +1036,7 @@ __device__ void phase_emit(const BatchParams& P, uint32_t groups, uint32_t shift
                 const uint32_t inc_hi = windows > 32u ? warp_inclusive(__popc(bits_hi)) : 0u;
                 const uint32_t n_lo = __shfl_sync(0xffffffffu, inc_lo, 31);
                 const uint32_t count = n_lo + __shfl_sync(0xffffffffu, inc_hi, 31);
-                const uint32_t slot0 = cur.goff - group_offset(P, groups, first_group);
+                const uint32_t slot0 = __reduce_add_sync(0xffffffffu, cur.before_lo + cur.before_hi);
                 if (lane == 0) {
                     atomicAdd(counters + 0, count);
                     const unsigned long long end = (unsigned long long)slot0 + count;
@@ -1244,7 +1272,6 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
 // barrier after the expansion.
 __global__ void __launch_bounds__(kBatchThreads, 5) batch_cull_kernel(BatchParams P) {
     extern __shared__ __align__(16) char sm[];
-    uint32_t* s_tmp = reinterpret_cast<uint32_t*>(sm + kSm2Misc);
     // A barrier of the first launch gave up: its span list may be incomplete.
     if (ld_cg(P.error) & kBatchErrTimeout) return;
     stamp(P, 4);
@@ -1254,8 +1281,6 @@ __global__ void __launch_bounds__(kBatchThreads, 5) batch_cull_kernel(BatchParam
     if (!grid_sync(P)) return;
     stamp(P, 5);
 
-    if (groups <= kLocalGroups) local_exclusive_scan(P.group_counts, groups, reinterpret_cast<uint32_t*>(sm), s_tmp);
-    else if (!grid_exclusive_scan(P, P.group_counts, P.group_offs, groups, s_tmp)) return;
     stamp(P, 6);
     phase_emit(P, groups, shift);
     // End of the launch: the latest block end (no barrier needed).

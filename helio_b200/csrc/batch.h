@@ -43,6 +43,18 @@ __host__ __device__ inline uint32_t span_view(const ActiveSpan& s) { return s.y 
 
 enum : uint32_t { kBatchErrTimeout = 1u, kBatchErrSpanCapacity = 2u };
 
+// Sums of the groups' visible meshlets: level k holds runs of 2^group_sum_shift(k) groups, counted
+// from their view's first group f. View v's runs start at entry (f >> shift) + v of the level, so
+// that no run holds groups of two views.
+constexpr uint32_t kGroupSumLevels = 3;
+__host__ __device__ constexpr uint32_t group_sum_shift(uint32_t level) { return level == 0u ? 4u : level == 1u ? 8u : 13u; }
+// Words of the levels below `levels`.
+__host__ __device__ inline uint32_t group_sum_words(uint32_t groups, uint32_t views, uint32_t levels) {
+    uint32_t words = 0;
+    for (uint32_t k = 0; k < levels; ++k) words += (groups >> group_sum_shift(k)) + views + 1u;
+    return words;
+}
+
 struct BatchParams {
     VgSceneDev scene;
     const uint32_t* scene_bounds;  // [2] bounds of launch_scene_update
@@ -71,8 +83,9 @@ struct BatchParams {
     uint32_t* view_span_start;  // [view_count + 1] first span of each view (views padded to 32)
     ActiveSpan* spans;        // [span_capacity]
     uint32_t span_capacity;   // multiple of 32
-    uint32_t* group_counts;   // [span_capacity / 8] visible meshlets per group of 32, 16 or 8 spans
-    uint32_t* group_offs;     // [span_capacity / 8 + 1]
+    uint2* group_counts;      // [span_capacity / 8] per group of 32, 16 or 8 spans: visible meshlets | view << 16,
+                              // the first group of its view
+    uint32_t* group_sums;     // [group_sum_words] visible meshlets per run of groups
     uint32_t* group_bits;     // [span_capacity / 32 * kWindowsPerWarp] window ballots
     uint32_t* span_vis;       // [span_capacity * 2] per-span visibility words, or null
     unsigned long long* phase_ns;  // [kBatchPhaseStamps] %globaltimer at launch and after each phase

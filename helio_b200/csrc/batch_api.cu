@@ -49,7 +49,7 @@ struct helio_batch {
     uint32_t view_count = 0;
     std::vector<helio::BatchViewDev> host_views;
     DevBuf views, cviews, lod, levels, out_indirect, out_draws, clear, chunk_counts, chunk_vis, vis_list, chunk_offs, seg_totals,
-        view_span_start, spans, group_counts, group_offs, group_bits, span_vis;
+        view_span_start, spans, group_counts, group_sums, group_bits, span_vis;
     size_t clear_bytes = 0;
     uint32_t grid = 0, object_chunks = 0, hiz_tiles = 0, span_capacity = 0, lod_pitch = 0;
     std::vector<size_t> out_offset;  // first draw of each view in out_indirect / out_draws
@@ -62,7 +62,7 @@ struct helio_batch {
     DevBuf& buf(int k) {
         DevBuf* all[] = {&levels, &out_indirect, &out_draws, &clear, &views, &cviews, &lod, &chunk_counts,
                          &chunk_vis, &vis_list, &chunk_offs, &seg_totals, &view_span_start, &spans,
-                         &group_counts, &group_offs, &group_bits, &span_vis};
+                         &group_counts, &group_sums, &group_bits, &span_vis};
         return *all[k];
     }
 
@@ -129,7 +129,7 @@ int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects
 // Device buffers of a batch, in helio_batch::buf order.
 enum {
     kBufLevels, kBufIndirect, kBufDraws, kBufClear, kBufViews, kBufCViews, kBufLod, kBufChunkCounts, kBufChunkVis,
-    kBufVisList, kBufChunkOffs, kBufSegTotals, kBufViewSpanStart, kBufSpans, kBufGroupCounts, kBufGroupOffs,
+    kBufVisList, kBufChunkOffs, kBufSegTotals, kBufViewSpanStart, kBufSpans, kBufGroupCounts, kBufGroupSums,
     kBufGroupBits, kBufSpanVis, kBatchBufs
 };
 
@@ -203,8 +203,8 @@ int32_t plan_batch(const helio_batch_config& cfg, const helio_vg_scene* sc, uint
     p.need[kBufSegTotals] = (size_t)std::max(p.grid, helio::batch_cull_max_grid()) * 4;
     p.need[kBufViewSpanStart] = (size_t)(n + 1) * 4;
     p.need[kBufSpans] = (size_t)p.span_capacity * sizeof(helio::ActiveSpan);
-    p.need[kBufGroupCounts] = (groups * 4 + 1) * 4;  // groups of 8 spans at the least
-    p.need[kBufGroupOffs] = (groups * 4 + 1) * 4;
+    p.need[kBufGroupCounts] = groups * 4 * sizeof(uint2);  // groups of 8 spans at the least
+    p.need[kBufGroupSums] = (size_t)helio::group_sum_words((uint32_t)groups * 4u, n, helio::kGroupSumLevels) * 4;
     p.need[kBufGroupBits] = (groups + 1) * helio::kWindowsPerWarp * 4;
     p.need[kBufSpanVis] = (cfg.flags & HELIO_BATCH_SPAN_VISIBILITY) ? (size_t)p.span_capacity * 8 : 0;
     for (size_t& x : p.need) x = x ? x : 16;  // DevBuf::ensure allocates at least 16 bytes
@@ -470,7 +470,7 @@ int32_t helio_batch_device_bytes(const helio_batch* b, uint64_t* bytes) {
     *bytes = b->views.bytes + b->cviews.bytes + b->lod.bytes + b->levels.bytes + b->out_indirect.bytes +
              b->out_draws.bytes + b->clear.bytes + b->chunk_counts.bytes + b->chunk_vis.bytes + b->vis_list.bytes +
              b->chunk_offs.bytes + b->seg_totals.bytes + b->view_span_start.bytes + b->spans.bytes +
-             b->group_counts.bytes + b->group_offs.bytes + b->group_bits.bytes + b->span_vis.bytes;
+             b->group_counts.bytes + b->group_sums.bytes + b->group_bits.bytes + b->span_vis.bytes;
     return HELIO_OK;
 }
 
@@ -544,8 +544,8 @@ int32_t helio_batch_execute(helio_batch* b, void* stream) {
     P.view_span_start = b->view_span_start.as<uint32_t>();
     P.spans = b->spans.as<helio::ActiveSpan>();
     P.span_capacity = b->span_capacity;
-    P.group_counts = b->group_counts.as<uint32_t>();
-    P.group_offs = b->group_offs.as<uint32_t>();
+    P.group_counts = b->group_counts.as<uint2>();
+    P.group_sums = b->group_sums.as<uint32_t>();
     P.group_bits = b->group_bits.as<uint32_t>();
     P.span_vis = (b->cfg.flags & HELIO_BATCH_SPAN_VISIBILITY) ? b->span_vis.as<uint32_t>() : nullptr;
     P.phase_ns = b->stamps();

@@ -63,7 +63,8 @@ struct CullView {
     HizView hiz;
     uint32_t screen_height;
     uint32_t hiz_mip_count;
-    uint32_t pad[2];
+    uint32_t first_span;  // batches: the view's first span in the span list
+    uint32_t pad;
 };
 static_assert(sizeof(CullView) % 16 == 0, "CullView is copied as 16-byte words");
 

@@ -272,7 +272,7 @@ __device__ __forceinline__ void view_setup_warp(const ViewSetupParams& P, CullVi
         v.lod_threshold_px = P.lod_threshold_px;
         v.screen_height = P.screen_height;
         v.hiz_mip_count = P.hiz_mip_count;
-        v.pad[0] = v.pad[1] = 0u;
+        v.first_span = v.pad = 0u;
     }
     __syncwarp();
 }

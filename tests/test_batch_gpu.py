@@ -197,3 +197,18 @@ def test_batch_scan_forms_match_oracle(cuda, views, objects):
     sc = S.make_scene(objects, objects, 3, 4, 0, 40.0)
     w = S.Workload(3, sc, S.multiview_set(S.SEED_BASE + 9, True, 0.05)[5:5 + views])
     _check_batch(w, w.views)
+
+
+@pytest.mark.parametrize("objects,views,cull_ctas", [(480, 3, 1), (512, 3, 1), (544, 3, 1), (8160, 2, 1), (8224, 2, 1),
+                                                     (131073, 1, 0)])
+def test_batch_group_sum_runs_match_oracle(cuda, objects, views, cull_ctas):
+    """A view's draws before a group, from the sums by runs of 16, 256 and 8,192 groups: views of 15, 16, 17,
+    255 and 257 groups of 32 spans, side by side, and one of 8,194 groups of 16."""
+    from helio_b200 import scene as S
+
+    sc = S.make_scene(objects, objects, 1, 1, 0, 40.0)
+    cam = S.orthographic((0, 0, 300), (0, 0, 0), (0, 1, 0), 100.0, 0.1, 600.0)
+    w = S.Workload(3, sc, [S.View(cam, 64, 64, np.ones((64, 64), np.float32), "ortho")] * views)
+    b, _, _ = run_batch(sc, w.views, cull_ctas=cull_ctas)
+    assert (np.diff(u32(b.spans()["view_span_start"]).astype(np.int64)) == (objects + 31) // 32 * 32).all()
+    _check_batch(w, w.views, cull_ctas=cull_ctas)
