@@ -13,7 +13,7 @@
 //      tested against a group of views; per (view, object) the selected LOD + 1 is
 //      stored and per (view, 256-object chunk) the number of active 64-meshlet spans
 //      and of visible objects. An object whose world centre lies outside a view's
-//      reject box fails that view's sphere test for certain (see reject_box_warp)
+//      reject box fails that view's sphere test for certain (see the reject box below)
 //      and skips it; the remaining (object, view) pairs are compacted per warp into
 //      full 32-lane batches for the exact test and the LOD choice
 //   2  exclusive scan of the (view, chunk) span counts
@@ -272,36 +272,80 @@ __device__ __forceinline__ PlaneD pushed_plane(const Planes& pl, int i, double r
     return q;
 }
 
-// s_q: six planes of shared memory, one built by each of lanes 0..5 (a double square root apiece,
-// where every use of a length had one of its own).
-__device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, PlaneD* s_q, float box[6]) {
+// Three-bit digits: digit k of kTripleA / B / C and kPairA / B are the planes of the k-th triple
+// a < b < c and the k-th pair a < b.
+constexpr uint64_t combination_digits(int size, int which) {
+    uint64_t digits = 0;
+    int k = 0;
+    for (int a = 0; a < 6; ++a)
+        for (int b = a + 1; b < 6; ++b)
+            for (int c = b + 1; c < (size == 3 ? 6 : b + 2); ++c, ++k)
+                digits |= (uint64_t)(which == 0 ? a : which == 1 ? b : c) << (3 * k);
+    return digits;
+}
+constexpr uint64_t kTripleA = combination_digits(3, 0), kTripleB = combination_digits(3, 1),
+                   kTripleC = combination_digits(3, 2), kPairA = combination_digits(2, 0),
+                   kPairB = combination_digits(2, 1);
+__device__ __forceinline__ int digit(uint64_t digits, int k) { return (int)(digits >> (3 * k)) & 7; }
+
+// An order-preserving map of floats (no NaN) to unsigned integers, and back.
+__device__ __forceinline__ uint32_t float_key(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+}
+__device__ __forceinline__ float key_float(uint32_t k) {
+    return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+}
+
+// The planes with pushed-out offsets into s_q, one built by each of lanes 0..5; false if an input
+// is not finite.
+__device__ bool pushed_planes_warp(const Planes& pl, float rmax, float cl1, PlaneD* s_q) {
     const int lane = threadIdx.x & 31;
-    bool finite = isfinite(rmax_f) && isfinite(cl1_f);
-    const double rmax = rmax_f, cl1 = cl1_f;
+    bool finite = isfinite(rmax) && isfinite(cl1);
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         const float4 p = pl.p[i];
         finite = finite && isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(p.w);
     }
+    if (lane < 6) s_q[lane] = pushed_plane(pl, lane, rmax, cl1);
+    __syncwarp();
+    return finite;
+}
+
+// True if Q is unbounded.
+__device__ bool reject_box_unbounded_warp(const PlaneD* s_q) {
+    const int lane = threadIdx.x & 31;
+    bool bad = false;
+    if (lane < 15) {
+        const PlaneD A = s_q[digit(kPairA, lane)], B = s_q[digit(kPairB, lane)];
+        const double d[3] = {A.y * B.z - A.z * B.y, A.z * B.x - A.x * B.z, A.x * B.y - A.y * B.x};
+        const double len = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        if (len > 1e-12 * A.len * B.len) {
+            bool up = true, down = true;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const PlaneD q = s_q[j];
+                const double along = q.x * d[0] + q.y * d[1] + q.z * d[2], tol = -1e-9 * q.len * len;
+                up = up && along >= tol;
+                down = down && -along >= tol;
+            }
+            bad = up || down;
+        }
+    }
+    return __any_sync(0xffffffffu, bad);
+}
+
+// The bounds of Q's vertices, rounded outward to float, in lo and hi; false if the box has to be
+// disabled for what the triples show.
+__device__ bool reject_box_vertices_warp(const PlaneD* s_q, float lo[3], float hi[3]) {
+    const int lane = threadIdx.x & 31;
     auto scale = [&](const PlaneD& q, double x, double y, double z) {
         return (fabs(x) + fabs(y) + fabs(z)) * q.len + fabs(q.w) + 1e-30;
     };
-    if (lane < 6) s_q[lane] = pushed_plane(pl, lane, rmax, cl1);
-    __syncwarp();
-    bool bad = !finite;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    if (finite && lane < 20) {
-        // lane -> (a < b < c)
-        int a = 0, b = 1, c = 2;
-        for (int k = 0; k < lane; ++k) {
-            if (++c == 6) {
-                if (++b == 5) {
-                    ++a;
-                    b = a + 1;
-                }
-                c = b + 1;
-            }
-        }
+    bool bad = false, vertex = false;
+    double p[3] = {0.0, 0.0, 0.0};
+    if (lane < 20) {
+        const int a = digit(kTripleA, lane), b = digit(kTripleB, lane), c = digit(kTripleC, lane);
         const PlaneD A = s_q[a], B = s_q[b], Cc = s_q[c];
         const double bc[3] = {B.y * Cc.z - B.z * Cc.y, B.z * Cc.x - B.x * Cc.z, B.x * Cc.y - B.y * Cc.x};
         const double ca[3] = {Cc.y * A.z - Cc.z * A.y, Cc.z * A.x - Cc.x * A.z, Cc.x * A.y - Cc.y * A.x};
@@ -309,7 +353,6 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, Pla
         const double det = A.x * bc[0] + A.y * bc[1] + A.z * bc[2];
         const double rel = fabs(det) / (A.len * B.len * Cc.len + 1e-300);
         const bool corner = a < 2 && b >= 2 && b < 4 && c >= 4;
-        double p[3] = {0.0, 0.0, 0.0};
         bool feasible = false, loose = false;
         if (rel > 1e-12) {
 #pragma unroll
@@ -324,63 +367,31 @@ __device__ void reject_box_warp(const Planes& pl, float rmax_f, float cl1_f, Pla
                 loose = loose && sl >= -1e-3 * sc;
             }
         }
-        if (corner && !(rel > 1e-4 && feasible)) bad = true;
-        if (!corner && rel > 1e-12 && rel <= 1e-4 && loose) bad = true;
-        if (rel > 1e-4 && feasible)
-            for (int k = 0; k < 3; ++k) lo[k] = hi[k] = p[k];
+        bad = (corner && !(rel > 1e-4 && feasible)) || (!corner && rel > 1e-12 && rel <= 1e-4 && loose);
+        vertex = rel > 1e-4 && feasible;
     }
-    if (finite && lane < 15) {
-        int a = 0, b = 1;
-        for (int k = 0; k < lane; ++k)
-            if (++b == 6) {
-                ++a;
-                b = a + 1;
-            }
-        const PlaneD A = s_q[a], B = s_q[b];
-        const double d[3] = {A.y * B.z - A.z * B.y, A.z * B.x - A.x * B.z, A.x * B.y - A.y * B.x};
-        const double len = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-        if (len > 1e-12 * A.len * B.len) {
-            for (int sgn = -1; sgn <= 1; sgn += 2) {
-                bool ray = true;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const PlaneD q = s_q[j];
-                    ray = ray && sgn * (q.x * d[0] + q.y * d[1] + q.z * d[2]) >= -1e-9 * q.len * len;
-                }
-                if (ray) bad = true;
-            }
-        }
-    }
-    bad = __any_sync(0xffffffffu, bad);
+    // Rounding is monotone, so that the least of the rounded values is the least value rounded.
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-            hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
-        }
-        if (bad || !(lo[k] <= hi[k])) {
-            box[k] = -INFINITY;
-            box[3 + k] = INFINITY;
-        } else {
-            const double pad = 1e-6 * (fabs(lo[k]) + fabs(hi[k]) + rmax + 1.0);
-            box[k] = __double2float_rd(lo[k] - pad);
-            box[3 + k] = __double2float_ru(hi[k] + pad);
-        }
+        lo[k] = key_float(__reduce_min_sync(0xffffffffu, float_key(vertex ? __double2float_rd(p[k]) : INFINITY)));
+        hi[k] = key_float(__reduce_max_sync(0xffffffffu, float_key(vertex ? __double2float_ru(p[k]) : -INFINITY)));
     }
+    return !__any_sync(0xffffffffu, bad);
 }
 
 // ── Phase 0: view constants ──────────────────────────────────────────────────
-// One warp per view. The constants are put together in shared memory by all lanes and stored
-// as 16-byte words; lane 0 then publishes the view.
+// One warp per view. The constants are put together in shared memory by all lanes and stored as
+// 16-byte words; lane 0 then publishes the view. The select units of a small batch wait for this: a
+// serial chain of loads and double-precision divisions and roots (5.1 us with 46 views, 7.2 when the
+// planes of a lane's triple were counted up in loops and the bounds reduced as doubles).
 __device__ void phase_setup(const BatchParams& P) {
     __shared__ CullView s_c;
     __shared__ PlaneD s_q[6];
     if (threadIdx.x >= 32) return;
-    const uint32_t lane = threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t v = blockIdx.x; v < P.view_count; v += gridDim.x) {
         BatchViewDev& V = P.views[v];
-        const uint32_t rad = __ldg(P.scene_bounds), far1 = __ldg(P.scene_bounds + 1);
+        const float rmax = __uint_as_float(__ldg(P.scene_bounds)), cl1 = __uint_as_float(__ldg(P.scene_bounds + 1));
         if (lane >= 8 && lane < 8 + HELIO_HIZ_MAX_MIPS) {
             const uint32_t l = lane - 8;
             s_c.hiz.level[l] = HizLevel{V.hiz.levels[l], V.hiz.lw[l], V.hiz.lh[l]};
@@ -398,17 +409,22 @@ __device__ void phase_setup(const BatchParams& P) {
             s_c.first_span = s_c.pad = 0u;  // (phase_expand sets the first span)
         }
         publish_planes_warp(V.camera.view_proj, s_c.planes);
-        float box[6];
-        reject_box_warp(s_c.planes, __uint_as_float(rad), __uint_as_float(far1), s_q, box);
         const uint4* src = reinterpret_cast<const uint4*>(&s_c);
         uint4* dst = reinterpret_cast<uint4*>(P.cviews + v);
         for (uint32_t k = lane; k < sizeof(CullView) / 16; k += 32u) dst[k] = src[k];
+        float lo[3], hi[3];
+        const bool finite = pushed_planes_warp(s_c.planes, rmax, cl1, s_q);
+        bool use = reject_box_vertices_warp(s_q, lo, hi) && finite;
+        use = use && !reject_box_unbounded_warp(s_q);
 #pragma unroll
-        for (uint32_t k = 0; k < 6; ++k)
-            if (lane == k) V.reject_box[k] = box[k];
+        for (int k = 0; k < 3; ++k) {
+            const bool on = use && lo[k] <= hi[k];
+            const double pad = 1e-6 * ((double)fabsf(lo[k]) + (double)fabsf(hi[k]) + (double)rmax + 1.0);
+            if ((int)lane == k) V.reject_box[k] = on ? __double2float_rd((double)lo[k] - pad) : -INFINITY;
+            if ((int)lane == 3 + k) V.reject_box[3 + k] = on ? __double2float_ru((double)hi[k] + pad) : INFINITY;
+        }
         __syncwarp();
         if (lane == 0) red_add_release(P.setup_done, 1u);  // the select units wait for every view
-        __syncwarp();
     }
 }
 
@@ -1177,7 +1193,10 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
         // Hi-Z tiles (memory bound) and select units (arithmetic bound) are spread
         // evenly through one work queue, so that the CTAs sharing an SM overlap the two
         // kinds of work and CTAs that draw cheap units draw more of them. Thread 0
-        // claims the next unit while the block works on the current one. The first h0
+        // claims the next unit while the block works on the current one, unless the queue is short
+        // (up to six units per CTA): there a CTA's second unit is often a long one, a select unit after a
+        // wait for the setup, that another CTA has time for (40 views at 0.38 of their full sizes: 66.4 ->
+        // 62.9 us a pass; long queues are 1 us slower without the claim ahead). The first h0
         // units are Hi-Z tiles (two per CTA: time for the view setup to finish); the
         // last h1 units are Hi-Z tiles too (the cheaper kind, so that the queue ends on
         // short units); between them, unit h0 + u is a select unit iff
@@ -1195,6 +1214,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
         if (threadIdx.x == 0) {
             *s_unit = atomicAdd(P.work, 1u);
             s_tmp[0] = ~0u;  // no HizJob in shared memory yet
+            s_tmp[9] = units + P.shadow_blocks > 6u * gridDim.x;
         }
         __syncthreads();
         unsigned long long t_hiz = 0, t_sel = 0, t0, t1;
@@ -1209,12 +1229,12 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
             const uint32_t q = *s_unit;
             if (q >= queue) break;
             uint32_t next = 0;
-            if (threadIdx.x == 0) next = atomicAdd(P.work, 1u);
+            if (threadIdx.x == 0 && s_unit[1]) next = atomicAdd(P.work, 1u);
             if (S && (q + 1u) % K == 0u && (q + 1u) / K <= S) {
                 shadow_test_block(P.shadow, (q + 1u) / K - 1u, 0u, 1u,
                                   *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
                 __syncthreads();  // every thread has read *s_unit
-                if (threadIdx.x == 0) *s_unit = next;
+                if (threadIdx.x == 0) *s_unit = s_unit[1] ? next : atomicAdd(P.work, 1u);
                 __syncthreads();
                 continue;
             }
@@ -1238,7 +1258,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
             (is_hiz ? t_hiz : t_sel) += t1 - t0;
             __syncthreads();  // every thread has read *s_unit
-            if (threadIdx.x == 0) *s_unit = next;
+            if (threadIdx.x == 0) *s_unit = s_unit[1] ? next : atomicAdd(P.work, 1u);
             __syncthreads();
         }
         if (threadIdx.x == 0) {
