@@ -15,8 +15,9 @@
 //      and of visible objects. An object whose world centre lies outside a view's
 //      reject box fails that view's sphere test for certain (see the reject box below)
 //      and skips it; the remaining (object, view) pairs are compacted per warp into
-//      full 32-lane batches for the exact test and the LOD choice
-//   2  exclusive scan of the (view, chunk) span counts
+//      full 32-lane batches for the exact test and the LOD choice (the span counts
+//      are also added to sums over runs of a view's chunks)
+//   2  the scan stage of an attached shadow cull
 //   3  expansion into one list of active spans, view-major, each view padded to a
 //      multiple of 32 spans so every group of 32 spans belongs to one view
 //   4  meshlet tests: a warp takes a group of 32 spans (16 or 8 in small batches) and packs
@@ -81,10 +82,7 @@ constexpr size_t kSmTestBits = kSmTestViews + sizeof(CullView) * 8;      // u32[
 constexpr int kBits = kWindowsPerWarp + 2;
 constexpr size_t kSmTestQueue = kSmTestBits + 8 * kBits * 4;            // u16[8][64]
 constexpr size_t kSmVStart = 0;                                          // u32[kBatchMaxViews + 1]
-// Phases 2 and 3 of a small batch: the chunk offsets in shared memory (local_exclusive_scan).
-constexpr size_t kSmOffs = 1024;                                         // u32[kLocalChunks + 1]
-constexpr uint32_t kLocalChunks = (uint32_t)((kSmSelLod - kSmOffs) / 4) - 1;
-static_assert(kSmVStart + 4 * (kBatchMaxViews + 1) <= kSmOffs, "the view starts lie below the offsets");
+static_assert(kSmVStart + 4 * (kBatchMaxViews + 1) <= kSmSelLod, "the view starts lie in the select's region");
 constexpr size_t kSmTestSpheres = ((kSmTestQueue + 8 * 64 * 2) + 15) / 16 * 16;  // float4[8][64]
 // The cull kernel (phases 4 and 5) has its own, small layout: the test phase's region.
 constexpr size_t kSm2Total = kSmTestSpheres + 8 * 64 * 16;
@@ -149,20 +147,6 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
     return x;
 }
 
-// Sum over the CTA; every thread gets the result. s: 9 words of shared memory.
-__device__ uint32_t block_sum(uint32_t x, uint32_t* s) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    __syncthreads();
-    if (lane == 0) s[warp] = x;
-    __syncthreads();
-    uint32_t t = 0;
-#pragma unroll
-    for (int w = 0; w < (int)(kBatchThreads / 32); ++w) t += s[w];
-    return t;
-}
-
 // Exclusive scan over the CTA; `total` receives the CTA sum. s: 9 words.
 __device__ uint32_t block_exclusive(uint32_t x, uint32_t* s, uint32_t& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -179,62 +163,6 @@ __device__ uint32_t block_exclusive(uint32_t x, uint32_t* s, uint32_t& total) {
         total += t;
     }
     return before + inc - x;
-}
-
-// out[i] = sum of in[0..i) for i <= n, over the whole grid (two grid barriers).
-// Returns false when a barrier timed out (the CTA must end).
-__device__ bool grid_exclusive_scan(const BatchParams& P, const uint32_t* in, uint32_t* out, uint32_t n,
-                                    uint32_t* s_tmp) {
-    const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-    const uint32_t seg = (n + G - 1) / G;
-    const uint32_t b0 = min(n, b * seg), b1 = min(n, b0 + seg);
-    uint32_t sum = 0;
-    for (uint32_t i = b0 + tid; i < b1; i += kBatchThreads) sum += ld_cg(in + i);
-    sum = block_sum(sum, s_tmp);
-    if (tid == 0) P.seg_totals[b] = sum;
-    if (!grid_sync(P)) return false;
-    uint32_t base = 0;
-    for (uint32_t k = tid; k < b; k += kBatchThreads) base += ld_cg(P.seg_totals + k);
-    base = block_sum(base, s_tmp);
-    for (uint32_t t0 = b0; t0 < b1; t0 += kBatchThreads) {
-        const uint32_t i = t0 + tid;
-        const uint32_t x = i < b1 ? ld_cg(in + i) : 0u;
-        uint32_t total;
-        const uint32_t ex = block_exclusive(x, s_tmp, total);
-        if (i < b1) out[i] = base + ex;
-        base += total;
-    }
-    if (b == G - 1 && tid == 0) out[n] = base;
-    return grid_sync(P);
-}
-
-// The same sums in shared memory (n + 1 words of s_out), by every CTA for itself: no grid barrier
-// after the one that ended the phase of the counts. For counts that fit a CTA's shared memory; at a
-// few thousand, loading them costs each CTA one round trip where the two barriers cost 5 us.
-__device__ void local_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* s_out, uint32_t* s_tmp) {
-    const uint32_t tid = threadIdx.x;
-    constexpr uint32_t kPer = 8;  // counts per thread and round
-    uint32_t base = 0;
-    for (uint32_t t0 = 0; t0 < n; t0 += kPer * kBatchThreads) {
-        uint32_t x[kPer], sum = 0, total;
-#pragma unroll
-        for (uint32_t k = 0; k < kPer; ++k) {
-            const uint32_t i = t0 + tid * kPer + k;
-            x[k] = i < n ? ld_cg(in + i) : 0u;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kPer; ++k) sum += x[k];
-        uint32_t at = base + block_exclusive(sum, s_tmp, total);
-#pragma unroll
-        for (uint32_t k = 0; k < kPer; ++k) {
-            const uint32_t i = t0 + tid * kPer + k;
-            if (i < n) s_out[i] = at;
-            at += x[k];
-        }
-        base += total;
-    }
-    if (tid == 0) s_out[n] = base;
-    __syncthreads();
 }
 
 // ── Reject box of a view ──────────────────────────────────────────────────────
@@ -483,6 +411,12 @@ __device__ void phase_hiz_tile(const BatchParams& P, uint32_t tile, char* sm) {
     else if (threadIdx.x == 32 && has1) hiz_quad_level6(J, t1, s_l5 + 4);
 }
 
+// The sums over runs of chunks that the select keeps, level by level (0: 32 chunks, 1: 1,024).
+__device__ __forceinline__ uint32_t* chunk_sum_row(const BatchParams& P, uint32_t v, uint32_t level) {
+    const uint32_t n0 = chunk_runs(P.object_chunks, 0u), n1 = chunk_runs(P.object_chunks, 1u);
+    return P.chunk_sums + (level ? (size_t)P.view_count * n0 + (size_t)v * n1 : (size_t)v * n0);
+}
+
 // ── Phase 1b: object select against a group of views (vg_cull.wgsl:282-352) ──
 // Unit = (256-object chunk, group of at most kSelectMaxViews views); lane j of warp
 // w holds object chunk * 256 + 32 w + j. Each lane tests its object's world centre
@@ -583,6 +517,8 @@ __device__ void select_write_lists(const BatchParams& P, uint32_t chunk, uint32_
     if (w == 7u) {
         P.chunk_counts[u] = s_spans[k];
         P.chunk_vis[u] = inc;
+    } else if (w < 2u && s_spans[k]) {
+        atomicAdd(chunk_sum_row(P, v, w) + (chunk >> (w ? 10u : 5u)), s_spans[k]);
     }
     const uint32_t* st = s_stats + k * 9u;
     uint32_t* counters = P.views[v].counters;
@@ -659,19 +595,55 @@ __device__ void phase_select_chunk(const BatchParams& P, uint32_t chunk, uint32_
 }
 
 // ── Phase 3: expansion into the view-major list of active spans ──────────────
-// offs: the chunk offsets in shared memory, or null (then P.chunk_offs holds them).
-__device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* sm) {
+// Active spans of the view before the chunk, for the (view, chunk) units of lanes 0..7, four lanes
+// to a unit: the counts of the chunk's run of 32 and the runs of 32 of its run of 1,024, all in
+// flight together, and the runs of 1,024. Every lane takes part; the units of `live` lanes count.
+// The select adds to the runs, so that no scan stands between it and the expansion: a scan over the
+// grid cost two grid barriers (6.8 us of a pass of 35 to 85 views, whose expansion is 1.5 to 2.5 us
+// longer for this: passes of 74 views over 22,871 instances 66.5 -> 60.9 us, of 85 over 200,000
+// 224.3 -> 221.9), and one by each CTA for itself, in shared memory, was no faster for the
+// smallest batches (27 views, 486 counts: 52.2 us either way) and slower above (35 views, 4,620
+// counts: 65 -> 59).
+__device__ __forceinline__ uint32_t chunk_prefixes(const BatchParams& P, uint32_t v, uint32_t ch, bool live) {
+    static_assert(kExpandBatch == 8, "four lanes to a unit");
+    const uint32_t lane = threadIdx.x & 31u, j = lane >> 2, part = lane & 3u;
+    const uint32_t vj = __shfl_sync(0xffffffffu, v, j), cj = __shfl_sync(0xffffffffu, ch, j);
+    const uint32_t* counts = P.chunk_counts + (size_t)vj * P.object_chunks + (cj & ~31u);
+    const uint32_t* runs = chunk_sum_row(P, vj, 0u) + ((cj >> 5) & ~31u);
+    const bool on = __shfl_sync(0xffffffffu, (int)live, j);
+    const uint32_t nc = on ? cj & 31u : 0u, nr = on ? (cj >> 5) & 31u : 0u;
+    uint32_t x = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 32u; k += 4u) {
+        if (k + part < nc) x += ld_cg(counts + k + part);
+        if (k + part < nr) x += ld_cg(runs + k + part);
+    }
+    if (on)
+        for (uint32_t k = part; k < cj >> 10; k += 4u) x += ld_cg(chunk_sum_row(P, vj, 1u) + k);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    return __shfl_sync(0xffffffffu, x, (lane & 7u) * 4u);
+}
+
+// Active spans of view v in its first `runs` runs of 1,024 chunks.
+__device__ __forceinline__ uint32_t chunk_runs_total(const BatchParams& P, uint32_t v, uint32_t runs) {
+    const uint32_t* top = chunk_sum_row(P, v, 1u);
+    uint32_t total = 0;
+    for (uint32_t i = 0; i < runs; ++i) total += ld_cg(top + i);
+    return total;
+}
+
+__device__ void phase_expand(const BatchParams& P, char* sm) {
     uint32_t* s_vstart = reinterpret_cast<uint32_t*>(sm + kSmVStart);
     uint32_t* s_tmp = reinterpret_cast<uint32_t*>(sm + kSmMisc);
     const uint32_t V = P.view_count, C = P.object_chunks, tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
-    auto offset_of = [&](size_t i) { return offs ? offs[i] : ld_cg(P.chunk_offs + i); };
+    auto spans_of = [&](uint32_t v) { return chunk_runs_total(P, v, chunk_runs(C, 1u)); };
     // Padded first span of every view (a multiple of 32).
     {
         uint32_t padded = 0;
         if (tid < V) {
-            const uint32_t a = offset_of((size_t)tid * C), e = offset_of((size_t)(tid + 1) * C);
-            padded = (e - a + 31u) & ~31u;
+            padded = (spans_of(tid) + 31u) & ~31u;
         }
         uint32_t total;
         const uint32_t ex = block_exclusive(padded, s_tmp, total);
@@ -742,8 +714,8 @@ __device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* s
         const uint32_t vis = live ? ld_cg(P.chunk_vis + u) : 0u;
         if (!__any_sync(0xffffffffu, vis != 0u)) continue;
         const uint32_t v = live ? (uint32_t)(u / C) : 0u, ch = live ? (uint32_t)(u - (size_t)v * C) : 0u;
-        uint32_t pos = 0;  // the unit's first span in the view-major list
-        if (vis) pos = s_vstart[v] + (offset_of(u) - offset_of((size_t)v * C));
+        // The unit's first span in the view-major list.
+        const uint32_t pos = s_vstart[v] + chunk_prefixes(P, v, ch, vis != 0u);
         const uint32_t inc_vis = warp_inclusive(vis);
         const uint32_t first_e = inc_vis - vis, total = __shfl_sync(0xffffffffu, inc_vis, 31);
         uint32_t written = 0;  // spans this lane's unit has written in earlier rounds
@@ -752,7 +724,6 @@ __device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* s
             const int j = owner_lane(first_e, e);  // the unit (lane) owning entry e
             const uint32_t jfirst = __shfl_sync(0xffffffffu, first_e, j);
             const uint32_t jv = __shfl_sync(0xffffffffu, v, j), jch = __shfl_sync(0xffffffffu, ch, j);
-            const uint32_t jpos = __shfl_sync(0xffffffffu, pos, j), jdone = __shfl_sync(0xffffffffu, written, j);
             const size_t ju = bq + (size_t)j * NB;
             uint32_t count = 0, first = 0, inst = 0, lod = 0, o = 0;
             if (e < total) {
@@ -771,6 +742,7 @@ __device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* s
             // Every lane takes part in the shuffle (its source differs per lane).
             const uint32_t inc_before_lead = __shfl_sync(0xffffffffu, inc, lead ? lead - 1u : 0u);
             const uint32_t before = lead ? inc_before_lead : 0u;
+            const uint32_t jpos = __shfl_sync(0xffffffffu, pos, j), jdone = __shfl_sync(0xffffffffu, written, j);
             uint32_t p = jpos + jdone + (inc - ns - before);
             for (uint32_t q = 0; q < ns; ++q, ++p) {
                 if (p < P.span_capacity)
@@ -786,8 +758,7 @@ __device__ void phase_expand(const BatchParams& P, const uint32_t* offs, char* s
     }
     // Padding spans (n = 0) complete every view to a multiple of 32.
     for (uint32_t v = blockIdx.x; v < V; v += gridDim.x) {
-        const uint32_t end = offset_of((size_t)(v + 1) * C) - offset_of((size_t)v * C);
-        for (uint32_t p = s_vstart[v] + end + tid; p < s_vstart[v + 1]; p += kBatchThreads)
+        for (uint32_t p = s_vstart[v] + spans_of(v) + tid; p < s_vstart[v + 1]; p += kBatchThreads)
             if (p < P.span_capacity) P.spans[p] = make_uint4(0u, v << 16, 0u, 0u);
     }
     // The attached shadow cull's placement: after their expansion, CTAs claim blocks of
@@ -1269,24 +1240,15 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
     if (!grid_sync(P)) return;
     stamp(P, 2);
     // The attached shadow cull's scan: CTA j takes the j-th chunk of dirty faces, CTA 0 also
-    // clears the clean faces' counts; done before the phase's last barrier (so an attached pass
-    // always takes the scan with barriers).
+    // clears the clean faces' counts; the placement, after the expansion, needs all of it.
     if (P.shadow_blocks) {
         if (blockIdx.x == 0) shadow_clear_clean(P.shadow);
         for (uint32_t j = blockIdx.x; j < kShadowChunks; j += gridDim.x)
             shadow_scan_chunk(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
-    }
-
-    const uint32_t n_chunks = P.view_count * P.object_chunks;
-    uint32_t* offs = n_chunks <= kLocalChunks && P.shadow_blocks == 0u ? reinterpret_cast<uint32_t*>(sm + kSmOffs) : nullptr;
-    if (offs) {
-        __syncthreads();  // the region is the select's
-        local_exclusive_scan(P.chunk_counts, n_chunks, offs, s_tmp);
-    } else if (!grid_exclusive_scan(P, P.chunk_counts, P.chunk_offs, n_chunks, s_tmp)) {
-        return;
+        if (!grid_sync(P)) return;
     }
     stamp(P, 3);
-    phase_expand(P, offs, sm);
+    phase_expand(P, sm);
 }
 
 // Phases 4 and 5 as a second cooperative launch: the meshlet tests need fewer registers

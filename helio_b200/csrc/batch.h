@@ -55,6 +55,13 @@ __host__ __device__ inline uint32_t group_sum_words(uint32_t groups, uint32_t vi
     return words;
 }
 
+// Sums of the active spans over runs of 32 and of 1,024 chunks of a view: the runs of all views,
+// view after view, level 0 first.
+__host__ __device__ inline uint32_t chunk_runs(uint32_t chunks, uint32_t level) { return (chunks >> (5u + 5u * level)) + 1u; }
+__host__ __device__ inline size_t chunk_sum_words(uint32_t chunks, uint32_t views) {
+    return (size_t)views * (chunk_runs(chunks, 0u) + chunk_runs(chunks, 1u));
+}
+
 struct BatchParams {
     VgSceneDev scene;
     const uint32_t* scene_bounds;  // [2] bounds of launch_scene_update
@@ -78,8 +85,7 @@ struct BatchParams {
     uint32_t* chunk_vis;      // [view_count * object_chunks] visible objects per (view, chunk)
     uint16_t* vis_list;       // [view_count * object_chunks * kBatchChunk] per (view, chunk): its
                               // visible objects in object order, slot | LOD << 8
-    uint32_t* chunk_offs;     // [view_count * object_chunks + 1]
-    uint32_t* seg_totals;     // [gridDim.x]
+    uint32_t* chunk_sums;     // [chunk_sum_words] active spans per run of a view's chunks, zero before the launch
     uint32_t* view_span_start;  // [view_count + 1] first span of each view (views padded to 32)
     ActiveSpan* spans;        // [span_capacity]
     uint32_t span_capacity;   // multiple of 32

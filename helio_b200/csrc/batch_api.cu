@@ -48,7 +48,7 @@ struct helio_batch {
     const helio_vg_scene* scene = nullptr;
     uint32_t view_count = 0;
     std::vector<helio::BatchViewDev> host_views;
-    DevBuf views, cviews, lod, levels, out_indirect, out_draws, clear, chunk_counts, chunk_vis, vis_list, chunk_offs, seg_totals,
+    DevBuf views, cviews, lod, levels, out_indirect, out_draws, clear, chunk_counts, chunk_vis, vis_list,
         view_span_start, spans, group_counts, group_sums, group_bits, span_vis;
     size_t clear_bytes = 0;
     uint32_t grid = 0, object_chunks = 0, hiz_tiles = 0, span_capacity = 0, lod_pitch = 0;
@@ -61,13 +61,13 @@ struct helio_batch {
     // Buffer k of the plan's order (kBuf* below).
     DevBuf& buf(int k) {
         DevBuf* all[] = {&levels, &out_indirect, &out_draws, &clear, &views, &cviews, &lod, &chunk_counts,
-                         &chunk_vis, &vis_list, &chunk_offs, &seg_totals, &view_span_start, &spans,
+                         &chunk_vis, &vis_list, &view_span_start, &spans,
                          &group_counts, &group_sums, &group_bits, &span_vis};
         return *all[k];
     }
 
     // Cleared region: counters (16 words per view) | barrier (2) | error (1) |
-    // work queue (1) | phase stamps (u64, 8-byte aligned).
+    // work queue (1) | phase stamps (u64, 8-byte aligned) | sums over runs of chunks.
     uint32_t* counters(uint32_t v) const { return clear.as<uint32_t>() + 16u * v; }
     uint32_t* barrier() const { return clear.as<uint32_t>() + 16u * view_count; }
     uint32_t* error() const { return barrier() + 2; }
@@ -80,6 +80,7 @@ struct helio_batch {
     unsigned long long* stamps() const {
         return reinterpret_cast<unsigned long long*>(clear.as<char>() + stamps_offset());
     }
+    uint32_t* chunk_sums() const { return reinterpret_cast<uint32_t*>(stamps() + helio::kBatchPhaseStamps); }
 };
 
 namespace {
@@ -129,7 +130,7 @@ int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects
 // Device buffers of a batch, in helio_batch::buf order.
 enum {
     kBufLevels, kBufIndirect, kBufDraws, kBufClear, kBufViews, kBufCViews, kBufLod, kBufChunkCounts, kBufChunkVis,
-    kBufVisList, kBufChunkOffs, kBufSegTotals, kBufViewSpanStart, kBufSpans, kBufGroupCounts, kBufGroupSums,
+    kBufVisList, kBufViewSpanStart, kBufSpans, kBufGroupCounts, kBufGroupSums,
     kBufGroupBits, kBufSpanVis, kBatchBufs
 };
 
@@ -192,15 +193,14 @@ int32_t plan_batch(const helio_batch_config& cfg, const helio_vg_scene* sc, uint
     p.need[kBufLevels] = level_floats * sizeof(float);
     p.need[kBufIndirect] = p.out_offset[n] * sizeof(HelioDrawIndexedIndirectArgs);
     p.need[kBufDraws] = p.out_offset[n] * sizeof(HelioGpuVgDraw);
-    p.need[kBufClear] = (((16u * n + 8u) * 4u + 7u) & ~(size_t)7u) + helio::kBatchPhaseStamps * 8u;
+    p.need[kBufClear] = (((16u * n + 8u) * 4u + 7u) & ~(size_t)7u) + helio::kBatchPhaseStamps * 8u +
+                        helio::chunk_sum_words(p.object_chunks, n) * 4u;
     p.need[kBufViews] = n * sizeof(helio::BatchViewDev);
     p.need[kBufCViews] = n * sizeof(helio::CullView);
     p.need[kBufLod] = (size_t)n * (p.lod_pitch ? p.lod_pitch : helio::kBatchChunk);
     p.need[kBufChunkCounts] = (units + 1) * 4;
     p.need[kBufChunkVis] = (units + 1) * 4;
     p.need[kBufVisList] = std::max<size_t>(1, units) * helio::kBatchChunk * sizeof(uint16_t);
-    p.need[kBufChunkOffs] = (units + 1) * 4;
-    p.need[kBufSegTotals] = (size_t)std::max(p.grid, helio::batch_cull_max_grid()) * 4;
     p.need[kBufViewSpanStart] = (size_t)(n + 1) * 4;
     p.need[kBufSpans] = (size_t)p.span_capacity * sizeof(helio::ActiveSpan);
     p.need[kBufGroupCounts] = groups * 4 * sizeof(uint2);  // groups of 8 spans at the least
@@ -469,7 +469,7 @@ int32_t helio_batch_device_bytes(const helio_batch* b, uint64_t* bytes) {
     HELIO_ARG(b && bytes, "null pointer");
     *bytes = b->views.bytes + b->cviews.bytes + b->lod.bytes + b->levels.bytes + b->out_indirect.bytes +
              b->out_draws.bytes + b->clear.bytes + b->chunk_counts.bytes + b->chunk_vis.bytes + b->vis_list.bytes +
-             b->chunk_offs.bytes + b->seg_totals.bytes + b->view_span_start.bytes + b->spans.bytes +
+             b->view_span_start.bytes + b->spans.bytes +
              b->group_counts.bytes + b->group_sums.bytes + b->group_bits.bytes + b->span_vis.bytes;
     return HELIO_OK;
 }
@@ -539,8 +539,7 @@ int32_t helio_batch_execute(helio_batch* b, void* stream) {
     P.chunk_counts = b->chunk_counts.as<uint32_t>();
     P.chunk_vis = b->chunk_vis.as<uint32_t>();
     P.vis_list = b->vis_list.as<uint16_t>();
-    P.chunk_offs = b->chunk_offs.as<uint32_t>();
-    P.seg_totals = b->seg_totals.as<uint32_t>();
+    P.chunk_sums = b->chunk_sums();
     P.view_span_start = b->view_span_start.as<uint32_t>();
     P.spans = b->spans.as<helio::ActiveSpan>();
     P.span_capacity = b->span_capacity;

@@ -212,3 +212,15 @@ def test_batch_group_sum_runs_match_oracle(cuda, objects, views, cull_ctas):
     b, _, _ = run_batch(sc, w.views, cull_ctas=cull_ctas)
     assert (np.diff(u32(b.spans()["view_span_start"]).astype(np.int64)) == (objects + 31) // 32 * 32).all()
     _check_batch(w, w.views, cull_ctas=cull_ctas)
+
+
+@pytest.mark.parametrize("objects,views", [(31 * 256, 3), (32 * 256, 3), (33 * 256, 2), (1023 * 256, 1), (1025 * 256 + 1, 1)])
+def test_batch_chunk_sum_runs_match_oracle(cuda, objects, views):
+    """A view's spans before an object chunk, from the sums by runs of 32 and 1,024 chunks: views of 31, 32 and 33
+    chunks, side by side, and of 1,023 and 1,026."""
+    from helio_b200 import scene as S
+
+    sc = S.make_scene(objects, objects, 1, 1, 0, 40.0)
+    cam = S.orthographic((0, 0, 300), (0, 0, 0), (0, 1, 0), 30.0, 0.1, 600.0)
+    w = S.Workload(3, sc, [S.View(cam, 64, 64, np.ones((64, 64), np.float32), "ortho")] * views)
+    _check_batch(w, w.views)
