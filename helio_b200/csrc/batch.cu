@@ -781,7 +781,8 @@ __device__ void phase_expand(const BatchParams& P, char* sm) {
 // warp works through its group's windows one after the other; with few groups per warp that
 // chain, and the rounding of groups over warps, set the time, so small batches take smaller
 // groups: groups are halved while there is not one per warp. 2,880 groups of 32 on 5,920 warps
-// (9 views over 30,000 objects): tests 54 us, 43 as groups of 8, emission 14.8 -> 12.1. With
+// (9 views over 30,000 objects): tests 54 us, 43 as groups of 8, emission 14.8 -> 12.1 (40 and 9.6
+// with what has changed since). With
 // more than one group per warp halving gains nothing (11,895 groups: 72.4 us either way, the
 // emission 19.2 -> 22.3).
 constexpr uint32_t kMaxGroupShift = 2;
@@ -844,7 +845,8 @@ __device__ void phase_test(const BatchParams& P, uint32_t groups, uint32_t shift
     // they are done with the previous one. (Claiming the next group ahead ties it to a
     // warp that is still busy: the queue's last groups then wait.) The queue hands out
     // the groups from the last view's end backwards: the main view, whose groups are the
-    // lightest, then fills the queue's tail (89.8 against 93.0 us in view order).
+    // lightest, then fills the queue's tail (89.8 against 93.0 us in view order, when the phase took
+    // that long; 64 now).
     // With at most one group per warp there is nothing to balance: warp w takes group w, without the
     // round trips of the claims (a 20-view batch of 694 groups of 32: 8.3 -> 6.8 us).
     for (;;) {

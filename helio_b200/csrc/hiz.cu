@@ -25,9 +25,11 @@ namespace {
 
 // One tile per CTA of four warps, its level 0 loaded into registers (128-bit loads where the
 // rows allow them, else 32 independent 4-byte loads per lane). 1367x769, whose rows no wide load
-// fits: 8.2 us per launch back to back, 10.1 with 256 threads per tile, the job copied by one
-// thread and the tail level by level. 8 CTAs per SM hide the loads' latency; the job is copied to shared memory for the tail, whose fields of levels 7.. no tile
-// reads (from the parameter space each would wait for a cold constant-cache line).
+// fits: 6.4 us per launch back to back (8.2 while the kernels still signalled launch_dependents
+// early, 10.1 then with 256 threads per tile, the job copied by one thread and the tail level by
+// level). 8 CTAs per SM hide the loads' latency; the job is copied to shared memory for the tail,
+// whose fields of levels 7.. no tile reads (from the parameter space each would wait for a cold
+// constant-cache line).
 __global__ void __launch_bounds__(kHizBlockThreads, 8)
     hiz_build_kernel(const __grid_constant__ HizJob J, uint32_t* ticket) {
     __shared__ __align__(16) HizJob s_J;

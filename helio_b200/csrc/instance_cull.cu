@@ -263,8 +263,7 @@ void launch_instance_cull(const InstanceCullParams& p, bool frustum, bool occlus
     if (p.draw_count == 0) return;
     if (!frustum && !occlusion) return;
     // One wave of 4 blocks per SM; each takes its share of the draws. A million draws move 210 MB
-    // (whole 144-byte rows) in 42 us then; 45 us with 3 blocks per SM, 46 with 5 and 49 with 6: more
-    // rows in flight than that only spread the fetches over more DRAM pages.
+    // (whole 144-byte rows) in 42 us then; 45 us with 3 blocks per SM, 46 with 5 and 49 with 6.
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);  // a cached attribute query

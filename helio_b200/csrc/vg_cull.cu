@@ -480,10 +480,12 @@ __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t e
 // frustum test. In smaller scenes each warp's latency dominates, and the loads stay together.
 //
 // Bound by the latency of its dependent loads (item, object, instance, meshlet, pyramid texel)
-// and by the launch. Against a select, a test and an emission launch with the counters cleared
-// before them, a frame (Hi-Z build included) went 29.3 -> 21.7 us with 4,096 instances x 64
-// meshlets at 1024x1024, 42.1 -> 31.8 with 10,000 x 100 (500 of them moved) at 1920x1080, and
-// 60.3 -> 54.3 with 100,000 x 100 at 3840x2160 (46.8 with the objects' world records).
+// and by the launch. In place of a select, a test and an emission launch with the counters cleared
+// before them, it took a frame (Hi-Z build included) from 29.3 to 21.7 us with 4,096 instances x 64
+// meshlets at 1024x1024, from 42.1 to 31.8 with 10,000 x 100 (500 of them moved) at 1920x1080, and
+// from 60.3 to 54.3 with 100,000 x 100 at 3840x2160; with the objects' world records, tiles of up
+// to 512 items, the instances' records and the bounds' pairs these frames now take 16.9, 21.5 and
+// 38 us.
 template <bool kWide>
 __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const __grid_constant__ VgFrameParams P) {
     __shared__ CullView s_view;
