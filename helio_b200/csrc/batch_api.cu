@@ -203,7 +203,10 @@ int32_t plan_batch(const helio_batch_config& cfg, const helio_vg_scene* sc, uint
     p.need[kBufVisList] = std::max<size_t>(1, units) * helio::kBatchChunk * sizeof(uint16_t);
     p.need[kBufViewSpanStart] = (size_t)(n + 1) * 4;
     p.need[kBufSpans] = (size_t)p.span_capacity * sizeof(helio::ActiveSpan);
-    p.need[kBufGroupCounts] = groups * 4 * sizeof(uint2);  // groups of 8 spans at the least
+    // Groups are smaller than 32 spans only while there are fewer than warps of the test launch, so
+    // that halving them ends below twice that many; never below 8 spans.
+    const size_t small_groups = std::min<size_t>(groups * 4, (size_t)helio::batch_cull_max_grid() * (helio::kBatchThreads / 32u) * 2u);
+    p.need[kBufGroupCounts] = std::max(groups, small_groups) * sizeof(uint2);
     p.need[kBufGroupSums] = (size_t)helio::group_sum_words((uint32_t)groups * 4u, n, helio::kGroupSumLevels) * 4;
     p.need[kBufGroupBits] = (groups + 1) * helio::kWindowsPerWarp * 4;
     p.need[kBufSpanVis] = (cfg.flags & HELIO_BATCH_SPAN_VISIBILITY) ? (size_t)p.span_capacity * 8 : 0;
