@@ -1270,7 +1270,7 @@ def run_build(args, rank, world, local_rank):
     traffic = json.loads(tfile.read_text()).get("vgbuild", {}).get("vg_build") if tfile.exists() else None
     roofline = {"bound": "hbm", "kernel": "vg_build", "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
                 "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
-                "note": "the six launches of one rebuild and its two read-backs (totals, error word), between one "
+                "note": "the launches of one rebuild and its read-back (totals, error word), between one "
                         "pair of CUDA events"}
 
     e2e = None
