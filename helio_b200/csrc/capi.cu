@@ -189,6 +189,7 @@ struct helio_vg_pass {
     bool have_version = false;
     uint32_t num_tiles = 0;
     uint32_t tile_items = helio::kMaxTileItems;
+    uint32_t spin_limit = helio::kSpinLimit, withheld_tile = 0xFFFFFFFFu;  // helio_vg_set_wait_limit
 };
 
 // ════════════════════════════════════════════════════════════════════════════
@@ -724,6 +725,8 @@ int32_t helio_vg_execute(helio_vg_pass* p, const HelioGpuCameraUniforms* camera_
     fp.num_tiles = p->num_tiles;
     fp.tile_items = p->tile_items;
     fp.counter_count = p->counter_count;
+    fp.spin_limit = p->spin_limit;
+    fp.withheld_tile = p->withheld_tile;
     HELIO_CK(helio::launch_vg_frame(fp, s));
     HELIO_CK(cudaGetLastError());
     return HELIO_OK;
@@ -758,6 +761,13 @@ int32_t helio_vg_publish(const helio_vg_pass* p, helio_vg_outputs* out) {
     return HELIO_OK;
 }
 
+int32_t helio_vg_set_wait_limit(helio_vg_pass* p, uint32_t max_polls, uint32_t withheld) {
+    HELIO_ARG(p, "null pointer");
+    p->spin_limit = max_polls ? max_polls : helio::kSpinLimit;
+    p->withheld_tile = withheld - 1u;
+    return HELIO_OK;
+}
+
 int32_t helio_vg_device_status(helio_vg_pass* p, void* stream) {
     HELIO_ARG(p, "null pointer");
     uint32_t err = 0;
@@ -766,7 +776,10 @@ int32_t helio_vg_device_status(helio_vg_pass* p, void* stream) {
                                  as_stream(stream)));
     HELIO_CK(cudaStreamSynchronize(as_stream(stream)));
     HELIO_CK(cudaGetLastError());
-    if (err & helio::kDevTimeout) return fail(HELIO_ERR_TIMEOUT, "a meshlet tile's wait for the tiles before it gave up");
+    if (err & helio::kDevTimeout) {
+        HELIO_CK(cudaMemsetAsync(p->scratch.as<uint32_t>() + 16 + helio::kVgError, 0, 4, as_stream(stream)));
+        return fail(HELIO_ERR_TIMEOUT, "a meshlet tile's wait for the tiles before it gave up");
+    }
     return HELIO_OK;
 }
 

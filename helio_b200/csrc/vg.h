@@ -89,6 +89,7 @@ enum : uint32_t {
     kVgError = 2,   // kDevTimeout, sticky
     kVgDone = 3,    // object CTAs that have added their statistics (zero between launches)
     kVgHist = 4,    // 9 words: LOD histogram, largest lod_count (zero between launches)
+    kVgLost = 13,   // epoch of the latest launch in which a tile's wait gave up
     kVgStateWords = 16
 };
 
@@ -105,6 +106,8 @@ struct VgFrameParams {
     uint32_t num_tiles;
     uint32_t tile_items;  // work items per tile: a power of two, 8 to kMaxTileItems
     uint32_t counter_count;
+    uint32_t spin_limit;     // polls before a tile's wait gives up (kSpinLimit by default)
+    uint32_t withheld_tile;  // a tile that publishes nothing (0xFFFFFFFF: none; tests only)
 };
 
 // Work items per tile: 512 for large scenes; halved for smaller ones until about one CTA

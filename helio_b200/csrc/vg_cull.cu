@@ -414,7 +414,8 @@ __device__ __forceinline__ uint32_t item_at(const TileItems& t, uint32_t w) {
     return t.owner[w] + __popc(t.heads[w] & le & ~1u);
 }
 
-enum : uint32_t { kTileSum = 1u, kTilePrefix = 2u };  // a status holds the tile's count, or all up to it
+// A status holds the tile's count, or all up to it; or the tile's wait gave up.
+enum : uint32_t { kTileSum = 1u, kTilePrefix = 2u, kTileLost = 3u };
 
 __device__ __forceinline__ unsigned long long tile_status(uint32_t epoch, uint32_t kind, uint32_t value) {
     return ((unsigned long long)(epoch & 0x3FFFFFFFu) << 34) | ((unsigned long long)kind << 32) | value;
@@ -432,7 +433,8 @@ __device__ __forceinline__ void st_status(unsigned long long* p, unsigned long l
 // Visible meshlets of the tiles before `tile`, by the whole CTA: thread t waits (bounded) for
 // the status of tile hi - 1 - t; the nearest one that holds a prefix ends the walk, the counts
 // nearer than it are added. Every earlier ticket is held by a CTA that runs and publishes its
-// count without waiting, so the waits end. Returns false, uniformly, when one gave up.
+// count without waiting, so the waits end. Returns false, uniformly, when one gave up, here or in
+// a tile before this one.
 __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t epoch, uint32_t* s_red,
                                uint32_t& prefix) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -445,12 +447,13 @@ __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t e
             const unsigned long long* p = P.status + (hi - 1u - threadIdx.x);
             uint32_t polls = 0;
             while (st = ld_status(p), (uint32_t)(st >> 34) != (epoch & 0x3FFFFFFFu)) {
-                if (++polls > kSpinLimit) {
+                if (++polls > P.spin_limit) {
                     lost = 1;
                     break;
                 }
                 if (polls > 32u) __nanosleep(polls < 512u ? 32 : 256);
             }
+            if (((uint32_t)(st >> 32) & 3u) == kTileLost) lost = 1;
         }
         if (__syncthreads_or(lost)) return false;
         // The nearest prefix: the lowest thread that saw one.
@@ -473,6 +476,34 @@ __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t e
         __syncthreads();
     }
     return true;
+}
+
+// A wait that gave up must leave no draw count behind that covers draws nobody wrote: the draw side
+// reads the count on the device. The tile that gave up notes the launch's epoch and then zeroes the
+// count; the last tile stores the count and then looks for the note. Each side has a sequentially
+// consistent fence between its two steps, so that either the last tile sees the note (and stores
+// zero itself) or the zeroing comes after the count.
+__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
+
+__device__ __forceinline__ void publish_count(const VgFrameParams& P, uint32_t count) {
+    st_relaxed(P.counters, count);
+    st_relaxed(P.counters + 1, count > P.capacity ? count - P.capacity : 0u);
+}
+
+__device__ __forceinline__ void give_up(const VgFrameParams& P, uint32_t tile, uint32_t epoch) {
+    atomicOr(P.state + kVgError, (uint32_t)kDevTimeout);
+    st_relaxed(P.state + kVgLost, epoch);
+    fence_sc();
+    publish_count(P, 0u);
+    st_status(P.status + tile, tile_status(epoch, kTileLost, 0u));  // the tiles after it give up too
 }
 
 // kWide: the form for large scenes, whose launch has more CTAs than fit at four per SM: they
@@ -521,6 +552,10 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
         return;
     }
     const uint32_t tile = s_tile, epoch = s_epoch;
+    if (tile >= P.num_tiles) {  // uniform; only if launches of one pass ran at the same time, which they must not
+        if (tid == 0) atomicOr(P.state + kVgError, (uint32_t)kDevTimeout);
+        return;
+    }
 
     // The tile's items, in rounds of one per thread: the object's selected LOD and the item's share
     // of it.
@@ -596,7 +631,8 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
             before += c[k];
         }
     }
-    if (tid == 0) st_status(P.status + tile, tile_status(epoch, tile == 0u ? kTilePrefix : kTileSum, count));
+    if (tid == 0 && tile != P.withheld_tile)
+        st_status(P.status + tile, tile_status(epoch, tile == 0u ? kTilePrefix : kTileSum, count));
     // Per-work-item visibility words: bits [off, off + n) of the tile's window bits.
 #pragma unroll
     for (uint32_t r = 0; r < kItemRounds; ++r)
@@ -607,16 +643,15 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
 
     uint32_t base;
     if (!tile_look_back(P, tile, epoch, s_tmp, base)) {
-        if (tid == 0) atomicOr(P.state + kVgError, (uint32_t)kDevTimeout);
+        if (tid == 0) give_up(P, tile, epoch);
         return;
     }
-    if (tid == 0) {
-        if (tile != 0u) st_status(P.status + tile, tile_status(epoch, kTilePrefix, base + count));
-        if (last) {
-            const uint32_t all = base + count;
-            P.counters[0] = all;
-            P.counters[1] = all > P.capacity ? all - P.capacity : 0u;
-        }
+    if (tid == 0 && tile != 0u && tile != P.withheld_tile)
+        st_status(P.status + tile, tile_status(epoch, kTilePrefix, base + count));
+    if (last && tid == kThreads - 32u) {  // in the warp with the fewest windows: the fence takes a while
+        publish_count(P, base + count);
+        fence_sc();
+        if (ld_relaxed(P.state + kVgLost) == epoch) publish_count(P, 0u);
     }
     // Emission, four windows at a time per warp: their draw records are loaded before any is
     // written. (tile_look_back ended with s_pre visible to every thread.)

@@ -277,6 +277,7 @@ CULL_EXPORTS = {
     "helio_vg_set_lod_quality": (i32, [vp, u32]),
     "helio_vg_publish": (i32, [vp, C.POINTER(VgOutputs)]),
     "helio_vg_device_status": (i32, [vp, vp]),
+    "helio_vg_set_wait_limit": (i32, [vp, u32, u32]),
     "helio_vg_destroy": (None, [vp]),
     "helio_vg_scene_create": (i32, [C.POINTER(vp)]),
     "helio_vg_scene_upload": (i32, [vp, C.POINTER(VgFrameData), vp]),

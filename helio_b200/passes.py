@@ -586,6 +586,11 @@ class VirtualGeometryPass:
     def device_status(self, stream=None) -> None:
         N.check(self._lib.helio_vg_device_status(self._h, _stream_ptr(stream)))
 
+    def set_wait_limit(self, max_polls: int = 0, withheld: int = 0) -> None:
+        """Polls before a tile's wait for the tiles before it gives up (0 = default, about 1 s);
+        withheld = k > 0 keeps the k-th tile from publishing its count (tests of the bounded wait)."""
+        N.check(self._lib.helio_vg_set_wait_limit(self._h, max_polls, withheld))
+
     def outputs(self) -> dict:
         """Zero-copy torch views of the published buffers (int32 words)."""
         o = self.publish()

@@ -445,8 +445,8 @@ int32_t helio_vg_create(const helio_vg_config* config, helio_vg_pass** out);
  * instance_version change; recomputes InstanceCullData on the GPU for what changed.
  * Reference: rendering.rs:708-859. May allocate (growth). */
 int32_t helio_vg_prepare(helio_vg_pass* pass, const helio_vg_frame_data* frame, void* stream);
-/* Clears the counters, runs object select then meshlet cull with deterministic
- * compaction: the visible draws are stored in (work item, lane) order and
+/* Object select, meshlet cull and deterministic compaction in one launch that writes every
+ * counter: the visible draws are stored in (work item, lane) order and
  * first_instance = slot. camera: device pointer. hiz: published pyramid.
  * Returns HELIO_ERR_CAPACITY only if the caller asks for it via
  * helio_vg_check_overflow(); execute itself never reads back. */
@@ -457,8 +457,15 @@ int32_t helio_vg_set_lod_quality(helio_vg_pass* pass, uint32_t lod_quality);
 int32_t helio_vg_publish(const helio_vg_pass* pass, helio_vg_outputs* out);
 /* Synchronises `stream` and reports any asynchronous CUDA error of the queued work, or
  * HELIO_ERR_TIMEOUT when a tile's bounded wait for the draw counts of the tiles before it
- * gave up in an execute since the last full upload (that execute's outputs are invalid). */
+ * gave up in an execute since the last full upload or report. Such an execute publishes a draw count of 0
+ * (counters[0] and [1]), so that a draw side which reads the count on the device draws nothing;
+ * the next execute starts clean. */
 int32_t helio_vg_device_status(helio_vg_pass* pass, void* stream);
+/* Bounds of that wait, from the next execute on: it gives up after max_polls polls (0 = the
+ * default, about 1 s). withheld = k > 0 keeps the k-th tile of work items from publishing its
+ * count, so that the tiles after it wait in vain: a way to run the wait out in tests (0 in normal
+ * use). */
+int32_t helio_vg_set_wait_limit(helio_vg_pass* pass, uint32_t max_polls, uint32_t withheld);
 void helio_vg_destroy(helio_vg_pass* pass);
 
 /* ════════════════════════════════════════════════════════════════════════════
