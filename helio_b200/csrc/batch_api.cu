@@ -97,7 +97,7 @@ constexpr size_t kBoundsBytes = 8 + 3 * 8;
 
 // Runs the update `u` with the instances [first, first + count) of a scene of `objects` objects from
 // `src` (the caller's rows of that range) and the scene's bounds; with `totals` also the sums of
-// launch_scene_update, read back (waits for the stream). Device rows that 16-byte loads
+// launch_scene_update, read back (waits for the stream). Rows of this device that 16-byte loads
 // can read are copied by the update itself. (Summing the objects on the host, read back
 // whole, took 15 to 33 ms for 475,000 objects.)
 int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects, uint32_t first, uint32_t count,
@@ -111,7 +111,7 @@ int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects
     u.first = first;
     u.count = count;
     u.rows = src;
-    if (count && !(memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16))) {
+    if (count && !(memory == HELIO_MEM_DEVICE && helio::caller_array(helio::reads_directly, src, 16))) {
         u.rows = sc->row_staging.as<HelioGpuInstanceData>();
         int32_t st = copy_in(sc->row_staging.ptr, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
         if (st) return st;
@@ -238,11 +238,11 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->row_staging.ensure(O * sizeof(HelioGpuInstanceData)));
         HELIO_CK(sc->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
-        // Device arrays that 16-byte loads can read are copied by the update launch itself.
+        // Arrays of this device that 16-byte loads can read are copied by the update launch itself.
         helio::SceneUpdate u{};
         const bool device = f->memory == HELIO_MEM_DEVICE;
         u.src_meshlets = f->meshlets;
-        if (M && !(device && helio::update_reads(f->meshlets, 16))) {
+        if (M && !(device && helio::caller_array(helio::reads_mapped, f->meshlets, 16))) {
             HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
             HELIO_CK(sc->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
             if ((st = copy_in(sc->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
@@ -252,7 +252,7 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         u.m_bounds = sc->m_bounds.as<float4>();
         u.m_axis = sc->m_axis.as<float4>();
         u.m_draw = sc->m_draw.as<uint4>();
-        if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
+        if (device && helio::caller_array(helio::reads_directly, f->objects, 16)) u.src_objects = f->objects;
         else if ((st = copy_in(sc->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
         // With the per-object span bound and LOD0 size, for capacities and the metric; the wait
         // for them also ends the use of the staging copy.

@@ -599,7 +599,7 @@ static int32_t vg_rows(helio_vg_pass* p, helio::SceneUpdate* u, uint32_t objects
     u->first = first;
     u->count = count;
     u->rows = src;
-    if (count == 0 || (memory == HELIO_MEM_DEVICE && helio::update_reads(src, 16))) return HELIO_OK;
+    if (count == 0 || (memory == HELIO_MEM_DEVICE && helio::caller_array(helio::reads_directly, src, 16))) return HELIO_OK;
     u->rows = p->row_staging.as<HelioGpuInstanceData>();
     return vg_copy(p->row_staging.ptr, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
 }
@@ -621,11 +621,11 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
         HELIO_CK(p->visibility.ensure(W * 8));
-        // Device arrays that 16-byte loads can read are copied by the update launch itself.
+        // Arrays of this device that 16-byte loads can read are copied by the update launch itself.
         helio::SceneUpdate u{};
         const bool device = f->memory == HELIO_MEM_DEVICE;
         u.src_meshlets = f->meshlets;
-        if (M && !(device && helio::update_reads(f->meshlets, 16))) {
+        if (M && !(device && helio::caller_array(helio::reads_mapped, f->meshlets, 16))) {
             HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
             HELIO_CK(p->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
             if ((st = vg_copy(p->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
@@ -635,11 +635,11 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         u.m_bounds = p->m_bounds.as<float4>();
         u.m_axis = p->m_axis.as<float4>();
         u.m_draw = p->m_draw.as<uint4>();
-        if (device && helio::update_reads(f->objects, 16)) u.src_objects = f->objects;
+        if (device && helio::caller_array(helio::reads_directly, f->objects, 16)) u.src_objects = f->objects;
         else if ((st = vg_copy(p->objects.ptr, f->objects, O * sizeof(HelioGpuVgObject), f->memory, s))) return st;
         u.items = p->items.as<HelioGpuVgWorkItem>();
         u.item_count = f->work_item_count;
-        if (device && helio::update_reads(f->work_items, 8)) u.src_items = f->work_items;
+        if (device && helio::caller_array(helio::reads_directly, f->work_items, 8)) u.src_items = f->work_items;
         else if ((st = vg_copy(p->items.ptr, f->work_items, W * sizeof(HelioGpuVgWorkItem), f->memory, s))) return st;
         if ((st = vg_rows(p, &u, f->object_count, 0, f->object_count, f->instances, f->memory, s))) return st;
         HELIO_CK(helio::launch_scene_update(u, s));

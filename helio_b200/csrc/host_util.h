@@ -63,6 +63,29 @@ struct DevBuf {
     }
 };
 
+// Whether kernels read a caller's array of "device memory" themselves, with loads of `align` bytes.
+// An array of another device is copied instead: a copy crosses devices, a kernel only with peer
+// access; and so is one that is not device memory at all, which the copy turns into an error.
+inline bool reads_directly(const cudaPointerAttributes& a, int device, const void* p, size_t align) {
+    return p && (reinterpret_cast<uintptr_t>(p) & (align - 1)) == 0 && a.type == cudaMemoryTypeDevice && a.device == device;
+}
+// The same for an array that no copy brought in before: only what kernels cannot read is copied.
+inline bool reads_mapped(const cudaPointerAttributes& a, int device, const void* p, size_t align) {
+    return reads_directly(a, device, p, align) ||
+           (p && (reinterpret_cast<uintptr_t>(p) & (align - 1)) == 0 &&
+            (a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeHost && a.devicePointer == p)));
+}
+// One of the two for an array on the current device.
+inline bool caller_array(bool (*rule)(const cudaPointerAttributes&, int, const void*, size_t), const void* p, size_t align) {
+    cudaPointerAttributes a{};
+    int device = -1;
+    if (!p || cudaGetDevice(&device) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return rule(a, device, p, align);
+}
+
 // Launches `kernel` with programmatic stream serialization: its CTAs are scheduled as those of the
 // stream's previous kernel end, and wait in pdl_wait before their first global access, which
 // hides a launch gap.

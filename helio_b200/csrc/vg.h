@@ -154,8 +154,6 @@ struct SceneUpdate {
     uint32_t* bounds;
     unsigned long long* totals;
 };
-// Whether the update kernel can read an array of device memory itself.
-inline bool update_reads(const void* p, size_t align) { return p && (reinterpret_cast<uintptr_t>(p) & (align - 1)) == 0; }
 cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream);
 // Object select, meshlet cull and emission of one view, in one launch.
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream);
