@@ -18,8 +18,8 @@ using helio::DevBuf;
 
 struct helio_vg_scene {
     DevBuf m_bounds, m_axis, m_draw, objects, xform, world;
-    DevBuf staging;      // meshlets on their way to the update launch
-    DevBuf row_staging;  // instance rows on their way there, for the whole scene: a patch never allocates
+    DevBuf staging;      // meshlets, and a host upload's rows, on their way to the update launch
+    DevBuf row_staging, patch_staging;  // instance rows on their way there (RowStaging)
     DevBuf bounds;  // launch_scene_update of the current objects and instances: u32[2], then u64[3] totals
     uint32_t meshlet_count = 0, object_count = 0;
     uint64_t lod0_meshlets = 0, max_spans = 0, max_draw_count = 0;
@@ -97,11 +97,12 @@ constexpr size_t kBoundsBytes = 8 + 3 * 8;
 
 // Runs the update `u` with the instances [first, first + count) of a scene of `objects` objects from
 // `src` (the caller's rows of that range) and the scene's bounds; with `totals` also the sums of
-// launch_scene_update, read back (waits for the stream). Rows of this device that 16-byte loads
-// can read are copied by the update itself. (Summing the objects on the host, read back
+// launch_scene_update, read back (waits for the stream). (Summing the objects on the host, read back
 // whole, took 15 to 33 ms for 475,000 objects.)
 int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects, uint32_t first, uint32_t count,
-                     const HelioGpuInstanceData* src, uint32_t memory, uint64_t* totals, cudaStream_t s) {
+                     const HelioGpuInstanceData* src, uint32_t memory, const helio::RowStaging& staging,
+                     uint64_t* totals, cudaStream_t s) {
+    HELIO_ARG(count == 0 || src, "frame data array missing");
     HELIO_CK(sc->bounds.ensure(kBoundsBytes));
     HELIO_CK(cudaMemsetAsync(sc->bounds.ptr, 0, kBoundsBytes, s));
     u.scene = sc->dev();
@@ -110,16 +111,10 @@ int32_t scene_update(helio_vg_scene* sc, helio::SceneUpdate& u, uint32_t objects
     u.world = sc->world.as<uint4>();
     u.first = first;
     u.count = count;
-    u.rows = src;
-    if (count && !(memory == HELIO_MEM_DEVICE && helio::caller_array(helio::reads_directly, src, 16))) {
-        u.rows = sc->row_staging.as<HelioGpuInstanceData>();
-        int32_t st = copy_in(sc->row_staging.ptr, src, (size_t)count * sizeof(HelioGpuInstanceData), memory, s);
-        if (st) return st;
-    }
     unsigned long long* sums = reinterpret_cast<unsigned long long*>(sc->bounds.as<char>() + 8);
     u.bounds = sc->bounds.as<uint32_t>();
     u.totals = totals ? sums : nullptr;
-    HELIO_CK(helio::launch_scene_update(u, s));
+    HELIO_CK(helio::launch_scene_update_from(u, src, memory, staging, s));
     if (totals) {
         HELIO_CK(cudaMemcpyAsync(totals, sums, 3 * 8, cudaMemcpyDeviceToHost, s));
         HELIO_CK(cudaStreamSynchronize(s));
@@ -235,16 +230,18 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->m_axis.ensure(M * 16));
         HELIO_CK(sc->m_draw.ensure(M * 16));
         HELIO_CK(sc->objects.ensure(O * sizeof(HelioGpuVgObject)));
-        HELIO_CK(sc->row_staging.ensure(O * sizeof(HelioGpuInstanceData)));
+        HELIO_CK(sc->row_staging.ensure(helio::staging_rows(f->object_count) * sizeof(HelioGpuInstanceData)));
         HELIO_CK(sc->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
         // Arrays of this device that 16-byte loads can read are copied by the update launch itself.
         helio::SceneUpdate u{};
         const bool device = f->memory == HELIO_MEM_DEVICE;
+        uint32_t rows = 0;  // that the staging copy has room for behind the meshlets
         u.src_meshlets = f->meshlets;
         if (M && !(device && helio::caller_array(helio::reads_mapped, f->meshlets, 16))) {
             HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
-            HELIO_CK(sc->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
+            if (!device) rows = std::min(f->object_count, helio::kPatchStagingRows);
+            HELIO_CK(sc->staging.ensure(M * sizeof(HelioGpuMeshletEntry) + (size_t)rows * sizeof(HelioGpuInstanceData)));
             if ((st = copy_in(sc->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
             u.src_meshlets = sc->staging.as<HelioGpuMeshletEntry>();
         }
@@ -257,7 +254,10 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         // With the per-object span bound and LOD0 size, for capacities and the metric; the wait
         // for them also ends the use of the staging copy.
         uint64_t totals[3] = {0, 0, 0};
-        if ((st = scene_update(sc, u, f->object_count, 0, f->object_count, f->instances, f->memory, totals, s))) return st;
+        helio::RowStaging staging{sc->row_staging, nullptr, nullptr, rows};
+        if (rows) staging.upload = reinterpret_cast<HelioGpuInstanceData*>(sc->staging.as<HelioGpuMeshletEntry>() + M);
+        if ((st = scene_update(sc, u, f->object_count, 0, f->object_count, f->instances, f->memory, staging, totals, s)))
+            return st;
         sc->staging.release();
         sc->meshlet_count = f->meshlet_count;
         sc->object_count = f->object_count;
@@ -272,7 +272,8 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_ARG(count > 0 && start + count <= sc->object_count, "invalid dirty instance range");
         helio::SceneUpdate u{};
         if ((st = scene_update(sc, u, sc->object_count, (uint32_t)start, (uint32_t)count,
-                               f->instances ? f->instances + start : nullptr, f->memory, nullptr, s)))
+                               f->instances ? f->instances + start : nullptr, f->memory,
+                               helio::RowStaging{sc->row_staging, &sc->patch_staging, nullptr, 0}, nullptr, s)))
             return st;
         sc->instance_version = f->instance_version;
     }
@@ -286,7 +287,7 @@ int32_t helio_vg_scene_info_get(const helio_vg_scene* sc, helio_vg_scene_info* o
     out->lod0_meshlets = sc->lod0_meshlets;
     out->max_spans = sc->max_spans;
     out->device_bytes = sc->m_bounds.bytes + sc->m_axis.bytes + sc->m_draw.bytes +
-                        sc->objects.bytes + sc->row_staging.bytes + sc->xform.bytes + sc->world.bytes;
+                        sc->objects.bytes + sc->row_staging.bytes + sc->patch_staging.bytes + sc->xform.bytes + sc->world.bytes;
     return HELIO_OK;
 }
 

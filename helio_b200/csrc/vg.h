@@ -1,6 +1,8 @@
 // vg.h — launch parameters of the virtual-geometry kernels.
 #pragma once
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace helio {
@@ -155,6 +157,27 @@ struct SceneUpdate {
     unsigned long long* totals;
 };
 cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream);
+// Instance rows that the update kernel does not read itself go through a staging buffer, in pieces of
+// what it holds. A scene keeps one for a fifth of its rows from its upload on: with the records no
+// more memory per object than rows and cull data took (285 bytes, 288 then), and at most 4.7 MB, since
+// larger pieces copy no faster.
+struct DevBuf;
+struct RowStaging {
+    DevBuf& kept;
+    DevBuf* patch;  // for a patch of more rows in a small scene, allocated by the first one (null: an upload)
+    HelioGpuInstanceData* upload;  // an upload's own, released after it, of kPatchStagingRows at most (null: none)
+    uint32_t upload_rows;
+};
+inline uint32_t staging_rows(uint32_t objects) { return std::min(std::max(objects / 5u, 1u), 32768u); }
+// Rows of the others: every piece costs a copy and a launch (4,000 rows of a 4,000-object scene: 75 us
+// as five pieces, 37 as one).
+constexpr uint32_t kPatchStagingRows = 4096;
+// The update `u` with its rows [u.first, u.first + u.count) in `src`, memory of the caller (HELIO_MEM_*),
+// null if there are none. Rows of this device that 16-byte loads can read are read by the kernel.
+// Others are copied to the staging piece by piece, each with an update of its own, the last with u's
+// bounds and totals.
+cudaError_t launch_scene_update_from(SceneUpdate u, const HelioGpuInstanceData* src, uint32_t memory,
+                                     const RowStaging& staging, cudaStream_t stream);
 // Object select, meshlet cull and emission of one view, in one launch.
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream);
 

@@ -711,6 +711,52 @@ cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream) {
     return e;
 }
 
+cudaError_t launch_scene_update_from(SceneUpdate u, const HelioGpuInstanceData* src, uint32_t memory,
+                                     const RowStaging& staging, cudaStream_t stream) {
+    u.rows = src;
+    const bool device = memory == HELIO_MEM_DEVICE;
+    if (u.count == 0 || (device && caller_array(reads_directly, src, 16))) return launch_scene_update(u, stream);
+    auto rows_in = [](const DevBuf& b) { return (uint32_t)std::min<size_t>(b.bytes / sizeof(HelioGpuInstanceData), 0xFFFFFFFFu); };
+    const DevBuf* buf = &staging.kept;
+    const uint32_t wanted = std::min(u.scene.object_count, kPatchStagingRows);
+    if (staging.patch && u.count > rows_in(*buf) && wanted > rows_in(*buf)) {
+        // Not under capture: nothing may be allocated there, and a graph must not hold a buffer that a
+        // later patch may replace.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+        if (e != cudaSuccess) return e;
+        if (capture == cudaStreamCaptureStatusNone) {
+            const cudaError_t grown = staging.patch->ensure(wanted * sizeof(HelioGpuInstanceData));
+            if (grown != cudaSuccess) return grown;
+            buf = staging.patch;
+        }
+    }
+    const bool own = staging.upload_rows > rows_in(*buf);
+    HelioGpuInstanceData* rows = own ? staging.upload : buf->as<HelioGpuInstanceData>();
+    const uint32_t room = own ? staging.upload_rows : rows_in(*buf);
+    if (!room) return cudaErrorInvalidValue;  // (a scene of at least one object has room for a row)
+    const uint32_t first = u.first, count = u.count;
+    uint32_t* const bounds = u.bounds;
+    unsigned long long* const totals = u.totals;
+    u.rows = rows;
+    for (uint32_t done = 0; done < count;) {
+        u.first = first + done;
+        u.count = std::min(room, count - done);
+        cudaError_t e = cudaMemcpyAsync(rows, src + done, (size_t)u.count * sizeof(HelioGpuInstanceData),
+                                        device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream);
+        if (e != cudaSuccess) return e;
+        done += u.count;
+        u.bounds = done == count ? bounds : nullptr;
+        u.totals = done == count ? totals : nullptr;
+        if ((e = launch_scene_update(u, stream)) != cudaSuccess) return e;
+        // The first piece has copied the rest of the scene.
+        u.src_objects = nullptr;
+        u.src_items = nullptr;
+        u.src_meshlets = nullptr;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream) {
     if (!p.num_tiles) return cudaSuccess;
     int dev = 0, sms = 0;

@@ -87,3 +87,75 @@ def test_moved_instances_reach_every_object_that_names_them(cuda, memory, start,
     for i in range(2):
         got = gather(b, i, n)
         check_view(new, v, got, None, None, got["capacity"])
+
+
+@pytest.mark.parametrize("memory", ["host", "device"])
+@pytest.mark.parametrize("n", [5, 1003, 200001])
+def test_scene_memory_per_object(cuda, memory, n):
+    """The bytes that a server's memory budget is charged for a scene: at most the objects (128),
+    a row (144) and 16 more per object, and 64 per meshlet, and after a patch of host rows 4,096 rows
+    more at most."""
+    import torch
+    from helio_b200 import native as N
+    from helio_b200 import scene as S
+    from helio_b200.passes import ServeLoop, VgScene
+
+    sc = S.make_scene(5, n, 8, 1, 0, 50.0, mesh_library=2)
+    host = (sc.meshlets, sc.objects, sc.instances, sc.work_items)
+    dev = {k: torch.from_numpy(a.view(np.uint8).reshape(-1).copy()).cuda()
+           for k, a in zip(("meshlets", "objects", "instances", "work_items"), host)}
+    vs = VgScene()
+    vs.upload(S.frame_data(sc, device=dev if memory == "device" else None))
+    most = 288 * n + 64 * len(sc.meshlets)
+    assert vs.info().device_bytes <= most
+    ServeLoop(hbm_budget_bytes=most).add_scene(vs)  # fits a budget of exactly that
+    vs.upload(S.frame_data(sc, instance_version=2, dirty=(0, n)))
+    assert vs.info().device_bytes <= most + 144 * 4096
+
+
+def test_patches_of_device_and_pinned_rows_replay_from_a_graph(cuda):
+    """A patch allocates nothing and waits for nothing: a captured patch and frame follow the rows as
+    they are at each replay, whether they are read by the update or staged."""
+    import torch
+    from helpers import gpu_hiz, oracle_vg_view, u32
+    from helio_b200 import native as N
+    from helio_b200 import scene as S
+    from helio_b200.passes import VirtualGeometryPass, camera_bytes
+    from oracle import oracle as O
+
+    n = 2000
+    sc = S.make_scene(7, n, 40, 4, 0, 20.0)
+    v = S.main_view(5, 200, 120, 30)
+    levels = O.hiz_build(v.depth)
+    hz, _ = gpu_hiz(v.depth)
+    cam = torch.from_numpy(camera_bytes(v.camera)).cuda()
+    frame = S.frame_data(sc)
+    raw = sc.instances.view(np.uint8).reshape(-1)
+    for memory in ("device", "unaligned", "pinned"):
+        at = 4 if memory == "unaligned" else 0
+        rows = torch.zeros(n * 144 + 16, dtype=torch.uint8)
+        rows = rows.pin_memory() if memory == "pinned" else rows.cuda()
+        rows[at:at + n * 144] = torch.from_numpy(raw)
+        vg = VirtualGeometryPass(v.width, v.height)
+        vg.prepare(frame)
+        torch.cuda.synchronize()
+        patch = N.VgFrameData(frame.meshlets, frame.objects, rows.data_ptr() + at, frame.work_items, frame.meshlet_count,
+                              frame.object_count, frame.work_item_count, frame.max_draw_count, 1, 2, 100, 1500,
+                              N.HELIO_MEM_HOST if memory == "pinned" else N.HELIO_MEM_DEVICE, 0)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            vg.prepare(patch)
+            vg.execute(cam, hz.publish())
+        for seed in (21, 22):
+            new = S.Scene(sc.meshlets, sc.objects, sc.instances.copy(), sc.work_items, sc.aabbs, sc.draw_calls,
+                          sc.max_draw_count, sc.lod0_meshlets)
+            new.instances[100:1600] = S.make_scene(seed, n, 40, 4, 0, 20.0).instances[100:1600]
+            rows[at:at + n * 144] = torch.from_numpy(new.instances.view(np.uint8).reshape(-1))
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            want = oracle_vg_view(new, v, levels)
+            out = vg.outputs()
+            np.testing.assert_array_equal(u32(out["counters"]), want["counters"])
+            np.testing.assert_array_equal(u32(out["draws"])[: want["counters"][0]], want["draws"])
+        del g
