@@ -91,7 +91,6 @@ enum : uint32_t {
     kVgError = 2,   // kDevTimeout, sticky
     kVgDone = 3,    // object CTAs that have added their statistics (zero between launches)
     kVgHist = 4,    // 9 words: LOD histogram, largest lod_count (zero between launches)
-    kVgLost = 13,   // epoch of the latest launch in which a tile's wait gave up
     kVgStateWords = 16
 };
 
@@ -100,7 +99,7 @@ struct VgFrameParams {
     ViewSetupParams setup;
     HelioDrawIndexedIndirectArgs* indirect;
     HelioGpuVgDraw* draws;
-    uint32_t* counters;          // [counter_count], written whole by every launch
+    uint32_t* counters;          // [counter_count], written whole by every launch; 8-byte aligned
     uint32_t* visibility;        // [2 * work_item_count]
     uint32_t* state;             // [kVgStateWords]
     unsigned long long* status;  // [num_tiles] epoch << 34 | kind << 32 | visible meshlets

@@ -479,30 +479,20 @@ __device__ bool tile_look_back(const VgFrameParams& P, uint32_t tile, uint32_t e
 }
 
 // A wait that gave up must leave no draw count behind that covers draws nobody wrote: the draw side
-// reads the count on the device. The tile that gave up notes the launch's epoch and then zeroes the
-// count; the last tile stores the count and then looks for the note. Each side has a sequentially
-// consistent fence between its two steps, so that either the last tile sees the note (and stores
-// zero itself) or the zeroing comes after the count.
-__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// reads the count on the device. The tile that gave up stores a count of zero, marked with the launch
+// in the word behind it; the last tile stores the count. Both exchange the two words as one, so that
+// either the last tile gets the mark back (and then stores zeros), or the zero is stored after its
+// count. No fence, and the exchange is on its way during the emission. (A fence between the count and
+// a look for the mark: frames of 4,096 objects 17.3 us, 16.9 with the exchange, 16.7 without either.)
+__device__ __forceinline__ unsigned long long swap_count(const VgFrameParams& P, uint32_t count, uint32_t rejected) {
+    return atomicExch(reinterpret_cast<unsigned long long*>(P.counters), ((unsigned long long)rejected << 32) | count);
 }
-__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
-
-__device__ __forceinline__ void publish_count(const VgFrameParams& P, uint32_t count) {
-    st_relaxed(P.counters, count);
-    st_relaxed(P.counters + 1, count > P.capacity ? count - P.capacity : 0u);
-}
+// Never the words of a finished launch, where a count of zero has nothing rejected, nor another launch's.
+__device__ __forceinline__ uint32_t lost_mark(uint32_t epoch) { return 0x80000000u | epoch; }
 
 __device__ __forceinline__ void give_up(const VgFrameParams& P, uint32_t tile, uint32_t epoch) {
     atomicOr(P.state + kVgError, (uint32_t)kDevTimeout);
-    st_relaxed(P.state + kVgLost, epoch);
-    fence_sc();
-    publish_count(P, 0u);
+    swap_count(P, 0u, lost_mark(epoch));
     st_status(P.status + tile, tile_status(epoch, kTileLost, 0u));  // the tiles after it give up too
 }
 
@@ -648,11 +638,9 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     }
     if (tid == 0 && tile != 0u && tile != P.withheld_tile)
         st_status(P.status + tile, tile_status(epoch, kTilePrefix, base + count));
-    if (last && tid == kThreads - 32u) {  // in the warp with the fewest windows: the fence takes a while
-        publish_count(P, base + count);
-        fence_sc();
-        if (ld_relaxed(P.state + kVgLost) == epoch) publish_count(P, 0u);
-    }
+    const uint32_t all = base + count;
+    unsigned long long held = 0;
+    if (last && tid == 0) held = swap_count(P, all, all > P.capacity ? all - P.capacity : 0u);
     // Emission, four windows at a time per warp: their draw records are loaded before any is
     // written. (tile_look_back ended with s_pre visible to every thread.)
     __syncthreads();
@@ -684,6 +672,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
             reinterpret_cast<uint4*>(P.draws)[slot] = make_uint4(s_it.inst[k[q]], mi[q], s_it.lod[k[q]], 0u);
         }
     }
+    if (last && tid == 0 && held == (unsigned long long)lost_mark(epoch) << 32) swap_count(P, 0u, 0u);
 }
 
 }  // namespace

@@ -457,9 +457,9 @@ int32_t helio_vg_set_lod_quality(helio_vg_pass* pass, uint32_t lod_quality);
 int32_t helio_vg_publish(const helio_vg_pass* pass, helio_vg_outputs* out);
 /* Synchronises `stream` and reports any asynchronous CUDA error of the queued work, or
  * HELIO_ERR_TIMEOUT when a tile's bounded wait for the draw counts of the tiles before it
- * gave up in an execute since the last full upload or report. Such an execute publishes a draw count of 0
- * (counters[0] and [1]), so that a draw side which reads the count on the device draws nothing;
- * the next execute starts clean. */
+ * gave up in an execute since the last full upload or report. Such an execute publishes a draw
+ * count of 0 (counters[0]; [1] has no meaning then), so that a draw side which reads the count on
+ * the device draws nothing; the next execute starts clean. */
 int32_t helio_vg_device_status(helio_vg_pass* pass, void* stream);
 /* Bounds of that wait, from the next execute on: it gives up after max_polls polls (0 = the
  * default, about 1 s). withheld = k > 0 keeps the k-th tile of work items from publishing its
