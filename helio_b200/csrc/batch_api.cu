@@ -230,7 +230,7 @@ int32_t helio_vg_scene_upload(helio_vg_scene* sc, const helio_vg_frame_data* f, 
         HELIO_CK(sc->m_axis.ensure(M * 16));
         HELIO_CK(sc->m_draw.ensure(M * 16));
         HELIO_CK(sc->objects.ensure(O * sizeof(HelioGpuVgObject)));
-        HELIO_CK(sc->row_staging.ensure(helio::staging_rows(f->object_count) * sizeof(HelioGpuInstanceData)));
+        HELIO_CK(sc->row_staging.ensure(helio::scene_staging_rows(f->object_count) * sizeof(HelioGpuInstanceData)));
         HELIO_CK(sc->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(sc->world.ensure(O * sizeof(helio::ObjectWorld)));
         // Arrays of this device that 16-byte loads can read are copied by the update launch itself.

@@ -178,8 +178,8 @@ struct helio_vg_pass {
     uint32_t counter_count = HELIO_VG_COUNTER_COUNT;
     // Scene (device resident).
     DevBuf m_bounds, m_axis, m_draw, objects, xform, world, items;
-    DevBuf staging;      // meshlets, and a host upload's rows, on their way to the update launch
-    DevBuf row_staging, patch_staging;  // instance rows on their way there (RowStaging)
+    DevBuf staging;      // meshlets on their way to the update launch
+    DevBuf row_staging;  // instance rows on their way there (RowStaging)
     // Outputs and scratch.
     DevBuf indirect, draws, visibility;
     DevBuf scratch;  // published counters (16 words) | kVgStateWords state words | tile statuses
@@ -591,8 +591,7 @@ static int32_t vg_copy(void* dst, const void* src, size_t bytes, uint32_t memory
 // Runs the update `u` of the pass's buffers with the instances [first, first + count) of a scene of
 // `objects` objects from `src` (the caller's rows of that range).
 static int32_t vg_update(helio_vg_pass* p, helio::SceneUpdate& u, uint32_t objects, uint32_t first, uint32_t count,
-                         const HelioGpuInstanceData* src, uint32_t memory, const helio::RowStaging& staging,
-                         cudaStream_t s) {
+                         const HelioGpuInstanceData* src, uint32_t memory, cudaStream_t s) {
     HELIO_ARG(count == 0 || src, "frame data array missing");
     u.scene.objects = p->objects.as<HelioGpuVgObject>();
     u.scene.object_count = u.scene.instance_count = objects;
@@ -600,7 +599,7 @@ static int32_t vg_update(helio_vg_pass* p, helio::SceneUpdate& u, uint32_t objec
     u.xform = p->xform.as<float4>();
     u.first = first;
     u.count = count;
-    HELIO_CK(helio::launch_scene_update_from(u, src, memory, staging, s));
+    HELIO_CK(helio::launch_scene_update_from(u, src, memory, helio::RowStaging{p->row_staging, nullptr, nullptr, 0}, s));
     return HELIO_OK;
 }
 
@@ -616,7 +615,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->m_axis.ensure(M * 16));
         HELIO_CK(p->m_draw.ensure(M * 16));
         HELIO_CK(p->objects.ensure(O * sizeof(HelioGpuVgObject)));
-        HELIO_CK(p->row_staging.ensure(helio::staging_rows(f->object_count) * sizeof(HelioGpuInstanceData)));
+        HELIO_CK(p->row_staging.ensure(std::min(f->object_count, helio::kMaxStagingRows) * sizeof(HelioGpuInstanceData)));
         HELIO_CK(p->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
@@ -624,12 +623,10 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         // Arrays of this device that 16-byte loads can read are copied by the update launch itself.
         helio::SceneUpdate u{};
         const bool device = f->memory == HELIO_MEM_DEVICE;
-        uint32_t rows = 0;  // that the staging copy has room for behind the meshlets
         u.src_meshlets = f->meshlets;
         if (M && !(device && helio::caller_array(helio::reads_mapped, f->meshlets, 16))) {
             HELIO_ARG(f->meshlets, device ? "meshlet array missing" : "frame data array missing");
-            if (!device) rows = std::min(f->object_count, helio::kPatchStagingRows);
-            HELIO_CK(p->staging.ensure(M * sizeof(HelioGpuMeshletEntry) + (size_t)rows * sizeof(HelioGpuInstanceData)));
+            HELIO_CK(p->staging.ensure(M * sizeof(HelioGpuMeshletEntry)));
             if ((st = vg_copy(p->staging.ptr, f->meshlets, M * sizeof(HelioGpuMeshletEntry), f->memory, s))) return st;
             u.src_meshlets = p->staging.as<HelioGpuMeshletEntry>();
         }
@@ -643,9 +640,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         u.item_count = f->work_item_count;
         if (device && helio::caller_array(helio::reads_directly, f->work_items, 8)) u.src_items = f->work_items;
         else if ((st = vg_copy(p->items.ptr, f->work_items, W * sizeof(HelioGpuVgWorkItem), f->memory, s))) return st;
-        helio::RowStaging staging{p->row_staging, nullptr, nullptr, rows};
-        if (rows) staging.upload = reinterpret_cast<HelioGpuInstanceData*>(p->staging.as<HelioGpuMeshletEntry>() + M);
-        if ((st = vg_update(p, u, f->object_count, 0, f->object_count, f->instances, f->memory, staging, s))) return st;
+        if ((st = vg_update(p, u, f->object_count, 0, f->object_count, f->instances, f->memory, s))) return st;
         if (p->staging.ptr) {
             // The staging copy is consumed by the update; release it once it ran.
             HELIO_CK(cudaStreamSynchronize(s));
@@ -677,8 +672,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_ARG(count > 0 && start + count <= p->object_count, "invalid dirty instance range");
         helio::SceneUpdate u{};
         if ((st = vg_update(p, u, p->object_count, (uint32_t)start, (uint32_t)count,
-                            f->instances ? f->instances + start : nullptr, f->memory,
-                            helio::RowStaging{p->row_staging, &p->patch_staging, nullptr, 0}, s)))
+                            f->instances ? f->instances + start : nullptr, f->memory, s)))
             return st;
         p->last_instance_version = f->instance_version;
     }

@@ -157,19 +157,19 @@ struct SceneUpdate {
 };
 cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream);
 // Instance rows that the update kernel does not read itself go through a staging buffer, in pieces of
-// what it holds. A scene keeps one for a fifth of its rows from its upload on: with the records no
-// more memory per object than rows and cull data took (285 bytes, 288 then), and at most 4.7 MB, since
-// larger pieces copy no faster.
+// what it holds. Every piece costs a copy and a launch (4,000 rows as five pieces 75 us, 37 as one), but
+// pieces of more than 4.7 MB copy no faster. A pass keeps that much from its upload on. A batch's
+// scene, whose bytes count against a server's budget, keeps a fifth of its rows (with the records 285
+// bytes per object, where rows and cull data took 288).
 struct DevBuf;
 struct RowStaging {
     DevBuf& kept;
-    DevBuf* patch;  // for a patch of more rows in a small scene, allocated by the first one (null: an upload)
+    DevBuf* patch;  // for a patch of more rows in a small scene, allocated by the first one (null: none)
     HelioGpuInstanceData* upload;  // an upload's own, released after it, of kPatchStagingRows at most (null: none)
     uint32_t upload_rows;
 };
-inline uint32_t staging_rows(uint32_t objects) { return std::min(std::max(objects / 5u, 1u), 32768u); }
-// Rows of the others: every piece costs a copy and a launch (4,000 rows of a 4,000-object scene: 75 us
-// as five pieces, 37 as one).
+constexpr uint32_t kMaxStagingRows = 32768;
+inline uint32_t scene_staging_rows(uint32_t objects) { return std::min(std::max(objects / 5u, 1u), kMaxStagingRows); }
 constexpr uint32_t kPatchStagingRows = 4096;
 // The update `u` with its rows [u.first, u.first + u.count) in `src`, memory of the caller (HELIO_MEM_*),
 // null if there are none. Rows of this device that 16-byte loads can read are read by the kernel.
