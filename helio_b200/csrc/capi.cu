@@ -178,6 +178,7 @@ struct helio_vg_pass {
     uint32_t counter_count = HELIO_VG_COUNTER_COUNT;
     // Scene (device resident).
     DevBuf m_bounds, m_axis, m_draw, objects, xform, world, items;
+    DevBuf names;        // the objects' instance indices, of large scenes (SceneUpdate::names)
     DevBuf staging;      // meshlets on their way to the update launch
     DevBuf row_staging;  // instance rows on their way there (RowStaging)
     // Outputs and scratch.
@@ -597,6 +598,7 @@ static int32_t vg_update(helio_vg_pass* p, helio::SceneUpdate& u, uint32_t objec
     u.scene.object_count = u.scene.instance_count = objects;
     u.scene.world = u.world = p->world.as<uint4>();
     u.xform = p->xform.as<float4>();
+    u.names = objects > helio::kPatchObjects ? p->names.as<uint32_t>() : nullptr;
     u.first = first;
     u.count = count;
     HELIO_CK(helio::launch_scene_update_from(u, src, memory, helio::RowStaging{p->row_staging, nullptr, nullptr, 0}, s));
@@ -618,6 +620,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         HELIO_CK(p->row_staging.ensure(std::min(f->object_count, helio::kMaxStagingRows) * sizeof(HelioGpuInstanceData)));
         HELIO_CK(p->xform.ensure(O * sizeof(helio::InstanceXform)));
         HELIO_CK(p->world.ensure(O * sizeof(helio::ObjectWorld)));
+        if (O > helio::kPatchObjects) HELIO_CK(p->names.ensure(O * 4));
         HELIO_CK(p->items.ensure(W * sizeof(HelioGpuVgWorkItem)));
         HELIO_CK(p->visibility.ensure(W * 8));
         // Arrays of this device that 16-byte loads can read are copied by the update launch itself.
@@ -671,6 +674,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
         const uint64_t start = f->instance_dirty_start, count = f->instance_dirty_count;
         HELIO_ARG(count > 0 && start + count <= p->object_count, "invalid dirty instance range");
         helio::SceneUpdate u{};
+        u.patch = true;
         if ((st = vg_update(p, u, p->object_count, (uint32_t)start, (uint32_t)count,
                             f->instances ? f->instances + start : nullptr, f->memory, s)))
             return st;

@@ -140,6 +140,9 @@ void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, Hel
 // bounds[1] = largest |c.x| + |c.y| + |c.z| of a world centre c. With `totals` (u64[3], zero before
 // the launch), sums over all objects: totals[0] = lod_meshlet_counts[0], totals[1] = 64-meshlet
 // spans and totals[2] = meshlets of the largest of the object's LODs.
+// Objects above which a pass keeps their names: in smaller scenes the update kernel has the objects'
+// fields on their way beside the rows instead of a round trip after the names.
+constexpr uint32_t kPatchObjects = 65536;
 struct SceneUpdate {
     VgSceneDev scene;  // object_count, instance_count, objects (written too, with src_objects) and world
     const HelioGpuInstanceData* rows;         // [count], 16-byte aligned
@@ -152,6 +155,11 @@ struct SceneUpdate {
     float4 *m_bounds, *m_axis;
     uint4* m_draw;
     uint32_t first, count, item_count, meshlet_count;
+    // [object_count] each object's instance_index, written by an update that is no patch, or null. With it a
+    // `patch` (rows only, no bounds or totals) looks for the objects to derive in 4 bytes per object
+    // (kPatchObjects)
+    uint32_t* names;
+    bool patch;
     uint32_t* bounds;
     unsigned long long* totals;
 };

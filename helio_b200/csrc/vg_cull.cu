@@ -143,6 +143,38 @@ __device__ __forceinline__ void update_meshlets(const SceneUpdate& U, uint32_t b
     }
 }
 
+// The InstanceXform of instance first + k from its row.
+__device__ __forceinline__ void put_xform(const SceneUpdate& U, uint32_t k) {
+    const float4* row = reinterpret_cast<const float4*>(U.rows + k);
+    const Mat4 m{__ldg(row), __ldg(row + 1), __ldg(row + 2), __ldg(row + 3)};
+    const float4 n0 = __ldg(row + 4), n1 = __ldg(row + 5), n2 = __ldg(row + 6);
+    const HelioInstanceCullData cd = cull_data_of(m);
+    const uint32_t flags = (cd.valid_transform ? 1u : 0u) | (cd.cone_cull_enabled ? 2u : 0u);
+    float4* x = U.xform + 6u * (size_t)(U.first + k);
+    st_pair(x, make_float4(m.c0.x, m.c0.y, m.c0.z, cd.max_scale),
+            make_float4(m.c1.x, m.c1.y, m.c1.z, __uint_as_float(flags)));
+    st_pair(x + 2, make_float4(m.c2.x, m.c2.y, m.c2.z, n0.x), make_float4(m.c3.x, m.c3.y, m.c3.z, n0.y));
+    st_pair(x + 4, make_float4(n0.z, n1.x, n1.y, n1.z), make_float4(n2.x, n2.y, n2.z, 0.0f));
+}
+
+// The ObjectWorld of object i, of `lods` LODs and the local sphere lb, which names row k. Returns the
+// LODs of the record (0: the object is never visible) and its world sphere.
+__device__ __forceinline__ uint32_t put_world(const SceneUpdate& U, uint32_t i, uint32_t k, uint32_t lods, float4 lb,
+                                              float4& sphere) {
+    const Mat4 model = ldg_mat4(U.rows[k].model);
+    const HelioInstanceCullData cd = cull_data_of(model);
+    uint32_t live = 0;
+    if (lods && cd.valid_transform) {
+        const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
+        sphere = make_float4(c.x, c.y, c.z, fmaxf(fmul(lb.w, cd.max_scale), 0.0f));
+        live = lods;
+    }
+    U.world[2u * (size_t)i] = make_uint4(__float_as_uint(sphere.x), __float_as_uint(sphere.y),
+                                         __float_as_uint(sphere.z), __float_as_uint(sphere.w));
+    U.world[2u * (size_t)i + 1u] = make_uint4(__float_as_uint(cd.max_scale), live, U.first + k, 0u);
+    return live;
+}
+
 template <bool kTotals>
 __global__ void __launch_bounds__(kUpdateThreads, 4)
     scene_update_kernel(const __grid_constant__ SceneUpdate U, uint32_t object_blocks, uint32_t item_blocks) {
@@ -155,7 +187,6 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
         return;
     }
     const uint32_t i0 = blockIdx.x * kUpdateThreads, i = i0 + threadIdx.x;
-    const HelioGpuInstanceData* rows = U.rows;  // row k = instance first + k
     if (U.src_objects && i0 < S.object_count)
         copy_words<8>(reinterpret_cast<uint4*>(S.objects + i0), reinterpret_cast<const uint4*>(U.src_objects + i0),
                       min(kUpdateThreads, S.object_count - i0) * (uint32_t)(sizeof(HelioGpuVgObject) / 16));
@@ -167,18 +198,7 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
         head = __ldg(reinterpret_cast<const uint2*>(obj));
         lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
     }
-    if (i < U.count) {
-        const float4* row = reinterpret_cast<const float4*>(rows + i);
-        const Mat4 m{__ldg(row), __ldg(row + 1), __ldg(row + 2), __ldg(row + 3)};
-        const float4 n0 = __ldg(row + 4), n1 = __ldg(row + 5), n2 = __ldg(row + 6);
-        const HelioInstanceCullData cd = cull_data_of(m);
-        const uint32_t flags = (cd.valid_transform ? 1u : 0u) | (cd.cone_cull_enabled ? 2u : 0u);
-        float4* x = U.xform + 6u * (size_t)(U.first + i);
-        st_pair(x, make_float4(m.c0.x, m.c0.y, m.c0.z, cd.max_scale),
-                make_float4(m.c1.x, m.c1.y, m.c1.z, __uint_as_float(flags)));
-        st_pair(x + 2, make_float4(m.c2.x, m.c2.y, m.c2.z, n0.x), make_float4(m.c3.x, m.c3.y, m.c3.z, n0.y));
-        st_pair(x + 4, make_float4(n0.z, n1.x, n1.y, n1.z), make_float4(n2.x, n2.y, n2.z, 0.0f));
-    }
+    if (i < U.count) put_xform(U, i);
     uint32_t rad = 0u, far1 = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
     unsigned long long lod0 = 0, spans = 0, draws = 0;
     if (i < S.object_count) {
@@ -197,17 +217,9 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
         float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t live = 0;
         const bool named = head.x < S.instance_count;
+        if (U.names) U.names[i] = head.x;
         if (named && head.x - U.first < U.count) {
-            const Mat4 model = ldg_mat4(rows[head.x - U.first].model);
-            const HelioInstanceCullData cd = cull_data_of(model);
-            if (lods && cd.valid_transform) {
-                const F3 c = mat4_point3(model, f3(lb.x, lb.y, lb.z));
-                sphere = make_float4(c.x, c.y, c.z, fmaxf(fmul(lb.w, cd.max_scale), 0.0f));
-                live = lods;
-            }
-            U.world[2u * (size_t)i] = make_uint4(__float_as_uint(sphere.x), __float_as_uint(sphere.y),
-                                                 __float_as_uint(sphere.z), __float_as_uint(sphere.w));
-            U.world[2u * (size_t)i + 1u] = make_uint4(__float_as_uint(cd.max_scale), live, head.x, 0u);
+            live = put_world(U, i, head.x - U.first, lods, lb, sphere);
         } else if (!named) {
             U.world[2u * (size_t)i] = U.world[2u * (size_t)i + 1u] = make_uint4(0u, 0u, 0u, 0u);
         } else if (U.bounds) {
@@ -249,6 +261,32 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
     __syncthreads();
     if (U.bounds && threadIdx.x < 2 && s_max[threadIdx.x]) atomicMax(U.bounds + threadIdx.x, s_max[threadIdx.x]);
     if (kTotals && threadIdx.x < 3 && s_sum[threadIdx.x]) atomicAdd(U.totals + threadIdx.x, s_sum[threadIdx.x]);
+}
+
+// A patch: a thread per row, and the objects' names over the grid, four loads in flight per thread; the
+// objects that name a row in the range are derived again. Reading every object's head and bounds for
+// that made a patch of one row as slow as the scene is large (a million objects: 19.4 us, 5.1 with
+// the names).
+__global__ void __launch_bounds__(kUpdateThreads) scene_patch_kernel(const __grid_constant__ SceneUpdate U) {
+    const VgSceneDev& S = U.scene;
+    pdl_wait();
+    const uint32_t i = blockIdx.x * kUpdateThreads + threadIdx.x, step = gridDim.x * kUpdateThreads;
+    if (i < U.count) put_xform(U, i);  // (a thread per row at the least)
+    for (uint64_t o0 = i; o0 < S.object_count; o0 += 4ull * step) {
+        uint32_t k[4];  // the row that object o0 + j * step names
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            k[j] = o0 + (uint64_t)j * step < S.object_count ? U.names[o0 + (uint64_t)j * step] - U.first : 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            if (k[j] >= U.count) continue;
+            const uint32_t o = (uint32_t)(o0 + (uint64_t)j * step);
+            const uint32_t lods = min(__ldg(&S.objects[o].lod_count), 8u);
+            const float4 lb = __ldg(reinterpret_cast<const float4*>(S.objects[o].local_bounds));
+            float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
+            put_world(U, o, k[j], lods, lb, sphere);
+        }
+    }
 }
 
 // ── View constants ────────────────────────────────────────────────────────────
@@ -694,6 +732,17 @@ cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream) {
     const uint32_t meshlets = u.src_meshlets ? blocks(u.meshlet_count, kUpdateMeshlets) : 0u;
     if (objects + items + meshlets == 0u) return cudaSuccess;
     helio_launch_begin("scene_update", stream);
+    if (u.patch && u.names) {
+        // A thread per row, and for the names at most one wave.
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const uint32_t grid = std::max(blocks(u.count, kUpdateThreads),
+                                       std::min(blocks(u.scene.object_count, kUpdateThreads), 8u * (uint32_t)std::max(sms, 1)));
+        const cudaError_t e = launch_after(scene_patch_kernel, grid, kUpdateThreads, 0, stream, u);
+        helio_launch_end(stream);
+        return e;
+    }
     const cudaError_t e = launch_after(u.totals ? scene_update_kernel<true> : scene_update_kernel<false>,
                                        objects + items + meshlets, kUpdateThreads, 0, stream, u, objects, items);
     helio_launch_end(stream);
@@ -738,7 +787,8 @@ cudaError_t launch_scene_update_from(SceneUpdate u, const HelioGpuInstanceData* 
         u.bounds = done == count ? bounds : nullptr;
         u.totals = done == count ? totals : nullptr;
         if ((e = launch_scene_update(u, stream)) != cudaSuccess) return e;
-        // The first piece has copied the rest of the scene.
+        // The first piece has copied the rest of the scene, and written the names.
+        u.patch = !bounds && !totals;
         u.src_objects = nullptr;
         u.src_items = nullptr;
         u.src_meshlets = nullptr;
