@@ -204,3 +204,36 @@ def test_shadow_cull_launch_forms(cuda, draws, faces):
         ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf, dst=ref_dst, counts=ref_counts)
         assert ran
         check_frame(dst, counts, ref_dst, ref_counts, np.nonzero(dirty)[0])
+
+
+# The decision is taken from the sign bits of the distances, for which a NaN distance (visible, as
+# every comparison with it fails) must not carry one: spheres and matrices of both signs of NaN with
+# several payloads, infinities, values whose sums and products overflow, zeros of both signs and
+# subnormals, alone and mixed into ordinary ones.
+@pytest.mark.parametrize("draws", [900, 2048, 5000])
+@pytest.mark.parametrize("share", [0.05, 0.5])
+def test_shadow_cull_of_special_values(cuda, draws, share):
+    rng = np.random.default_rng(draws + int(100 * share))
+    special = np.concatenate([
+        np.array([0x7FC00000, 0xFFC00000, 0x7F800001, 0xFF800001, 0x7FFFFFFF, 0xFFFFFFFF, 0x7FD12345, 0xFFD12345],
+                 np.uint32).view(np.float32),
+        np.array([np.inf, -np.inf, 3e38, -3e38, 1e20, -1e20, 0.0, -0.0, 1e-45, -1e-45, 1e-39, -1e-39], np.float32)])
+    mats, nf = shadow_faces(11)
+    inst, src = shadow_scene(12, 3000, draws)
+
+    def mix(a):
+        flat = a.reshape(-1).view(np.uint32).copy()
+        at = rng.random(flat.size) < share
+        flat[at] = special.view(np.uint32)[rng.integers(0, len(special), int(at.sum()))]
+        return flat.view(np.float32).reshape(a.shape)
+
+    inst["bounds"] = mix(np.ascontiguousarray(inst["bounds"]))
+    mats = np.concatenate([mats[:nf // 2], mix(mats[nf // 2:])])  # half the faces with ordinary matrices
+    dirty = np.zeros(256, np.uint32)
+    dirty[:nf] = 1
+    dst, counts = Gpu().run(mats, inst, src, dirty, nf)
+    ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf)
+    assert ran
+    check_frame(dst, counts, ref_dst, ref_counts, range(nf))
+    live = inst["bounds"][np.minimum(src[:, 4], 2999)]
+    assert np.isnan(live).any() and 0 < ref_counts[:nf // 2].sum()
