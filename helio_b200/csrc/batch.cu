@@ -325,7 +325,7 @@ __device__ void phase_setup(const BatchParams& P) {
             s_c.hiz.level[l] = HizLevel{V.hiz.levels[l], V.hiz.lw[l], V.hiz.lh[l]};
             s_c.hiz.pitch[l] = V.hiz.lpitch[l];
         } else if (lane == 0) {
-            s_c.vp = ldg_mat4(V.camera.view_proj);
+            s_c.vp = ld_mat4(V.camera.view_proj);
             s_c.pos_near = __ldg(reinterpret_cast<const float4*>(V.camera.position_near));
             s_c.p00 = __ldg(&V.camera.proj[0]);
             s_c.p11 = __ldg(&V.camera.proj[5]);
@@ -1302,7 +1302,7 @@ __global__ void __launch_bounds__(kBatchThreads) pack_draws_kernel(const BatchVi
     static_assert(kBatchMaxViews <= kBatchThreads, "one thread per view");
     const uint32_t tid = threadIdx.x;
     pdl_wait();
-    const uint32_t n = tid < V ? min(__ldg(views[tid].counters), views[tid].capacity) : 0u;
+    const uint32_t n = tid < V ? min(ld_weak(views[tid].counters), views[tid].capacity) : 0u;
     // A published count is at most 2^32 - 1 draws and V at most 128: the low and high halves
     // are scanned apart, so that the 64-bit bases are exact.
     uint32_t lo_total, hi_total, units;
@@ -1343,9 +1343,9 @@ __global__ void __launch_bounds__(kBatchThreads) pack_draws_kernel(const BatchVi
 #pragma unroll
         for (uint32_t k = 0; k < 5; ++k) {
             const uint32_t i = k * kPackUnit + tid;
-            w[k] = i < count * 5u ? __ldg(src_i + i) : 0u;
+            w[k] = i < count * 5u ? ld_weak(src_i + i) : 0u;
         }
-        if (tid < count) rec = __ldg(src_d + tid);
+        if (tid < count) rec = ld_weak(src_d + tid);
 #pragma unroll
         for (uint32_t k = 0; k < 5; ++k) {
             const uint32_t i = k * kPackUnit + tid;

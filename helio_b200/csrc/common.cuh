@@ -75,6 +75,23 @@ __device__ __forceinline__ bool quotient_le(float a, float b, float r, const Quo
     return fdiv(a, b) <= q.thr;
 }
 
+// A load of what an earlier kernel of the stream, or its caller's, may have written. An ordinary one: the
+// read-only path (ld.global.nc, __ldg) promises that nothing is written while the kernel runs, which
+// a kernel launched as a dependent cannot, since it may be resident before the one that writes has
+// ended; and no fence or clobber keeps a load of that kind behind pdl_wait.
+template <typename T>
+__device__ __forceinline__ T ld_weak(const T* p) {
+    return *p;
+}
+// (The cull kernels use __ldca, the same load as a function of its own, which the compiler keeps where
+// the code has it: as ordinary loads of structures' pointers they cost the frame kernel 276 bytes of
+// spills, and frames of 100,000 objects 43.7 instead of 37.7 us.)
+// x, known to the compiler only behind the wait before it (volatile statements keep their order).
+__device__ __forceinline__ uint32_t after_wait(uint32_t x) {
+    asm volatile("" : "+r"(x));
+    return x;
+}
+
 // Column-major 4x4 matrix held as four columns.
 struct Mat4 {
     float4 c0, c1, c2, c3;
@@ -84,9 +101,9 @@ __device__ __forceinline__ Mat4 load_mat4(const float* m) {
     const float4* p = reinterpret_cast<const float4*>(m);
     return Mat4{p[0], p[1], p[2], p[3]};
 }
-__device__ __forceinline__ Mat4 ldg_mat4(const float* m) {
+__device__ __forceinline__ Mat4 ld_mat4(const float* m) {
     const float4* p = reinterpret_cast<const float4*>(m);
-    return Mat4{__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3)};
+    return Mat4{ld_weak(p), ld_weak(p + 1), ld_weak(p + 2), ld_weak(p + 3)};
 }
 
 // (M * vec4(p, 1)).xyz
@@ -153,7 +170,7 @@ __device__ __forceinline__ float hiz_sample(const HizView& hz, float u, float v,
     ix = min(max(ix, 0), (int)w - 1);
     iy = min(max(iy, 0), (int)h - 1);
     const float* p = lv.texels + (size_t)iy * hz.pitch[l] + ix;
-    return kCoherent ? __ldcg(p) : __ldg(p);
+    return kCoherent ? __ldcg(p) : __ldca(p);
 }
 
 // Frustum planes as published by vg_cull.wgsl:266-280 (GPU form, no length guard).
@@ -191,10 +208,10 @@ __device__ __forceinline__ void publish_planes_warp(const float* vp, Planes& out
         float p[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float r3 = __ldg(vp + c * 4 + 3);
-            const float rr = __ldg(vp + c * 4 + (lane >> 1));  // rows 0,0,1,1,2,2
-            if (lane == 4) p[c] = __ldg(vp + c * 4 + 2);
-            else if (lane == 5) p[c] = fsub(r3, __ldg(vp + c * 4 + 2));
+            const float r3 = ld_weak(vp + c * 4 + 3);
+            const float rr = ld_weak(vp + c * 4 + (lane >> 1));  // rows 0,0,1,1,2,2
+            if (lane == 4) p[c] = ld_weak(vp + c * 4 + 2);
+            else if (lane == 5) p[c] = fsub(r3, ld_weak(vp + c * 4 + 2));
             else if (lane & 1) p[c] = fsub(r3, rr);
             else p[c] = fadd(r3, rr);
         }

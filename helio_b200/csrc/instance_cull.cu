@@ -45,7 +45,7 @@ __device__ float static_hiz_sample(const InstanceCullParams& P, float x, float y
     const uint32_t W = P.static_dims[0], H = P.static_dims[1], D = P.static_dims[2] * 6u;
     const StaticTap tx = static_tap(x, W), ty = static_tap(y, H), tz = static_tap(z, D);
     const float* T = P.static_texels;
-    auto at = [&](uint32_t i, uint32_t j, uint32_t k) { return __ldg(T + ((size_t)k * H + j) * W + i); };
+    auto at = [&](uint32_t i, uint32_t j, uint32_t k) { return ld_weak(T + ((size_t)k * H + j) * W + i); };
     const float c00 = static_lerp(at(tx.i0, ty.i0, tz.i0), at(tx.i1, ty.i0, tz.i0), tx.w);
     const float c10 = static_lerp(at(tx.i0, ty.i1, tz.i0), at(tx.i1, ty.i1, tz.i0), tx.w);
     const float c01 = static_lerp(at(tx.i0, ty.i0, tz.i1), at(tx.i1, ty.i0, tz.i1), tx.w);
@@ -97,17 +97,17 @@ __device__ __forceinline__ uint32_t cull_draw(const InstanceCullParams& P, const
     } else if (active) {
         const HelioGpuDrawCall dc = P.draw_calls[idx];
         const uint32_t ii = dc.first_instance;
-        const float4 bounds = __ldg(reinterpret_cast<const float4*>(P.instances[ii].bounds));
-        const uint32_t flags = __ldg(&P.instances[ii].flags);
+        const float4 bounds = ld_weak(reinterpret_cast<const float4*>(P.instances[ii].bounds));
+        const uint32_t flags = ld_weak(&P.instances[ii].flags);
         const HelioGpuCameraUniforms* cam = P.camera;
-        const Mat4 vp = ldg_mat4(cam->view_proj);
+        const Mat4 vp = ld_mat4(cam->view_proj);
         const F3 center = f3(bounds.x, bounds.y, bounds.z);
         const float radius = bounds.w;
         uint32_t instance_count_out = 0u;  // value of indirect[idx].instance_count after the frustum stage
 
         if (kFrustum) {
-            const float4 amin = __ldg(reinterpret_cast<const float4*>(P.aabbs[ii].min));
-            const float4 amax = __ldg(reinterpret_cast<const float4*>(P.aabbs[ii].max));
+            const float4 amin = ld_weak(reinterpret_cast<const float4*>(P.aabbs[ii].min));
+            const float4 amax = ld_weak(reinterpret_cast<const float4*>(P.aabbs[ii].max));
             // aabb_in_frustum (:88-98)
             bool aabb_visible = true;
 #pragma unroll
@@ -134,7 +134,7 @@ __device__ __forceinline__ uint32_t cull_draw(const InstanceCullParams& P, const
             if (visible) {
                 const float4 clip = mat4_point4(vp, center);
                 if (clip.w > 0.0f) {
-                    const float p11 = __ldg(&cam->proj[5]);
+                    const float p11 = ld_weak(&cam->proj[5]);
                     float r_ndc = fabsf(fdiv(fmul(radius, p11), clip.w));
                     if (r_ndc < 0.001f) should_draw = false;
                 }
@@ -164,7 +164,7 @@ __device__ __forceinline__ uint32_t cull_draw(const InstanceCullParams& P, const
             if (radius > 0.0f) {
                 const float4 clip = mat4_point4(vp, center);
                 if (clip.w > 0.0f) {
-                    const float p00 = __ldg(&cam->proj[0]), p11 = __ldg(&cam->proj[5]);
+                    const float p00 = ld_weak(&cam->proj[0]), p11 = ld_weak(&cam->proj[5]);
                     const float ndc_x = fdiv(clip.x, clip.w), ndc_y = fdiv(clip.y, clip.w);
                     const float uv_x = fadd(fmul(ndc_x, 0.5f), 0.5f), uv_y = fadd(fmul(ndc_y, -0.5f), 0.5f);
                     const float ndc_r = fmaxf(fabsf(fdiv(fmul(radius, p00), clip.w)), fabsf(fdiv(fmul(radius, p11), clip.w)));
@@ -172,7 +172,7 @@ __device__ __forceinline__ uint32_t cull_draw(const InstanceCullParams& P, const
                                      fadd(ndc_y, ndc_r) < -1.0f || fsub(ndc_y, ndc_r) > 1.0f;
                     if (!off) {
                         // sphere_near_depth (:124-140)
-                        const float4 pn = __ldg(reinterpret_cast<const float4*>(cam->position_near));
+                        const float4 pn = ld_weak(reinterpret_cast<const float4*>(cam->position_near));
                         const F3 tc = sub3(center, f3(pn.x, pn.y, pn.z));
                         const float dist_sq = dot3(tc, tc);
                         float near_z = 0.0f;

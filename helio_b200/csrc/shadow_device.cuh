@@ -95,7 +95,7 @@ __device__ __forceinline__ float4 shadow_normalize(float4 p) {
 // of the (256-thread) block calls it.
 __device__ __forceinline__ uint32_t shadow_list_dirty(const uint32_t* face_dirty, ShadowSmem& s) {
     const uint32_t f = threadIdx.x, lane = f & 31u, warp = f >> 5;
-    const bool dirty = __ldg(face_dirty + f) != 0u;
+    const bool dirty = ld_weak(face_dirty + f) != 0u;
     const uint32_t bal = __ballot_sync(0xffffffffu, dirty);
     __syncthreads();  // the block's previous use of s is over
     if (lane == 0) s.warp[warp] = __popc(bal);
@@ -132,9 +132,9 @@ __device__ __forceinline__ float4 shadow_face_plane(const float* m, uint32_t i) 
 __device__ __forceinline__ float4 shadow_draw_sphere(const ShadowDev& D, uint32_t d, bool& live) {
     live = false;
     if (d >= D.draw_count) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t fi = __ldg(&D.src[d].first_instance);
+    const uint32_t fi = ld_weak(&D.src[d].first_instance);
     if (fi >= D.instance_count) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 b = __ldg(reinterpret_cast<const float4*>(D.instances[fi].bounds));
+    const float4 b = ld_weak(reinterpret_cast<const float4*>(D.instances[fi].bounds));
     live = !(b.w <= 0.0f);
     return b;
 }
@@ -311,7 +311,7 @@ static __device__ __noinline__ void shadow_scan_chunk(const ShadowDev& D, uint32
 
 // The counts of the clean faces are cleared (lib.rs:266-270); one block calls it.
 __device__ __forceinline__ void shadow_clear_clean(const ShadowDev& D) {
-    if (__ldg(D.face_dirty + threadIdx.x) == 0u) D.face_counts[threadIdx.x] = 0u;
+    if (ld_weak(D.face_dirty + threadIdx.x) == 0u) D.face_counts[threadIdx.x] = 0u;
 }
 
 // Stores the warp's visible draws (bit i of lane j's word: draw i in face j) at lane j's `at` +

@@ -74,7 +74,7 @@ __device__ __forceinline__ HelioInstanceCullData cull_data_of(const Mat4& mm) {
 __global__ void instance_cull_data_kernel(const HelioGpuInstanceData* __restrict__ inst, uint32_t n,
                                           HelioInstanceCullData* __restrict__ out) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = cull_data_of(ldg_mat4(inst[i].model));
+        out[i] = cull_data_of(ld_mat4(inst[i].model));
 }
 
 // launch_scene_update. CTAs come in three kinds: one per 256 rows and 256 objects (the same
@@ -101,7 +101,7 @@ __device__ __forceinline__ void copy_words(uint4* dst, const uint4* src, uint32_
     uint4 x[kEach];
 #pragma unroll
     for (int k = 0; k < kEach; ++k)
-        if (k * kUpdateThreads + threadIdx.x < n) x[k] = __ldg(src + k * kUpdateThreads + threadIdx.x);
+        if (k * kUpdateThreads + threadIdx.x < n) x[k] = ld_weak(src + k * kUpdateThreads + threadIdx.x);
 #pragma unroll
     for (int k = 0; k < kEach; ++k)
         if (k * kUpdateThreads + threadIdx.x < n) dst[k * kUpdateThreads + threadIdx.x] = x[k];
@@ -114,7 +114,7 @@ __device__ __forceinline__ void update_items(const SceneUpdate& U, uint32_t bloc
     const uint64_t i0 = (uint64_t)block * kUpdateItems + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        if (i0 + k * kUpdateThreads < U.item_count) x[k] = __ldg(src + i0 + k * kUpdateThreads);
+        if (i0 + k * kUpdateThreads < U.item_count) x[k] = ld_weak(src + i0 + k * kUpdateThreads);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
         if (i0 + k * kUpdateThreads < U.item_count) dst[i0 + k * kUpdateThreads] = x[k];
@@ -146,8 +146,8 @@ __device__ __forceinline__ void update_meshlets(const SceneUpdate& U, uint32_t b
 // The InstanceXform of instance first + k from its row.
 __device__ __forceinline__ void put_xform(const SceneUpdate& U, uint32_t k) {
     const float4* row = reinterpret_cast<const float4*>(U.rows + k);
-    const Mat4 m{__ldg(row), __ldg(row + 1), __ldg(row + 2), __ldg(row + 3)};
-    const float4 n0 = __ldg(row + 4), n1 = __ldg(row + 5), n2 = __ldg(row + 6);
+    const Mat4 m{ld_weak(row), ld_weak(row + 1), ld_weak(row + 2), ld_weak(row + 3)};
+    const float4 n0 = ld_weak(row + 4), n1 = ld_weak(row + 5), n2 = ld_weak(row + 6);
     const HelioInstanceCullData cd = cull_data_of(m);
     const uint32_t flags = (cd.valid_transform ? 1u : 0u) | (cd.cone_cull_enabled ? 2u : 0u);
     float4* x = U.xform + 6u * (size_t)(U.first + k);
@@ -161,7 +161,7 @@ __device__ __forceinline__ void put_xform(const SceneUpdate& U, uint32_t k) {
 // LODs of the record (0: the object is never visible) and its world sphere.
 __device__ __forceinline__ uint32_t put_world(const SceneUpdate& U, uint32_t i, uint32_t k, uint32_t lods, float4 lb,
                                               float4& sphere) {
-    const Mat4 model = ldg_mat4(U.rows[k].model);
+    const Mat4 model = ld_mat4(U.rows[k].model);
     const HelioInstanceCullData cd = cull_data_of(model);
     uint32_t live = 0;
     if (lods && cd.valid_transform) {
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
         else update_meshlets(U, b - item_blocks);
         return;
     }
-    const uint32_t i0 = blockIdx.x * kUpdateThreads, i = i0 + threadIdx.x;
+    const uint32_t i0 = blockIdx.x * kUpdateThreads, i = after_wait(i0 + threadIdx.x);
     if (U.src_objects && i0 < S.object_count)
         copy_words<8>(reinterpret_cast<uint4*>(S.objects + i0), reinterpret_cast<const uint4*>(U.src_objects + i0),
                       min(kUpdateThreads, S.object_count - i0) * (uint32_t)(sizeof(HelioGpuVgObject) / 16));
@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
     uint2 head = make_uint2(0u, 0u);  // instance_index, lod_count
     float4 lb = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < S.object_count) {
-        head = __ldg(reinterpret_cast<const uint2*>(obj));
-        lb = __ldg(reinterpret_cast<const float4*>(obj->local_bounds));
+        head = ld_weak(reinterpret_cast<const uint2*>(obj));
+        lb = ld_weak(reinterpret_cast<const float4*>(obj->local_bounds));
     }
     if (i < U.count) put_xform(U, i);
     uint32_t rad = 0u, far1 = 0u;  // bits of the largest radius and centre (non-negative floats order like their bits)
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(kUpdateThreads, 4)
     if (i < S.object_count) {
         const uint32_t lods = min(head.y, 8u);
         if (kTotals) {
-            const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts));
-            const uint4 c1 = __ldg(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts + 4));
+            const uint4 c0 = ld_weak(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts));
+            const uint4 c1 = ld_weak(reinterpret_cast<const uint4*>(obj->lod_meshlet_counts + 4));
             const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
             uint32_t mx = 0;
 #pragma unroll
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kUpdateThreads) scene_patch_kernel(const __gri
         for (uint32_t j = 0; j < 4; ++j) {
             if (k[j] >= U.count) continue;
             const uint32_t o = (uint32_t)(o0 + (uint64_t)j * step);
-            const uint32_t lods = min(__ldg(&S.objects[o].lod_count), 8u);
-            const float4 lb = __ldg(reinterpret_cast<const float4*>(S.objects[o].local_bounds));
+            const uint32_t lods = min(ld_weak(&S.objects[o].lod_count), 8u);
+            const float4 lb = ld_weak(reinterpret_cast<const float4*>(S.objects[o].local_bounds));
             float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
             put_world(U, o, k[j], lods, lb, sphere);
         }
@@ -302,10 +302,10 @@ __device__ __forceinline__ void view_setup_warp(const ViewSetupParams& P, CullVi
         reinterpret_cast<uint32_t*>(&v.hiz)[k] = reinterpret_cast<const uint32_t*>(&P.hiz)[k];
     if (lane == 0) {
         const HelioGpuCameraUniforms* cam = P.camera;
-        v.vp = ldg_mat4(cam->view_proj);
-        v.pos_near = __ldg(reinterpret_cast<const float4*>(cam->position_near));
-        v.p00 = __ldg(&cam->proj[0]);
-        v.p11 = __ldg(&cam->proj[5]);
+        v.vp = ld_mat4(cam->view_proj);
+        v.pos_near = ld_weak(reinterpret_cast<const float4*>(cam->position_near));
+        v.p00 = ld_weak(&cam->proj[0]);
+        v.p11 = ld_weak(&cam->proj[5]);
         v.focal = fmul(fmul(fabsf(v.p11), (float)P.screen_height), 0.5f);
         v.lod_threshold_px = P.lod_threshold_px;
         v.screen_height = P.screen_height;
@@ -329,8 +329,8 @@ __device__ __forceinline__ Selected select_object(const VgSceneDev& S, const Cul
     const float wr = w.sphere.w;
     if (w.lod_count == 0u || !sphere_visible_vg(view.planes, c, wr)) return r;
     const HelioGpuVgObject* o = S.objects + i;
-    const float4 e0 = __ldg(reinterpret_cast<const float4*>(o->lod_errors));
-    const float4 e1 = __ldg(reinterpret_cast<const float4*>(o->lod_errors + 4));
+    const float4 e0 = __ldca(reinterpret_cast<const float4*>(o->lod_errors));
+    const float4 e1 = __ldca(reinterpret_cast<const float4*>(o->lod_errors + 4));
     const float4 pn = view.pos_near;
     const F3 d = sub3(c, f3(pn.x, pn.y, pn.z));
     const float dist = fsqrt(dot3(d, d));
@@ -359,7 +359,7 @@ constexpr uint32_t kObjectBlock = kObjectRounds * kCullWarps * 32u;
 __device__ void object_block(const VgFrameParams& P, const CullView& view, uint32_t block, uint32_t blocks,
                              uint32_t* s_hist, uint32_t* s_flag) {
     const VgSceneDev& S = P.scene;
-    const uint32_t i0 = block * kObjectBlock + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t i0 = after_wait(block * kObjectBlock + threadIdx.x), lane = threadIdx.x & 31u;
     if (threadIdx.x < 9) s_hist[threadIdx.x] = 0u;
     Selected r[kObjectRounds];
 #pragma unroll
@@ -593,15 +593,15 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
     for (uint32_t r = 0; r < kItemRounds; ++r) {
         n[r] = first[r] = inst[r] = lod[r] = 0u;
         if (r * kThreads + tid >= P.tile_items || w0 + r * kThreads >= S.work_item_count) continue;
-        const uint2 it = __ldg(reinterpret_cast<const uint2*>(S.items + w0 + r * kThreads));  // object, local meshlet base
+        const uint2 it = __ldca(reinterpret_cast<const uint2*>(S.items + w0 + r * kThreads));  // object, local meshlet base
         if (it.x >= S.object_count) continue;
         const HelioGpuVgObject* o = S.objects + it.x;
         const Selected sel = select_object(S, s_view, it.x);
         if (!sel.sel) continue;
-        const uint32_t count = __ldg(&o->lod_meshlet_counts[sel.sel - 1u]);
+        const uint32_t count = __ldca(&o->lod_meshlet_counts[sel.sel - 1u]);
         if (it.y >= count) continue;
         n[r] = min(64u, count - it.y);
-        first[r] = __ldg(&o->lod_first_meshlets[sel.sel - 1u]) + it.y;
+        first[r] = __ldca(&o->lod_first_meshlets[sel.sel - 1u]) + it.y;
         inst[r] = sel.instance;
         lod[r] = sel.sel - 1u;
     }
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
             if ((b[q] >> lane) & 1u) {
                 k[q] = item_at(s_it, w);
                 mi[q] = s_it.first[k[q]] + (w * 32u + lane - s_it.off[k[q]]);
-                d[q] = __ldg(S.m_draw + mi[q]);
+                d[q] = __ldca(S.m_draw + mi[q]);
             }
         }
 #pragma unroll

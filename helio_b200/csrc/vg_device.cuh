@@ -7,9 +7,9 @@
 
 namespace helio {
 
-// 32 bytes in one load (sm_100); p is 32-byte aligned.
-__device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+// 32 bytes in one load (sm_100); p is 32-byte aligned. (Not of the read-only path: see ld_weak.)
+__device__ __forceinline__ void ld_pair(const float4* p, float4& a, float4& b) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
         : "l"(p));
 }
@@ -26,14 +26,14 @@ struct InstanceView {
 __device__ __forceinline__ InstanceView load_instance(const VgSceneDev& S, uint32_t i) {
     const float4* p = S.xform + 6u * (size_t)i;
     InstanceView v;
-    ldg_pair(p, v.model.c0, v.model.c1);
-    ldg_pair(p + 2, v.model.c2, v.model.c3);
+    ld_pair(p, v.model.c0, v.model.c1);
+    ld_pair(p + 2, v.model.c2, v.model.c3);
     return v;
 }
 
 // The rest of the normal matrix of instance i.
 __device__ __forceinline__ void load_normal(const VgSceneDev& S, uint32_t i, float4& na, float4& nb) {
-    ldg_pair(S.xform + 6u * (size_t)i + 4u, na, nb);
+    ld_pair(S.xform + 6u * (size_t)i + 4u, na, nb);
 }
 
 // mat3(normal matrix) * axis, in the order of mat3_vec.
@@ -43,7 +43,7 @@ __device__ __forceinline__ F3 normal_vec(const InstanceView& v, float4 na, float
 }
 
 __device__ __forceinline__ ObjectWorld load_world(const VgSceneDev& S, uint32_t o) {
-    const uint4 a = __ldg(S.world + 2u * (size_t)o), b = __ldg(S.world + 2u * (size_t)o + 1u);
+    const uint4 a = __ldca(S.world + 2u * (size_t)o), b = __ldca(S.world + 2u * (size_t)o + 1u);
     ObjectWorld w;
     w.sphere = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w));
     w.max_scale = __uint_as_float(b.x);
@@ -95,9 +95,9 @@ __device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const Vg
                                                      uint32_t instance, F3& c, float& wr) {
     const InstanceView in = load_instance(S, instance);
     float4 b, cone, axis, na, nb;
-    ldg_pair(S.m_bounds + 2u * (size_t)mi, b, cone);
+    ld_pair(S.m_bounds + 2u * (size_t)mi, b, cone);
     if (!kLazyCone) {
-        axis = __ldg(S.m_axis + mi);
+        axis = __ldca(S.m_axis + mi);
         load_normal(S, instance, na, nb);
     }
     if (!in.valid()) return false;
@@ -112,7 +112,7 @@ __device__ __forceinline__ bool meshlet_frustum_cone(const CullView& C, const Vg
         const float guard = fmul(wr, 1.5f);
         if (cam_dist_sq > fmul(guard, guard) && cone.w <= 1.0f) {
             if (kLazyCone) {
-                axis = __ldg(S.m_axis + mi);
+                axis = __ldca(S.m_axis + mi);
                 load_normal(S, instance, na, nb);
             }
             const F3 a = normal_vec(in, na, nb, axis);
