@@ -1360,30 +1360,23 @@ cudaError_t launch_pack_draws(const BatchViewDev* views, uint32_t view_count, He
     if (!view_count) return cudaGetLastError();
     // As many CTAs as stay resident: the totals are known on the device only, and a CTA without
     // units leaves after the table.
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return launch_after(pack_draws_kernel, (uint32_t)(sms > 0 ? sms : 1) * 8u, kBatchThreads, 0, stream, views,
+    return launch_after(pack_draws_kernel, device_sms() * 8u, kBatchThreads, 0, stream, views,
                         view_count, indirect, draws, offsets, capacity);
 }
 
 size_t batch_dynamic_smem() { return kSmTotal; }
 
 uint32_t batch_max_grid() {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per_sm = 0;
     cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmTotal);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, kBatchThreads, kSmTotal);
-    return (uint32_t)(sms * per_sm);
+    return device_sms() * (uint32_t)per_sm;
 }
 
 uint32_t batch_cull_max_grid() {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_cull_kernel, kBatchThreads, kSm2Total);
-    return (uint32_t)(sms * per_sm);
+    return device_sms() * (uint32_t)per_sm;
 }
 
 namespace {

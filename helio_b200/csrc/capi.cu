@@ -661,7 +661,7 @@ int32_t helio_vg_prepare(helio_vg_pass* p, const helio_vg_frame_data* f, void* s
             p->capacity = cap;
         }
         p->max_draw_count = bounded;
-        p->tile_items = helio::vg_tile_items(p->work_item_count);
+        p->tile_items = helio::vg_tile_items(p->work_item_count, helio::device_sms());
         p->num_tiles = helio::vg_tiles(p->work_item_count, p->tile_items);
         const size_t scratch_bytes = (16 + helio::kVgStateWords) * 4 + (size_t)p->num_tiles * 8;
         HELIO_CK(p->scratch.ensure(scratch_bytes));

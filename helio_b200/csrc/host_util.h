@@ -86,6 +86,14 @@ inline bool caller_array(bool (*rule)(const cudaPointerAttributes&, int, const v
     return rule(a, device, p, align);
 }
 
+// SMs of the current device (a cached attribute query), at least 1.
+inline uint32_t device_sms() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? (uint32_t)sms : 1u;
+}
+
 // Launches `kernel` with programmatic stream serialization: its CTAs are scheduled as those of the
 // stream's previous kernel end, and wait in pdl_wait before their first global access, which
 // hides a launch gap.

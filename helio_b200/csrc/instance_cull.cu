@@ -265,11 +265,7 @@ void launch_instance_cull(const InstanceCullParams& p, bool frustum, bool occlus
     // One wave of 4 blocks per SM; each takes its share of the draws. A million draws move 210 MB
     // (whole 144-byte rows): 40.9 us through the fused launch, 42.3 with 8 blocks per SM, the pyramid
     // descriptor copied by one thread and no early scheduling.
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);  // a cached attribute query
-    if (sms < 1) sms = 1;
-    const uint32_t blocks = std::min<uint32_t>((p.draw_count + 255u) / 256u, (uint32_t)sms * 4u);
+    const uint32_t blocks = std::min<uint32_t>((p.draw_count + 255u) / 256u, device_sms() * 4u);
     helio_launch_begin(frustum && occlusion ? "instance_cull_fused" : frustum ? "indirect_dispatch" : "occlusion_cull",
                        stream);
     launch_after(frustum && occlusion ? instance_cull_kernel<true, true>

@@ -124,7 +124,7 @@ cudaError_t launch_shadow(const ShadowDev& D, cudaStream_t s) {
     }
     // One CTA takes all chunks of its draws when the blocks alone fill the device; below that the
     // chunks are shared out, so that a CTA's chain of loads and planes is not repeated per chunk.
-    const dim3 grid(D.blocks, std::max(1u, std::min(kChunks, 148u * 6u / D.blocks)));
+    const dim3 grid(D.blocks, std::max(1u, std::min(kChunks, device_sms() * 6u / D.blocks)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);

@@ -119,9 +119,9 @@ struct VgFrameParams {
 // once); 51.5, 44.0 and 40.2 us with at most 128, 256 and 512 items (782 tiles of 256 did not fit the
 // device at once, 391 of 512 do).
 constexpr uint32_t kTilesPerSm = 1;
-inline uint32_t vg_tile_items(uint32_t work_items) {
+inline uint32_t vg_tile_items(uint32_t work_items, uint32_t sms) {
     uint32_t n = kMaxTileItems;
-    while (n > 8u && (uint64_t)work_items < 148ull * kTilesPerSm * n) n >>= 1;
+    while (n > 8u && (uint64_t)work_items < (uint64_t)sms * kTilesPerSm * n) n >>= 1;
     return n;
 }
 inline uint32_t vg_tiles(uint32_t work_items, uint32_t tile_items) {

@@ -595,7 +595,7 @@ int32_t helio_vg_builder_run(helio_vg_builder* b, const helio_vg_build_inputs* i
                                             *in, w, b->block_base.as<uint64_t>(), o);
         helio_launch_note();
         if (r != cudaSuccess) return r;
-        const uint32_t mesh_ctas = std::min(M, 148u * 8u);
+        const uint32_t mesh_ctas = std::min(M, helio::device_sms() * 8u);
         r = helio::launch_after(outputs_kernel, mesh_ctas + (uint32_t)(((uint64_t)S + kThreads - 1) / kThreads), kThreads,
                                 0, s, *in, o, mesh_ctas, w.error);
         helio_launch_note();

@@ -718,8 +718,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 5 : 4) vg_frame_kernel(const
 void launch_instance_cull_data(const HelioGpuInstanceData* inst, uint32_t n, HelioInstanceCullData* out,
                                cudaStream_t stream) {
     if (!n) return;
-    uint32_t blocks = (n + 255u) / 256u;
-    if (blocks > 148u * 16u) blocks = 148u * 16u;
+    const uint32_t blocks = std::min((n + 255u) / 256u, device_sms() * 16u);
     helio_launch_begin("instance_cull_data", stream);
     instance_cull_data_kernel<<<blocks, 256, 0, stream>>>(inst, n, out);
     helio_launch_end(stream);
@@ -734,11 +733,8 @@ cudaError_t launch_scene_update(const SceneUpdate& u, cudaStream_t stream) {
     helio_launch_begin("scene_update", stream);
     if (u.patch && u.names) {
         // A thread per row, and for the names at most one wave.
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const uint32_t grid = std::max(blocks(u.count, kUpdateThreads),
-                                       std::min(blocks(u.scene.object_count, kUpdateThreads), 8u * (uint32_t)std::max(sms, 1)));
+                                       std::min(blocks(u.scene.object_count, kUpdateThreads), 8u * device_sms()));
         const cudaError_t e = launch_after(scene_patch_kernel, grid, kUpdateThreads, 0, stream, u);
         helio_launch_end(stream);
         return e;
@@ -798,11 +794,8 @@ cudaError_t launch_scene_update_from(SceneUpdate u, const HelioGpuInstanceData* 
 
 cudaError_t launch_vg_frame(const VgFrameParams& p, cudaStream_t stream) {
     if (!p.num_tiles) return cudaSuccess;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t grid = p.num_tiles + (uint32_t)(((uint64_t)p.scene.object_count + kObjectBlock - 1) / kObjectBlock);
-    const bool wide = grid > 4u * (uint32_t)std::max(sms, 1);
+    const bool wide = grid > 4u * device_sms();
     helio_launch_begin("vg_frame", stream);
     const cudaError_t e = launch_after(wide ? vg_frame_kernel<true> : vg_frame_kernel<false>, grid, kThreads, 0, stream, p);
     helio_launch_end(stream);
