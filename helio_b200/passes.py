@@ -85,8 +85,12 @@ def device_view(ptr: int, shape, dtype: str = "<i4", strides=None) -> torch.Tens
 def _stream_ptr(stream) -> int:
     # The raw handle: building torch's Stream object takes 3 us, as long as the launch of a pass
     # (4,099 draws through both instance passes: 20.4 -> 14.5 us a pass with the handle alone).
+    # It is not of torch's public interface, so that a build without it takes the object.
     if stream is None:
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is None:
+            return torch.cuda.current_stream().cuda_stream
+        return raw(torch.cuda.current_device())
     return stream.cuda_stream
 
 
