@@ -43,8 +43,10 @@ constexpr uint32_t kErrOffset = 2u;  // an LOD descriptor offset exceeds u32
 // Mesh records are read as 16-byte words (the API requires them 16-byte aligned): a
 // warp's lanes usually name different meshes, so every load instruction touches up to
 // 32 lines, and wide loads keep the number of such instructions down.
+// (Not of the read-only path, see ld_weak; as ordinary loads they waited for the stores before them: 2M slots
+// 259 -> 271 us.)
 __device__ __forceinline__ uint4 mesh_word(const HelioVgMeshRecord* meshes, uint32_t m, int k) {
-    return helio::ld_weak(reinterpret_cast<const uint4*>(meshes + m) + k);
+    return __ldca(reinterpret_cast<const uint4*>(meshes + m) + k);
 }
 
 // Word 0 of the record: first_meshlet, meshlet_count, lod_count, max_meshlet_count.
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(kThreads) first_ref_kernel(const __grid_consta
 __global__ void __launch_bounds__(kThreads) fold_kernel(const __grid_constant__ helio_vg_build_inputs in,
                                                         const __grid_constant__ BuildWork w) {
     helio::pdl_wait();
-    const uint32_t m = blockIdx.x * kThreads + threadIdx.x;
+    const uint32_t m = helio::after_wait(blockIdx.x * kThreads + threadIdx.x);
     if (m < in.mesh_count) fold_mesh(in, w, m);
 }
 
@@ -351,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 4) place_kernel(const __grid_constan
         const bool ok = m[j] < in.mesh_count;
         h[j] = ok ? mesh_word(in.meshes, m[j], 0) : make_uint4(0u, 0u, 0u, 0u);
         // Through L1: past it, a small library's table is a few L2 lines that every slot asks for.
-        fr[j] = ok ? helio::ld_weak(w.first_ref + m[j]) : 0u;
+        fr[j] = ok ? __ldca(w.first_ref + m[j]) : 0u;
     }
     uint32_t ex[kSub][4];  // exclusive within the warp and round
 #pragma unroll
@@ -450,7 +452,7 @@ __device__ __forceinline__ void write_objects(const helio_vg_build_inputs& in, c
         const uint32_t mk = __shfl_sync(0xffffffffu, m, __shfl_sync(0xffffffffu, nth, k));
         if (k >= n_used) continue;
         x[r] = mesh_word(in.meshes, mk, (int)w);
-        base[r] = w == 4u || w == 5u ? helio::ld_weak(out.mesh_base + mk) : 0u;
+        base[r] = w == 4u || w == 5u ? __ldca(out.mesh_base + mk) : 0u;
     }
     bool over = false;
 #pragma unroll
@@ -486,7 +488,7 @@ __device__ __forceinline__ void copy_descriptors(const helio_vg_build_inputs& in
             uint4 x[4];
 #pragma unroll
             for (uint32_t k = 0; k < 4; ++k)
-                if (i0 + k * kThreads < words) x[k] = helio::ld_weak(src + i0 + k * kThreads);
+                if (i0 + k * kThreads < words) x[k] = __ldca(src + i0 + k * kThreads);
 #pragma unroll
             for (uint32_t k = 0; k < 4; ++k)
                 if (i0 + k * kThreads < words) dst[i0 + k * kThreads] = x[k];
