@@ -213,3 +213,38 @@ def test_build_forms_match_oracle(cuda, slots, meshes):
     for _ in range(2):
         _, host, _ = gpu_build(lib, b)
         assert_same(host, ref)
+
+
+@pytest.mark.parametrize("meshes", [1183, 2367, 2368, 2369, 3552, 18944, 40000])
+def test_descriptor_copies_of_many_meshes(cuda, meshes):
+    """Libraries around the sizes from which a CTA copies several meshes at a time (two per 8 CTAs of
+    148 SMs, and 16): meshes of 0 to 5 descriptors and a few of hundreds, half of them used."""
+    import torch
+    from helio_b200 import scene as S
+    from helio_b200.passes import VgBuilder
+
+    rng = np.random.default_rng(meshes)
+    m = np.zeros(meshes, S.DT_MESH)
+    m["meshlet_count"] = rng.integers(0, 6, meshes)
+    m["meshlet_count"][rng.integers(0, meshes, 5)] = rng.integers(300, 1500, 5)
+    end = np.cumsum(m["meshlet_count"], dtype=np.int64)
+    m["first_meshlet"] = end - m["meshlet_count"]
+    m["lod_count"] = 1
+    m["max_meshlet_count"] = m["meshlet_count"]
+    m["lod_meshlet_counts"][:, 0] = m["meshlet_count"]
+    pool = np.frombuffer(rng.integers(0, 2**32, size=(int(end[-1]) + 1) * 16, dtype=np.uint32).tobytes(), S.DT_MESHLET)
+    slot_mesh = rng.integers(0, meshes, 2 * meshes).astype(np.uint32)
+    slot_mesh[slot_mesh % 2 == 1] = meshes  # past the table
+    inst = np.zeros(len(slot_mesh), S.DT_INSTANCE)
+    dev = [torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy()).cuda()
+           for a in (pool, m, slot_mesh, inst)]
+    b = VgBuilder()
+    b.run(*dev)
+    got = b.outputs()["meshlets"].cpu().numpy().view(S.DT_MESHLET)
+    used = slot_mesh[slot_mesh < meshes]
+    _, at = np.unique(used, return_index=True)
+    order = used[np.sort(at)]  # first references in slot order
+    order = order[m["meshlet_count"][order] > 0]
+    rows = np.concatenate([np.arange(f, f + c) for f, c in zip(m["first_meshlet"][order], m["meshlet_count"][order])])
+    assert len(got) == len(rows)
+    assert got.tobytes() == pool[rows].tobytes()
