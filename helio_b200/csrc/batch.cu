@@ -1246,7 +1246,8 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_kernel(const __grid_co
     if (P.shadow_blocks) {
         if (blockIdx.x == 0) shadow_clear_clean(P.shadow);
         for (uint32_t j = blockIdx.x; j < kShadowChunks; j += gridDim.x)
-            shadow_scan_chunk(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow));
+            shadow_scan_chunk<kShadowWarps>(P.shadow, j, *reinterpret_cast<ShadowSmem*>(sm + kSmShadow),
+                                            reinterpret_cast<ShadowSmem*>(sm + kSmShadow)->word);
         if (!grid_sync(P)) return;
     }
     stamp(P, 3);

@@ -92,13 +92,14 @@ __device__ __forceinline__ float4 shadow_normalize(float4 p) {
 }
 
 // The dirty faces in ascending order into s.active; returns their number. Every thread
-// of the (256-thread) block calls it.
+// of the block, of kWarps >= kShadowWarps warps, calls it.
+template <uint32_t kWarps = kShadowWarps>
 __device__ __forceinline__ uint32_t shadow_list_dirty(const uint32_t* face_dirty, ShadowSmem& s) {
     const uint32_t f = threadIdx.x, lane = f & 31u, warp = f >> 5;
-    const bool dirty = ld_weak(face_dirty + f) != 0u;
+    const bool dirty = (kWarps == kShadowWarps || f < kShadowFaces) && ld_weak(face_dirty + f) != 0u;
     const uint32_t bal = __ballot_sync(0xffffffffu, dirty);
     __syncthreads();  // the block's previous use of s is over
-    if (lane == 0) s.warp[warp] = __popc(bal);
+    if (lane == 0 && (kWarps == kShadowWarps || warp < kShadowWarps)) s.warp[warp] = __popc(bal);
     __syncthreads();
     uint32_t before = 0, n = 0;
     for (uint32_t w = 0; w < kShadowWarps; ++w) {
@@ -266,37 +267,40 @@ __device__ __forceinline__ void shadow_sum_before(const ShadowDev& D, uint32_t c
 }
 
 // Scan stage of chunk c (nothing when it holds no dirty face): counts become the draws of each
-// face before each block, and the faces' totals are written. Every thread of the block calls it.
-static __device__ __noinline__ void shadow_scan_chunk(const ShadowDev& D, uint32_t c, ShadowSmem& s) {
-    const uint32_t n_active = shadow_list_dirty(D.face_dirty, s);
+// face before each block, and the faces' totals are written. Every thread of the block of kWarps
+// warps calls it; sums: a row per warp.
+template <uint32_t kWarps>
+static __device__ __noinline__ void shadow_scan_chunk(const ShadowDev& D, uint32_t c, ShadowSmem& s,
+                                                      uint32_t (*sums)[kShadowChunk]) {
+    const uint32_t n_active = shadow_list_dirty<kWarps>(D.face_dirty, s);
     if (c * kShadowChunk >= n_active) return;  // uniform over the block
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     // Each warp takes a run of blocks: its sum, then its prefixes.
-    const uint32_t run = (D.blocks + kShadowWarps - 1) / kShadowWarps;
+    const uint32_t run = (D.blocks + kWarps - 1) / kWarps;
     const uint32_t b0 = min(D.blocks, warp * run), b1 = min(D.blocks, b0 + run);
     __syncthreads();
     {
         const uint32_t* in = D.counts + (size_t)c * D.blocks * 32u + lane;
         uint32_t n = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (uint32_t b = b0; b < b1; ++b) n += __ldcg(in + (size_t)b * 32u);
-        s.word[warp][lane] = n;
+        sums[warp][lane] = n;
     }
     __syncthreads();
     uint32_t at = 0, total = 0;
 #pragma unroll
-    for (uint32_t w = 0; w < kShadowWarps; ++w) {
-        if (w < warp) at += s.word[w][lane];
-        total += s.word[w][lane];
+    for (uint32_t w = 0; w < kWarps; ++w) {
+        if (w < warp) at += sums[w][lane];
+        total += sums[w][lane];
     }
     uint32_t* counts = D.counts + (size_t)c * D.blocks * 32u + lane;
     uint32_t b = b0;
-    for (; b + 8u <= b1; b += 8u) {
-        uint32_t n[8];
+    for (; b + 16u <= b1; b += 16u) {
+        uint32_t n[16];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) n[k] = __ldcg(counts + (size_t)(b + k) * 32u);
+        for (uint32_t k = 0; k < 16; ++k) n[k] = __ldcg(counts + (size_t)(b + k) * 32u);
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
+        for (uint32_t k = 0; k < 16; ++k) {
             counts[(size_t)(b + k) * 32u] = at;
             at += n[k];
         }

@@ -237,3 +237,16 @@ def test_shadow_cull_of_special_values(cuda, draws, share):
     check_frame(dst, counts, ref_dst, ref_counts, range(nf))
     live = inst["bounds"][np.minimum(src[:, 4], 2999)]
     assert np.isnan(live).any() and 0 < ref_counts[:nf // 2].sum()
+
+
+@pytest.mark.parametrize("draws", [393217, 1000001])
+def test_shadow_cull_of_large_lists(cuda, draws):
+    """Lists whose scan gives every warp a run of blocks of several rounds and a remainder."""
+    mats, nf = shadow_faces(13)
+    inst, src = shadow_scene(14, 5000, draws)
+    dirty = np.zeros(256, np.uint32)
+    dirty[[0, 3, 17, nf - 1]] = 1
+    dst, counts = Gpu().run(mats, inst, src, dirty, nf)
+    ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf)
+    assert ran and ref_counts[3] > 4096
+    check_frame(dst, counts, ref_dst, ref_counts, np.nonzero(dirty)[0])
