@@ -224,3 +224,16 @@ def test_batch_chunk_sum_runs_match_oracle(cuda, objects, views):
     cam = S.orthographic((0, 0, 300), (0, 0, 0), (0, 1, 0), 30.0, 0.1, 600.0)
     w = S.Workload(3, sc, [S.View(cam, 64, 64, np.ones((64, 64), np.float32), "ortho")] * views)
     _check_batch(w, w.views)
+
+
+# One CTA, so 8 warps: (view, chunk) units just below, at and above one and several per warp, which
+# the expansion hands out by index (at most one batch per warp) or by claims, in batches of 1 to 8.
+@pytest.mark.parametrize("views,chunks", [(1, 7), (1, 8), (1, 9), (3, 3), (1, 15), (2, 8), (1, 17), (3, 8), (1, 25), (1, 63),
+                                          (2, 32), (1, 65), (3, 24), (1, 129)])
+def test_batch_expansion_batches_match_oracle(cuda, views, chunks):
+    from helio_b200 import scene as S
+
+    objects = 256 * chunks - 13
+    sc = S.make_scene(views * chunks, objects, 3, 4, 0, 40.0)
+    w = S.Workload(3, sc, S.multiview_set(S.SEED_BASE + 10, True, 0.05)[5:5 + views])
+    _check_batch(w, w.views, max_ctas=1)

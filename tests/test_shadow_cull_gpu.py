@@ -250,3 +250,20 @@ def test_shadow_cull_of_large_lists(cuda, draws):
     ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf)
     assert ran and ref_counts[3] > 4096
     check_frame(dst, counts, ref_dst, ref_counts, np.nonzero(dirty)[0])
+
+
+@pytest.mark.parametrize("blocks,extra", [(110, 0), (111, 0), (111, 1), (126, 1), (147, 1), (148, 0), (296, 1), (444, 0), (444, 1),
+                                          (1024, 0)])
+def test_shadow_cull_chunk_shares(cuda, blocks, extra):
+    """All 256 faces dirty at the block counts where the number of CTAs that share the chunks of a block
+    changes (eight down to one on 148 SMs), and the largest list whose place blocks sum the counts."""
+    from helio_b200 import scene as S
+
+    mats, nf = S.shadow_faces(15, 12, 40)
+    draws = 256 * blocks + extra
+    inst, src = shadow_scene(16, 4000, draws, spread=150.0)
+    dirty = np.ones(256, np.uint32)
+    dst, counts = Gpu().run(mats, inst, src, dirty, nf)
+    ref_dst, ref_counts, ran = O.shadow_cull(mats, inst, src, dirty, nf)
+    assert ran
+    check_frame(dst, counts, ref_dst, ref_counts, range(256))
