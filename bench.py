@@ -159,6 +159,14 @@ def union_meshlets(scene, lods: np.ndarray) -> int:
     return total
 
 
+def object_bytes(scene, visible: np.ndarray) -> tuple[int, int]:
+    """Bytes that the select and the meshlet tests cannot do without, once per scene, given which
+    objects some view selects (bool per object): the select reads the 32-byte world record of
+    every object, and of a selected one its 8 LOD errors and the first meshlet and count of a LOD
+    (40 B); the tests read the 96-byte record of each instance that a selected object names."""
+    return 32 * len(scene.objects) + 40 * int(visible.sum()), 96 * len(np.unique(scene.objects["instance_index"][visible]))
+
+
 # ── Workloads ─────────────────────────────────────────────────────────────────
 
 def _u32(t) -> np.ndarray:
@@ -251,11 +259,11 @@ class PlainWorkload:
 
     def kernel_bytes(self) -> tuple[dict, int]:
         """Bytes an ideal implementation must move per launch, from the step's outputs:
-        hiz_build = depth read + level-0 copy + levels 1.. written; vg_frame = 148 B per
-        object (64 B head / bounds / LOD errors, 64 B model, 16 B InstanceCullData, 4 B
-        selected-LOD write) + 16 B per work item (item, visibility words) + 44 B per tested
-        meshlet (centre, radius, cone apex, cutoff, axis) + 48 B per visible draw (12 B read,
-        36 B written)."""
+        hiz_build = depth read + level-0 copy + levels 1.. written; vg_frame = object_bytes
+        (records of the objects and of the instances tested) + 4 B per object (selected LOD
+        written) + 16 B per work item (item, visibility words) + 44 B per tested meshlet
+        (centre, radius, cone apex, cutoff, axis) + 48 B per visible draw (12 B read, 36 B
+        written)."""
         v, depth, cam, hz, vg = self.passes[0]
         o = vg.outputs()
         counters = o["counters"].cpu().numpy().view(np.uint32)
@@ -268,7 +276,8 @@ class PlainWorkload:
         tested = int(n.sum())
         hz = hiz_bytes(v.width, v.height, True)  # the TMA form or the 128-bit-load form, whichever ran
         return {"hiz_build_tma": hz, "hiz_build": hz,
-                "vg_frame": 148 * len(obj) + 16 * len(items) + 44 * tested + 48 * visible}, visible
+                "vg_frame": sum(object_bytes(self.scene, selected > 0)) + 4 * len(obj) + 16 * len(items)
+                            + 44 * tested + 48 * visible}, visible
 
     def e2e(self):
         import torch
@@ -456,20 +465,21 @@ class BatchedWorkload:
 
     def kernel_bytes(self) -> tuple[dict, int]:
         """Algorithmic bytes of the batched kernel: per view the Hi-Z (depth read + levels
-        1.. written) and the per-object LOD byte, the scene's object stage once per batch
-        (176 B per object: 96 B object fields, 64 B model, 16 B InstanceCullData), 44 B
-        per meshlet of the union over views of each object's selected LOD range, 32 B per
-        active span (16 B written, 16 B read) plus 8 B of span visibility, and 48 B per
-        visible draw (12 B read, 36 B written). Split by launch: batch_kernel (phases 0-3:
-        Hi-Z, LOD bytes, objects, span records written), batch_cull_kernel (phases 4-6:
-        meshlets, span records read, visibility, draws)."""
+        1.. written) and the per-object LOD byte, the records of the scene's objects and of
+        the instances tested once per batch (object_bytes), 44 B per meshlet of the union
+        over views of each object's selected LOD range, 32 B per active span (16 B written,
+        16 B read) plus 8 B of span visibility, and 48 B per visible draw (12 B read, 36 B
+        written). Split by launch: batch_kernel (phases 0-3: Hi-Z, LOD bytes, objects, span
+        records written), batch_cull_kernel (phases 4-5: instances, meshlets, span records
+        read, visibility, draws)."""
         lods, visible = self.outputs()
         spans = sum(active_spans(self.scene, lods[v])[0] for v in range(len(self.views)))
         k1 = sum(hiz_bytes(v.width, v.height, False) for v in self.views)
         k1 += lods.size  # LOD bytes
-        k1 += 176 * len(self.scene.objects)
+        objects, instances = object_bytes(self.scene, (lods > 0).any(axis=0))
+        k1 += objects
         k1 += 16 * spans  # span records written by the expansion
-        k2 = 44 * union_meshlets(self.scene, lods) + 24 * spans + 48 * visible
+        k2 = instances + 44 * union_meshlets(self.scene, lods) + 24 * spans + 48 * visible
         return {"batch_kernel": k1, "batch_cull_kernel": k2}, visible
 
     # The two cooperative launches of one step, reported together as the step's roofline.
