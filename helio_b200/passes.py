@@ -447,6 +447,8 @@ class BatchedCull:
         every grid barrier wait for CTAs that never arrive (tests of the bounded waits)."""
         N.check(self._lib.helio_batch_set_wait_limit(self._h, max_polls, extra_arrivals))
 
+    # The names are part of the interface. "span_count_scan" is the scan of an attached shadow cull now,
+    # and "group_count_scan" is empty: neither the spans' nor the groups' counts are scanned.
     PHASES = ("view_setup", "hiz_and_select", "span_count_scan", "span_expand", "meshlet_test",
               "group_count_scan", "emit", "max_cta_hiz_busy", "max_cta_select_busy")
 

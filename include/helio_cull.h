@@ -443,7 +443,10 @@ typedef struct helio_vg_pass helio_vg_pass;
 int32_t helio_vg_create(const helio_vg_config* config, helio_vg_pass** out);
 /* Uploads on buffer_version change, else patches [instance_dirty_start, +count) on
  * instance_version change; recomputes InstanceCullData on the GPU for what changed.
- * Reference: rendering.rs:708-859. May allocate (growth). */
+ * Arrays of memory HELIO_MEM_DEVICE on the current device are read by the update kernel
+ * itself (16-byte aligned ones, work items 8-byte aligned); others, of another device for
+ * instance, are copied first. Reference: rendering.rs:708-859. A full upload may allocate
+ * (growth), a patch does not. */
 int32_t helio_vg_prepare(helio_vg_pass* pass, const helio_vg_frame_data* frame, void* stream);
 /* Object select, meshlet cull and deterministic compaction in one launch that writes every
  * counter: the visible draws are stored in (work item, lane) order and
@@ -486,6 +489,8 @@ typedef struct helio_vg_scene_info {
     uint64_t device_bytes;
 } helio_vg_scene_info;
 int32_t helio_vg_scene_create(helio_vg_scene** out);
+/* May allocate: a full upload (growth), and the first patch of many rows that have to be staged in
+ * a small scene (at most 4,096 rows; not while the stream is captured). */
 int32_t helio_vg_scene_upload(helio_vg_scene* scene, const helio_vg_frame_data* frame, void* stream);
 int32_t helio_vg_scene_info_get(const helio_vg_scene* scene, helio_vg_scene_info* out);
 void helio_vg_scene_destroy(helio_vg_scene* scene);
@@ -567,9 +572,10 @@ int32_t helio_batch_pack_draws(const helio_batch* batch, HelioDrawIndexedIndirec
                                uint32_t* offsets, uint64_t capacity, void* stream);
 /* Tracing: device time (us) of the phases of the last execute, read from timer
  * stamps the kernel takes at its grid barriers (synchronises `stream`). Order:
- * view setup, Hi-Z + object select, span-count scan, span expansion, meshlet tests,
- * group-count scan, emission; then the largest per-CTA busy time on Hi-Z tiles and
- * on object chunks within the Hi-Z + select phase. */
+ * view setup, Hi-Z + object select, the scan of an attached shadow cull (else about
+ * nothing), span expansion, meshlet tests, a phase that no longer exists (always about
+ * nothing: the groups' counts need no scan), emission; then the largest per-CTA busy time
+ * on Hi-Z tiles and on object chunks within the Hi-Z + select phase. */
 int32_t helio_batch_get_phase_times(helio_batch* batch, double* us_out, uint32_t capacity, uint32_t* count,
                                     void* stream);
 /* Synchronises `stream`; HELIO_ERR_TIMEOUT if a bounded grid barrier gave up,
