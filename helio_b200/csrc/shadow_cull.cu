@@ -13,7 +13,7 @@
 // Stages and layout: shadow_device.cuh. Up to 2,048 draws one launch does everything, a cluster
 // of 8 CTAs per chunk of 32 dirty faces; beyond that a test and a place launch, with a scan
 // between them from 1,024 blocks of 256 draws on. Against three launches in every case: 2,000
-// draws x 10 dirty faces 16.4 -> 6.7 us a pass, 4,188 x 19 18.4 -> 8.7, 100,000 x 44 35.5 -> 20.8.
+// draws x 10 dirty faces 16.4 -> 6.3 us a pass, 4,188 x 19 18.4 -> 8.7, 100,000 x 44 35.5 -> 22.0.
 
 #include <algorithm>
 #include <new>
