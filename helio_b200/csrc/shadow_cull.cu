@@ -63,8 +63,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kThreads)
     shadow_put_sphere(s.sphere[warp], sphere);
     const ShadowPlanes p = shadow_chunk_planes(D, c * kShadowChunk, nf, width, s);
     uint32_t word = 0u;
-    const uint64_t minus_zero = pack2(D.minus_zero, D.minus_zero);
-    if (live_mask) word = shadow_test_word(p, s.sphere[warp], width, minus_zero) & live_mask;  // uniform over the warp
+    if (live_mask) word = shadow_test_word(p, s.sphere[warp], width) & live_mask;  // uniform over the warp
     if (lane >= nf) word = 0u;
     s_cnt[warp][lane] = __popc(word);
     __syncthreads();
@@ -177,7 +176,6 @@ bool helio::shadow_dev(const helio_shadow_cull_pass* p, ShadowDev* out) {
     D.face_dirty = p->in.face_dirty;
     D.instance_count = p->in.instance_count;
     D.draw_count = p->in.draw_count;
-    D.minus_zero = -0.0f;
     D.blocks = p->blocks;
     D.words = p->words;
     D.bits = p->bits.as<uint32_t>();

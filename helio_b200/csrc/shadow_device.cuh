@@ -51,7 +51,6 @@ struct ShadowDev {
     uint32_t* counts;  // [kShadowChunks][blocks][32]
     HelioDrawIndexedIndirectArgs* dst;  // [256][4096]
     uint32_t* face_counts;              // [256]
-    float minus_zero;                   // -0.0f (fmul2)
 };
 
 // Shared memory of one block running a stage.
@@ -74,13 +73,17 @@ __device__ __forceinline__ uint64_t pack2(float a, float b) {
 __device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-// A product of its own, as a multiply-add of a -0 that the compiler does not know (ShadowDev::minus_zero):
-// the assembler joins a packed multiply (also one whose -0 is a constant) and the packed addition that
-// takes it into one operation with one rounding, in spite of .rn and of its switch for that, and then
-// spheres within a rounding of a plane changed sides (1 of 24.8 million draw-face decisions).
-__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b, uint64_t minus_zero) {
+// A product of its own, as a multiply-add of a -0 that the compiler does not know: the assembler joins a
+// packed multiply (also one whose -0 is a constant) and the packed addition that takes it into one
+// operation with one rounding, in spite of .rn and of its switch for that, and then spheres within a
+// rounding of a plane changed sides (1 of 24.8 million draw-face decisions). In constant memory, since
+// the batched kernel has no register for it (as a parameter it cost that kernel 40 bytes of spills and
+// 2% of its time).
+static __constant__ float2 c_minus_zero = {-0.0f, -0.0f};
+
+__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
     uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(minus_zero));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(pack2(c_minus_zero.x, c_minus_zero.y)));
     return r;
 }
 __device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
@@ -191,10 +194,9 @@ __device__ __forceinline__ uint32_t shadow_width(uint32_t nf) { return nf > 1u ?
 // positive or NaN, so a distance is never -0 and a NaN distance is the canonical one, whose sign
 // bit is clear: the sign bits decide. Lane j of each group of `width` lanes tests the pairs
 // g, g + 32 / width, ... of its group g; the groups' bits are brought together at the end.
-__device__ __forceinline__ uint32_t shadow_test_word(const ShadowPlanes& p, const float4* spheres, uint32_t width,
-                                                     uint64_t minus_zero) {
+__device__ __forceinline__ uint32_t shadow_test_word(const ShadowPlanes& p, const float4* spheres, uint32_t width) {
     const uint32_t lane = threadIdx.x & 31u, groups = 32u / width, g = lane / width;
-    uint32_t out = 0;  // bits of the draws that are out
+    uint32_t in = 0;
 #pragma unroll 2
     for (uint32_t k = g; k < 16u; k += groups) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(spheres + 2u * k);
@@ -203,17 +205,13 @@ __device__ __forceinline__ uint32_t shadow_test_word(const ShadowPlanes& p, cons
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
             float d0, d1;
-            const uint64_t x = fmul2(p.x[i], a.x, minus_zero), y = fmul2(p.y[i], a.y, minus_zero),
-                           z = fmul2(p.z[i], b.x, minus_zero);
+            const uint64_t x = fmul2(p.x[i], a.x), y = fmul2(p.y[i], a.y), z = fmul2(p.z[i], b.x);
             unpack2(fadd2(fadd2(fadd2(fadd2(x, y), z), p.w[i]), b.y), d0, d1);
             n0 |= __float_as_uint(d0);
             n1 |= __float_as_uint(d1);
         }
-        out |= ((n0 >> 31) | (n1 >> 31 << 1)) << (2u * k);
+        in |= (3u ^ ((n0 >> 31) | (n1 >> 31 << 1))) << (2u * k);
     }
-    uint32_t in = 0;
-    for (uint32_t k = g; k < 16u; k += groups) in |= 3u << (2u * k);
-    in &= ~out;
     for (uint32_t d = width; d < 32u; d <<= 1) in |= __shfl_xor_sync(0xffffffffu, in, d);
     return in;
 }
@@ -233,8 +231,7 @@ static __device__ __noinline__ void shadow_test_block(const ShadowDev& D, uint32
         const uint32_t nf = min(kShadowChunk, n_active - c * kShadowChunk);
         const uint32_t width = shadow_width(nf);
         const ShadowPlanes p = shadow_chunk_planes(D, c * kShadowChunk, nf, width, s);
-        const uint32_t all =
-            shadow_test_word(p, s.sphere[warp], width, pack2(D.minus_zero, D.minus_zero)) & live_mask;
+        const uint32_t all = shadow_test_word(p, s.sphere[warp], width) & live_mask;
         const uint32_t word = lane < nf ? all : 0u;
         D.bits[((size_t)c * D.words + block * kShadowWarps + warp) * 32u + lane] = word;
         __syncthreads();  // the planes are read: their region takes the counts
