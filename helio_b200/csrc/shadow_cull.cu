@@ -13,7 +13,7 @@
 // Stages and layout: shadow_device.cuh. Up to 2,048 draws one launch does everything, a cluster
 // of 8 CTAs per chunk of 32 dirty faces; beyond that a test and a place launch, with a scan
 // between them from 1,024 blocks of 256 draws on. Against three launches in every case: 2,000
-// draws x 10 dirty faces 16.4 -> 6.3 us a pass, 4,188 x 19 18.4 -> 8.7, 100,000 x 44 35.5 -> 22.0.
+// draws x 10 dirty faces 16.4 -> 6.3 us a pass, 4,188 x 19 18.4 -> 8.7, 100,000 x 44 35.5 -> 21.7.
 
 #include <algorithm>
 #include <new>
@@ -36,8 +36,8 @@ constexpr uint32_t kChunks = kShadowChunks;
 // Small draw lists in one launch: cluster y is chunk y, its CTA x takes the draws [256 x, ...), one
 // per thread, and learns the counts of the CTAs before it through distributed shared memory, so
 // that nothing but the results touches global memory. Bound by latency: the dirty list, the draws'
-// instances and spheres, the planes and one cluster barrier. Up to 2,048 draws it takes 5.5 to 9.2
-// us on the device (10 to 60 dirty faces), the two launches below 6.9 to 10.2; with several draws
+// instances and spheres, the planes and one cluster barrier. Up to 2,048 draws it takes 5.6 to 8.6
+// us on the device (10 to 60 dirty faces), the two launches below 6.9 to 10.0; with several draws
 // per thread it fell behind them (3,000 draws x 19 faces: 12.5 against 8.9 us).
 constexpr uint32_t kClusterCtas = 8;
 constexpr uint32_t kClusterDraws = kClusterCtas * kThreads;

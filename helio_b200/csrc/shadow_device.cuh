@@ -18,7 +18,7 @@
 // word by itself (no ballots, one shared load per 32 tests instead of six), and two draws go
 // through each packed multiply or add. A last chunk of at most 16 faces repeats them in the
 // warp's other lanes, which take every second (fourth, ...) pair of draws. The test is bound by
-// instruction issue (100,000 draws x 44 faces: 7.0M warp instructions, 20M with a lane per draw
+// instruction issue (100,000 draws x 44 faces: 6.5M warp instructions, 20M with a lane per draw
 // and the planes read from shared memory). Stages (no atomics on the data path):
 //   test   block of 256 draws: per chunk and warp the lanes' words, per chunk the block's
 //          counts, both stored lane by lane;
